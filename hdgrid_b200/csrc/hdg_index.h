@@ -174,8 +174,10 @@ struct hdg_index {
     uint64_t last_q = 0, last_ncand = 0;
     uint64_t last_stats[10] = {0};
     float last_beta = 0.f;
-    // learned per-query schedule: f32 master | Adam m | Adam v | gradient | bf16 weights
+    // learned per-query schedule: f32 master | Adam m | Adam v | bf16 weights
     hdg::DeviceBuffer mlp;
+    hdg::DeviceBuffer mlp_work;    // partial gradients of a training pass (one call at a time)
+    std::mutex mlp_mu;             // guards mlp_work
     bool mlp_ready = false;
     uint64_t mlp_step = 0;
     hdg_index() = default;

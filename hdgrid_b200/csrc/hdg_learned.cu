@@ -26,7 +26,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <random>
+#include <type_traits>
 #include <vector>
 
 #include "hdg_device.cuh"
@@ -35,8 +37,6 @@
 namespace hdg {
 
 namespace {
-
-constexpr int kTile = 32;  // samples per forward block
 
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
@@ -187,49 +187,76 @@ __global__ void __launch_bounds__(128) k_features(IndexDev D, GridMeta g, const 
     if (t < kMlpFeatures) feats[qi * kMlpFeatures + t] = s_f[t];
 }
 
-// ---- forward ---------------------------------------------------------------------------
-// 128 threads (one hidden unit each), persistent over tiles of kTile samples: the weights are
-// staged once per block, unit-major with rows padded by one word (49 and 129), so that both
-// the staging writes and the reads of unit t's row across the threads are conflict-free;
-// inputs are broadcast.
+// ---- forward and backward ----------------------------------------------------------------
+// One kernel for inference and for a training step's whole forward and backward pass: 256
+// threads, one tile of TS samples at a time, persistent over the tiles.  The weights are staged
+// once per block, unit-major with rows padded by one word (49 and 129), so that both the staging
+// writes and the reads of unit t's row across the threads are conflict-free.  Activations are
+// unit-major rows of TS samples padded by 4 words: 16-byte reads, 8 consecutive rows on
+// different banks.
+//
+// Training (GRAD): the tile's activations never leave shared memory.  The loss gradient, the
+// two hidden gradients and the tile's share of every weight gradient follow from them, the
+// weight gradients in registers (8 x 8 of W2 and 8 x 3 of W1 per thread) across the block's
+// tiles; each block writes one partial row of all parameters, which k_grad_reduce sums.  A
+// separate pass per layer, each output one serial sum over the batch, took 4.2 ms at 4,096 rows
+// (one chain of dependent FMAs and loads per weight, 128 blocks, eight allocations a call);
+// gradients plus a forward call now take 78 us together.
+// Bound: FMA issue of one block per SM (about 2 M FMAs per 32 samples) and, below one tile per
+// SM, the latency of one tile.
 struct FwdOut {
     float* z;            // [n x 2]
-    float* a1;           // [n x 128] hidden 1 (bf16-rounded), training only
-    float* a2;           // [n x 128] hidden 2, training only
     uint32_t* nprobe;    // inference: per-query lists to probe
     uint8_t* sched;      // inference: per-query schedule flag
     int allow_sched;
     uint32_t max_probe;
+    const float* y;      // training: targets [rows x 2]
+    const uint32_t* rows;  // training: row of sample b in x and y (nullptr: b)
+    float* part;         // training: [blocks x kMlpParams] partial gradients
+    double* loss;        // training: [blocks] partial loss sums
 };
 
-__global__ void __launch_bounds__(kMlpHidden) k_mlp_forward(Params P, const float* __restrict__ x, uint64_t n,
-                                                            FwdOut o) {
+constexpr int kFwdThreads = 256;
+
+template <int TS, bool GRAD>
+constexpr size_t forward_smem() {
+    return sizeof(float) * ((kMlpFeatures + 1) * kMlpHidden + (kMlpHidden + 1) * kMlpHidden + kMlpOut * kMlpHidden +
+                            (kMlpFeatures + (GRAD ? 3 : 2) * kMlpHidden) * (TS + 4) + kMlpOut * TS);
+}
+
+template <int TS, bool GRAD>
+__global__ void __launch_bounds__(kFwdThreads) k_mlp(Params P, const float* __restrict__ x, uint64_t n, FwdOut o) {
     constexpr int S1 = kMlpFeatures + 1, S2 = kMlpHidden + 1;  // padded weight rows
-    constexpr int SH = kTile + 4;  // activation rows: 16-byte aligned, 4-way conflicts at most on the writes
+    constexpr int SH = TS + 4;                                 // activation rows
+    constexpr int TH = TS / 2;                                 // samples per thread in a hidden layer
     extern __shared__ __align__(16) float sm[];
-    float* w1p = sm;                                   // [128][49]: unit-major W1
+    float* xs = sm;                                    // [48][SH]: feature-major inputs
+    float* h1 = xs + kMlpFeatures * SH;                // [128][SH]: unit-major activations
+    float* h2 = h1 + kMlpHidden * SH;                  // [128][SH]
+    float* g2 = h2 + kMlpHidden * SH;                  // [128][SH] (GRAD): gradient at hidden 2
+    float* dz = g2 + (GRAD ? kMlpHidden * SH : 0);     // [2][TS] loss gradient at the outputs
+    float* w1p = dz + kMlpOut * TS;                    // [128][49]: unit-major W1
     float* w2p = w1p + kMlpHidden * S1;                // [128][129]
     float* w3 = w2p + kMlpHidden * S2;                 // [2][128]
-    float* xs = w3 + kMlpOut * kMlpHidden;             // [48][kTile]: feature-major inputs
-    float* h1 = xs + kMlpFeatures * kTile;             // [128][SH]: unit-major activations
-    float* h2 = h1 + kMlpHidden * SH;                  // [128][SH]
-    const int t = threadIdx.x;
-    for (int e = t; e < kMlpHidden * kMlpFeatures; e += blockDim.x)
+    __shared__ double s_loss[kFwdThreads / 32];
+    const int t = threadIdx.x, u = t & (kMlpHidden - 1), half = t / kMlpHidden;
+    for (int e = t; e < kMlpHidden * kMlpFeatures; e += kFwdThreads)
         w1p[(e / kMlpFeatures) * S1 + e % kMlpFeatures] = __bfloat162float(P.w[kMlpW1 + e]);
-    for (int e = t; e < kMlpHidden * kMlpHidden; e += blockDim.x)
+    for (int e = t; e < kMlpHidden * kMlpHidden; e += kFwdThreads)
         w2p[(e / kMlpHidden) * S2 + e % kMlpHidden] = __bfloat162float(P.w[kMlpW2 + e]);
-    for (int e = t; e < kMlpOut * kMlpHidden; e += blockDim.x) w3[e] = __bfloat162float(P.w[kMlpW3 + e]);
-    const float bias1 = P.master[kMlpB1 + t], bias2 = P.master[kMlpB2 + t];
-    // one hidden layer: acc[b] = sum over r of w[r] * in[r][b], in order r = 0, 1, ... (the
-    // sample's inputs read four at a time as broadcasts)
-    auto layer = [&](const float* wrow, const float* in, int rows, int ld, float (&acc)[kTile]) {
+    for (int e = t; e < kMlpOut * kMlpHidden; e += kFwdThreads) w3[e] = __bfloat162float(P.w[kMlpW3 + e]);
+    const float bias1 = P.master[kMlpB1 + u], bias2 = P.master[kMlpB2 + u];
+    // acc[b] = sum over r of w[r * ws] * in[r][b], in order r = 0, 1, ..., for this thread's half
+    // of the samples (read four at a time as broadcasts)
+    auto layer = [&](const float* w, int ws, const float* in, int rows, float (&acc)[TH]) {
 #pragma unroll
-        for (int b = 0; b < kTile; b++) acc[b] = 0.f;
+        for (int b = 0; b < TH; b++) acc[b] = 0.f;
+#pragma unroll 4
         for (int r = 0; r < rows; r++) {
-            const float wv = wrow[r];
-            const float4* v = reinterpret_cast<const float4*>(in + r * ld);
+            const float wv = w[r * ws];
+            const float4* v = reinterpret_cast<const float4*>(in + r * SH + half * TH);
 #pragma unroll
-            for (int b4 = 0; b4 < kTile / 4; b4++) {
+            for (int b4 = 0; b4 < TH / 4; b4++) {
                 const float4 a = v[b4];
                 acc[4 * b4] = fmaf(wv, a.x, acc[4 * b4]);
                 acc[4 * b4 + 1] = fmaf(wv, a.y, acc[4 * b4 + 1]);
@@ -238,34 +265,70 @@ __global__ void __launch_bounds__(kMlpHidden) k_mlp_forward(Params P, const floa
             }
         }
     };
-    for (uint64_t b0 = (uint64_t)blockIdx.x * kTile; b0 < n; b0 += (uint64_t)gridDim.x * kTile) {
-        __syncthreads();  // the weights are staged; the previous tile's reads are done
-        for (int e = t; e < kTile * kMlpFeatures; e += blockDim.x) {
-            const int i = e / kTile, b = e % kTile;
-            xs[e] = b0 + b < n ? bf16r(x[(b0 + b) * kMlpFeatures + i]) : 0.f;
+    auto put = [&](float* row, const float (&v)[TH]) {
+#pragma unroll
+        for (int b4 = 0; b4 < TH / 4; b4++)
+            reinterpret_cast<float4*>(row + half * TH)[b4] =
+                make_float4(v[4 * b4], v[4 * b4 + 1], v[4 * b4 + 2], v[4 * b4 + 3]);
+    };
+    // GRAD: the block's weight gradients so far.  Rows to*8 .. +7 (outputs), columns ti + 16 k
+    const int ti = t & 15, to = t >> 4;
+    float gw2[GRAD ? 8 : 1][8], gw1[GRAD ? 8 : 1][3];
+    float gw3 = 0.f, gb = 0.f, gb3 = 0.f;  // W3[half][u]; b1 (half 0) or b2 (half 1) of unit u; b3[t]
+    double lsum = 0.0;
+    if constexpr (GRAD) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) gw2[i][k] = 0.f;
+#pragma unroll
+            for (int k = 0; k < 3; k++) gw1[i][k] = 0.f;
         }
-        __syncthreads();
-        float acc[kTile];
-        layer(w1p + t * S1, xs, kMlpFeatures, kTile, acc);
+    }
+    // tile share of dW[to*8 + i][ti + 16 k] = sum_b dy[row][b] * in[col][b]
+    auto outer = [&](const float* dy, const float* in, auto& acc, auto kc) {
+        constexpr int K = decltype(kc)::value;
+#pragma unroll 1
+        for (int b4 = 0; b4 < TS / 4; b4++) {
+            float4 dv[8], av[K];
 #pragma unroll
-        for (int b = 0; b < kTile; b++) h1[t * SH + b] = bf16r(fmaxf(acc[b] + bias1, 0.f));
-        __syncthreads();
-        layer(w2p + t * S2, h1, kMlpHidden, SH, acc);
+            for (int i = 0; i < 8; i++) dv[i] = reinterpret_cast<const float4*>(dy + (to * 8 + i) * SH)[b4];
 #pragma unroll
-        for (int b = 0; b < kTile; b++) h2[t * SH + b] = bf16r(fmaxf(acc[b] + bias2, 0.f));
-        __syncthreads();
-        if (o.a1) {
-            for (int e = t; e < kTile * kMlpHidden; e += blockDim.x) {
-                const int b = e / kMlpHidden, u = e % kMlpHidden;
-                if (b0 + b < n) {
-                    o.a1[(b0 + b) * kMlpHidden + u] = h1[u * SH + b];
-                    o.a2[(b0 + b) * kMlpHidden + u] = h2[u * SH + b];
+            for (int k = 0; k < K; k++) av[k] = reinterpret_cast<const float4*>(in + (ti + 16 * k) * SH)[b4];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    acc[i][k] = fmaf(dv[i].x, av[k].x, acc[i][k]);
+                    acc[i][k] = fmaf(dv[i].y, av[k].y, acc[i][k]);
+                    acc[i][k] = fmaf(dv[i].z, av[k].z, acc[i][k]);
+                    acc[i][k] = fmaf(dv[i].w, av[k].w, acc[i][k]);
                 }
-            }
         }
-        if (t < kTile * kMlpOut) {
+    };
+    auto row_of = [&](uint64_t b) -> uint64_t { return GRAD && o.rows ? (uint64_t)o.rows[b] : b; };
+    for (uint64_t b0 = (uint64_t)blockIdx.x * TS; b0 < n; b0 += (uint64_t)gridDim.x * TS) {
+        __syncthreads();  // the weights are staged; the previous tile's reads are done
+        for (int e = t; e < TS * kMlpFeatures; e += kFwdThreads) {
+            const int b = e / kMlpFeatures, i = e % kMlpFeatures;
+            xs[i * SH + b] = b0 + b < n ? bf16r(x[row_of(b0 + b) * kMlpFeatures + i]) : 0.f;
+        }
+        __syncthreads();
+        float acc[TH];
+        layer(w1p + u * S1, 1, xs, kMlpFeatures, acc);
+#pragma unroll
+        for (int b = 0; b < TH; b++) acc[b] = bf16r(fmaxf(acc[b] + bias1, 0.f));
+        put(h1 + u * SH, acc);
+        __syncthreads();
+        layer(w2p + u * S2, 1, h1, kMlpHidden, acc);
+#pragma unroll
+        for (int b = 0; b < TH; b++) acc[b] = bf16r(fmaxf(acc[b] + bias2, 0.f));
+        put(h2 + u * SH, acc);
+        __syncthreads();
+        if (t < TS * kMlpOut) {
             const int b = t >> 1, c = t & 1;
             float z = 0.f;
+#pragma unroll 8
             for (int j2 = 0; j2 < kMlpHidden; j2++) z = fmaf(w3[c * kMlpHidden + j2], h2[j2 * SH + b], z);
             z += P.master[kMlpB3 + c];
             const uint64_t bi = b0 + b;
@@ -277,71 +340,131 @@ __global__ void __launch_bounds__(kMlpHidden) k_mlp_forward(Params P, const floa
                 }
                 if (c == 1 && o.sched) o.sched[bi] = (o.allow_sched && z > 0.f) ? 1 : 0;
             }
+            if constexpr (GRAD) {
+                // loss = mean over the batch of (z0 - y0)^2 + BCE(sigmoid(z1), y1); a tile's missing
+                // samples have gradient 0
+                float g = 0.f;
+                if (bi < n) {
+                    const float yv = o.y[row_of(bi) * kMlpOut + c];
+                    const float inv = 1.f / (float)n;
+                    if (c == 0) {
+                        g = 2.f * (z - yv) * inv;
+                        lsum += (double)(z - yv) * (z - yv);
+                    } else {
+                        const float s = 1.f / (1.f + expf(-z));
+                        g = (s - yv) * inv;
+                        // numerically stable BCE with logits: max(z,0) - z*y + log(1 + exp(-|z|))
+                        lsum += (double)(fmaxf(z, 0.f) - z * yv + log1pf(expf(-fabsf(z))));
+                    }
+                }
+                dz[c * TS + b] = g;
+            }
+        }
+        if constexpr (GRAD) {
+            __syncthreads();
+            // hidden 2: g2[u][b] = (dz[0][b] W3[0][u] + dz[1][b] W3[1][u]) where h2 > 0; W3 and b3
+            {
+                const float w30 = w3[u], w31 = w3[kMlpHidden + u];
+                float g[TH], s = 0.f;
+#pragma unroll
+                for (int b = 0; b < TH; b++) {
+                    const int bb = half * TH + b;
+                    g[b] = h2[u * SH + bb] > 0.f ? fmaf(dz[TS + bb], w31, dz[bb] * w30) : 0.f;
+                }
+                put(g2 + u * SH, g);
+#pragma unroll
+                for (int b = 0; b < TS; b++) s = fmaf(dz[half * TS + b], h2[u * SH + b], s);
+                gw3 += s;
+                if (t < kMlpOut) {
+                    float sb = 0.f;
+#pragma unroll
+                    for (int b = 0; b < TS; b++) sb += dz[t * TS + b];
+                    gb3 += sb;
+                }
+            }
+            __syncthreads();
+            // hidden 1: sum over o of g2[o][b] W2[o][u] where h1 > 0, kept in h2's place (its last
+            // readers are behind the barrier)
+            layer(w2p + u, S2, g2, kMlpHidden, acc);
+#pragma unroll
+            for (int b = 0; b < TH; b++) acc[b] = h1[u * SH + half * TH + b] > 0.f ? acc[b] : 0.f;
+            put(h2 + u * SH, acc);
+            outer(g2, h1, gw2, std::integral_constant<int, 8>());
+            __syncthreads();
+            outer(h2, xs, gw1, std::integral_constant<int, 3>());
+            const float* gr = (half ? g2 : h2) + u * SH;
+            float s = 0.f;
+#pragma unroll
+            for (int b = 0; b < TS; b++) s += gr[b];
+            gb += s;
+        }
+    }
+    if constexpr (GRAD) {
+        float* p = o.part + (uint64_t)blockIdx.x * kMlpParams;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) p[kMlpW2 + (to * 8 + i) * kMlpHidden + ti + 16 * k] = gw2[i][k];
+#pragma unroll
+            for (int k = 0; k < 3; k++) p[kMlpW1 + (to * 8 + i) * kMlpFeatures + ti + 16 * k] = gw1[i][k];
+        }
+        p[kMlpW3 + half * kMlpHidden + u] = gw3;
+        p[(half ? kMlpB2 : kMlpB1) + u] = gb;
+        if (t < kMlpOut) p[kMlpB3 + t] = gb3;
+        for (int k = 16; k > 0; k >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, k);
+        if ((t & 31) == 0) s_loss[t >> 5] = lsum;
+        __syncthreads();
+        if (t == 0) {
+            double l = 0.0;
+            for (int k = 0; k < kFwdThreads / 32; k++) l += s_loss[k];
+            o.loss[blockIdx.x] = l;
         }
     }
 }
 
-// ---- loss and backward -----------------------------------------------------------------
-// loss = mean over the batch of (z0 - y0)^2 + BCE(sigmoid(z1), y1)
-__global__ void k_loss_grad(const float* __restrict__ z, const float* __restrict__ y, uint64_t n,
-                            float* __restrict__ dz, double* __restrict__ loss) {
-    const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    double l = 0.0;
-    if (b < n) {
-        const float z0 = z[2 * b], z1 = z[2 * b + 1], y0 = y[2 * b], y1 = y[2 * b + 1];
-        const float inv = 1.f / (float)n;
-        dz[2 * b] = 2.f * (z0 - y0) * inv;
-        const float s = 1.f / (1.f + expf(-z1));
-        dz[2 * b + 1] = (s - y1) * inv;
-        // numerically stable BCE with logits: max(z,0) - z*y + log(1 + exp(-|z|))
-        l = (double)(z0 - y0) * (z0 - y0) + (double)(fmaxf(z1, 0.f) - z1 * y1 + log1pf(expf(-fabsf(z1))));
-    }
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l / (double)n);
-}
+// One Adam update (b1, b2, eps; c1, c2 the bias corrections); lr 0 with m = nullptr: none.
+struct AdamStep {
+    float *p, *m, *v;
+    float lr, b1, b2, eps, c1, c2;
+    __nv_bfloat16* pw;
+};
 
-// dW[o][i] = sum_b dY[b][o] * X[b][i], db[o] = sum_b dY[b][o]; one block per output row o
-__global__ void __launch_bounds__(128) k_grad_w(const float* __restrict__ dy, int n_out, const float* __restrict__ xin,
-                                                int n_in, uint64_t n, float* __restrict__ dw, float* __restrict__ db) {
-    const int o = blockIdx.x, t = threadIdx.x;
-    for (int i = t; i < n_in; i += blockDim.x) {
-        float s = 0.f;
-        for (uint64_t b = 0; b < n; b++) s = fmaf(dy[b * n_out + o], xin[b * n_in + i], s);
-        dw[(uint64_t)o * n_in + i] = s;
+// Gradient = sum of the blocks' partial rows, then the Adam update when a.m is given.  32
+// parameters per block, 8 threads each over every 8th row (up to 19 loads in flight per thread),
+// in a fixed order.  Bound: the partial rows' L2 reads (13 MB at 148 rows).
+__global__ void __launch_bounds__(256) k_grad_reduce(const float* __restrict__ part, int nb,
+                                                     const double* __restrict__ lpart, uint64_t n, int accumulate,
+                                                     float* __restrict__ grad, double* __restrict__ loss, AdamStep a) {
+    __shared__ float s_p[8][33];
+    const int lane = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    float s = 0.f;
+    if (i < kMlpParams) {
+#pragma unroll 4
+        for (int r = y; r < nb; r += 8) s += __ldcg(part + (uint64_t)r * kMlpParams + i);
     }
-    if (t < 32) {
-        float s = 0.f;
-        for (uint64_t b = t; b < n; b += 32) s += dy[b * n_out + o];
-        for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
-        if (t == 0) db[o] = s;
+    s_p[y][lane] = s;
+    __syncthreads();
+    if (y == 0 && i < kMlpParams) {
+        float g = ((s_p[0][lane] + s_p[1][lane]) + (s_p[2][lane] + s_p[3][lane])) +
+                  ((s_p[4][lane] + s_p[5][lane]) + (s_p[6][lane] + s_p[7][lane]));
+        if (grad) grad[i] = g;
+        if (a.m) {
+            const float mi = a.b1 * a.m[i] + (1.f - a.b1) * g;
+            const float vi = a.b2 * a.v[i] + (1.f - a.b2) * g * g;
+            a.m[i] = mi;
+            a.v[i] = vi;
+            const float pi = a.p[i] - a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+            a.p[i] = pi;
+            a.pw[i] = __float2bfloat16_rn(pi);
+        }
     }
-}
-
-// dX[b][j] = (sum_o dY[b][o] * W[o][j]) * (A[b][j] > 0); one block per sample
-__global__ void __launch_bounds__(128) k_grad_x(const float* __restrict__ dy, int n_out,
-                                                const __nv_bfloat16* __restrict__ w, int n_in,
-                                                const float* __restrict__ a, uint64_t n, float* __restrict__ dx) {
-    const uint64_t b = blockIdx.x;
-    for (int j = threadIdx.x; j < n_in; j += blockDim.x) {
-        float s = 0.f;
-        for (int o = 0; o < n_out; o++) s = fmaf(dy[b * n_out + o], __bfloat162float(w[(uint64_t)o * n_in + j]), s);
-        dx[b * n_in + j] = a[b * n_in + j] > 0.f ? s : 0.f;
+    if (blockIdx.x == 0 && y == 1) {  // the mean loss of the batch
+        double l = 0.0;
+        for (int r = lane; r < nb; r += 32) l += __ldcg(lpart + r);
+        for (int k = 16; k > 0; k >>= 1) l += __shfl_xor_sync(0xffffffffu, l, k);
+        if (lane == 0) *loss = (accumulate ? *loss : 0.0) + l / (double)n;
     }
-}
-
-__global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, int n, float lr, float b1, float b2, float eps, float c1, float c2,
-                       __nv_bfloat16* __restrict__ pw) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    p[i] = pi;
-    pw[i] = __float2bfloat16_rn(pi);
 }
 
 __global__ void k_to_bf16_params(const float* __restrict__ p, int n, __nv_bfloat16* __restrict__ pw) {
@@ -349,26 +472,15 @@ __global__ void k_to_bf16_params(const float* __restrict__ p, int n, __nv_bfloat
     if (i < n) pw[i] = __float2bfloat16_rn(p[i]);
 }
 
-__global__ void k_gather_batch(const float* __restrict__ x, const float* __restrict__ y,
-                               const uint32_t* __restrict__ idx, uint64_t n, float* __restrict__ xb,
-                               float* __restrict__ yb) {
-    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n * kMlpFeatures) return;
-    const uint64_t b = e / kMlpFeatures, i = e % kMlpFeatures;
-    const uint64_t src = idx[b];
-    xb[e] = x[src * kMlpFeatures + i];
-    if (i < kMlpOut) yb[b * kMlpOut + i] = y[src * kMlpOut + i];
-}
-
-// model buffer: master | adam m | adam v | grad (fp32, kMlpParams each) | bf16 copy
+// model buffer: master | adam m | adam v (fp32, kMlpParams each) | bf16 copy
 struct ModelPtrs {
-    float *master, *m, *v, *grad;
+    float *master, *m, *v;
     __nv_bfloat16* w;
 };
 
 ModelPtrs model_ptrs(hdg_index* idx) {
     if (!idx->mlp.ptr) {
-        idx->mlp.ensure(sizeof(float) * 4 * kMlpParams + sizeof(__nv_bfloat16) * kMlpParams + 256);
+        idx->mlp.ensure(sizeof(float) * 3 * kMlpParams + sizeof(__nv_bfloat16) * kMlpParams + 256);
         CK(cudaMemset(idx->mlp.ptr, 0, idx->mlp.bytes));
     }
     float* base = static_cast<float*>(idx->mlp.ptr);
@@ -376,50 +488,71 @@ ModelPtrs model_ptrs(hdg_index* idx) {
     p.master = base;
     p.m = base + kMlpParams;
     p.v = base + 2 * kMlpParams;
-    p.grad = base + 3 * kMlpParams;
-    p.w = reinterpret_cast<__nv_bfloat16*>(base + 4 * kMlpParams);
+    p.w = reinterpret_cast<__nv_bfloat16*>(base + 3 * kMlpParams);
     return p;
 }
 
-size_t forward_smem() {
-    return sizeof(float) * ((kMlpFeatures + 1) * kMlpHidden + (kMlpHidden + 1) * kMlpHidden + kMlpOut * kMlpHidden +
-                            kTile * kMlpFeatures + 2 * (kTile + 4) * kMlpHidden);
+// Blocks of a pass over n samples in tiles of ts: one per SM at most (the staged weights fill it)
+int mlp_blocks(uint64_t n, int ts) { return (int)std::min<uint64_t>((n + ts - 1) / ts, (uint64_t)sm_count()); }
+
+// Tile size for n samples: a tile costs a fixed part (about 12 samples' worth: staging, barriers,
+// the output layer's chain) plus its samples, and the pass lasts as long as the block with the
+// most tiles; the smallest such time wins.
+int mlp_tile(uint64_t n) {
+    int best = 8;
+    uint64_t cost = ~0ull;
+    for (int ts : {8, 16, 32}) {
+        const uint64_t tiles = (n + ts - 1) / ts, rounds = (tiles + sm_count() - 1) / sm_count();
+        if (rounds * (ts + 12) < cost) {
+            cost = rounds * (ts + 12);
+            best = ts;
+        }
+    }
+    return best;
 }
 
-void launch_forward(const ModelPtrs& mp, const float* x, uint64_t n, const FwdOut& o, cudaStream_t st) {
-    const size_t sm = forward_smem();
-    CK(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    // persistent over the tiles: as many blocks as fit at once (each stages the weights once)
-    int per_sm = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mlp_forward, kMlpHidden, sm));
-    const uint64_t tiles = (n + kTile - 1) / kTile;
-    const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)sm_count() * std::max(per_sm, 1)));
-    k_mlp_forward<<<(unsigned)blocks, kMlpHidden, sm, st>>>(Params{mp.master, mp.w}, x, n, o);
-    CK_LAUNCH();
+template <bool GRAD>
+int launch_mlp(const ModelPtrs& mp, const float* x, uint64_t n, const FwdOut& o, cudaStream_t st) {
+    auto go = [&](auto tsc) {
+        constexpr int TS = decltype(tsc)::value;
+        constexpr size_t sm = forward_smem<TS, GRAD>();
+        CK(cudaFuncSetAttribute(k_mlp<TS, GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        const int blocks = std::max(1, mlp_blocks(n, TS));
+        k_mlp<TS, GRAD><<<blocks, kFwdThreads, sm, st>>>(Params{mp.master, mp.w}, x, n, o);
+        CK_LAUNCH();
+        return blocks;
+    };
+    const int ts = mlp_tile(n);
+    if (ts == 8) return go(std::integral_constant<int, 8>());
+    if (ts == 16) return go(std::integral_constant<int, 16>());
+    return go(std::integral_constant<int, 32>());
 }
 
-// backward of one batch into mp.grad (forward activations a1, a2 and outputs z given)
-void launch_backward(const ModelPtrs& mp, const float* x, const float* y, uint64_t n, const float* z,
-                     const float* a1, const float* a2, float* dz, float* dh2, float* dh1, double* loss,
-                     cudaStream_t st) {
-    k_loss_grad<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(z, y, n, dz, loss);
-    CK_LAUNCH();
-    k_grad_w<<<kMlpOut, 128, 0, st>>>(dz, kMlpOut, a2, kMlpHidden, n, mp.grad + kMlpW3, mp.grad + kMlpB3);
-    CK_LAUNCH();
-    k_grad_x<<<(unsigned)n, 128, 0, st>>>(dz, kMlpOut, mp.w + kMlpW3, kMlpHidden, a2, n, dh2);
-    CK_LAUNCH();
-    k_grad_w<<<kMlpHidden, 128, 0, st>>>(dh2, kMlpHidden, a1, kMlpHidden, n, mp.grad + kMlpW2, mp.grad + kMlpB2);
-    CK_LAUNCH();
-    k_grad_x<<<(unsigned)n, 128, 0, st>>>(dh2, kMlpHidden, mp.w + kMlpW2, kMlpHidden, a1, n, dh1);
-    CK_LAUNCH();
-    // the layer-1 input is the bf16-rounded feature row, as in the forward pass
-    k_grad_w<<<kMlpHidden, 128, 0, st>>>(dh1, kMlpHidden, x, kMlpFeatures, n, mp.grad + kMlpW1, mp.grad + kMlpB1);
-    CK_LAUNCH();
+// Scratch of a training pass, kept in the index (14 MB at most): one partial gradient row and
+// loss sum per block, then the batch loss.
+struct TrainScratch {
+    float* part;
+    double *lpart, *loss;
+};
+TrainScratch train_scratch(hdg_index* idx) {
+    const size_t rows = (size_t)sm_count(), part = align_up(rows * kMlpParams * sizeof(float), 256);
+    idx->mlp_work.ensure(part + (rows + 1) * sizeof(double));
+    char* b = static_cast<char*>(idx->mlp_work.ptr);
+    TrainScratch t;
+    t.part = reinterpret_cast<float*>(b);
+    t.lpart = reinterpret_cast<double*>(b + part);
+    t.loss = t.lpart + rows;
+    return t;
 }
 
-__global__ void k_round_rows(const float* __restrict__ x, uint64_t n, float* __restrict__ out) {
-    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < n) out[e] = bf16r(x[e]);
+// Forward, backward and the summed gradient (into grad when given) of one batch; with a.m, the
+// Adam update too.  accumulate: the batch's mean loss is added to *s.loss instead of stored.
+void train_pass(const ModelPtrs& mp, const TrainScratch& s, const float* x, const float* y, const uint32_t* rows,
+                uint64_t n, int accumulate, float* grad, const AdamStep& a, cudaStream_t st) {
+    const FwdOut o{nullptr, nullptr, nullptr, 0, 0, y, rows, s.part, s.lpart};
+    const int nb = launch_mlp<true>(mp, x, n, o, st);
+    k_grad_reduce<<<(kMlpParams + 31) / 32, 256, 0, st>>>(s.part, nb, s.lpart, n, accumulate, grad, s.loss, a);
+    CK_LAUNCH();
 }
 
 }  // namespace
@@ -441,8 +574,8 @@ void learned_infer(hdg_index* idx, const float* feats, uint64_t q, uint32_t* npr
                    uint32_t max_probe, float* z, cudaStream_t st) {
     HDG_REQUIRE(idx->mlp_ready, HDG_ERR_STATE, "no trained model in this index");
     const ModelPtrs mp = model_ptrs(idx);
-    FwdOut o{z, nullptr, nullptr, nprobe, sched, allow_sched, max_probe};
-    launch_forward(mp, feats, q, o, st);
+    launch_mlp<false>(mp, feats, q, FwdOut{z, nprobe, sched, allow_sched, max_probe, nullptr, nullptr, nullptr, nullptr},
+                      st);
 }
 
 void mlp_init(hdg_index* idx, uint64_t seed) {
@@ -482,24 +615,18 @@ void mlp_get(hdg_index* idx, float* host, size_t count) {
 void mlp_forward(hdg_index* idx, const float* d_x, uint64_t n, float* d_z, cudaStream_t st) {
     HDG_REQUIRE(idx->mlp_ready, HDG_ERR_STATE, "no model in this index");
     const ModelPtrs mp = model_ptrs(idx);
-    launch_forward(mp, d_x, n, FwdOut{d_z, nullptr, nullptr, nullptr, nullptr, 0, 0}, st);
+    launch_mlp<false>(mp, d_x, n, FwdOut{d_z, nullptr, nullptr, 0, 0, nullptr, nullptr, nullptr, nullptr}, st);
 }
 
 double mlp_gradients(hdg_index* idx, const float* d_x, const float* d_y, uint64_t n, float* d_grad, cudaStream_t st) {
     HDG_REQUIRE(idx->mlp_ready, HDG_ERR_STATE, "no model in this index");
     HDG_REQUIRE(n > 0, HDG_ERR_INVALID_ARG, "empty batch");
     const ModelPtrs mp = model_ptrs(idx);
-    DevMem<float> z(n * kMlpOut), a1(n * kMlpHidden), a2(n * kMlpHidden), dz(n * kMlpOut);
-    DevMem<float> dh2(n * kMlpHidden), dh1(n * kMlpHidden), xr(n * kMlpFeatures);
-    DevMem<double> loss(1);
-    CK(cudaMemsetAsync(loss.p, 0, sizeof(double), st));
-    k_round_rows<<<(unsigned)((n * kMlpFeatures + 255) / 256), 256, 0, st>>>(d_x, n * kMlpFeatures, xr.p);
-    CK_LAUNCH();
-    launch_forward(mp, xr.p, n, FwdOut{z.p, a1.p, a2.p, nullptr, nullptr, 0, 0}, st);
-    launch_backward(mp, xr.p, d_y, n, z.p, a1.p, a2.p, dz.p, dh2.p, dh1.p, loss.p, st);
-    CK(cudaMemcpyAsync(d_grad, mp.grad, sizeof(float) * kMlpParams, cudaMemcpyDeviceToDevice, st));
+    std::lock_guard<std::mutex> lock(idx->mlp_mu);  // the scratch serves one call at a time
+    const TrainScratch ts = train_scratch(idx);
+    train_pass(mp, ts, d_x, d_y, nullptr, n, 0, d_grad, AdamStep{}, st);
     double h = 0.0;
-    CK(cudaMemcpyAsync(&h, loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&h, ts.loss, sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     return h;
 }
@@ -510,10 +637,9 @@ double mlp_train(hdg_index* idx, const float* d_x, const float* d_y, uint64_t n,
     HDG_REQUIRE(n > 0 && batch > 0 && epochs > 0, HDG_ERR_INVALID_ARG, "empty training run");
     const ModelPtrs mp = model_ptrs(idx);
     const uint64_t B = std::min<uint64_t>(batch, n);
-    DevMem<float> xb(B * kMlpFeatures), xr(B * kMlpFeatures), yb(B * kMlpOut), z(B * kMlpOut);
-    DevMem<float> a1(B * kMlpHidden), a2(B * kMlpHidden), dz(B * kMlpOut), dh2(B * kMlpHidden), dh1(B * kMlpHidden);
+    std::lock_guard<std::mutex> lock(idx->mlp_mu);
+    const TrainScratch ts = train_scratch(idx);
     DevMem<uint32_t> perm(n);
-    DevMem<double> loss(1);
     std::vector<uint32_t> order(n);
     for (uint64_t i = 0; i < n; i++) order[i] = (uint32_t)i;
     std::mt19937_64 rng(seed);
@@ -521,28 +647,18 @@ double mlp_train(hdg_index* idx, const float* d_x, const float* d_y, uint64_t n,
     for (uint32_t ep = 0; ep < epochs; ep++) {
         std::shuffle(order.begin(), order.end(), rng);
         CK(cudaMemcpyAsync(perm.p, order.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, st));
-        CK(cudaMemsetAsync(loss.p, 0, sizeof(double), st));
         uint64_t steps = 0;
         for (uint64_t s = 0; s + B <= n || (s < n && steps == 0); s += B) {
             const uint64_t nb = std::min<uint64_t>(B, n - s);
-            k_gather_batch<<<(unsigned)((nb * kMlpFeatures + 255) / 256), 256, 0, st>>>(d_x, d_y, perm.p + s, nb,
-                                                                                        xb.p, yb.p);
-            CK_LAUNCH();
-            k_round_rows<<<(unsigned)((nb * kMlpFeatures + 255) / 256), 256, 0, st>>>(xb.p, nb * kMlpFeatures,
-                                                                                      xr.p);
-            CK_LAUNCH();
-            launch_forward(mp, xr.p, nb, FwdOut{z.p, a1.p, a2.p, nullptr, nullptr, 0, 0}, st);
-            launch_backward(mp, xr.p, yb.p, nb, z.p, a1.p, a2.p, dz.p, dh2.p, dh1.p, loss.p, st);
             idx->mlp_step++;
             const float b1 = 0.9f, b2 = 0.999f;
             const float c1 = 1.f - std::pow(b1, (float)idx->mlp_step), c2 = 1.f - std::pow(b2, (float)idx->mlp_step);
-            k_adam<<<(kMlpParams + 255) / 256, 256, 0, st>>>(mp.master, mp.grad, mp.m, mp.v, kMlpParams, lr, b1, b2,
-                                                             1e-8f, c1, c2, mp.w);
-            CK_LAUNCH();
+            train_pass(mp, ts, d_x, d_y, perm.p + s, nb, steps > 0, nullptr,
+                       AdamStep{mp.master, mp.m, mp.v, lr, b1, b2, 1e-8f, c1, c2, mp.w}, st);
             steps++;
         }
         double h = 0.0;
-        CK(cudaMemcpyAsync(&h, loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(&h, ts.loss, sizeof(double), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         last = h / (double)std::max<uint64_t>(steps, 1);
     }
