@@ -436,10 +436,8 @@ hdg_status hdg_recover_filters(const hdg_filter_spec* spec, const float* d_query
     return guarded([&] {
         HDG_REQUIRE(spec && d_query_labels && d_ranges, HDG_ERR_INVALID_ARG, "null pointer");
         HDG_REQUIRE(spec->l >= 1 && spec->l <= HDG_MAX_LABEL_DIMS, HDG_ERR_INVALID_ARG, "bad l");
-        DeviceBuffer map;
-        map.ensure(std::max<size_t>(16, (size_t)spec->n_map * 4));
-        if (spec->n_map)
-            CK(cudaMemcpy(map.ptr, spec->interval_map, (size_t)spec->n_map * 4, cudaMemcpyHostToDevice));
+        HDG_REQUIRE(spec->n_map >= 0 && (spec->n_map == 0 || spec->interval_map), HDG_ERR_INVALID_ARG,
+                    "bad interval map");
         FilterDev f{};
         f.l = spec->l;
         bool range = false;
@@ -452,9 +450,17 @@ hdg_status hdg_recover_filters(const hdg_filter_spec* spec, const float* d_query
         }
         f.filter_dim = range ? 2 : 1;
         f.n_map = spec->n_map;
+        const cudaStream_t st = static_cast<cudaStream_t>(stream);
+        if (spec->n_map <= kMapArg) {
+            recover_filters_arg(f, spec->interval_map, d_query_labels, n_queries, d_ranges, st);
+            return;
+        }
+        DeviceBuffer map;
+        map.ensure((size_t)spec->n_map * 4);
+        CK(cudaMemcpy(map.ptr, spec->interval_map, (size_t)spec->n_map * 4, cudaMemcpyHostToDevice));
         f.map = static_cast<const float*>(map.ptr);
-        recover_filters(f, d_query_labels, n_queries, d_ranges, static_cast<cudaStream_t>(stream));
-        CK(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
+        recover_filters(f, d_query_labels, n_queries, d_ranges, st);
+        CK(cudaStreamSynchronize(st));
     });
 }
 

@@ -96,6 +96,10 @@ void label_mask(const float* ranges, const float* labels, uint32_t l, uint64_t n
                 const uint64_t* indices, uint64_t n_cand, int32_t* mask, cudaStream_t st);
 void recover_filters(const FilterDev& f, const float* qlabels, uint64_t nq, float* ranges,
                      cudaStream_t st);
+// the same with the map (at most kMapArg entries, host memory) passed as a kernel argument
+constexpr int kMapArg = 512;
+void recover_filters_arg(const FilterDev& f, const float* host_map, const float* qlabels, uint64_t nq, float* ranges,
+                         cudaStream_t st);
 void recover_filters_noalloc(const FilterDev& f, const float* host_map, const float* qlabels, uint64_t nq,
                              float* ranges, cudaStream_t st);
 // tcgen05 BF16 GEMM (hdg_gemm.cu)

@@ -33,3 +33,63 @@ def test_mlp_tiles(cuda, n):
     for name, _ in mo.SHAPES:
         rel = np.linalg.norm(gg[name] - oo[name]) / max(np.linalg.norm(oo[name]), 1e-12)
         assert rel <= (2e-2 if n < 32 else 5e-3), (name, rel)
+
+
+# one to four queries per shared-memory table, tables from one subspace to the largest that fits
+# (and past it: 256), candidate tiles of 128, candidates past the data set
+@pytest.mark.parametrize("m,q", [(1, 1), (7, 2), (25, 3), (32, 5), (33, 4), (50, 7), (64, 3), (128, 2), (200, 1), (256, 2)])
+@pytest.mark.parametrize("n,n_cand", [(1, 1), (127, 130), (128, 128), (2051, 2051), (40000, 33333)])
+def test_pq_adc_all_candidates(cuda, m, q, n, n_cand):
+    import torch
+    import hdgrid_b200 as hg
+    rng = np.random.default_rng(m * 1000 + n)
+    codes = rng.integers(0, 256, (m, n), dtype=np.uint8)
+    lut = rng.random((q, m, 256), dtype=np.float32)
+    out = torch.full((q, n_cand), -1.0, device=cuda)
+    hg.pq_adc(torch.from_numpy(codes).to(cuda), n, torch.from_numpy(lut).to(cuda), q, m, 256, None, n_cand, out)
+    got = out.cpu().numpy()
+    real = min(n, n_cand)
+    want = np.zeros((q, real))
+    for j in range(m):
+        want += lut[:, j, :].astype(np.float64)[:, codes[j, :real]]
+    # m positive terms summed in FP32 in some order: relative error below m * 2^-24
+    assert np.abs(got[:, :real] - want).max() <= m * 2.0 ** -24 * want.max()
+    assert np.all(got[:, real:] == np.finfo(np.float32).max)
+
+
+@pytest.mark.parametrize("l,q", [(1, 1), (3, 64), (4, 65), (4, 2), (8, 130)])
+@pytest.mark.parametrize("n,n_cand", [(1, 1), (5, 3), (1023, 1026), (4097, 4097), (5000, 4096)])
+def test_label_mask_all_candidates(cuda, l, q, n, n_cand):
+    import torch
+    import hdgrid_b200 as hg
+    rng = np.random.default_rng(l * 100 + q + n)
+    lab = rng.integers(0, 20, (n, l)).astype(np.float32)
+    lab[rng.random((n, l)) < 0.02] = np.nan  # a NaN label passes
+    lo = rng.integers(-1, 12, (q, l)).astype(np.float32)
+    hi = lo + rng.integers(0, 15, (q, l)).astype(np.float32)
+    box = np.stack([lo, hi], axis=2).reshape(q, 2 * l).copy()
+    out = torch.full((q, n_cand), 7, dtype=torch.int32, device=cuda)
+    hg.label_mask(torch.from_numpy(box).to(cuda), torch.from_numpy(lab).to(cuda), l, n, q, None, n_cand, out)
+    got = out.cpu().numpy()
+    real = min(n, n_cand)
+    bad = (lab[None, :real, :] < lo[:, None, :]) | (lab[None, :real, :] > hi[:, None, :])
+    assert np.array_equal(got[:, :real], (~bad.any(2)).astype(np.int32))
+    assert np.all(got[:, real:] == 0)
+
+
+@pytest.mark.parametrize("entries", [2, 512, 514, 70000])
+def test_recover_filters_map_sizes(cuda, entries):
+    import torch
+    import hdgrid_b200 as hg
+    rng = np.random.default_rng(entries)
+    table = rng.integers(0, 1 << 20, entries)
+    conf = "l = 1\nfilter0:\n\ttype = 1\n\tinterval_map = [" + ", ".join(map(str, table)) + "]\n"
+    ql = np.concatenate([[1.0, entries / 2, entries / 2 + 1], rng.integers(1, entries // 2 + 1, 200)]).astype(np.float32)
+    out = torch.empty((ql.size, 2), device=cuda)
+    hg.recover_filters(conf, torch.from_numpy(ql[:, None].copy()).to(cuda), out)
+    got = out.cpu().numpy()
+    v = (ql - 1).astype(np.int64)
+    ok = 2 * v + 1 < entries
+    assert np.array_equal(got[ok, 0], table[2 * v[ok]].astype(np.float32))
+    assert np.array_equal(got[ok, 1], table[2 * v[ok] + 1].astype(np.float32))
+    assert np.all(got[~ok, 0] > got[~ok, 1])  # outside the table: an empty box
