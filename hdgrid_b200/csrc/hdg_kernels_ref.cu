@@ -398,9 +398,18 @@ void recover_filters_noalloc(const FilterDev& f0, const float* host_map, const f
 }
 
 // ---- filtered exact kNN ------------------------------------------------------------------
-// Block = 256 threads, 32 queries x 64 base vectors per tile, each thread a 2 x 4 register
-// tile of f32 distances; per-query top-k buffers in shared memory with a running threshold.
-constexpr int BF_Q = 32, BF_V = 64, BF_K = 32, BF_CAP = 512;
+// An item is a group of queries and a span of base rows; a block of 16 warps streams the span
+// through shared memory in tiles of R rows (two tiles, copied ahead by cp.async).  A warp owns
+// `own` queries (or, with fewer queries than warps, a share of every tile's rows of one query): it
+// tests the tile's labels first, packs the rows that pass into a list and only then computes
+// distances, one (query, row) pair per lane, in dimension order as one FMA chain.  A key below the
+// query's running k-th goes to the query's buffer, which a warp sort cuts back to k when it fills.
+// An item leaves its k best keys per query; k_bf_merge takes the k smallest over the spans.
+// Bound: with many queries the shared-memory reads of the passing rows (16 bytes per pair and four
+// dimensions), with few the read of the base set.
+// One block per 32 queries that computed every pair and tested the labels afterwards took 352 ms
+// on 1,000 queries x 1 M x 128 (32 blocks, 10 % of the pairs pass); this takes BF_MS.
+constexpr int kBfThreads = 512, kBfWarps = kBfThreads / 32;
 
 __device__ void warp_bitonic_sort(uint64_t* keys, int n) {
     const int lane = threadIdx.x & 31;
@@ -419,128 +428,235 @@ __device__ void warp_bitonic_sort(uint64_t* keys, int n) {
         }
 }
 
-__global__ void __launch_bounds__(256) k_bruteforce(const float* __restrict__ data, uint64_t n, uint32_t d,
-                                                    const float* __restrict__ labels, uint32_t l,
-                                                    const float* __restrict__ queries, uint64_t nq,
-                                                    const float* __restrict__ ranges, uint32_t k,
-                                                    float* __restrict__ out_dist, uint64_t* __restrict__ out_ids) {
+struct BfShape {
+    int rows;      // R: rows per tile (a multiple of 32)
+    int pitch;     // floats per staged row (0: rows are read from global memory)
+    int cap;       // keys per query buffer (a power of two, at least k + 64)
+    int queries;   // queries per item
+    int share;     // warps per query (queries * share = 16 * own)
+    int staged_q;  // query vectors in shared memory
+    uint32_t spans;
+};
+
+static size_t bf_smem(const BfShape& b, uint32_t d, uint32_t l) {
+    return sizeof(uint64_t) * b.cap * std::max(b.queries * b.share, kBfWarps) + (b.staged_q ? sizeof(float) * b.queries * ((d + 3) / 4 * 4) : 0) +
+           sizeof(float) * 2 * b.rows * ((size_t)b.pitch + l) + sizeof(float) * b.queries * 2 * l +
+           kBfWarps * (size_t)b.rows;
+}
+
+__device__ __forceinline__ void bf_copy4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void bf_copy16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// VEC: d % 4 == 0 and 16-byte aligned base rows
+template <bool VEC>
+__global__ void __launch_bounds__(kBfThreads) k_bruteforce(const float* __restrict__ data, uint64_t n, uint32_t d,
+                                                           const float* __restrict__ labels, uint32_t l,
+                                                           const float* __restrict__ queries, uint64_t nq,
+                                                           const float* __restrict__ ranges, uint32_t k, BfShape b,
+                                                           uint64_t* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char smem[];
-    uint64_t* s_buf = reinterpret_cast<uint64_t*>(smem);  // [BF_Q][BF_CAP]
-    __shared__ float s_qt[BF_K][BF_Q + 1];
-    __shared__ float s_vt[BF_K][BF_V + 4];
-    __shared__ float s_lab[BF_V][kMaxDims];
-    __shared__ float s_rng[BF_Q][2 * kMaxDims];
-    __shared__ int s_cnt[BF_Q];
-    __shared__ uint64_t s_th[BF_Q];
-    __shared__ int s_need;
-    const int t = threadIdx.x, warp = t >> 5;
-    const int tq = t >> 4;  // 16 query pairs
-    const int tv = t & 15;  // 16 vector quads
-    const uint64_t q0 = (uint64_t)blockIdx.x * BF_Q;
-    for (int e = t; e < BF_Q * 2 * (int)l; e += blockDim.x) {
-        const int qq = e / (2 * l), c = e % (2 * l);
-        s_rng[qq][c] = (q0 + qq < nq) ? ranges[(q0 + qq) * 2 * l + c] : 1.f;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int R = b.rows, dq = (int)(d + 3) / 4 * 4;
+    const int nbuf = max(b.queries * b.share, kBfWarps), own = b.queries * b.share / kBfWarps;
+    uint64_t* s_buf = reinterpret_cast<uint64_t*>(smem);                        // [nbuf][cap]
+    float* s_q = reinterpret_cast<float*>(s_buf + (size_t)nbuf * b.cap);        // [queries][dq]
+    float* s_tile = s_q + (b.staged_q ? b.queries * dq : 0);                     // [2][R][pitch]
+    float* s_lab = s_tile + 2 * (size_t)R * b.pitch;                             // [2][R][l]
+    float* s_rng = s_lab + 2 * (size_t)R * l;                                    // [queries][2 l]
+    uint8_t* s_list = reinterpret_cast<uint8_t*>(s_rng + b.queries * 2 * l) + (size_t)warp * R;  // [R] rows that pass
+    const uint64_t group = blockIdx.x / b.spans, span = blockIdx.x % b.spans;
+    const uint64_t q0 = group * b.queries;
+    const int nqb = (int)min((uint64_t)b.queries, nq - q0);
+    for (int e = t; b.staged_q && e < b.queries * dq; e += kBfThreads) {
+        const int qq = e / dq, j = e % dq;
+        s_q[e] = qq < nqb && j < (int)d ? queries[(q0 + qq) * d + j] : 0.f;
     }
-    if (t < BF_Q) {
-        s_cnt[t] = 0;
-        s_th[t] = ~0ull;
-    }
-    const int K = (int)k;
-    for (uint64_t v0 = 0; v0 < n; v0 += BF_V) {
-        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        for (uint32_t k0 = 0; k0 < d; k0 += BF_K) {
-            __syncthreads();
-            for (int e = t; e < BF_Q * BF_K; e += blockDim.x) {
-                const int qq = e / BF_K, kk = e % BF_K;
-                s_qt[kk][qq] = (q0 + qq < nq && k0 + kk < d) ? queries[(q0 + qq) * d + k0 + kk] : 0.f;
-            }
-            for (int e = t; e < BF_V * BF_K; e += blockDim.x) {
-                const int vv = e / BF_K, kk = e % BF_K;
-                s_vt[kk][vv] = (v0 + vv < n && k0 + kk < d) ? data[(v0 + vv) * d + k0 + kk] : 0.f;
-            }
-            if (k0 == 0)
-                for (int e = t; e < BF_V * (int)l; e += blockDim.x) {
-                    const int vv = e / l, c = e % l;
-                    s_lab[vv][c] = (v0 + vv < n) ? labels[(v0 + vv) * l + c] : 0.f;
+    for (int e = t; e < nqb * 2 * (int)l; e += kBfThreads) s_rng[e] = ranges[q0 * 2 * l + e];
+    const uint64_t tiles = (n + R - 1) / R;
+    const uint64_t t0 = tiles * span / b.spans, t1 = tiles * (span + 1) / b.spans;
+    auto issue = [&](uint64_t tile, int st) {
+        const uint64_t v0 = tile * R;
+        const int rows = (int)min((uint64_t)R, n - v0);
+        float* dst = s_tile + (size_t)st * R * b.pitch;
+        if (b.pitch) {
+            if (VEC) {
+                const int d4 = (int)d / 4;
+                for (int e = t; e < rows * d4; e += kBfThreads) {
+                    const int r = e / d4, j = e % d4;
+                    bf_copy16(dst + (size_t)r * b.pitch + 4 * j, data + (v0 + r) * d + 4 * j);
                 }
-            __syncthreads();
-#pragma unroll 8
-            for (int kk = 0; kk < BF_K; kk++) {
-                const float a0 = s_qt[kk][2 * tq], a1 = s_qt[kk][2 * tq + 1];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float b = s_vt[kk][4 * tv + j];
-                    const float d0 = a0 - b, d1 = a1 - b;
-                    acc[0][j] = fmaf(d0, d0, acc[0][j]);
-                    acc[1][j] = fmaf(d1, d1, acc[1][j]);
-                }
-            }
-        }
-        // predicate + threshold + append (each query gets at most 64 appends per tile)
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const int qq = 2 * tq + i;
-            if (q0 + qq >= nq) continue;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int vv = 4 * tv + j;
-                const uint64_t id = v0 + vv;
-                if (id >= n) continue;
-                bool pass = true;
-                for (uint32_t c = 0; c < l; c++) {
-                    const float lv = s_lab[vv][c];
-                    if (lv < s_rng[qq][2 * c] || lv > s_rng[qq][2 * c + 1]) pass = false;
-                }
-                if (!pass) continue;
-                const uint64_t key = ((uint64_t)float_key(acc[i][j]) << 32) | (uint32_t)id;
-                if (key < s_th[qq]) {
-                    const int pos = atomicAdd(&s_cnt[qq], 1);
-                    s_buf[qq * BF_CAP + pos] = key;
-                }
-            }
-        }
-        __syncthreads();
-        if (t == 0) {
-            int need = 0;
-            for (int qq = 0; qq < BF_Q; qq++) need |= (s_cnt[qq] > BF_CAP - BF_V) ? 1 : 0;
-            s_need = need;
-        }
-        __syncthreads();
-        if (s_need) {
-            for (int qq = warp; qq < BF_Q; qq += 8) {
-                const int c = s_cnt[qq];
-                if (c <= BF_CAP - BF_V) continue;
-                uint64_t* buf = s_buf + qq * BF_CAP;
-                for (int i = c + (t & 31); i < BF_CAP; i += 32) buf[i] = ~0ull;
-                __syncwarp();
-                warp_bitonic_sort(buf, BF_CAP);
-                if ((t & 31) == 0) {
-                    s_cnt[qq] = min(c, K);
-                    if (c >= K) s_th[qq] = buf[K - 1];
-                }
-                __syncwarp();
-            }
-        }
-    }
-    __syncthreads();
-    for (int qq = warp; qq < BF_Q; qq += 8) {
-        if (q0 + qq >= nq) continue;
-        const int c = s_cnt[qq];
-        uint64_t* buf = s_buf + qq * BF_CAP;
-        for (int i = c + (t & 31); i < BF_CAP; i += 32) buf[i] = ~0ull;
-        __syncwarp();
-        warp_bitonic_sort(buf, BF_CAP);
-        const uint64_t q = q0 + qq;
-        for (int i = (t & 31); i < K; i += 32) {
-            const uint64_t key = buf[i];
-            if (i < c && key != ~0ull) {
-                out_dist[q * k + i] = key_float((uint32_t)(key >> 32));
-                out_ids[q * k + i] = (uint32_t)key;
             } else {
-                out_dist[q * k + i] = INFINITY;
-                out_ids[q * k + i] = ~0ull;
+                for (int e = t; e < rows * (int)d; e += kBfThreads) {
+                    const int r = e / (int)d, j = e % (int)d;
+                    bf_copy4(dst + (size_t)r * b.pitch + j, data + (v0 + r) * d + j);
+                }
             }
         }
+        for (int e = t; e < rows * (int)l; e += kBfThreads) bf_copy4(s_lab + (size_t)st * R * l + e, labels + v0 * l + e);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the buffers of this warp: slot warp * own + i, query (warp / share) * own + i (own > 1: share 1)
+    const int sub = warp % b.share, my_rows = R / b.share, r_lo = sub * my_rows;
+    constexpr int kOwn = 2;
+    int cnt[kOwn] = {0, 0};
+    uint64_t th[kOwn] = {~0ull, ~0ull};
+    if (t0 < t1) issue(t0, 0);
+    for (uint64_t tile = t0; tile < t1; tile++) {
+        const int st = (int)((tile - t0) & 1);
+        if (tile + 1 < t1) {
+            issue(tile + 1, st ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const uint64_t v0 = tile * R;
+        const int rows = (int)min((uint64_t)R, n - v0);
+        const float* tl = s_tile + (size_t)st * R * b.pitch;
+        const float* tlab = s_lab + (size_t)st * R * l;
+#pragma unroll
+        for (int o = 0; o < kOwn; o++) {
+            const int qq = (warp / b.share) * own + o;
+            if (o >= own || qq >= nqb) continue;
+            const float* rg = s_rng + qq * 2 * l;
+            int np = 0;
+            for (int r0 = r_lo; r0 < r_lo + my_rows; r0 += 32) {
+                const int r = r0 + lane;
+                bool ok = r < r_lo + my_rows && r < rows;
+                for (uint32_t i = 0; ok && i < l; i++) {
+                    const float v = tlab[r * l + i];
+                    if (v < rg[2 * i] || v > rg[2 * i + 1]) ok = false;
+                }
+                const unsigned bal = __ballot_sync(0xffffffffu, ok);
+                if (ok) s_list[np + __popc(bal & ((1u << lane) - 1u))] = (uint8_t)r;
+                np += __popc(bal);
+            }
+            __syncwarp();
+            uint64_t* buf = s_buf + (size_t)(warp * own + o) * b.cap;
+            const float* q = b.staged_q ? s_q + qq * dq : queries + (q0 + qq) * d;
+            for (int p0 = 0; p0 < np; p0 += 32) {
+                const bool v = p0 + lane < np;
+                const int r = s_list[v ? p0 + lane : p0];
+                const float* row = b.pitch ? tl + (size_t)r * b.pitch : data + (v0 + r) * d;
+                float acc = 0.f;
+                if (VEC) {
+#pragma unroll 4
+                    for (int j = 0; j < (int)d / 4; j++) {
+                        const float4 x = reinterpret_cast<const float4*>(q)[j], y = reinterpret_cast<const float4*>(row)[j];
+                        float e = x.x - y.x;
+                        acc = fmaf(e, e, acc);
+                        e = x.y - y.y;
+                        acc = fmaf(e, e, acc);
+                        e = x.z - y.z;
+                        acc = fmaf(e, e, acc);
+                        e = x.w - y.w;
+                        acc = fmaf(e, e, acc);
+                    }
+                } else {
+#pragma unroll 4
+                    for (int j = 0; j < (int)d; j++) {
+                        const float e = q[j] - row[j];
+                        acc = fmaf(e, e, acc);
+                    }
+                }
+                const uint64_t key = ((uint64_t)float_key(acc) << 32) | (uint32_t)(v0 + r);
+                const bool in = v && key < th[o];
+                const unsigned bal = __ballot_sync(0xffffffffu, in);
+                if (in) buf[cnt[o] + __popc(bal & ((1u << lane) - 1u))] = key;
+                cnt[o] += __popc(bal);
+                if (cnt[o] > b.cap - 32) {  // cut back to the k best
+                    for (int i = cnt[o] + lane; i < b.cap; i += 32) buf[i] = ~0ull;
+                    __syncwarp();
+                    warp_bitonic_sort(buf, b.cap);
+                    cnt[o] = (int)k;
+                    th[o] = buf[k - 1];
+                    __syncwarp();
+                }
+            }
+        }
+        __syncthreads();  // the tile's reads are done before its buffer is refilled
+    }
+    // every buffer sorted, its first k keys final
+#pragma unroll
+    for (int o = 0; o < kOwn; o++) {
+        if (o >= own) continue;
+        uint64_t* buf = s_buf + (size_t)(warp * own + o) * b.cap;
+        for (int i = cnt[o] + lane; i < b.cap; i += 32) buf[i] = ~0ull;
+        __syncwarp();
+        warp_bitonic_sort(buf, b.cap);
+        for (int i = (int)k + lane; i < b.cap; i += 32) buf[i] = ~0ull;
+    }
+    // the warps of one query merge pairwise (k <= cap / 2)
+    for (int step = 1; step < b.share; step <<= 1) {
+        __syncthreads();
+        if (sub % (2 * step) == 0) {
+            uint64_t* buf = s_buf + (size_t)warp * b.cap;
+            const uint64_t* other = buf + (size_t)step * b.cap;
+            for (int i = lane; i < (int)k; i += 32) buf[b.cap - 1 - i] = other[i];
+            __syncwarp();
+            warp_bitonic_sort(buf, b.cap);
+            for (int i = (int)k + lane; i < b.cap; i += 32) buf[i] = ~0ull;
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 0; o < kOwn; o++) {
+        const int qq = (warp / b.share) * own + o;
+        if (o >= own || qq >= nqb || sub) continue;
+        uint64_t* dst = part + ((q0 + qq) * b.spans + span) * k;
+        const uint64_t* buf = s_buf + (size_t)(warp * own + o) * b.cap;
+        for (int i = lane; i < (int)k; i += 32) dst[i] = buf[i];
+    }
+}
+
+// The k smallest keys of each query's spans * k, ascending.  A query's keys come in rounds into a
+// buffer of kBfMerge; once it is full, it is cut to its k smallest and the k-th bounds the rest.
+constexpr int kBfMerge = 2048;
+__global__ void __launch_bounds__(256) k_bf_merge(const uint64_t* __restrict__ part, uint32_t spans, uint32_t k,
+                                                  float* __restrict__ out_dist, uint64_t* __restrict__ out_ids) {
+    __shared__ uint64_t s_keys[kBfMerge];
+    __shared__ uint32_t s_hist[256], s_wc[32];
+    __shared__ unsigned long long s_sel[4];
+    __shared__ int s_cnt;
+    const uint64_t q = blockIdx.x;
+    const uint64_t* src = part + q * spans * k;
+    const uint32_t total = spans * k;
+    uint64_t th = ~0ull;
+    if (threadIdx.x == 0) s_cnt = 0;
+    __syncthreads();
+    for (uint32_t e0 = 0; e0 < total; e0 += 256) {
+        const uint32_t e = e0 + threadIdx.x;
+        const uint64_t key = e < total ? src[e] : ~0ull;
+        if (key < th) s_keys[atomicAdd(&s_cnt, 1)] = key;
+        __syncthreads();
+        const int c = s_cnt;
+        __syncthreads();
+        if (c > kBfMerge - 256) {
+            th = block_select_smallest(s_keys, c, (int)k, s_hist, s_wc, s_sel);
+            if (threadIdx.x == 0) s_cnt = (int)k;
+            __syncthreads();
+        }
+    }
+    int c = s_cnt;
+    __syncthreads();
+    if (c > (int)k) {
+        block_select_smallest(s_keys, c, (int)k, s_hist, s_wc, s_sel);
+        c = (int)k;
+    }
+    const int n2 = (int)next_pow2_dev((uint32_t)max(c, 2));
+    for (int i = c + (int)threadIdx.x; i < n2; i += blockDim.x) s_keys[i] = ~0ull;
+    __syncthreads();
+    block_bitonic_sort(s_keys, n2);
+    for (int i = threadIdx.x; i < (int)k; i += blockDim.x) {
+        const uint64_t key = i < c ? s_keys[i] : ~0ull;
+        out_dist[q * k + i] = key != ~0ull ? key_float((uint32_t)(key >> 32)) : INFINITY;
+        out_ids[q * k + i] = key != ~0ull ? (uint64_t)(uint32_t)key : ~0ull;
     }
 }
 
@@ -551,10 +667,69 @@ void bruteforce_knn(const float* data, uint64_t n, uint32_t d, const float* labe
     HDG_REQUIRE(l >= 1 && l <= (uint32_t)kMaxDims && d >= 1, HDG_ERR_INVALID_ARG, "bad dims");
     HDG_REQUIRE(n < (1ull << 32), HDG_ERR_INVALID_ARG, "n must be < 2^32");
     if (!q) return;
-    const size_t sm = sizeof(uint64_t) * BF_Q * BF_CAP;
-    CK(cudaFuncSetAttribute(k_bruteforce, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_bruteforce<<<nblk(q, BF_Q), 256, sm, st>>>(data, n, d, labels, l, queries, q, ranges, k, dist, ids);
-    CK_LAUNCH();
+    bool vec = d % 4 == 0 && (reinterpret_cast<uintptr_t>(data) & 15) == 0;
+    BfShape b{};
+    // two queries per warp (32 per item: the base set is streamed once per 32 queries) while their
+    // buffers are small, one for k > 128; fewer queries than warps share the warps out
+    b.cap = k <= 128 ? 256 : 512;
+    b.queries = k <= 128 ? 32 : 16;
+    b.share = 1;
+    b.staged_q = 1;
+    if (q <= 16) {
+        b.queries = 1;
+        while ((uint64_t)b.queries < q) b.queries *= 2;
+        b.share = kBfWarps / b.queries;
+    }
+    // the longest tile whose two buffers fit, its rows padded to an odd number of bank groups;
+    // rows too long for that are read from global memory, and so are queries of extreme length
+    const size_t most = 227 * 1024;
+    b.pitch = vec ? (int)(d + (d / 4 % 2 ? 0 : 4)) : (int)(d | 1);
+    for (b.rows = 128; b.rows >= 32 && bf_smem(b, d, l) > most; b.rows /= 2) {
+    }
+    if (b.rows < 32) {
+        b.rows = 128;
+        b.pitch = 0;
+        if (bf_smem(b, d, l) > most) {
+            b.staged_q = 0;
+            vec = false;
+        }
+    }
+    const size_t sm = bf_smem(b, d, l);
+    // spans: of one to four items per SM, the count that leaves the last round fullest
+    constexpr uint64_t kBfBatch = 65536;  // queries per launch: bounds the partial keys
+    const uint64_t sms = (uint64_t)sm_count(), tiles = std::max<uint64_t>(1, (n + b.rows - 1) / b.rows);
+    for (uint64_t a = 0; a < q; a += kBfBatch) {
+        const uint64_t nb = std::min(kBfBatch, q - a), groups = (nb + b.queries - 1) / b.queries;
+        uint64_t spans = 1;
+        double fill = 0.0;
+        for (uint64_t w = 1; w <= 4; w++) {
+            const uint64_t c = std::min(tiles, std::max<uint64_t>(1, sms * w / groups)), items = groups * c;
+            const double f = (double)items / (double)((items + sms - 1) / sms * sms);
+            if (f > fill + 0.02) {
+                fill = f;
+                spans = c;
+            }
+        }
+        b.spans = (uint32_t)spans;
+        uint64_t* part = nullptr;
+        CK(cudaMallocAsync(reinterpret_cast<void**>(&part), sizeof(uint64_t) * nb * spans * k, st));
+        auto launch = [&](auto kern) {
+            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            kern<<<(unsigned)(groups * spans), kBfThreads, sm, st>>>(data, n, d, labels, l, queries + a * d, nb,
+                                                                    ranges + a * 2 * l, k, b, part);
+            CK_LAUNCH();
+        };
+        try {
+            if (vec) launch(k_bruteforce<true>);
+            else launch(k_bruteforce<false>);
+            k_bf_merge<<<(unsigned)nb, 256, 0, st>>>(part, b.spans, k, dist + a * k, ids + a * k);
+            CK_LAUNCH();
+        } catch (...) {
+            cudaFreeAsync(part, st);
+            throw;
+        }
+        CK(cudaFreeAsync(part, st));
+    }
 }
 
 }  // namespace hdg

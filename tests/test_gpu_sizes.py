@@ -93,3 +93,36 @@ def test_recover_filters_map_sizes(cuda, entries):
     assert np.array_equal(got[ok, 0], table[2 * v[ok]].astype(np.float32))
     assert np.array_equal(got[ok, 1], table[2 * v[ok] + 1].astype(np.float32))
     assert np.all(got[~ok, 0] > got[~ok, 1])  # outside the table: an empty box
+
+
+# queries sharing warps (1 to 16) and two per warp, ragged groups; k at both buffer sizes; tiles of
+# 128 rows and their remainders; rows read as float4, as floats, and too long for a staged tile
+@pytest.mark.parametrize("q,k", [(1, 1), (2, 100), (3, 256), (9, 10), (16, 128), (17, 129), (33, 100), (70, 5)])
+@pytest.mark.parametrize("n,d,l", [(1, 4, 1), (31, 3, 4), (129, 100, 2), (5000, 128, 4), (20011, 96, 8), (1500, 384, 3),
+                                   (700, 1001, 1), (300, 6000, 2)])
+def test_bruteforce_shapes(cuda, q, k, n, d, l):
+    import torch
+    import hdgrid_b200 as hg
+    rng = np.random.default_rng(q * 31 + n)
+    base = rng.standard_normal((n, d), dtype=np.float32)
+    qs = rng.standard_normal((q, d), dtype=np.float32)
+    lab = rng.integers(0, 1000, (n, l)).astype(np.float32)
+    lo = np.where(rng.random((q, l)) < 0.6, 0, rng.integers(0, 1000, (q, l))).astype(np.float32)
+    hi = np.where(rng.random((q, l)) < 0.6, 1000, lo + rng.integers(0, 300, (q, l))).astype(np.float32)
+    box = np.stack([lo, hi], axis=2).reshape(q, 2 * l).copy()
+    dist = torch.full((q, k), -1.0, device=cuda)
+    ids = torch.full((q, k), 7, dtype=torch.int64, device=cuda)
+    hg.bruteforce_knn(torch.from_numpy(base).to(cuda), torch.from_numpy(lab).to(cuda), torch.from_numpy(qs).to(cuda),
+                      torch.from_numpy(box).to(cuda), k, dist, ids)
+    gd, gi = dist.cpu().numpy(), ids.cpu().numpy()
+    for i in range(q):
+        ok = np.all((lab >= lo[i]) & (lab <= hi[i]), axis=1)
+        e = ((base[ok].astype(np.float64) - qs[i].astype(np.float64)) ** 2).sum(1)
+        m = min(k, e.size)
+        tol = (d + 2) * 2.0 ** -24  # d positive terms, one FP32 chain
+        np.testing.assert_allclose(gd[i, :m], np.sort(e)[:m], rtol=tol)
+        full = np.full(n, np.inf)
+        full[ok] = e
+        np.testing.assert_allclose(full[gi[i, :m]], gd[i, :m], rtol=tol)
+        assert len(set(gi[i, :m].tolist())) == m
+        assert np.all(np.isinf(gd[i, m:])) and np.all(gi[i, m:] == -1)
