@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "hdg_device.cuh"
@@ -453,8 +454,44 @@ __device__ __forceinline__ void bf_copy16(void* dst, const void* src) {
                  : "memory");
 }
 
-// VEC: d % 4 == 0 and 16-byte aligned base rows
-template <bool VEC>
+// The squared distances of U rows per lane to one query, each one FMA chain in dimension order
+// (U independent chains hide the FMA and shared-memory latency; the query's reads are shared)
+template <bool VEC, int U>
+__device__ __forceinline__ void bf_dist(const float* q, const float* const (&row)[U], int d, float (&acc)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; u++) acc[u] = 0.f;
+    if (VEC) {
+#pragma unroll 4
+        for (int j = 0; j < d / 4; j++) {
+            const float4 x = reinterpret_cast<const float4*>(q)[j];
+            float4 y[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) y[u] = reinterpret_cast<const float4*>(row[u])[j];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const float e0 = x.x - y[u].x, e1 = x.y - y[u].y, e2 = x.z - y[u].z, e3 = x.w - y[u].w;
+                acc[u] = fmaf(e0, e0, acc[u]);
+                acc[u] = fmaf(e1, e1, acc[u]);
+                acc[u] = fmaf(e2, e2, acc[u]);
+                acc[u] = fmaf(e3, e3, acc[u]);
+            }
+        }
+    } else {
+#pragma unroll 4
+        for (int j = 0; j < d; j++) {
+            const float x = q[j];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const float e = x - row[u][j];
+                acc[u] = fmaf(e, e, acc[u]);
+            }
+        }
+    }
+}
+
+// VEC: d % 4 == 0 and 16-byte aligned base rows; LAB4: four label dims; STAGED: rows and queries in
+// shared memory (else rows, and queries of extreme length, are read from global memory)
+template <bool VEC, bool LAB4, bool STAGED>
 __global__ void __launch_bounds__(kBfThreads) k_bruteforce(const float* __restrict__ data, uint64_t n, uint32_t d,
                                                            const float* __restrict__ labels, uint32_t l,
                                                            const float* __restrict__ queries, uint64_t nq,
@@ -467,7 +504,7 @@ __global__ void __launch_bounds__(kBfThreads) k_bruteforce(const float* __restri
     uint64_t* s_buf = reinterpret_cast<uint64_t*>(smem);                        // [nbuf][cap]
     float* s_q = reinterpret_cast<float*>(s_buf + (size_t)nbuf * b.cap);        // [queries][dq]
     float* s_tile = s_q + (b.staged_q ? b.queries * dq : 0);                     // [2][R][pitch]
-    float* s_lab = s_tile + 2 * (size_t)R * b.pitch;                             // [2][R][l]
+    float* s_lab = s_tile + 2 * (size_t)R * b.pitch;                             // [2][R][l] (R % 32: 16-byte aligned)
     float* s_rng = s_lab + 2 * (size_t)R * l;                                    // [queries][2 l]
     uint8_t* s_list = reinterpret_cast<uint8_t*>(s_rng + b.queries * 2 * l) + (size_t)warp * R;  // [R] rows that pass
     const uint64_t group = blockIdx.x / b.spans, span = blockIdx.x % b.spans;
@@ -484,17 +521,14 @@ __global__ void __launch_bounds__(kBfThreads) k_bruteforce(const float* __restri
         const uint64_t v0 = tile * R;
         const int rows = (int)min((uint64_t)R, n - v0);
         float* dst = s_tile + (size_t)st * R * b.pitch;
-        if (b.pitch) {
-            if (VEC) {
-                const int d4 = (int)d / 4;
-                for (int e = t; e < rows * d4; e += kBfThreads) {
-                    const int r = e / d4, j = e % d4;
-                    bf_copy16(dst + (size_t)r * b.pitch + 4 * j, data + (v0 + r) * d + 4 * j);
-                }
-            } else {
-                for (int e = t; e < rows * (int)d; e += kBfThreads) {
-                    const int r = e / (int)d, j = e % (int)d;
-                    bf_copy4(dst + (size_t)r * b.pitch + j, data + (v0 + r) * d + j);
+        if (STAGED) {  // a warp copies whole rows: no division per element
+            for (int r = warp; r < rows; r += kBfWarps) {
+                float* to = dst + (size_t)r * b.pitch;
+                const float* from = data + (v0 + r) * d;
+                if (VEC) {
+                    for (int j = 4 * lane; j < (int)d; j += 128) bf_copy16(to + j, from + j);
+                } else {
+                    for (int j = lane; j < (int)d; j += 32) bf_copy4(to + j, from + j);
                 }
             }
         }
@@ -526,12 +560,21 @@ __global__ void __launch_bounds__(kBfThreads) k_bruteforce(const float* __restri
             if (o >= own || qq >= nqb) continue;
             const float* rg = s_rng + qq * 2 * l;
             int np = 0;
+#pragma unroll 4
             for (int r0 = r_lo; r0 < r_lo + my_rows; r0 += 32) {
                 const int r = r0 + lane;
                 bool ok = r < r_lo + my_rows && r < rows;
-                for (uint32_t i = 0; ok && i < l; i++) {
-                    const float v = tlab[r * l + i];
-                    if (v < rg[2 * i] || v > rg[2 * i + 1]) ok = false;
+                const int rr = ok ? r : 0;
+                if (LAB4) {
+                    const float4 v = reinterpret_cast<const float4*>(tlab)[rr];
+                    const float4 b0 = reinterpret_cast<const float4*>(rg)[0], b1 = reinterpret_cast<const float4*>(rg)[1];
+                    ok = ok && !(v.x < b0.x || v.x > b0.y) && !(v.y < b0.z || v.y > b0.w) &&
+                         !(v.z < b1.x || v.z > b1.y) && !(v.w < b1.z || v.w > b1.w);
+                } else {
+                    for (uint32_t i = 0; i < l; i++) {
+                        const float v = tlab[rr * l + i];
+                        if (v < rg[2 * i] || v > rg[2 * i + 1]) ok = false;
+                    }
                 }
                 const unsigned bal = __ballot_sync(0xffffffffu, ok);
                 if (ok) s_list[np + __popc(bal & ((1u << lane) - 1u))] = (uint8_t)r;
@@ -539,45 +582,42 @@ __global__ void __launch_bounds__(kBfThreads) k_bruteforce(const float* __restri
             }
             __syncwarp();
             uint64_t* buf = s_buf + (size_t)(warp * own + o) * b.cap;
-            const float* q = b.staged_q ? s_q + qq * dq : queries + (q0 + qq) * d;
-            for (int p0 = 0; p0 < np; p0 += 32) {
-                const bool v = p0 + lane < np;
-                const int r = s_list[v ? p0 + lane : p0];
-                const float* row = b.pitch ? tl + (size_t)r * b.pitch : data + (v0 + r) * d;
-                float acc = 0.f;
-                if (VEC) {
-#pragma unroll 4
-                    for (int j = 0; j < (int)d / 4; j++) {
-                        const float4 x = reinterpret_cast<const float4*>(q)[j], y = reinterpret_cast<const float4*>(row)[j];
-                        float e = x.x - y.x;
-                        acc = fmaf(e, e, acc);
-                        e = x.y - y.y;
-                        acc = fmaf(e, e, acc);
-                        e = x.z - y.z;
-                        acc = fmaf(e, e, acc);
-                        e = x.w - y.w;
-                        acc = fmaf(e, e, acc);
-                    }
-                } else {
-#pragma unroll 4
-                    for (int j = 0; j < (int)d; j++) {
-                        const float e = q[j] - row[j];
-                        acc = fmaf(e, e, acc);
+            const float* q = STAGED || b.staged_q ? s_q + qq * dq : queries + (q0 + qq) * d;
+            // U pairs per lane from list entry p0 on
+            auto pass = [&](int p0, auto uc) {
+                constexpr int U = decltype(uc)::value;
+                const float* row[U];
+                int r[U];
+                float acc[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int p = p0 + 32 * u + lane;
+                    r[u] = s_list[p < np ? p : p0];
+                    row[u] = STAGED ? tl + r[u] * b.pitch : data + (v0 + r[u]) * d;
+                }
+                bf_dist<VEC, U>(q, row, (int)d, acc);
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const uint64_t key = ((uint64_t)float_key(acc[u]) << 32) | (uint32_t)(v0 + r[u]);
+                    const bool in = p0 + 32 * u + lane < np && key < th[o];
+                    const unsigned bal = __ballot_sync(0xffffffffu, in);
+                    if (in) buf[cnt[o] + __popc(bal & ((1u << lane) - 1u))] = key;
+                    cnt[o] += __popc(bal);
+                    if (cnt[o] > b.cap - 32) {  // cut back to the k best
+                        for (int i = cnt[o] + lane; i < b.cap; i += 32) buf[i] = ~0ull;
+                        __syncwarp();
+                        warp_bitonic_sort(buf, b.cap);
+                        cnt[o] = (int)k;
+                        th[o] = buf[k - 1];
+                        __syncwarp();
                     }
                 }
-                const uint64_t key = ((uint64_t)float_key(acc) << 32) | (uint32_t)(v0 + r);
-                const bool in = v && key < th[o];
-                const unsigned bal = __ballot_sync(0xffffffffu, in);
-                if (in) buf[cnt[o] + __popc(bal & ((1u << lane) - 1u))] = key;
-                cnt[o] += __popc(bal);
-                if (cnt[o] > b.cap - 32) {  // cut back to the k best
-                    for (int i = cnt[o] + lane; i < b.cap; i += 32) buf[i] = ~0ull;
-                    __syncwarp();
-                    warp_bitonic_sort(buf, b.cap);
-                    cnt[o] = (int)k;
-                    th[o] = buf[k - 1];
-                    __syncwarp();
-                }
+            };
+            int p0 = 0;
+            for (; np - p0 > 64; p0 += 128) pass(p0, std::integral_constant<int, 4>());
+            for (; p0 < np; p0 += 64) {
+                if (np - p0 > 32) pass(p0, std::integral_constant<int, 2>());
+                else pass(p0, std::integral_constant<int, 1>());
             }
         }
         __syncthreads();  // the tile's reads are done before its buffer is refilled
@@ -720,8 +760,9 @@ void bruteforce_knn(const float* data, uint64_t n, uint32_t d, const float* labe
             CK_LAUNCH();
         };
         try {
-            if (vec) launch(k_bruteforce<true>);
-            else launch(k_bruteforce<false>);
+            if (!b.pitch) vec ? launch(k_bruteforce<true, false, false>) : launch(k_bruteforce<false, false, false>);
+            else if (vec) l == 4 ? launch(k_bruteforce<true, true, true>) : launch(k_bruteforce<true, false, true>);
+            else l == 4 ? launch(k_bruteforce<false, true, true>) : launch(k_bruteforce<false, false, true>);
             k_bf_merge<<<(unsigned)nb, 256, 0, st>>>(part, b.spans, k, dist + a * k, ids + a * k);
             CK_LAUNCH();
         } catch (...) {
