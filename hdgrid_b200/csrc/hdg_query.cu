@@ -906,10 +906,14 @@ __device__ __forceinline__ void store_lut(float* lut, int f16, uint64_t i, float
         lut[i] = v;
 }
 
-// Block = (64 queries, one group of 32 subspaces).  The group's codebook is staged once in
-// shared memory as [c*pq_len + t][33] (conflict-free stores from coalesced global reads and
-// conflict-free lane reads); lane = subspace column j, so a warp stores one contiguous
-// 128-byte LUT row per codeword.
+// Block = (64 queries, one group of 32 subspaces, a slice of the codewords).  The slice's codebook
+// rows are staged once in shared memory as [c*pq_len + t][33] (conflict-free stores from coalesced
+// global reads and conflict-free lane reads); lane = subspace column j, so a warp stores one
+// contiguous 128-byte LUT row per codeword.  The warps share out (query, part of the slice) pairs,
+// as many parts as it takes to give every warp one.  Bound: the LUT's writes.
+// The slice: the largest that still gives four blocks per SM (lut_slices); with the whole codebook
+// per block 1,000 queries ran on 16 blocks and one query on one warp.  Sliced, the stage went
+// 32 -> 8 us (1 query), 100 -> 27 us (1,000) and 192 -> 131 us (10,000, M = 32).
 __global__ void __launch_bounds__(512) k_lut(IndexDev D, const float* __restrict__ queries, uint64_t q, int G,
                                              float* __restrict__ lut, int f16, const uint32_t* __restrict__ item_off) {
     extern __shared__ float smem_lut[];
@@ -920,28 +924,34 @@ __global__ void __launch_bounds__(512) k_lut(IndexDev D, const float* __restrict
         if (!__syncthreads_or(need)) return;
     }
     const int g = blockIdx.y, pq_len = D.pq_len, d = D.d, M = D.M;
-    float* s_cb = smem_lut;                          // [(c * pq_len + t) * 33 + j]
-    const int n = 32 * kCodes * pq_len;
-    const float* src = D.pq_centers + (uint64_t)(32 * g) * kCodes * pq_len;
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-        const int j = e / (kCodes * pq_len), rem = e - j * (kCodes * pq_len);
-        s_cb[rem * 33 + j] = (32 * g + j < M) ? __ldg(src + e) : 0.f;
+    const int nc = kCodes / (int)gridDim.z, c0 = (int)blockIdx.z * nc;  // this slice's codewords
+    float* s_cb = smem_lut;                          // [((c - c0) * pq_len + t) * 33 + j]
+    const int n1 = nc * pq_len;                      // words per subspace
+    const float* src = D.pq_centers + (uint64_t)(32 * g) * kCodes * pq_len + (uint64_t)c0 * pq_len;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int j = warp; j < 32; j += nw) {
+        const bool real_j = 32 * g + j < M;
+        for (int r = lane; r < n1; r += 32)
+            s_cb[r * 33 + j] = real_j ? __ldg(src + (uint64_t)j * kCodes * pq_len + r) : 0.f;
     }
     __syncthreads();
-    // one warp per query: lane j keeps the query's slice of subspace 32g+j in registers
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int m = 32 * g + lane;
     const bool real = m < M;
-    for (int qq = warp; qq < kLutQ; qq += nw) {
-        const uint64_t qi = (uint64_t)blockIdx.x * kLutQ + qq;
-        if (qi >= q) break;
+    const int nq = (int)min((uint64_t)kLutQ, q - (uint64_t)blockIdx.x * kLutQ);
+    int parts = 1;  // parts of the slice per query (a power of two dividing nc)
+    while (parts < nc && parts * nq < nw) parts *= 2;
+    const int pc = nc / parts;
+    for (int u = warp; u < nq * parts; u += nw) {
+        const uint64_t qi = (uint64_t)blockIdx.x * kLutQ + u / parts;
         if (item_off[qi + 1] == item_off[qi]) continue;  // no ADC work: no LUT
+        // lane j keeps the query's slice of subspace 32g+j in registers
         float qv[kLutMaxPqLen];
 #pragma unroll
         for (int t = 0; t < kLutMaxPqLen; t++)
             qv[t] = (real && t < pq_len) ? queries[qi * d + (uint64_t)m * pq_len + t] : 0.f;
         const uint64_t row0 = (qi * G + g) * (kCodes * 32);
-        for (int c = 0; c < kCodes; c++) {
+        const int cb = u % parts * pc;
+        for (int c = cb; c < cb + pc; c++) {
             float s = 0.f;
 #pragma unroll
             for (int t = 0; t < kLutMaxPqLen; t++) {
@@ -950,9 +960,17 @@ __global__ void __launch_bounds__(512) k_lut(IndexDev D, const float* __restrict
                     s = fmaf(df, df, s);
                 }
             }
-            store_lut(lut, f16, row0 + c * 32 + lane, real ? s : 0.f);
+            store_lut(lut, f16, row0 + (uint64_t)(c0 + c) * 32 + lane, real ? s : 0.f);
         }
     }
+}
+
+// Codeword slices of k_lut: the fewest (at most 16) that give four blocks per SM
+static int lut_slices(uint64_t q, int G, int sms) {
+    const uint64_t blocks = (q + kLutQ - 1) / kLutQ * (uint64_t)G;
+    int s = 1;
+    while (s < 16 && blocks * s < 4ull * sms) s *= 2;
+    return s;
 }
 
 // Fallback for long subspaces: one query per block, thread = codeword, transposed store.
@@ -2812,10 +2830,11 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             // the LUTs of the queries that have ADC work items (a predicate-first query whose
             // budget takes every survivor has none)
             if (D.pq_len <= (uint32_t)kLutMaxPqLen) {
-                const size_t sm = sizeof(float) * kCodes * D.pq_len * 33;
+                const int slices = lut_slices(q, (int)G, sm_count());
+                const size_t sm = sizeof(float) * (kCodes / slices) * D.pq_len * 33;
                 CK(cudaFuncSetAttribute(k_lut, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-                k_lut<<<dim3((unsigned)((q + kLutQ - 1) / kLutQ), G), 512, sm, st>>>(D, c.queries, q, (int)G, w.lut,
-                                                                                    w.lut16, w.item_off);
+                k_lut<<<dim3((unsigned)((q + kLutQ - 1) / kLutQ), G, slices), 512, sm, st>>>(D, c.queries, q, (int)G,
+                                                                                            w.lut, w.lut16, w.item_off);
             } else {
                 k_lut_plain<<<dim3((unsigned)q, G), 256, sizeof(float) * D.d, st>>>(D, c.queries, (int)G, w.lut,
                                                                                   w.lut16, w.item_off);
