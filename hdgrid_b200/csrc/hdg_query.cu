@@ -37,7 +37,8 @@ namespace hdg {
 
 constexpr int kThreads = 256;
 constexpr uint32_t kInvalid = 0xffffffffu;
-constexpr uint32_t kChunk = 32768;  // default candidates per scan work item (SCAN_CHUNK)
+constexpr uint32_t kChunk = 32768;  // default most candidates per scan work item (SCAN_CHUNK)
+constexpr uint32_t kChunkMin = 1024;
 constexpr int kBins = 4096;         // select histogram
 constexpr int kBCap = 4096;         // boundary-bin buffer of the select
 constexpr uint32_t kPreChunk = 8192; // candidates per work item of the predicate pass
@@ -64,7 +65,7 @@ struct Workspace {
     uint32_t* nfin;          // [q] finite distances (predicate passed)
     uint32_t* lab_read;      // [q] candidates of the predicate pass whose labels were read
     uint32_t* rank_read;     // [q] candidates of the predicate pass whose label ranks were read
-    uint32_t* counter;       // [4] work counters: ADC scan, refine, predicate pass
+    uint32_t* counter;       // [4] work counters: ADC scan, refine, predicate pass; [3] candidates per scan item
     float* lut;              // [q x G x 256 x 32] f32, or __half when lut16
     int lut16;               // LUT stored in FP16 (LUT_FP16=1); the scan sums in FP32
     uint32_t* qbud;          // [q] candidate budget n_cand of each query (k_batch)
@@ -95,7 +96,8 @@ struct Workspace {
     uint32_t k_max;          // output row stride
     int mode;                // batch schedule: 0 pre-filter (exps0 <= 1), 1 post-filter, 2 single dim
     uint32_t exps0;
-    uint32_t chunk;          // candidates per scan work item
+    uint32_t chunk;          // candidates per scan work item (SCAN_CHUNK; 0: set by k_batch from the batch)
+    uint32_t scan_items;     // work items k_batch aims at when it sets the chunk
     int is_split;            // IS_SPLIT: trimmed Morton sub-ranges per probed list
     int nsplit;              // sub-ranges per probed list (n_split when is_split, else 1)
     uint64_t cap;            // distance-buffer capacity in candidates
@@ -144,6 +146,8 @@ __device__ __forceinline__ uint32_t q_budget(const Workspace& w, uint64_t qi) { 
 __device__ __forceinline__ bool takes_row(const Workspace& w, uint64_t qi) {
     return compacts(w, qi) && w.nfin[qi] <= q_budget(w, qi);
 }
+// Candidates per scan work item (k_batch sets the word)
+__device__ __forceinline__ uint32_t scan_chunk(const Workspace& w) { return w.counter[3]; }
 // The selected candidates (pool rows) of query qi: its row of the selection buffer, or its
 // distance row when it takes the row whole
 __device__ __forceinline__ uint32_t* sel_row(const Workspace& w, uint64_t qi) {
@@ -776,6 +780,7 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
     __shared__ unsigned long long s_tot[32], s_items[32], s_pitems[32], s_sel[32];
     __shared__ unsigned long long s_red[3], s_drop[2];
     __shared__ float s_beta;
+    __shared__ uint32_t s_chunk;
     const int t = threadIdx.x;
     if (t == 0) s_red[0] = s_red[1] = s_red[2] = s_drop[0] = s_drop[1] = 0;
     __syncthreads();
@@ -783,7 +788,26 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
     const uint64_t b = t * per, e = min(q, b + per);
     // a predicate-first query of the predicate pass has predicate items over its candidates
     // (its ADC items follow from its survivors, k_scan_plan); any other query has ADC items
-    auto n_items = [&](uint64_t i, uint32_t c) { return compacts(w, i) ? 0u : (c + w.chunk - 1) / w.chunk; };
+    // Candidates per scan item: SCAN_CHUNK, or the smallest power of two from kChunkMin to kChunk
+    // that leaves at most scan_items items.  A small batch then fills the SMs (37 queries of
+    // 73,000 candidates ran as 111 items of up to 32,768: SCAN_FIG); a large one keeps long
+    // items, since each loads its query's LUT.
+    if (w.chunk) {
+        if (t == 0) s_chunk = w.chunk;
+        __syncthreads();
+    } else {
+        unsigned long long c = 0, all = 0;
+        for (uint64_t i = b; i < e; i++) c += w.qstat[i * 4];
+        block_inclusive_sum(c, s_tot, &all);
+        if (t == 0) {
+            uint32_t ch = kChunkMin;
+            while (ch < kChunk && (unsigned long long)ch * w.scan_items < all) ch *= 2;
+            s_chunk = ch;
+        }
+        __syncthreads();
+    }
+    const uint32_t chunk = s_chunk;
+    auto n_items = [&](uint64_t i, uint32_t c) { return compacts(w, i) ? 0u : (c + chunk - 1) / chunk; };
     auto n_pitems = [&](uint64_t i, uint32_t c) { return compacts(w, i) ? (c + kPreChunk - 1) / kPreChunk : 0u; };
     unsigned long long cand = 0, items = 0, pitems = 0, exact = 0, mx = 0;
     for (uint64_t i = b; i < e; i++) {
@@ -850,6 +874,7 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
         s_beta = beta;
         w.counter[0] = 0;
         w.counter[2] = 0;
+        w.counter[3] = chunk;
     }
     __syncthreads();
     // each query's budget n_cand, now that the batch's beta and max_row are known, and the
@@ -1410,13 +1435,14 @@ __global__ void __launch_bounds__(1024) k_scan_plan(uint64_t q, Workspace w) {
     const int t = threadIdx.x;
     const uint64_t per = (q + blockDim.x - 1) / blockDim.x;
     const uint64_t b = t * per, e = min(q, b + per);
+    const uint32_t chunk = scan_chunk(w);
     auto n_items = [&](uint64_t i) {
         uint32_t c = compacts(w, i) ? w.cand_count[i] : w.qstat[i * 4];
         // a compact row that its budget takes whole needs no ADC distance (the select takes
         // every survivor and the re-rank orders them), unless the distances are the output
         // (the reference's pre-filter schedule)
         if (compacts(w, i) && w.mode != kPre && c <= w.qbud[i]) c = 0;
-        return (c + w.chunk - 1) / w.chunk;
+        return (c + chunk - 1) / chunk;
     };
     // such a row's survivors all count as passed (the ADC scan counts them for the others)
     for (uint64_t i = b; i < e; i++)
@@ -1447,7 +1473,7 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
     uint32_t* s_start = s_pre + Ps + 1;                                       // [Ps]
     __shared__ ScanShared s;
     const int t = threadIdx.x, lane = t & 31;
-    const uint32_t n_items = w.item_off[q];
+    const uint32_t n_items = w.item_off[q], chunk = scan_chunk(w);
     int cur = -1;
     for (;;) {
         if (t == 0) {
@@ -1469,7 +1495,7 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
         const int qq = s.query;
         const bool compact = compacts(w, qq);
         const uint32_t total = compact ? w.cand_count[qq] : w.qstat[(uint64_t)qq * 4];
-        const uint32_t e0 = (uint32_t)(item - w.item_off[qq]) * w.chunk;
+        const uint32_t e0 = (uint32_t)(item - w.item_off[qq]) * chunk;
         if (e0 >= total) {  // a query cut by the distance capacity
             __syncthreads();
             continue;
@@ -1505,7 +1531,7 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
             else __syncthreads();
             cur = qq;
         }
-        const uint32_t e1 = min(total, e0 + w.chunk);
+        const uint32_t e1 = min(total, e0 + chunk);
         float* dst = w.dist + w.qoff[qq];
         const uint32_t* srow = reinterpret_cast<const uint32_t*>(dst);  // compact: the survivors' pool rows
         const uint32_t* sp = w.spos + w.qoff[qq];
@@ -1620,7 +1646,7 @@ __global__ void __launch_bounds__(512) k_scan_generic(IndexDev D, int G, int Ps,
     __shared__ ScanShared s;
     __shared__ float s_box[2 * kMaxDims];
     const int t = threadIdx.x, lane = t & 31;
-    const uint32_t n_items = w.item_off[q];
+    const uint32_t n_items = w.item_off[q], chunk = scan_chunk(w);
     const int M = D.M;
     int cur = -1;
     for (;;) {
@@ -1642,7 +1668,7 @@ __global__ void __launch_bounds__(512) k_scan_generic(IndexDev D, int G, int Ps,
         if (item >= (int)n_items) break;
         const int qq = s.query;
         const uint32_t total = w.qstat[(uint64_t)qq * 4];
-        const uint32_t e0 = (uint32_t)(item - w.item_off[qq]) * w.chunk;
+        const uint32_t e0 = (uint32_t)(item - w.item_off[qq]) * chunk;
         if (e0 >= total) {  // a query cut by the distance capacity
             __syncthreads();
             continue;
@@ -1660,7 +1686,7 @@ __global__ void __launch_bounds__(512) k_scan_generic(IndexDev D, int G, int Ps,
             scan_load_query(w, Ps, qq, s_pre, s_start);  // ends with a barrier
             cur = qq;
         }
-        const uint32_t e1 = min(total, e0 + w.chunk);
+        const uint32_t e1 = min(total, e0 + chunk);
         float* dst = w.dist + w.qoff[qq];
         const bool preq = pre || q_prefilter(w, qq);
         uint32_t kmin = 0xffffffffu, kmax = 0u, nf = 0;
@@ -1801,15 +1827,18 @@ __global__ void __launch_bounds__(kSelThreads) k_select(IndexDev D, int Ps, int 
             if (sel_bin(d, s_lv[l].lo, s_lv[l].inv) != s_lv[l].bin) return false;
         return true;
     };
-    // First bin of s_hist whose cumulative count reaches need: s_bin, s_below (count before
-    // it) and s_cntb (its count).  Warp 0 scans; the caller synchronises.
+    // First bin of s_hist whose cumulative count reaches need: s_bin (-1: none), s_below (count
+    // before it) and s_cntb (its count).  Warp 0 scans 128 bins per step (one 16-byte read per
+    // lane) and stops at the bin; the caller synchronises.  (32 bins per step took up to 4 us; a
+    // scan by the whole block costs its barriers at every level and reads every bin.)
     auto find_bin = [&](uint32_t need) {
         if (t < 32) {
-            uint32_t run = 0, below = 0;
-            int found = -1;
-            for (int base = 0; base < kBins && found < 0; base += 32) {
-                const uint32_t v = s_hist[base + t];
-                uint32_t x = v;
+            uint32_t run = 0;
+            bool found = false;
+            for (int base = 0; base < kBins && !found; base += 128) {
+                const uint4 v = reinterpret_cast<const uint4*>(s_hist + base)[t];
+                const uint32_t sum = v.x + v.y + v.z + v.w;
+                uint32_t x = sum;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
                     const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -1817,16 +1846,23 @@ __global__ void __launch_bounds__(kSelThreads) k_select(IndexDev D, int Ps, int 
                 }
                 const unsigned hit = __ballot_sync(0xffffffffu, run + x >= need);
                 if (hit) {
-                    const int l0 = __ffs(hit) - 1;
-                    found = base + l0;
-                    below = run + __shfl_sync(0xffffffffu, x - v, l0);
+                    found = true;
+                    if (t == __ffs(hit) - 1) {
+                        const uint32_t c[4] = {v.x, v.y, v.z, v.w};
+                        uint32_t below = run + x - sum;
+                        int i = 0;
+                        while (i < 3 && below + c[i] < need) below += c[i++];
+                        s_bin = base + 4 * t + i;
+                        s_below = below;
+                        s_cntb = c[i];
+                    }
                 }
                 run += __shfl_sync(0xffffffffu, x, 31);
             }
-            if (t == 0) {
-                s_bin = found;
-                s_below = below;
-                s_cntb = found >= 0 ? s_hist[found] : 0;
+            if (t == 0 && !found) {
+                s_bin = -1;
+                s_below = 0;
+                s_cntb = 0;
             }
         }
     };
@@ -2718,7 +2754,8 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     w.k_max = k;
     w.mode = mode;
     w.exps0 = (uint32_t)std::min<uint64_t>(exps0, 1u << 20);
-    w.chunk = P.scan_chunk ? (uint32_t)P.scan_chunk : kChunk;
+    w.chunk = (uint32_t)P.scan_chunk;
+    w.scan_items = 8 * (uint32_t)sm_count();
     w.cap = sync_sizing ? ~0ull : cx.dist_buf.bytes / 4;
     if (sync_sizing) w.sel_cap = ~0ull;  // sized after k_batch
     const FilterDev f = filter_dev(idx);
