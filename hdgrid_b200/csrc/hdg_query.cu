@@ -790,7 +790,7 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
     // (its ADC items follow from its survivors, k_scan_plan); any other query has ADC items
     // Candidates per scan item: SCAN_CHUNK, or the smallest power of two from kChunkMin to kChunk
     // that leaves at most scan_items items.  A small batch then fills the SMs (37 queries of
-    // 73,000 candidates ran as 111 items of up to 32,768: SCAN_FIG); a large one keeps long
+    // 73,000 candidates ran as 111 items of up to 32,768 in 325 us, in 125 us this way); a large one keeps long
     // items, since each loads its query's LUT.
     if (w.chunk) {
         if (t == 0) s_chunk = w.chunk;
@@ -1637,10 +1637,14 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
         __syncthreads();
     }
 }
-// Generic ADC (any M): natural subspace order, LUT [G][256][32] in shared memory.
+// Generic ADC (any M): natural subspace order.  The LUT sits in shared memory by subspace, entry c
+// of subspace m at m * 256 + (c ^ (m & 31)): the lanes of a warp read one subspace at a time, and
+// their codes spread over the banks (codeword-major rows put every lane on the subspace's one
+// bank); the XOR keeps the staging writes free of conflicts.  Each warp takes a contiguous span of
+// the item and walks the ranges.  2.7 M candidates x 25 subspaces: 125 -> 66 us.
 __global__ void __launch_bounds__(512) k_scan_generic(IndexDev D, int G, int Ps, int pre, int lbl, uint64_t q,
                                                       Workspace w) {
-    extern __shared__ __align__(16) float s_lut[];  // [G][256][32]
+    extern __shared__ __align__(16) float s_lut[];  // [32 G][256], swizzled
     uint32_t* s_pre = reinterpret_cast<uint32_t*>(s_lut + G * kCodes * 32);
     uint32_t* s_start = s_pre + Ps + 1;
     __shared__ ScanShared s;
@@ -1648,6 +1652,11 @@ __global__ void __launch_bounds__(512) k_scan_generic(IndexDev D, int G, int Ps,
     const int t = threadIdx.x, lane = t & 31;
     const uint32_t n_items = w.item_off[q], chunk = scan_chunk(w);
     const int M = D.M;
+    // shared-memory place of entry e of the global LUT ([G][256][32])
+    auto lut_at = [](int e) {
+        const int m = (e >> 13) * 32 + (e & 31), c = (e >> 5) & (kCodes - 1);
+        return m * kCodes + (c ^ (m & 31));
+    };
     int cur = -1;
     for (;;) {
         if (t == 0) {
@@ -1677,10 +1686,10 @@ __global__ void __launch_bounds__(512) k_scan_generic(IndexDev D, int G, int Ps,
             const uint64_t src0 = (uint64_t)qq * G * kCodes * 32;
             if (w.lut16) {
                 const __half* src = reinterpret_cast<const __half*>(w.lut) + src0;
-                for (int e = t; e < G * kCodes * 32; e += blockDim.x) s_lut[e] = __half2float(src[e]);
+                for (int e = t; e < G * kCodes * 32; e += blockDim.x) s_lut[lut_at(e)] = __half2float(src[e]);
             } else {
                 const float* src = w.lut + src0;
-                for (int e = t; e < G * kCodes * 32; e += blockDim.x) s_lut[e] = src[e];
+                for (int e = t; e < G * kCodes * 32; e += blockDim.x) s_lut[lut_at(e)] = src[e];
             }
             if (t < 2 * lbl) s_box[t] = w.box[(uint64_t)qq * 2 * lbl + t];
             scan_load_query(w, Ps, qq, s_pre, s_start);  // ends with a barrier
@@ -1690,14 +1699,20 @@ __global__ void __launch_bounds__(512) k_scan_generic(IndexDev D, int G, int Ps,
         float* dst = w.dist + w.qoff[qq];
         const bool preq = pre || q_prefilter(w, qq);
         uint32_t kmin = 0xffffffffu, kmax = 0u, nf = 0;
-        for (uint32_t e = e0 + t; e < e1; e += blockDim.x) {
-            int lo = 0, hi = Ps - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (s_pre[mid] <= e) lo = mid;
+        const uint32_t nw = blockDim.x >> 5, span = ((e1 - e0 + nw - 1) / nw + 31) / 32 * 32;
+        const uint32_t wb = e0 + (uint32_t)(t >> 5) * span, we = min(e1, wb + span);
+        int rg = 0;
+        {
+            int hi = Ps - 1;
+            while (rg < hi) {
+                const int mid = (rg + hi + 1) >> 1;
+                if (s_pre[mid] <= wb + lane) rg = mid;
                 else hi = mid - 1;
             }
-            const uint32_t pool = s_start[lo] + (e - s_pre[lo]);
+        }
+        for (uint32_t e = wb + lane; e < we; e += 32) {
+            while (s_pre[rg + 1] <= e) rg++;
+            const uint32_t pool = s_start[rg] + (e - s_pre[rg]);
             bool pass = true;
             if (preq) {
                 const float* lab = D.labels + (uint64_t)pool * lbl;
@@ -1713,11 +1728,17 @@ __global__ void __launch_bounds__(512) k_scan_generic(IndexDev D, int G, int Ps,
                 for (int j = 0; j * 16 < M; j++) {
                     const uint4 v = __ldg(cp + (uint64_t)j * D.n);
                     const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
-                    for (int b = 0; b < 16 && j * 16 + b < M; b++) {
+                    const int nb = M - 16 * j;
+                    float x[16];
+#pragma unroll
+                    for (int b = 0; b < 16; b++) {
                         const int m = j * 16 + b;
                         const uint32_t c = (wv[b >> 2] >> (8 * (b & 3))) & 0xffu;
-                        sum += s_lut[(m >> 5) * (kCodes * 32) + c * 32 + (m & 31)];
+                        x[b] = b < nb ? s_lut[m * kCodes + (int)(c ^ (uint32_t)(m & 31))] : 0.f;
                     }
+#pragma unroll
+                    for (int b = 0; b < 16; b++)
+                        if (b < nb) sum += x[b];
                 }
                 const uint32_t key = float_key(sum);
                 kmin = min(kmin, key);
@@ -1750,7 +1771,9 @@ __global__ void __launch_bounds__(512) k_scan_generic(IndexDev D, int G, int Ps,
 // than kBCap is split again over its own min/max (at most kMaxLevels levels); a bin whose
 // entries all share one distance is resolved by position order.
 constexpr int kMaxLevels = 4;
-constexpr int kSelThreads = 512;
+// 512 threads and four loads in flight each; fewer queries than SMs (one block each) take 1,024
+// threads and eight loads (37 queries of 73,000 candidates: 88 -> 51 us)
+constexpr int kSelThreads = 512, kSelThreadsFew = 1024;
 
 struct SelLevel {
     float lo, inv;
@@ -1773,7 +1796,8 @@ __device__ __forceinline__ uint32_t pos_to_pool(const uint32_t* s_pre, const uin
     return s_start[lo] + (e - s_pre[lo]);
 }
 
-__global__ void __launch_bounds__(kSelThreads) k_select(IndexDev D, int Ps, int Kcap, int sorted_out, Workspace w,
+template <int NT, int U>
+__global__ void __launch_bounds__(NT) k_select(IndexDev D, int Ps, int Kcap, int sorted_out, Workspace w,
                                                         float* __restrict__ out_dist,
                                                         uint64_t* __restrict__ out_ids, int k_out) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1893,15 +1917,15 @@ __global__ void __launch_bounds__(kSelThreads) k_select(IndexDev D, int Ps, int 
                 s_nb = 0;
             }
             __syncthreads();
-            for (uint32_t e0 = t; e0 < total; e0 += 4 * blockDim.x) {
-                float dv[4];
+            for (uint32_t e0 = t; e0 < total; e0 += U * blockDim.x) {
+                float dv[U];
 #pragma unroll
-                for (int u = 0; u < 4; u++) {  // four independent loads in flight per thread
+                for (int u = 0; u < U; u++) {  // U independent loads in flight per thread
                     const uint32_t e = e0 + u * blockDim.x;
                     dv[u] = e < total ? __ldg(dist + e) : INFINITY;
                 }
 #pragma unroll
-                for (int u = 0; u < 4; u++)
+                for (int u = 0; u < U; u++)
                     if (dv[u] < INFINITY && inside(dv[u], level)) atomicAdd(&s_hist[sel_bin(dv[u], lo, inv)], 1u);
             }
             __syncthreads();
@@ -1909,15 +1933,15 @@ __global__ void __launch_bounds__(kSelThreads) k_select(IndexDev D, int Ps, int 
             __syncthreads();
             const int b = s_bin;
             const bool fits = s_cntb <= (uint32_t)kBCap;
-            for (uint32_t e0 = 0; e0 < total; e0 += 4 * blockDim.x) {  // block-uniform bound
-                float dv[4];
+            for (uint32_t e0 = 0; e0 < total; e0 += U * blockDim.x) {  // block-uniform bound
+                float dv[U];
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
+                for (int u = 0; u < U; u++) {
                     const uint32_t e = e0 + t + u * blockDim.x;
                     dv[u] = e < total ? __ldg(dist + e) : INFINITY;
                 }
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
+                for (int u = 0; u < U; u++) {
                     const float d = dv[u];
                     const uint32_t e = e0 + t + u * blockDim.x;
                     const bool in = d < INFINITY && inside(d, level);
@@ -2918,8 +2942,12 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     const int sorted_out = mode == kPre ? 1 : 0;
     const size_t sm_sel = sizeof(uint32_t) * kBins + sizeof(uint64_t) * kBCap +
                           (sorted_out ? sizeof(uint64_t) * next_pow2(std::max<uint32_t>(k, 2)) : 0) + sm_tab + 16;
-    CK(cudaFuncSetAttribute(k_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_sel));
-    k_select<<<(unsigned)q, kSelThreads, sm_sel, st>>>(D, R, (int)k, sorted_out, w, c.dist, c.ids, (int)k);
+    auto launch_sel = [&](auto kern, int nt) {
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_sel));
+        kern<<<(unsigned)q, nt, sm_sel, st>>>(D, R, (int)k, sorted_out, w, c.dist, c.ids, (int)k);
+    };
+    if (q <= (uint64_t)sm_count()) launch_sel(k_select<kSelThreadsFew, 8>, kSelThreadsFew);
+    else launch_sel(k_select<kSelThreads, 4>, kSelThreads);
     CK_LAUNCH();
     launches++;
     tm.mark("select");
