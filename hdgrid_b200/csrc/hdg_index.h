@@ -143,11 +143,25 @@ struct QueryCtx {
     uint64_t work_queries = 0;
     std::map<std::string, std::pair<size_t, size_t>> layout;  // name -> (offset, bytes)
     GraphState* graphs = nullptr;   // QUERY_GRAPH=1: graphs keyed by pointers and sizes
+    uint64_t* pinned = nullptr;     // [16] the batch scalars and the GEMM status word, read back per call
+    // the last call's scalars, still on the device (a call that needed no host read)
+    struct Lazy {
+        bool pending = false;
+        cudaEvent_t done = nullptr;  // after the call's k_batch
+        const uint64_t* scal = nullptr;
+        uint64_t q = 0, exps0 = 0, launches = 0;
+        uint32_t k = 0;
+        int mode = 0;
+    } lazy;
     std::mutex mu;
     QueryCtx() = default;
     QueryCtx(const QueryCtx&) = delete;
     QueryCtx& operator=(const QueryCtx&) = delete;
-    ~QueryCtx() { release_graphs(graphs); }
+    ~QueryCtx() {
+        release_graphs(graphs);
+        if (pinned) cudaFreeHost(pinned);
+        if (lazy.done) cudaEventDestroy(lazy.done);
+    }
 };
 
 }  // namespace hdg
@@ -164,6 +178,7 @@ struct hdg_index {
     // query contexts by stream (the last one used serves hdg_debug_fetch)
     std::map<void*, std::unique_ptr<hdg::QueryCtx>> ctxs;
     hdg::QueryCtx* last_ctx = nullptr;
+    hdg::QueryCtx* lazy_ctx = nullptr;  // context whose last call's stats are still on the device (stats_mu)
     std::mutex ctx_mu;             // guards ctxs and last_ctx
     std::mutex stats_mu;           // guards the last-query stats and stage times
     int device = 0;

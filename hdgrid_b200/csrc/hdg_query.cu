@@ -226,6 +226,7 @@ __global__ void __launch_bounds__(kThreads) k_prologue(IndexDev D, GridMeta g, F
     const int t = threadIdx.x;
     const int l = g.l;
     const uint32_t L = D.n_lists;
+    if (qi == 0 && t == 0) *w.gemm_err = 0;
     if (t < 4) s_rank[t] = 0;
     if (t < l) {
         float lo, hi;
@@ -2471,7 +2472,7 @@ static Workspace carve(hdg_index* idx, QueryCtx& cx, uint64_t q, bool record) {
     w.S = (float*)take("gemm_s", q * (C + L) * 4);
     w.qnorm = (float*)take("qnorm", q * 4);
     w.qbf = take("qbf", q * idx->dev.d * 2);
-    w.gemm_err = (int*)take("gemm_err", 16);
+    w.gemm_err = reinterpret_cast<int*>(w.scal + 8);  // in the scalars' padding: one copy reads both
     w.feats = (float*)take("features", q * kMlpFeatures * 4);
     w.lq_ps = (uint32_t*)take("learned_nprobe", q * 4);
     w.lq_sched = (uint8_t*)take("learned_schedule", q);
@@ -2518,13 +2519,35 @@ static size_t workspace_bytes(hdg_index* idx, QueryCtx& cx, uint64_t q) {
     return need;
 }
 
+static void resolve_lazy(hdg_index* idx, QueryCtx& cx);
 static void reserve_ctx(hdg_index* idx, QueryCtx& cx, uint64_t q) {
     HDG_REQUIRE(idx->built, HDG_ERR_STATE, "index not built");
     const size_t need = workspace_bytes(idx, cx, q);
     if (cx.work.ptr && cx.work.bytes >= need) return;
+    resolve_lazy(idx, cx);
     cx.work.reset();
     cx.work.ensure(need);
     cx.work_queries = q;
+}
+
+// Batches of up to this many (query, point) pairs get candidate buffers for every pair (at
+// most 80 MiB each for distances, positions and selection), so the host need not read the candidate total
+// before it enqueues the scan: one query went
+// from 100 to 69 us without the wait.
+constexpr uint64_t kUnsizedPairs = 16ull << 20;
+
+// Candidate buffers of a batch whose totals are known to be at most coarse / selected entries
+static void ensure_candidates(QueryCtx& cx, uint64_t q, uint32_t k, uint64_t coarse, uint64_t selected) {
+    if (cx.dist_buf.bytes < std::max<uint64_t>(coarse, 1) * 4) {
+        invalidate_ctx_graphs(cx);  // their distance pointer dies with the old buffer
+        resize_rows(cx, std::max<uint64_t>(coarse, 1) * 4 * 5 / 4);
+    }
+    if (cx.sel_buf.bytes < std::max<uint64_t>(selected, 1) * 4) {
+        invalidate_ctx_graphs(cx);  // and their selection pointer with this one
+        cx.sel_buf.reset();
+        cx.sel_buf.ensure(std::max<uint64_t>(selected, 1) * 4 * 5 / 4);
+    }
+    ensure_part_buf(cx, q, k);
 }
 
 // The query context of a stream (created on first use); it becomes the last one used.
@@ -2540,6 +2563,9 @@ void reserve_workspace(hdg_index* idx, uint64_t q, cudaStream_t st) {
     QueryCtx& cx = query_ctx(idx, st);
     std::lock_guard<std::mutex> g(cx.mu);
     reserve_ctx(idx, cx, q);
+    // a small batch's candidate buffers too: its calls then allocate nothing
+    const uint64_t pairs = q * (uint64_t)idx->dev.n, k = idx->params.topk;
+    if (pairs <= kUnsizedPairs && k >= 1 && k <= 2048) ensure_candidates(cx, q, (uint32_t)k, pairs, pairs);
 }
 
 FilterDev filter_dev(const hdg_index* idx) {
@@ -2726,6 +2752,7 @@ static void fill_stats(hdg_index* idx, uint64_t q, uint32_t k, int mode, uint64_
     } else if (mode == kL1) {
         K = exps0 * k;
     }
+    idx->lazy_ctx = nullptr;  // these are the newest stats
     idx->last_ncand = K;  // no cap: the budget the reference computes is the one used
     idx->last_beta = beta;
     idx->last_q = q;
@@ -2733,6 +2760,21 @@ static void fill_stats(hdg_index* idx, uint64_t q, uint32_t k, int mode, uint64_
     std::memcpy(&bits, &beta, 4);
     const uint64_t s[10] = {q, idx->last_ncand, K, coarse, real, max_row, bits, (uint64_t)mode, launches, sc[5]};
     std::memcpy(idx->last_stats, s, sizeof(s));
+}
+
+// Reads back the scalars that the context's last call left on the device (cx.mu held) and, if
+// they are still the index's newest, makes them its stats.
+static void resolve_lazy(hdg_index* idx, QueryCtx& cx) {
+    if (!cx.lazy.pending) return;
+    cx.lazy.pending = false;
+    {
+        std::lock_guard<std::mutex> g(idx->stats_mu);
+        if (idx->lazy_ctx != &cx) return;
+    }
+    uint64_t sc[8];
+    CK(cudaEventSynchronize(cx.lazy.done));
+    CK(cudaMemcpy(sc, cx.lazy.scal, sizeof(sc), cudaMemcpyDeviceToHost));
+    fill_stats(idx, cx.lazy.q, cx.lazy.k, cx.lazy.mode, cx.lazy.exps0, sc, cx.lazy.launches);
 }
 
 // Enqueues one query batch on st.  sync_sizing: one host read after k_batch sizes the
@@ -2764,6 +2806,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     HDG_REQUIRE(mode == kPre || c.data, HDG_ERR_INVALID_ARG, "d_data is required for the re-rank");
     HDG_REQUIRE(mode != kPre || !c.qsched, HDG_ERR_INVALID_ARG,
                 "per-query schedules need exps0 > 1 (the pre-filter schedule has no re-rank)");
+    cx.lazy.pending = false;  // superseded by this call
     if (!cx.work.ptr || cx.work.bytes < workspace_bytes(idx, cx, q)) {
         HDG_REQUIRE(sync_sizing, HDG_ERR_STATE, "workspace too small for a captured query");
         reserve_ctx(idx, cx, q);
@@ -2803,7 +2846,6 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     // tensor-core estimates of every query-centroid dot product, used to prune the exact
     // ranking when n_list or sub_lists leaves part of the candidates out (COARSE_BF16=1)
     const bool use_gemm = P.coarse_bf16 != 0 && D.d % 8 == 0 && (Pc < (int)D.C || Ps < Pc * (int)D.S_max);
-    CK(cudaMemsetAsync(w.gemm_err, 0, sizeof(int), st));
     if (use_gemm) {
         rows_to_bf16(c.queries, q, (int)D.d, w.qbf, w.qnorm, st);
         umma_dot(w.qbf, q, D.centers_bf16, D.C, (int)D.d, w.S, w.ldS, w.gemm_err, st);
@@ -2835,25 +2877,31 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     CK_LAUNCH();
     launches++;
     uint64_t sc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    // no host read: a small batch whose caller needs no totals and whose coarse stage has no
+    // tensor-core status to report
+    bool lazy = sync_sizing && !use_gemm && !coarse_out && P.break_down == 0 && q * (uint64_t)D.n <= kUnsizedPairs;
+    if (lazy) {  // (a stream under capture is refused by the read below, as it always was)
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(st, &cap));
+        lazy = cap == cudaStreamCaptureStatusNone;
+    }
     if (sync_sizing) {
-        int gemm_err = 0;
-        CK(cudaMemcpyAsync(sc, w.scal, sizeof(sc), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&gemm_err, w.gemm_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        HDG_REQUIRE(gemm_err == 0, HDG_ERR_TIMEOUT, "tensor-core wait expired in the coarse GEMM");
-        const uint64_t coarse = sc[0], selected = sc[7];
+        uint64_t coarse = q * (uint64_t)D.n, selected = coarse;  // at most every point of every query
+        if (lazy) {
+            if (!cx.lazy.done) CK(cudaEventCreateWithFlags(&cx.lazy.done, cudaEventDisableTiming));
+            CK(cudaEventRecord(cx.lazy.done, st));
+        } else {
+            if (!cx.pinned) CK(cudaMallocHost(reinterpret_cast<void**>(&cx.pinned), 16 * sizeof(uint64_t)));
+            CK(cudaMemcpyAsync(cx.pinned, w.scal, 9 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            std::memcpy(sc, cx.pinned, sizeof(sc));
+            HDG_REQUIRE((uint32_t)cx.pinned[8] == 0, HDG_ERR_TIMEOUT, "tensor-core wait expired in the coarse GEMM");
+            coarse = sc[0];
+            selected = sc[7];
+        }
         if (coarse_out) *coarse_out = coarse;
         if (sel_out) *sel_out = selected;
-        if (cx.dist_buf.bytes < std::max<uint64_t>(coarse, 1) * 4) {
-            invalidate_ctx_graphs(cx);  // their distance pointer dies with the old buffer
-            resize_rows(cx, std::max<uint64_t>(coarse, 1) * 4 * 5 / 4);
-        }
-        if (cx.sel_buf.bytes < std::max<uint64_t>(selected, 1) * 4) {
-            invalidate_ctx_graphs(cx);  // and their selection pointer with this one
-            cx.sel_buf.reset();
-            cx.sel_buf.ensure(std::max<uint64_t>(selected, 1) * 4 * 5 / 4);
-        }
-        ensure_part_buf(cx, q, k);
+        ensure_candidates(cx, q, k, coarse, selected);
     } else {
         HDG_REQUIRE(cx.dist_buf.ptr && cx.sel_buf.ptr && cx.part_buf.bytes >= part_bytes(cx, q, k), HDG_ERR_STATE,
                     "no candidate buffers for a captured query");
@@ -2868,7 +2916,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     // candidate ranges per query: one per probed list, or n_split per list when is_split
     const int R = Ps * w.nsplit;
     const size_t sm_tab = sizeof(uint32_t) * (2 * R + 1);
-    if (!sync_sizing || sc[3] > 0) {
+    if (!sync_sizing || lazy || sc[3] > 0) {
         if (fast && (pre || w.qsched)) {
             // the predicate pass of the predicate-first queries, then the ADC items that
             // follow from their survivors
@@ -2967,11 +3015,22 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
         tm.mark("refine");
     }
     if (!sync_sizing && pinned) {
-        CK(cudaMemcpyAsync(pinned, w.scal, 8 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(pinned + 8, w.gemm_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(pinned, w.scal, 9 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     }
     if (launches_out) *launches_out = launches;
-    if (sync_sizing) fill_stats(idx, q, k, mode, exps0, sc, launches);
+    if (lazy) {
+        cx.lazy.pending = true;
+        cx.lazy.scal = w.scal;
+        cx.lazy.q = q;
+        cx.lazy.k = k;
+        cx.lazy.mode = mode;
+        cx.lazy.exps0 = exps0;
+        cx.lazy.launches = launches;
+        std::lock_guard<std::mutex> g(idx->stats_mu);
+        idx->lazy_ctx = &cx;
+    } else if (sync_sizing) {
+        fill_stats(idx, q, k, mode, exps0, sc, launches);
+    }
     tm.finish();
 }
 
@@ -2997,6 +3056,7 @@ hdg_status finish_async_query(hdg_index* idx) {
     for (QueryCtx* cx : all) {
         std::lock_guard<std::mutex> g(cx->mu);
         const hdg_status s = finish_ctx(idx, *cx);
+        resolve_lazy(idx, *cx);
         if (worst == HDG_OK) worst = s;
     }
     return worst;
@@ -3091,6 +3151,9 @@ void run_query(hdg_index* idx, const float* d_queries, uint64_t q, const float* 
     CK(cudaStreamWaitEvent(st, g->ev_out, 0));
     g->last = *hit;
     g->pending = true;
+    cx.lazy.pending = false;
+    std::lock_guard<std::mutex> gs(idx->stats_mu);
+    idx->lazy_ctx = nullptr;
 }
 
 void query_features(hdg_index* idx, const float* d_queries, uint64_t q, const float* d_query_labels,
@@ -3104,6 +3167,7 @@ void query_features(hdg_index* idx, const float* d_queries, uint64_t q, const fl
                 "query label columns must equal l * filter_dim");
     QueryCtx& cx = query_ctx(idx, st);
     std::lock_guard<std::mutex> lock(cx.mu);
+    resolve_lazy(idx, cx);  // this call lays the workspace out for its own q
     if (!cx.work.ptr || cx.work.bytes < workspace_bytes(idx, cx, q)) reserve_ctx(idx, cx, q);
     Workspace w = carve(idx, cx, q, true);
     const FilterDev f = filter_dev(idx);

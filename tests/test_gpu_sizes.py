@@ -126,3 +126,42 @@ def test_bruteforce_shapes(cuda, q, k, n, d, l):
         np.testing.assert_allclose(full[gi[i, :m]], gd[i, :m], rtol=tol)
         assert len(set(gi[i, :m].tolist())) == m
         assert np.all(np.isinf(gd[i, m:])) and np.all(gi[i, m:] == -1)
+
+
+# small batches are enqueued without a host read: their stats are read on demand, whatever ran since
+@pytest.mark.parametrize("q", [1, 5, 64])
+def test_small_batch_stats_on_demand(cuda, q):
+    import torch
+    import hdgrid_b200 as hg
+    from tests.helpers import build_gpu
+    ws = datasets.config1(scale=0.1, n_queries=64)
+    idx, base, _ = build_gpu(ws, cuda)
+    qs, ql = torch.from_numpy(ws["queries"]).to(cuda), torch.from_numpy(ws["query_labels"]).to(cuda)
+
+    def call(n, stream=None):
+        d = torch.empty((n, 20), device=cuda)
+        i = torch.empty((n, 20), dtype=torch.int64, device=cuda)
+        idx.query(hg.query_input_t(base, qs[:n].contiguous(), ql[:n].contiguous()), hg.query_output_t(d, i), stream=stream)
+        return d, i
+
+    idx.set_param("BREAK_DOWN", 1)  # timed calls read the scalars at once
+    d0, i0 = call(q)
+    want = idx.last_query_stats()
+    call(17)
+    other = idx.last_query_stats()
+    idx.set_param("BREAK_DOWN", 0)
+    d1, i1 = call(q)
+    assert idx.last_query_stats() == want
+    assert torch.equal(d0, d1) and torch.equal(i0, i1)
+    call(17)
+    idx.query_features(qs, ql, 20)  # reuses the workspace: the call's stats are kept
+    assert idx.last_query_stats() == other
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    call(17)
+    call(q, side)  # the newest call counts, on whichever stream
+    assert idx.last_query_stats() == want
+    call(17, side)
+    call(q)
+    assert idx.last_query_stats() == want
+    torch.cuda.synchronize()
