@@ -25,6 +25,7 @@
 #include <random>
 
 #include "hdg_device.cuh"
+#include "hdg_est.cuh"
 #include "hdg_internal.h"
 
 namespace hdg {
@@ -338,6 +339,31 @@ __global__ void k_gather_codes_labels(const uint8_t* __restrict__ codes_by_id, i
     uint4* dst = reinterpret_cast<uint4*>(codes + r * M_pad);
     for (int v = 0; v < M_pad / 16; v++) dst[v] = src[v];
     for (int i = 0; i < l; i++) labels[r * l + i] = labels_by_id[id * l + i];
+}
+
+// A point's PQ approximation (the codewords its codes name) in BF16, and its constants for the
+// distance estimates; one warp per pool row, lane = subspace (mod 32).
+__global__ void k_decode_rows(IndexDev D, uint16_t* __restrict__ out, float4* __restrict__ cst) {
+    const uint64_t r = (uint64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    const int lane = threadIdx.x & 31;
+    if (r >= D.n) return;
+    const int L = D.pq_len;
+    float s = 0.f, e = 0.f;
+    for (int m = lane; m < (int)D.M; m += 32) {
+        const uint32_t c = D.codes[((uint64_t)(m >> 4) * D.n + r) * 16 + (m & 15)];
+        const float* x = D.pq_centers + ((uint64_t)m * kCodes + c) * L;
+        for (int t = 0; t < L; t++) {
+            const float v = __ldg(x + t);
+            const __nv_bfloat16 h = __float2bfloat16_rn(v);
+            const float df = v - __bfloat162float(h);
+            s = fmaf(v, v, s);
+            e = fmaf(df, df, e);
+            out[r * D.d + m * L + t] = __bfloat16_as_ushort(h);
+        }
+    }
+    s = warp_sum(s);
+    e = warp_sum(e);
+    if (lane == 0) cst[r] = make_float4(s * (1.f - kEstSlack), sqrtf(s) * (1.f + kEstSlack), sqrtf(e) * (1.f + kEstSlack), 0.f);
 }
 
 __global__ void k_to_bf16(const float* __restrict__ x, uint64_t n, __nv_bfloat16* __restrict__ y) {
@@ -811,6 +837,9 @@ void label_rank_thresholds(const float* labels, uint64_t n, int l, int bits, flo
     }
 }
 
+constexpr uint64_t kDecodedMax = 16ull << 30;
+constexpr uint64_t kDecodedMinPoints = 16384;  // smaller sets never reach the estimate pass
+
 // Copy the host index into one device arena and fill idx->dev.
 void upload_index(hdg_index* idx, cudaStream_t st) {
     HostIndex& H = idx->host;
@@ -943,6 +972,22 @@ void upload_index(hdg_index* idx, cudaStream_t st) {
     D.S_max = 0;
     for (uint64_t c = 0; c < H.C; c++)
         D.S_max = std::max<uint32_t>(D.S_max, H.cluster_off[c + 1] - H.cluster_off[c]);
+    // the estimate pass of the post-filter scan reads the points' PQ approximations as tensor-core
+    // operands (2 d + 16 bytes per point; not kept past kDecodedMax, where the full scan runs)
+    D.decoded = nullptr;
+    D.decoded_c = nullptr;
+    idx->decoded.reset();
+    const uint64_t dec = align_up((uint64_t)H.n * H.d * 2, 256);
+    if (H.d % 8 == 0 && H.M % 32 == 0 && H.M <= 96 && H.M * H.pq_len == H.d && H.n >= kDecodedMinPoints &&
+        dec <= kDecodedMax) {
+        idx->decoded.ensure(dec + (uint64_t)H.n * sizeof(float4));
+        char* p = static_cast<char*>(idx->decoded.ptr);
+        k_decode_rows<<<blocks_for(H.n, 8), 256, 0, st>>>(D, reinterpret_cast<uint16_t*>(p),
+                                                         reinterpret_cast<float4*>(p + dec));
+        CK_LAUNCH();
+        D.decoded = reinterpret_cast<const uint16_t*>(p);
+        D.decoded_c = reinterpret_cast<const float4*>(p + dec);
+    }
     idx->grid = gp;
     CK(cudaStreamSynchronize(st));
     CK_LAUNCH();

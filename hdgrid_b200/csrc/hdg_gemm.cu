@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include "hdg_internal.h"
+#include "hdg_umma.cuh"
 
 namespace hdg {
 
@@ -28,11 +29,6 @@ constexpr int kGemmThreads = 128;
 constexpr uint32_t kStage = 16 * 1024;         // one 128 x 64 bf16 chunk in the canonical layout
 constexpr uint32_t kLBO = (GM / 8) * 128;      // bytes between the two 8-element K chunks
 constexpr uint32_t kSBO = 128;                 // bytes between 8-row groups
-constexpr long long kSpinLimit = 1ll << 26;
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
 
 // K-major, no-swizzle UMMA shared-memory descriptor (layout of cute::UMMA::SmemDescriptor:
 // start>>4 [0,14), LBO>>4 [16,30), SBO>>4 [32,46), version 1 [46,48), layout 0 [61,64)).
@@ -53,21 +49,6 @@ constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GN 
 __device__ __forceinline__ uint32_t canon_off(int row, int k) {
     return (uint32_t)(k >> 3) * kLBO + (uint32_t)(row >> 3) * kSBO + (uint32_t)(row & 7) * 16u +
            (uint32_t)(k & 7) * 2u;
-}
-
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase) {
-    for (long long it = 0; it < kSpinLimit; it++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred P1;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, P1;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(phase)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
 }
 
 // out[r][n] = sum_k A[r][k] * B[n][k]; A [rows x d] bf16, B [cols x d] bf16, out row stride ldo.
@@ -198,23 +179,6 @@ __global__ void __launch_bounds__(kGemmThreads) k_umma_dot(const __nv_bfloat16* 
 // BN = 64 or 128 output columns per CTA (64 when 128-wide tiles would leave SMs idle).
 constexpr int kTStages = 4;
 constexpr uint32_t kTileA = GM * GK * 2;  // 16 KB per stage
-
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3fff);
-    d |= (uint64_t)1 << 16;                   // leading byte offset (unused by K-major SW128)
-    d |= (uint64_t)(1024 >> 4) << 32;         // stride byte offset: 8 rows x 128 bytes
-    d |= (uint64_t)1 << 46;                   // descriptor version (sm100)
-    d |= (uint64_t)2 << 61;                   // SWIZZLE_128B
-    return d;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
 
 template <int BN>
 __global__ void __launch_bounds__(kGemmThreads) k_umma_tma(const __grid_constant__ CUtensorMap mapA, uint64_t rows,
@@ -391,7 +355,7 @@ static EncodeTiledFn encode_tiled() {
 
 // Tensor map of a row-major bf16 [n x d] matrix read in boxes of 64 (K) x box_rows, 128-byte
 // swizzle, zero fill past the edges.
-static CUtensorMap bf16_rows_map(const void* base, uint64_t n, int d, uint32_t box_rows) {
+CUtensorMap bf16_rows_map(const void* base, uint64_t n, int d, uint32_t box_rows) {
     HDG_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0 && d % 8 == 0, HDG_ERR_UNSUPPORTED,
                 "TMA operands need 16-byte aligned rows");
     CUtensorMap m;

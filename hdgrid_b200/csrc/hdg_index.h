@@ -104,6 +104,8 @@ struct IndexDev {
     const float* pq_centers;
     const uint32_t* prefix;        // dense prefix counts (nullptr when the rows form or prefix16 is used)
     const uint16_t* prefix16;      // the dense counts in 16 bits, kept when no list exceeds 65535 points
+    const uint16_t* decoded;       // [n x d] the points' PQ approximations in BF16, pool order (nullptr: not kept)
+    const float4* decoded_c;       // [n] their constants for the distance estimates (hdg_est.cuh)
     const uint64_t* prefix_off;    // compressed rows (nullptr when dense)
     const uint64_t* prefix_rows;
 };
@@ -140,6 +142,7 @@ struct QueryCtx {
     DeviceBuffer pos_buf;           // u32 candidate positions of compact rows (same capacity)
     DeviceBuffer sel_buf;           // u32 selected candidates: min(n_cand, candidates) per query
     DeviceBuffer part_buf;          // u64 best keys of the refine work items
+    DeviceBuffer est_buf;           // thresholds and row-tile entries of the estimate pass
     uint64_t work_queries = 0;
     std::map<std::string, std::pair<size_t, size_t>> layout;  // name -> (offset, bytes)
     GraphState* graphs = nullptr;   // QUERY_GRAPH=1: graphs keyed by pointers and sizes
@@ -174,6 +177,8 @@ struct hdg_index {
     hdg::GridMeta grid;
     hdg::IndexDev dev{};
     hdg::DeviceBuffer arena;       // all index arrays
+    hdg::DeviceBuffer decoded;     // derived at upload, not stored in the index file: the points'
+                                   // PQ approximations in BF16 and their estimate constants
     hdg::DeviceBuffer map_buf;     // filter interval map
     // query contexts by stream (the last one used serves hdg_debug_fetch)
     std::map<void*, std::unique_ptr<hdg::QueryCtx>> ctxs;

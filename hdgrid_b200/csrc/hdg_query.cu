@@ -23,14 +23,17 @@
 //                exact f32 re-rank and top-k (refine.cu:36-120).
 // There is no dense [q x max_row_len] candidate table and one host round trip per batch
 // (the candidate total and the batch-wide budget).
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <type_traits>
 
 #include "hdg_device.cuh"
+#include "hdg_est.cuh"
 #include "hdg_internal.h"
 
 namespace hdg {
@@ -56,8 +59,10 @@ struct Workspace {
     uint32_t* range_len;     // [q x Ps]
     uint32_t* range_pre;     // [q x (Ps + 1)] exclusive prefix of range_len (last: the candidate total)
     uint32_t* qstat;         // [q x 4]: cand_total, exact_total, n_lists, n_clusters
+    uint32_t* qtiles;        // [q] row tiles (kEstM pool rows) that the query's candidate ranges touch
     uint64_t* scal;          // [8]: cand sum, exact sum, max cand, items, beta (f32 bits),
-                             //      queries dropped by a capacity, kept candidates, selected sum
+                             //      queries dropped by a capacity, kept candidates, selected sum;
+                             //      then (in its padding) the GEMM status word and the row-tile sum
     uint64_t* qoff;          // [q + 1] candidate offsets into dist
     uint32_t* item_off;      // [q + 1] work-item offsets of the ADC scan
     uint32_t* pitem_off;     // [q + 1] work-item offsets of the predicate pass (predicate-first queries)
@@ -81,6 +86,13 @@ struct Workspace {
     int surv_list;           // 1: the predicate pass lists each predicate-first query's survivors
     float* dist;             // [sum of candidates]
     uint32_t* spos;          // [sum of candidates] candidate position of each entry of a compact row
+    // the estimate pass of post-filter queries (nullptr: not run)
+    uint32_t* prq;           // [q] 0: every candidate scanned; 1: only the candidates its estimate keeps; 2: scanned
+                             //     in full after all (the threshold turned out too low)
+    float* thr;              // [q] ADC threshold: every candidate at or below it is kept
+    uint32_t* nle;           // [q] kept candidates whose ADC distance is at or below the threshold
+    float4* est_qc;          // [q] constants of the estimate test
+    int round;               // 2: the scan and select of the prq == 2 queries
     float* S;                // [q x (C + L)] tensor-core dot products (nullptr: exact path only)
     uint64_t ldS;
     float* qnorm;            // [q] squared query norms
@@ -116,6 +128,9 @@ __device__ __forceinline__ bool q_prefilter(const Workspace& w, uint64_t qi) {
 // true when query qi's row is compact: the predicate pass lists its survivors (position and
 // pool row), the ADC scan replaces each pool row by the survivor's distance
 __device__ __forceinline__ bool compacts(const Workspace& w, uint64_t qi) { return w.surv_list && q_prefilter(w, qi); }
+// true when query qi's row holds only the candidates that the estimate pass kept (positions and
+// pool rows, as a compacting query's survivors)
+__device__ __forceinline__ bool pruned(const Workspace& w, uint64_t qi) { return w.prq && w.prq[qi] == 1; }
 // Candidate budget n_cand of query qi given the batch's beta and max_row_len: the query's k for
 // the reference pre-filter schedule (exps0 <= 1), exps0 * k for the single-dim schedule and the
 // predicate-first schedule, and the reference's min(exps0 * k * beta, max_row_len) for the
@@ -535,7 +550,7 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(IndexDev D, GridMeta 
     float* s_lo = reinterpret_cast<float*>(s_keys + max(sort_n1, sort_n2));
     float* s_q = s_lo + max(sort_n1, sort_n2);
     __shared__ uint32_t s_chosen[1024];
-    __shared__ uint32_t s_red[2];
+    __shared__ uint32_t s_red[3];
     __shared__ uint32_t s_wc[32];
     __shared__ unsigned long long s_scan[32];
     __shared__ uint32_t s_hist[256];
@@ -549,7 +564,7 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(IndexDev D, GridMeta 
     for (int i = t; i < d; i += blockDim.x) s_q[i] = queries[qi * d + i];
     if (t == 0) {
         s_nvalid = 0;
-        s_red[0] = s_red[1] = 0;
+        s_red[0] = s_red[1] = s_red[2] = 0;
     }
     __syncthreads();
     // One pass over the clusters: those with a non-zero filtered count (filter_none_zero_data
@@ -688,7 +703,10 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(IndexDev D, GridMeta 
         }
     }
     const uint64_t zlo = w.zrange[qi * 2], zhi = w.zrange[qi * 2 + 1];
-    uint32_t my_cand = 0, my_exact = 0;
+    uint32_t my_cand = 0, my_exact = 0, my_tiles = 0;
+    auto tiles_of = [](uint32_t start, uint32_t len) {
+        return len ? (start + len - 1) / (uint32_t)kEstM - start / (uint32_t)kEstM + 1u : 0u;
+    };
     const int ns = w.nsplit;
     int box[2 * kMaxDims];
     if (w.is_split)
@@ -732,6 +750,7 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(IndexDev D, GridMeta 
                 w.range_start[r0] = start;
                 w.range_len[r0] = len;
                 my_cand += len;
+                my_tiles += tiles_of(start, len);
             } else {
                 for (int sp = 0; sp < ns; sp++) {
                     uint32_t st = kInvalid, ln = 0;
@@ -739,12 +758,19 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(IndexDev D, GridMeta 
                     w.range_start[r0 + sp] = st;
                     w.range_len[r0 + sp] = ln;
                     my_cand += ln;
+                    my_tiles += tiles_of(st, ln);
                 }
             }
         }
     }
-    atomicAdd(&s_red[0], my_cand);
-    atomicAdd(&s_red[1], my_exact);
+    my_cand = __reduce_add_sync(0xffffffffu, my_cand);
+    my_exact = __reduce_add_sync(0xffffffffu, my_exact);
+    my_tiles = __reduce_add_sync(0xffffffffu, my_tiles);
+    if ((t & 31) == 0) {
+        atomicAdd(&s_red[0], my_cand);
+        atomicAdd(&s_red[1], my_exact);
+        atomicAdd(&s_red[2], my_tiles);
+    }
     __syncthreads();
     // the exclusive prefix of the ranges' lengths (its last entry the candidate total): the
     // predicate pass, the scan and the select find a position's range by searching it
@@ -770,6 +796,7 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(IndexDev D, GridMeta 
         w.qstat[qi * 4 + 1] = s_red[1];
         w.qstat[qi * 4 + 2] = nps;
         w.qstat[qi * 4 + 3] = npc;
+        w.qtiles[qi] = s_red[2];
     }
 }
 
@@ -779,11 +806,11 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(IndexDev D, GridMeta 
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
     __shared__ unsigned long long s_tot[32], s_items[32], s_pitems[32], s_sel[32];
-    __shared__ unsigned long long s_red[3], s_drop[2];
+    __shared__ unsigned long long s_red[4], s_drop[2];
     __shared__ float s_beta;
     __shared__ uint32_t s_chunk;
     const int t = threadIdx.x;
-    if (t == 0) s_red[0] = s_red[1] = s_red[2] = s_drop[0] = s_drop[1] = 0;
+    if (t == 0) s_red[0] = s_red[1] = s_red[2] = s_red[3] = s_drop[0] = s_drop[1] = 0;
     __syncthreads();
     const uint64_t per = (q + blockDim.x - 1) / blockDim.x;
     const uint64_t b = t * per, e = min(q, b + per);
@@ -810,8 +837,9 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
     const uint32_t chunk = s_chunk;
     auto n_items = [&](uint64_t i, uint32_t c) { return compacts(w, i) ? 0u : (c + chunk - 1) / chunk; };
     auto n_pitems = [&](uint64_t i, uint32_t c) { return compacts(w, i) ? (c + kPreChunk - 1) / kPreChunk : 0u; };
-    unsigned long long cand = 0, items = 0, pitems = 0, exact = 0, mx = 0;
+    unsigned long long cand = 0, items = 0, pitems = 0, exact = 0, mx = 0, rtiles = 0;
     for (uint64_t i = b; i < e; i++) {
+        rtiles += w.qtiles[i];
         const uint32_t c = w.qstat[i * 4];
         cand += c;
         items += n_items(i, c);
@@ -858,7 +886,9 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
     cand = warp_sum_u64(cand);
     exact = warp_sum_u64(exact);
     mx = warp_max_u64(mx);
+    rtiles = warp_sum_u64(rtiles);
     if ((t & 31) == 0) {
+        atomicAdd(&s_red[3], rtiles);
         atomicAdd(&s_red[0], cand);
         atomicAdd(&s_red[1], exact);
         atomicMax(&s_red[2], mx);
@@ -869,6 +899,7 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
         w.scal[1] = s_red[1];
         w.scal[2] = s_red[2];
         w.scal[3] = tot_i + tot_p;
+        w.scal[9] = s_red[3];
         // beta = coarse / real as the reference computes it (Super-Grid-IVF_PQ.cu:1219)
         const float beta = s_red[1] == 0 ? INFINITY : __fdiv_rn((float)s_red[0], (float)s_red[1]);
         w.scal[4] = __float_as_uint(beta);
@@ -1438,7 +1469,8 @@ __global__ void __launch_bounds__(1024) k_scan_plan(uint64_t q, Workspace w) {
     const uint64_t b = t * per, e = min(q, b + per);
     const uint32_t chunk = scan_chunk(w);
     auto n_items = [&](uint64_t i) {
-        uint32_t c = compacts(w, i) ? w.cand_count[i] : w.qstat[i * 4];
+        if (w.round == 2) return w.prq[i] == 2 ? (w.qstat[i * 4] + chunk - 1) / chunk : 0u;
+        uint32_t c = compacts(w, i) || pruned(w, i) ? w.cand_count[i] : w.qstat[i * 4];
         // a compact row that its budget takes whole needs no ADC distance (the select takes
         // every survivor and the re-rank orders them), unless the distances are the output
         // (the reference's pre-filter schedule)
@@ -1447,7 +1479,7 @@ __global__ void __launch_bounds__(1024) k_scan_plan(uint64_t q, Workspace w) {
     };
     // such a row's survivors all count as passed (the ADC scan counts them for the others)
     for (uint64_t i = b; i < e; i++)
-        if (compacts(w, i) && w.mode != kPre && w.cand_count[i] <= w.qbud[i]) w.nfin[i] = w.cand_count[i];
+        if (w.round != 2 && compacts(w, i) && w.mode != kPre && w.cand_count[i] <= w.qbud[i]) w.nfin[i] = w.cand_count[i];
     unsigned long long items = 0;
     for (uint64_t i = b; i < e; i++) items += n_items(i);
     unsigned long long tot = 0;
@@ -1494,7 +1526,8 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
         const int item = s.item;
         if (item >= (int)n_items) break;
         const int qq = s.query;
-        const bool compact = compacts(w, qq);
+        const bool prn = pruned(w, qq), compact = compacts(w, qq) || prn;
+        const float thr = prn ? w.thr[qq] : 0.f;
         const uint32_t total = compact ? w.cand_count[qq] : w.qstat[(uint64_t)qq * 4];
         const uint32_t e0 = (uint32_t)(item - w.item_off[qq]) * chunk;
         if (e0 >= total) {  // a query cut by the distance capacity
@@ -1536,7 +1569,7 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
         float* dst = w.dist + w.qoff[qq];
         const uint32_t* srow = reinterpret_cast<const uint32_t*>(dst);  // compact: the survivors' pool rows
         const uint32_t* sp = w.spos + w.qoff[qq];
-        uint32_t kmin = 0xffffffffu, kmax = 0u, nf = 0;
+        uint32_t kmin = 0xffffffffu, kmax = 0u, nf = 0, nl = 0;
         // each warp takes a contiguous span of the item (a multiple of 32 * CPT entries, so in
         // a full row position mod 32 stays the lane), so a lane's walk to its candidate's range
         // crosses few range boundaries per step
@@ -1620,6 +1653,7 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
                     kmin = min(kmin, key);
                     kmax = max(kmax, key);
                     nf++;
+                    nl += sum[u] <= thr ? 1u : 0u;
                 }
                 dst[e] = sum[u];
             }
@@ -1634,6 +1668,10 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
             atomicMin(&w.mm[2 * qq], kmin);
             atomicMax(&w.mm[2 * qq + 1], kmax);
             atomicAdd(&w.nfin[qq], nf);
+        }
+        if (prn) {
+            nl = __reduce_add_sync(0xffffffffu, nl);
+            if (lane == 0 && nl) atomicAdd(&w.nle[qq], nl);
         }
         __syncthreads();
     }
@@ -1819,7 +1857,21 @@ __global__ void __launch_bounds__(NT) k_select(IndexDev D, int Ps, int Kcap, int
     // A predicate-first query of the predicate pass has a compact row: its survivors' distances
     // in arrival order with their candidate positions beside them (cand_count entries); any
     // other query's row holds one distance per candidate position.
-    const bool compact = compacts(w, qi);
+    // A query of the estimate pass has a compact row too: the candidates its estimates kept.  They
+    // hold its K smallest if K of them lie at or below the threshold; else (or when the pass
+    // reports an expired wait) the query is marked, scanned in full and selected in round 2.
+    if (w.round == 2 && w.prq[qi] != 2) return;
+    const bool prn = pruned(w, qi), compact = compacts(w, qi) || prn;
+    if (prn && ((uint32_t)K > w.nle[qi] || *w.gemm_err != 0)) {
+        __syncthreads();  // every thread has read prq
+        if (t == 0) {
+            w.prq[qi] = 2;
+            w.nfin[qi] = 0;
+            w.mm[2 * qi] = 0xffffffffu;
+            w.mm[2 * qi + 1] = 0u;
+        }
+        return;
+    }
     if (!sorted_out && takes_row(w, qi)) return;  // the selection is the row (cand_count entries)
     const uint32_t total = compact ? w.cand_count[qi] : w.qstat[qi * 4];
     const float* dist = w.dist + w.qoff[qi];
@@ -2417,6 +2469,267 @@ __global__ void __launch_bounds__(kThreads, 5) k_refine(IndexDev D, const float*
 }
 
 // ------------------------------------------------------------------------------------
+// The estimate pass: which candidates of a post-filter query can be among its n_cand smallest
+// ------------------------------------------------------------------------------------
+// The post-filter schedule needs the n_cand smallest ADC distances of a query's candidates, a few
+// percent of them.  An ADC distance is the distance to the candidate's PQ approximation, so a
+// tensor-core product of queries and approximations bounds it from below (hdg_est.cuh):
+//   k_est_thr    a threshold per query from a strided sample of its candidates' ADC distances: a
+//                sample rank past n_cand's share by four standard deviations;
+//   k_est_count / k_est_scan / k_est_fill   the (query, range) entries of every tile of kEstM pool
+//                rows, so that a tile meets only the queries whose ranges touch it;
+//   k_est        every candidate whose bound is not above the threshold goes to its query's row;
+//   k_scan_fast  the exact ADC of those (the compact-row path);
+//   k_select     if n_cand of them lie at or below the threshold, the n_cand smallest are among
+//                them: the selection is the full scan's.  A query whose threshold was too low is
+//                scanned in full (round 2).
+// 10,000 queries x 227,000 candidates x 32 subspaces (n_cand 9,384): EST_FIG.
+constexpr int kThrThreads = 512;
+constexpr uint32_t kThrMax = 4096;  // sampled candidates at most
+constexpr int kThrBins = 2048;
+
+template <int G>
+__global__ void __launch_bounds__(kThrThreads) k_est_thr(IndexDev D, int R, const float* __restrict__ queries, Workspace w) {
+    extern __shared__ __align__(16) float s_lut[];  // [G][256][32]
+    float* s_d = s_lut + G * kCodes * 32;                                // [kThrMax]
+    uint32_t* s_hist = reinterpret_cast<uint32_t*>(s_d + kThrMax);      // [kThrBins]
+    uint32_t* s_pre = s_hist + kThrBins;                                  // [R + 1]
+    uint32_t* s_start = s_pre + R + 1;                                    // [R]
+    __shared__ unsigned long long s_scan[32];
+    __shared__ float s_red[3];
+    __shared__ uint32_t s_mm[2];
+    __shared__ int s_bin;
+    const uint64_t qi = blockIdx.x;
+    const int t = threadIdx.x, lane = t & 31;
+    const uint32_t N = w.qstat[qi * 4];
+    const uint32_t K = w.qbud[qi];
+    // sample size: the cost of a sampled candidate against the extra candidates that a coarser
+    // threshold lets through, about 2.5 (5 sqrt(K N))^(2/3) of either
+    uint32_t ms = 0, rank = 0;
+    if (N >= 4096 && (uint64_t)K * 3 <= N) {
+        ms = (uint32_t)powf(5.f * sqrtf((float)K * (float)N), 2.f / 3.f);
+        ms = min(kThrMax, max(512u, ms));
+        const float r = (float)K * (float)ms / (float)N;
+        rank = (uint32_t)(r + 4.f * sqrtf(r) + 4.f);
+    }
+    if (t == 0) {
+        w.prq[qi] = 0;
+        w.nle[qi] = 0;
+    }
+    if (ms == 0 || rank >= ms) return;  // block-uniform
+    if (t == 0) {
+        s_mm[0] = 0xffffffffu;
+        s_mm[1] = 0u;
+        s_red[0] = s_red[1] = s_red[2] = 0.f;
+        s_bin = -1;
+    }
+    if (w.lut16) {
+        const uint2* src = reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(w.lut) + qi * G * kCodes * 32);
+        for (int e = t; e < G * kCodes * 8; e += kThrThreads) {
+            const uint2 v = __ldg(src + e);
+            const float2 a = __half22float2(reinterpret_cast<const __half2&>(v.x)),
+                         b = __half22float2(reinterpret_cast<const __half2&>(v.y));
+            reinterpret_cast<float4*>(s_lut)[e] = make_float4(a.x, a.y, b.x, b.y);
+        }
+    } else {
+        const float4* src = reinterpret_cast<const float4*>(w.lut + qi * G * kCodes * 32);
+        for (int e = t; e < G * kCodes * 8; e += kThrThreads) reinterpret_cast<float4*>(s_lut)[e] = __ldg(src + e);
+    }
+    for (int i = t; i < kThrBins; i += kThrThreads) s_hist[i] = 0;
+    const uint32_t* pre = w.range_pre + qi * (R + 1);
+    for (int i = t; i <= R; i += kThrThreads) s_pre[i] = pre[i];
+    for (int i = t; i < R; i += kThrThreads) s_start[i] = w.range_start[qi * R + i];
+    __syncthreads();
+    // the query's norms (for the estimate's constants)
+    {
+        float qn = 0.f, q2 = 0.f, rq = 0.f;
+        for (int i = t; i < (int)D.d; i += kThrThreads) {
+            const float v = queries[qi * D.d + i], h = __bfloat162float(__float2bfloat16_rn(v)), e = v - h;
+            qn = fmaf(v, v, qn);
+            q2 = fmaf(h, h, q2);
+            rq = fmaf(e, e, rq);
+        }
+        qn = warp_sum(qn);
+        q2 = warp_sum(q2);
+        rq = warp_sum(rq);
+        if (lane == 0 && t < (int)((D.d + 31) / 32 * 32)) {
+            atomicAdd(&s_red[0], qn);
+            atomicAdd(&s_red[1], q2);
+            atomicAdd(&s_red[2], rq);
+        }
+    }
+    const uint4* planes = reinterpret_cast<const uint4*>(D.codes);
+    uint32_t kmin = 0xffffffffu, kmax = 0u;
+    for (uint32_t i = t; i < ms; i += kThrThreads) {
+        const uint32_t e = (uint32_t)(((uint64_t)i * N + N / 2) / ms);
+        int lo = 0, hi = R - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (s_pre[mid] <= e) lo = mid;
+            else hi = mid - 1;
+        }
+        const uint4* cp = planes + s_start[lo] + (e - s_pre[lo]);
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            // lane r goes round from subspace r: the lanes of a warp read different banks
+            const uint4 a = __ldg(cp + (uint64_t)(2 * g) * D.n), b = __ldg(cp + (uint64_t)(2 * g + 1) * D.n);
+            uint32_t wv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            rotate_words(wv, (uint32_t)lane >> 2);
+            const uint32_t sh = 8u * (lane & 3);
+            const char* L = reinterpret_cast<const char*>(s_lut + g * kCodes * 32);
+#pragma unroll
+            for (int st = 0; st < 32; st += 2) {
+                const uint32_t x = __funnelshift_r(wv[st >> 2], wv[((st >> 2) + 1) & 7], sh);
+                const uint32_t c0 = (x >> (8 * (st & 3))) & 255u, c1 = (x >> (8 * ((st + 1) & 3))) & 255u;
+                s0 += *reinterpret_cast<const float*>(L + (c0 << 7) + ((4 * lane + 4 * st) & 127));
+                s1 += *reinterpret_cast<const float*>(L + (c1 << 7) + ((4 * lane + 4 * st + 4) & 127));
+            }
+        }
+        const float d = s0 + s1;
+        s_d[i] = d;
+        const uint32_t key = float_key(d);
+        if (d < INFINITY) {
+            kmin = min(kmin, key);
+            kmax = max(kmax, key);
+        }
+    }
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    if (lane == 0) {
+        atomicMin(&s_mm[0], kmin);
+        atomicMax(&s_mm[1], kmax);
+    }
+    __syncthreads();
+    if (s_mm[0] > s_mm[1]) return;  // no finite distance
+    // the threshold: the upper edge of the bin that holds the sample's rank-th distance
+    const float lo = key_float(s_mm[0]), hi = key_float(s_mm[1]);
+    const float inv = hi > lo ? (float)kThrBins / (hi - lo) : 0.f;
+    for (uint32_t i = t; i < ms; i += kThrThreads) {
+        const float d = s_d[i];
+        if (d < INFINITY) atomicAdd(&s_hist[min(kThrBins - 1, max(0, (int)((d - lo) * inv)))], 1u);
+    }
+    __syncthreads();
+    constexpr int kPer = kThrBins / kThrThreads;
+    uint32_t c[kPer], sum = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+        c[i] = s_hist[t * kPer + i];
+        sum += c[i];
+    }
+    unsigned long long tot = 0;
+    uint32_t run = (uint32_t)block_inclusive_sum(sum, s_scan, &tot) - sum;
+    if (run < rank && rank <= run + sum) {
+        int i = 0;
+        while (i < kPer - 1 && run + c[i] < rank) run += c[i++];
+        s_bin = t * kPer + i;
+    }
+    __syncthreads();
+    if (t == 0 && s_bin >= 0) {
+        const float T = s_bin == kThrBins - 1 || !(inv > 0.f) ? hi : lo + (float)(s_bin + 1) / inv;
+        const float qn = s_red[0], qh = sqrtf(s_red[1]) * (1.f + kEstSlack), rq = sqrtf(s_red[2]) * (1.f + kEstSlack);
+        // the bound holds for the distance itself: an ADC distance at or below T may be off by its
+        // own rounding -- FP32 sums, and with FP16 tables each entry by 2^-11 (or 2^-25)
+        const float Tb = w.lut16 ? T * (1.f + 1.1e-3f) + 1e-7f * (float)D.M : T * (1.f + kEstSlack);
+        if (T < INFINITY) {
+            w.thr[qi] = T;
+            w.est_qc[qi] = make_float4(2.f * (rq + kEstAcc * (float)D.d * sqrtf(qn)) * (1.f + kEstSlack), 2.f * qh,
+                                       qn * (1.f - kEstSlack) - Tb, 0.f);
+            w.prq[qi] = 1;
+        }
+    }
+}
+
+// +1 / -1 at the first row tile of every candidate range of the pass's queries and past its last
+__global__ void k_est_count(uint64_t q, int R, Workspace w, int* __restrict__ diff) {
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= q * R) return;
+    if (w.prq[e / R] != 1) return;
+    const uint32_t len = w.range_len[e], start = w.range_start[e];
+    if (!len) return;
+    atomicAdd(&diff[start / kEstM], 1);
+    atomicAdd(&diff[(start + len - 1) / kEstM + 1], -1);
+}
+
+// Entries of every row tile (the running sum of diff), their prefix, and the prefix of their query
+// tiles; cursor: a copy of the entries' prefix for the fill.  One block.
+__global__ void __launch_bounds__(1024) k_est_scan(const int* __restrict__ diff, uint32_t tiles,
+                                                   uint32_t* __restrict__ ent_off, uint32_t* __restrict__ nt_off,
+                                                   uint32_t* __restrict__ cursor) {
+    __shared__ unsigned long long s_a[32], s_b[32], s_c[32];
+    const int t = threadIdx.x;
+    const uint32_t per = (tiles + blockDim.x - 1) / blockDim.x, b = min(tiles, t * per), e = min(tiles, b + per);
+    long long d = 0;
+    for (uint32_t i = b; i < e; i++) d += diff[i];
+    unsigned long long tot = 0;
+    const long long c0 = (long long)block_inclusive_sum((unsigned long long)d, s_a, &tot) - d;  // (wraps like the sums)
+    unsigned long long ne = 0, nt = 0;
+    long long c = c0;
+    for (uint32_t i = b; i < e; i++) {
+        c += diff[i];
+        ne += (unsigned long long)c;
+        nt += (unsigned long long)(c + kEstN - 1) / kEstN;
+    }
+    unsigned long long pe = block_inclusive_sum(ne, s_b, &tot) - ne;
+    unsigned long long pn = block_inclusive_sum(nt, s_c, &tot) - nt;
+    c = c0;
+    for (uint32_t i = b; i < e; i++) {
+        c += diff[i];
+        ent_off[i] = cursor[i] = (uint32_t)pe;
+        nt_off[i] = (uint32_t)pn;
+        pe += (unsigned long long)c;
+        pn += (unsigned long long)(c + kEstN - 1) / kEstN;
+    }
+    if (e == tiles && b < e) {
+        ent_off[tiles] = (uint32_t)pe;
+        nt_off[tiles] = (uint32_t)pn;
+    }
+}
+
+// The entries themselves.  A warp takes 32 ranges and shares their tiles out evenly: entry k of
+// the warp belongs to the range whose prefix of tile counts holds k.
+__global__ void __launch_bounds__(256) k_est_fill(uint64_t q, int R, Workspace w, uint32_t* __restrict__ cursor,
+                                                  uint4* __restrict__ ent) {
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    uint32_t qi = 0, start = 0, len = 0, pre = 0;
+    if (e < q * R) {
+        qi = (uint32_t)(e / R);
+        if (w.prq[qi] == 1) {
+            len = w.range_len[e];
+            start = w.range_start[e];
+            pre = w.range_pre[(uint64_t)qi * (R + 1) + (uint32_t)(e % R)];
+        }
+    }
+    const uint32_t t0 = start / kEstM, n = len ? (start + len - 1) / kEstM - t0 + 1u : 0u;
+    uint32_t inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
+    for (uint32_t k0 = 0; k0 < total; k0 += 32) {
+        const uint32_t k = k0 + lane;
+        int r = 0;  // the first lane whose inclusive prefix passes k
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const uint32_t v = __shfl_sync(0xffffffffu, inc, r + o - 1);
+            if (v <= k) r += o;
+        }
+        r = min(r, 31);
+        const uint32_t rs = __shfl_sync(0xffffffffu, start, r), rl = __shfl_sync(0xffffffffu, len, r),
+                       rp = __shfl_sync(0xffffffffu, pre, r), rq = __shfl_sync(0xffffffffu, qi, r),
+                       ri = __shfl_sync(0xffffffffu, inc, r), rn = __shfl_sync(0xffffffffu, n, r);
+        if (k < total) {
+            const uint32_t tile = rs / kEstM + (k - (ri - rn)), base = tile * kEstM;
+            const uint32_t lo = max(rs, base) - base, hi = min(rs + rl, base + kEstM) - base;
+            ent[atomicAdd(&cursor[tile], 1u)] = make_uint4(rq, lo | (hi << 16), rp - rs, 0u);
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------
 // host orchestration
 // ------------------------------------------------------------------------------------
 static uint32_t lut_groups(const IndexDev& D) { return (D.M + 31) / 32; }
@@ -2450,6 +2763,7 @@ static Workspace carve(hdg_index* idx, QueryCtx& cx, uint64_t q, bool record) {
     w.is_split = P.is_split ? 1 : 0;
     w.nsplit = (int)ns;
     w.qstat = (uint32_t*)take("qstat", q * 4 * 4);
+    w.qtiles = (uint32_t*)take("row_tiles", q * 4);
     w.scal = (uint64_t*)take("scalars", 8 * 8);
     w.qoff = (uint64_t*)take("qoff", (q + 1) * 8);
     w.item_off = (uint32_t*)take("item_off", (q + 1) * 4);
@@ -2777,6 +3091,75 @@ static void resolve_lazy(hdg_index* idx, QueryCtx& cx) {
     fill_stats(idx, cx.lazy.q, cx.lazy.k, cx.lazy.mode, cx.lazy.exps0, sc, cx.lazy.launches);
 }
 
+// The estimate pass pays from this many candidates in the batch and on the average query:
+// EST_RULE
+constexpr uint64_t kEstMinCands = 32ull << 20, kEstMinRow = 8192;
+
+// Thresholds, row-tile entries (`entries` of them at most), estimates and the scan's work items.
+static void estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const QueryCall& c, int R, uint32_t G,
+                          uint64_t entries, cudaStream_t st) {
+    const IndexDev& D = idx->dev;
+    const uint64_t q = c.q;
+    const uint32_t tiles = (D.n + kEstM - 1) / kEstM;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off += align_up(bytes, 256);
+        return o;
+    };
+    const size_t o_prq = take(q * 4), o_thr = take(q * 4), o_nle = take(q * 4), o_qc = take(q * sizeof(float4));
+    const size_t o_diff = take((tiles + 1) * 4ull), o_eo = take((tiles + 1) * 4ull), o_no = take((tiles + 1) * 4ull),
+                 o_cur = take((tiles + 1) * 4ull), o_ent = take(std::max<uint64_t>(entries, 1) * sizeof(uint4));
+    if (cx.est_buf.bytes < off) {
+        cx.est_buf.reset();
+        cx.est_buf.ensure(off + off / 4);
+    }
+    char* b = static_cast<char*>(cx.est_buf.ptr);
+    w.prq = reinterpret_cast<uint32_t*>(b + o_prq);
+    w.thr = reinterpret_cast<float*>(b + o_thr);
+    w.nle = reinterpret_cast<uint32_t*>(b + o_nle);
+    w.est_qc = reinterpret_cast<float4*>(b + o_qc);
+    int* diff = reinterpret_cast<int*>(b + o_diff);
+    EstArgs a{};
+    a.rowc = D.decoded_c;
+    a.qc = w.est_qc;
+    a.qb = static_cast<const uint16_t*>(w.qbf);
+    a.ldq = D.d;
+    a.n_rows = D.n;
+    a.tiles = tiles;
+    uint32_t* ent_off = reinterpret_cast<uint32_t*>(b + o_eo);
+    uint32_t* nt_off = reinterpret_cast<uint32_t*>(b + o_no);
+    uint32_t* cursor = reinterpret_cast<uint32_t*>(b + o_cur);
+    uint4* ent = reinterpret_cast<uint4*>(b + o_ent);
+    a.ent_off = ent_off;
+    a.nt_off = nt_off;
+    a.ent = ent;
+    a.qoff = w.qoff;
+    a.drow = reinterpret_cast<uint32_t*>(w.dist);
+    a.prow = w.spos;
+    a.cnt = w.cand_count;
+    CK(cudaMemsetAsync(diff, 0, (tiles + 1) * 4ull, st));
+    const size_t sm = sizeof(float) * (G * kCodes * 32 + kThrMax + kThrBins) + sizeof(uint32_t) * (2 * R + 1);
+    auto thr = [&](auto kern) {
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        kern<<<(unsigned)q, kThrThreads, sm, st>>>(D, R, c.queries, w);
+        CK_LAUNCH();
+    };
+    if (G == 1) thr(k_est_thr<1>);
+    else if (G == 2) thr(k_est_thr<2>);
+    else thr(k_est_thr<3>);
+    const unsigned blocks = (unsigned)((q * R + 255) / 256);
+    k_est_count<<<blocks, 256, 0, st>>>(q, R, w, diff);
+    CK_LAUNCH();
+    k_est_scan<<<1, 1024, 0, st>>>(diff, tiles, ent_off, nt_off, cursor);
+    CK_LAUNCH();
+    k_est_fill<<<blocks, 256, 0, st>>>(q, R, w, cursor, ent);
+    CK_LAUNCH();
+    est_ranges(a, D.decoded, (int)D.d, w.gemm_err, st);
+    k_scan_plan<<<1, 1024, 0, st>>>(q, w);
+    CK_LAUNCH();
+}
+
 // Enqueues one query batch on st.  sync_sizing: one host read after k_batch sizes the
 // distance buffer and fills the stats (the plain path).  Otherwise nothing waits on the
 // host (the CUDA-graph path): the distance buffer keeps its capacity, queries past it are
@@ -2823,6 +3206,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     w.exps0 = (uint32_t)std::min<uint64_t>(exps0, 1u << 20);
     w.chunk = (uint32_t)P.scan_chunk;
     w.scan_items = 8 * (uint32_t)sm_count();
+    w.round = 1;
     w.cap = sync_sizing ? ~0ull : cx.dist_buf.bytes / 4;
     if (sync_sizing) w.sel_cap = ~0ull;  // sized after k_batch
     const FilterDev f = filter_dev(idx);
@@ -2892,7 +3276,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             CK(cudaEventRecord(cx.lazy.done, st));
         } else {
             if (!cx.pinned) CK(cudaMallocHost(reinterpret_cast<void**>(&cx.pinned), 16 * sizeof(uint64_t)));
-            CK(cudaMemcpyAsync(cx.pinned, w.scal, 9 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+            CK(cudaMemcpyAsync(cx.pinned, w.scal, 10 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             std::memcpy(sc, cx.pinned, sizeof(sc));
             HDG_REQUIRE((uint32_t)cx.pinned[8] == 0, HDG_ERR_TIMEOUT, "tensor-core wait expired in the coarse GEMM");
@@ -2916,6 +3300,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     // candidate ranges per query: one per probed list, or n_split per list when is_split
     const int R = Ps * w.nsplit;
     const size_t sm_tab = sizeof(uint32_t) * (2 * R + 1);
+    std::function<void(const Workspace&)> scan;  // the ADC scan as launched
     if (!sync_sizing || lazy || sc[3] > 0) {
         if (fast && (pre || w.qsched)) {
             // the predicate pass of the predicate-first queries, then the ADC items that
@@ -2952,6 +3337,19 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             launches++;
             tm.mark("lut");
         }
+        // post-filter queries with many more candidates than budget: the estimate pass (not in a
+        // captured graph, whose entry count is not known)
+        const bool prune = sync_sizing && !lazy && mode == kPost && !w.qsched && fast && D.decoded && sc[0] >= kEstMinCands &&
+                           sc[0] / q >= kEstMinRow && cx.pinned[9] < (1ull << 32);
+        if (prune) {
+            if (!use_gemm) {
+                rows_to_bf16(c.queries, q, (int)D.d, w.qbf, w.qnorm, st);
+                launches++;
+            }
+            estimate_pass(idx, cx, w, c, R, G, cx.pinned[9], st);
+            launches += 6;
+            tm.mark("estimate");
+        }
         if (fast) {
             // threads x candidates-per-thread (SCAN_CPT, chosen by the autotuner; 0 = 1)
             const int cpt = (P.scan_cpt == 1 || P.scan_cpt == 2 || P.scan_cpt == 4) ? (int)P.scan_cpt : 1;
@@ -2960,7 +3358,8 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             auto launch = [&](auto kern, int nt) {
                 CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
                 const int blocks = sm_count() * occupancy_blocks(kern, nt, sm);
-                kern<<<blocks, nt, sm, st>>>(D, R, q, w);
+                scan = [=](const Workspace& ww) { kern<<<blocks, nt, sm, st>>>(D, R, q, ww); };
+                scan(w);
             };
             if (G == 1) {
                 if (cpt == 1) launch(k_scan_fast<1, 512, 1>, 512);
@@ -2993,6 +3392,17 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     auto launch_sel = [&](auto kern, int nt) {
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_sel));
         kern<<<(unsigned)q, nt, sm_sel, st>>>(D, R, (int)k, sorted_out, w, c.dist, c.ids, (int)k);
+        if (!w.prq) return;
+        // queries whose threshold was too low (usually none): scanned and selected in full
+        CK_LAUNCH();
+        w.round = 2;
+        k_scan_plan<<<1, 1024, 0, st>>>(q, w);
+        CK_LAUNCH();
+        scan(w);
+        CK_LAUNCH();
+        kern<<<(unsigned)q, nt, sm_sel, st>>>(D, R, (int)k, sorted_out, w, c.dist, c.ids, (int)k);
+        w.round = 1;
+        launches += 3;
     };
     if (q <= (uint64_t)sm_count()) launch_sel(k_select<kSelThreadsFew, 8>, kSelThreadsFew);
     else launch_sel(k_select<kSelThreads, 4>, kSelThreads);

@@ -165,3 +165,86 @@ def test_small_batch_stats_on_demand(cuda, q):
     call(q)
     assert idx.last_query_stats() == want
     torch.cuda.synchronize()
+
+
+def _plain_and_full(cuda, ws, k, conf=()):
+    """A batch through the plain call (estimate pass) and through a graph replay (full scan)."""
+    import torch
+    import hdgrid_b200 as hg
+    from tests.helpers import build_gpu
+    idx, base, _ = build_gpu(ws, cuda)
+    for key, v in conf:
+        idx.set_param(key, v)
+    q, ql = torch.from_numpy(ws["queries"]).to(cuda), torch.from_numpy(ws["query_labels"]).to(cuda)
+    out = []
+    for graph in (0, 1):
+        idx.set_param("QUERY_GRAPH", graph)
+        d = torch.full((q.shape[0], k), -1.0, device=cuda)
+        i = torch.full((q.shape[0], k), 7, dtype=torch.int64, device=cuda)
+        for _ in range(2):
+            idx.query(hg.query_input_t(base, q, ql), hg.query_output_t(d, i))
+        if graph:
+            idx.status()
+            d.fill_(-1.0)
+            i.fill_(7)
+            idx.query(hg.query_input_t(base, q, ql), hg.query_output_t(d, i))
+            idx.status()
+        else:
+            idx.set_param("BREAK_DOWN", 1)
+            idx.query(hg.query_input_t(base, q, ql), hg.query_output_t(d, i))
+            stages = idx.stage_times()
+            idx.set_param("BREAK_DOWN", 0)
+        torch.cuda.synchronize()
+        out.append((d, i))
+    return idx, stages, out
+
+
+# one to three groups of 32 subspaces (K of 128, 64 + a remainder chunk, 384), FP16 tables, split
+# ranges, ragged query tiles; the estimate pass must select what the full scan selects
+@pytest.mark.parametrize("case", ["m32", "m64", "m96", "fp16", "split", "few", "d96"])
+def test_estimate_pass_equals_full_scan(cuda, case):
+    import torch
+    if case in ("m96", "fp16"):
+        ws = datasets.config2(scale=0.4, n_queries=2001, max_grids=30_000, lut_fp16=1 if case == "fp16" else 0)
+    else:
+        ws = datasets.config4(scale=0.04, n_queries=129 if case == "few" else 1500, clusters=16, sub_clusters=8,
+                              n_list=16, sub_lists=100, exps0=8, max_grids=16384, pq_dim=64 if case == "m64" else 32,
+                              is_split=1 if case == "split" else 0, n_split=3 if case == "split" else 1)
+        if case == "few":  # long rows from few queries: open boxes
+            ws["query_labels"][:, 0::2] = 0
+            ws["query_labels"][:, 1::2] = 1_000_000
+        if case == "d96":  # K of 96: one whole chunk of 64 and half of one
+            ws["base"] = np.ascontiguousarray(ws["base"][:, :96])
+            ws["queries"] = np.ascontiguousarray(ws["queries"][:, :96])
+    idx, stages, out = _plain_and_full(cuda, ws, 100)
+    assert "estimate" in stages, stages
+    assert torch.equal(out[0][1], out[1][1]) and torch.equal(out[0][0], out[1][0])
+
+
+def test_estimate_pass_threshold_too_low(cuda):
+    """One list whose position order is the id order, with the near points exactly at the sampled
+    positions: the threshold lies below the budget's share and every query is scanned in full."""
+    import torch
+    n, d, nq, k, exps0 = 1 << 17, 64, 300, 100, 4
+    rng = np.random.default_rng(3)
+    base = (rng.standard_normal((n, d)) * 0.1 + 5.0).astype(np.float32)
+    K = exps0 * k
+    for ms in range(int((5 * np.sqrt(K * n)) ** (2 / 3)) - 1, int((5 * np.sqrt(K * n)) ** (2 / 3)) + 3):
+        pos = (np.arange(ms, dtype=np.int64) * n + n // 2) // ms
+        base[pos[:: max(1, ms // 24)]] -= 5.0
+    ws = dict(base=base, labels=np.full((n, 2), 10, np.float32),
+              queries=(rng.standard_normal((nq, d)) * 0.1).astype(np.float32),
+              query_labels=np.full((nq, 2), 10, np.float32),
+              hdgrid_conf=datasets.hdgrid_conf(clusters=1, sub_clusters=1, pq_dim=32, max_grids=16, n_list=1, sub_lists=1,
+                                               exps0=exps0, topk=k),
+              filter_conf="l = 2\nfilter0:\n\ttype = 0\n\tshift_val = [5, 5]\nfilter1:\n\ttype = 0\n\tshift_val = [5, 5]\n")
+    idx, stages, out = _plain_and_full(cuda, ws, k)
+    assert "estimate" in stages, stages
+    assert torch.equal(out[0][1], out[1][1]) and torch.equal(out[0][0], out[1][0])
+    # every query's kept count was below its budget's share, so every candidate was scanned
+    import hdgrid_b200 as hg
+    idx.set_param("QUERY_GRAPH", 0)
+    b, q, ql = (torch.from_numpy(ws[x]).to(cuda) for x in ("base", "queries", "query_labels"))
+    idx.query(hg.query_input_t(b, q, ql), hg.query_output_t(*out[0]))
+    nfin = np.frombuffer(idx.debug_fetch("nfin").tobytes(), np.uint32)[:nq]
+    assert np.all(nfin == n), nfin
