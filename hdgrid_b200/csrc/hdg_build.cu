@@ -18,6 +18,7 @@
 // k-means results are not pinned by any reference test (RAFT is not vendored), so the
 // build uses its own seeded Lloyd iterations.
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <algorithm>
 #include <cmath>
@@ -341,29 +342,40 @@ __global__ void k_gather_codes_labels(const uint8_t* __restrict__ codes_by_id, i
     for (int i = 0; i < l; i++) labels[r * l + i] = labels_by_id[id * l + i];
 }
 
-// A point's PQ approximation (the codewords its codes name) in BF16, and its constants for the
+// A point's PQ approximation (the codewords its codes name) in FP16, and its constants for the
 // distance estimates; one warp per pool row, lane = subspace (mod 32).
-__global__ void k_decode_rows(IndexDev D, uint16_t* __restrict__ out, float4* __restrict__ cst) {
+__global__ void k_decode_rows(IndexDev D, uint16_t* __restrict__ out, float4* __restrict__ cst,
+                              uint32_t* __restrict__ mx) {
+    __shared__ uint32_t s_mx[3];
+    if (threadIdx.x < 3) s_mx[threadIdx.x] = 0u;
+    __syncthreads();
     const uint64_t r = (uint64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int lane = threadIdx.x & 31;
-    if (r >= D.n) return;
     const int L = D.pq_len;
     float s = 0.f, e = 0.f;
-    for (int m = lane; m < (int)D.M; m += 32) {
+    for (int m = lane; r < D.n && m < (int)D.M; m += 32) {
         const uint32_t c = D.codes[((uint64_t)(m >> 4) * D.n + r) * 16 + (m & 15)];
         const float* x = D.pq_centers + ((uint64_t)m * kCodes + c) * L;
         for (int t = 0; t < L; t++) {
             const float v = __ldg(x + t);
-            const __nv_bfloat16 h = __float2bfloat16_rn(v);
-            const float df = v - __bfloat162float(h);
+            const __half h = __float2half_rn(v);
+            const float df = v - __half2float(h);
             s = fmaf(v, v, s);
             e = fmaf(df, df, e);
-            out[r * D.d + m * L + t] = __bfloat16_as_ushort(h);
+            out[r * D.d + m * L + t] = __half_as_ushort(h);
         }
     }
     s = warp_sum(s);
     e = warp_sum(e);
-    if (lane == 0) cst[r] = make_float4(s * (1.f - kEstSlack), sqrtf(s) * (1.f + kEstSlack), sqrtf(e) * (1.f + kEstSlack), 0.f);
+    if (lane == 0 && r < D.n) {
+        const float4 v = make_float4(s * (1.f - kEstSlack), sqrtf(s) * (1.f + kEstSlack), sqrtf(e) * (1.f + kEstSlack), 0.f);
+        cst[r] = v;
+        atomicMax(&s_mx[0], __float_as_uint(v.x));  // (non-negative floats order as their bits; NaN above all)
+        atomicMax(&s_mx[1], __float_as_uint(v.y));
+        atomicMax(&s_mx[2], __float_as_uint(v.z));
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) atomicMax(&mx[threadIdx.x], s_mx[threadIdx.x]);
 }
 
 __global__ void k_to_bf16(const float* __restrict__ x, uint64_t n, __nv_bfloat16* __restrict__ y) {
@@ -976,15 +988,20 @@ void upload_index(hdg_index* idx, cudaStream_t st) {
     // operands (2 d + 16 bytes per point; not kept past kDecodedMax, where the full scan runs)
     D.decoded = nullptr;
     D.decoded_c = nullptr;
+    D.decoded_max = nullptr;
     idx->decoded.reset();
     const uint64_t dec = align_up((uint64_t)H.n * H.d * 2, 256);
     if (H.d % 8 == 0 && H.M % 32 == 0 && H.M <= 96 && H.M * H.pq_len == H.d && H.n >= kDecodedMinPoints &&
         dec <= kDecodedMax) {
-        idx->decoded.ensure(dec + (uint64_t)H.n * sizeof(float4));
+        const uint64_t cst = (uint64_t)H.n * sizeof(float4);
+        idx->decoded.ensure(dec + cst + 16);
         char* p = static_cast<char*>(idx->decoded.ptr);
+        uint32_t* mx = reinterpret_cast<uint32_t*>(p + dec + cst);
+        CK(cudaMemsetAsync(mx, 0, 16, st));
         k_decode_rows<<<blocks_for(H.n, 8), 256, 0, st>>>(D, reinterpret_cast<uint16_t*>(p),
-                                                         reinterpret_cast<float4*>(p + dec));
+                                                         reinterpret_cast<float4*>(p + dec), mx);
         CK_LAUNCH();
+        D.decoded_max = mx;
         D.decoded = reinterpret_cast<const uint16_t*>(p);
         D.decoded_c = reinterpret_cast<const float4*>(p + dec);
     }

@@ -1,23 +1,24 @@
 // Distance estimates on the tensor cores (hdg_est.cuh).
 //
-// Persistent, one CTA per SM, 12 warps: 0-7 epilogue, 8 MMA issue and TMEM, 9 the rows by TMA
-// (a tile's rows are consecutive), 10-11 the queries by cp.async (any queries, gathered by id into
-// the 128-byte-swizzled layout).  A work item is one tile of 128 rows x 128 queries; every CTA
-// takes an equal, consecutive span of them, so successive items share their rows in L2.  K runs in
-// chunks of 64 through a ring of stages (full barriers: one for the TMA bytes, one for the two
-// gathering warps; the tcgen05.commit of a chunk's MMAs frees its stage).  Two accumulators of 128
-// TMEM columns let the MMAs of item i + 1 run under the epilogue of item i.
+// Persistent, one CTA per SM, 20 warps: 0-15 epilogue (two groups of eight, taking turns at the
+// items), 16 MMA issue and TMEM, 17 the rows by TMA (a tile's rows are consecutive), 18-19 the
+// queries by cp.async (any queries, gathered by id into the 128-byte-swizzled layout).  A work item
+// is one tile of 128 rows x 128 queries; every CTA takes an equal, consecutive span of them, so
+// successive items share their rows in L2.  K runs in chunks of 64 through a ring of stages (full
+// barriers: one for the TMA bytes, one for the two gathering warps; the tcgen05.commit of a
+// chunk's MMAs frees its stage).  Four accumulators of 128 TMEM columns keep the MMAs ahead.
 //
-// Epilogue of item i: thread = row, loop over columns (queries): three FMAs and a compare per pair
-// against the query's constants, broadcast from shared memory; a ballot per column and warp gives
-// the column's 128-bit mask.  One thread per column then reserves the kept rows' slots with one
-// atomic, whose latency runs under item i + 1; after that item's masks the rows of item i are
-// written, a warp per column, consecutive slots by consecutive lanes.
-// Bound: the epilogue's issue slots (about 8 instructions per 32 pairs and the writes); the MMAs
-// take half of that at K = 128.  Every wait is bounded: on expiry the kernel sets *err, lets its
-// copies land, frees TMEM and returns.
+// Epilogue of an item: thread = row, loop over columns (queries), two at a time in packed FP32
+// FMAs against the queries' constants, broadcast from shared memory; a ballot per column and warp
+// gives the column's 128-bit mask.  Two threads per column then reserve the kept rows' slots with
+// one atomic, whose latency runs under the group's next item, after whose masks they walk the
+// mask's bits and write the kept rows.
+// Bound: the epilogue's issue slots (about 7 instructions per column and warp, and the writes).
+// 145,000 items of K = 128 (10,000 queries x 227,000 candidates): 6.6 ms with one epilogue group
+// and a warp per column writing its kept rows (15,000 warp instructions an item, half of them for
+// the writes, 35 % issue), K_EST_MS as it stands.  Every wait is bounded: on expiry the kernel sets
+// *err, lets its copies land, frees TMEM and returns.
 #include <cuda.h>
-#include <cuda_bf16.h>
 
 #include <algorithm>
 
@@ -29,20 +30,30 @@ namespace hdg {
 
 namespace {
 
-constexpr int kEstThreads = 384, kEpiThreads = 256;
-constexpr uint32_t kChunkBytes = 128 * 64 * 2;  // one 128 x 64 bf16 operand chunk
-constexpr int kEstStages = 5;
-constexpr int kSlots = 3;  // column constants: read through the following item
+constexpr int kEpiThreads = 256, kGroups = 2, kAccs = 4;  // threads per epilogue group
+constexpr int kEstThreads = kGroups * kEpiThreads + 128;
+constexpr uint32_t kChunkBytes = 128 * 64 * 2;  // one 128 x 64 FP16 operand chunk
+constexpr int kMaxStages = 4;
+// ring stages: the steps of two pending items per group take the fourth stage's room
+constexpr int est_stages(bool ranges) { return ranges ? 3 : 4; }
+constexpr int kSlots = 3;  // column constants: read through the group's following item
 
-struct EstShared {
-    float4 col[kSlots][kEstN];
+struct EstGroup {  // of one epilogue group
+    float4 ab[kSlots][kEstN / 2];    // {a0, a1, b0, b1} of a pair of columns
+    float4 zs[kSlots][kEstN / 2];    // {z0, z1, steps0, steps1}
+    float2 sb[kSlots][kEstN / 2];    // the steps' bias: 2^23 + 1 - z * steps
     uint64_t off[kSlots][kEstN];     // ranges: the query's row offset
     uint32_t qid[kSlots][kEstN];
     uint32_t delta[kSlots][kEstN];
     uint32_t lohi[kSlots][kEstN];
     uint4 mask[2][kEstN];
-    uint32_t base[2][kEstN];
-    uint64_t full_a[kEstStages], full_b[kEstStages], empty[kEstStages], acc_full[2], acc_empty[2];
+    uint32_t base[2][kEstN];         // the query's slot of its first kept row
+    uint32_t pre[2][kEstN];          // kept rows of the columns before, within the column's warp
+    uint32_t wsum[2][kEstN / 32];    // kept rows of 32 columns
+};
+struct EstShared {
+    EstGroup grp[kGroups];
+    uint64_t full_a[kMaxStages], full_b[kMaxStages], empty[kMaxStages], acc_full[kAccs], acc_empty[kAccs];
     uint32_t tmem;
     int fail;
 };
@@ -72,20 +83,26 @@ __device__ __forceinline__ void est_commit(uint64_t& bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&bar))
                  : "memory");
 }
-__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,"
-        "%30,%31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(addr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+__device__ __forceinline__ void epi_bar(int group) { asm volatile("bar.sync %0, 256;" ::"r"(1 + group) : "memory"); }
+// (d0, d1) = (a0, a1) * (b0, b1) + (c0, c1), each rounded like one fmaf
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 ra, rb, rc;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+        "fma.rn.f32x2 ra, ra, rb, rc;\n\tmov.b64 {%0, %1}, ra;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
 }
+
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(addr));
+}
+__device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // The items of this CTA in order: row tile t, its query tile j
 template <bool RANGES>
@@ -136,15 +153,19 @@ template <bool RANGES, int LT>
 __global__ void __launch_bounds__(kEstThreads, 1) k_est(const __grid_constant__ CUtensorMap map_rows, EstArgs a, int d,
                                                         int nk, int* __restrict__ err) {
     extern __shared__ unsigned char est_smem[];
-    // [stages][rows chunk, queries chunk], then the shared block, then (LT) the label boxes
+    // [stages][rows chunk, queries chunk], then the shared block, then the label boxes or the steps
     unsigned char* ring = est_smem + (1024 - (smem_u32(est_smem) & 1023)) % 1024;
+    constexpr int kEstStages = est_stages(RANGES);
     EstShared& s = *reinterpret_cast<EstShared*>(ring + kEstStages * 2 * kChunkBytes);
-    float* s_box = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(&s) + (sizeof(EstShared) + 15) / 16 * 16);
+    unsigned char* tail = reinterpret_cast<unsigned char*>(&s) + (sizeof(EstShared) + 15) / 16 * 16;
+    float* s_box = reinterpret_cast<float*>(tail);  // [group][2][column][2 l] label boxes (!RANGES)
+    unsigned char* s_step = tail;                   // [group][2][column][row] steps (RANGES)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rbase = smem_u32(ring);
-    if (warp == 8) {
+    constexpr int kMmaWarp = kGroups * kEpiThreads / 32;
+    if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem)),
-                     "r"(2 * kEstN));
+                     "r"(kAccs * kEstN));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
@@ -157,7 +178,7 @@ __global__ void __launch_bounds__(kEstThreads, 1) k_est(const __grid_constant__ 
             init(s.full_b[i], 2);
             init(s.empty[i], 1);
         }
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < kAccs; i++) {
             init(s.acc_full[i], 1);
             init(s.acc_empty[i], kEpiThreads / 32);
         }
@@ -172,7 +193,7 @@ __global__ void __launch_bounds__(kEstThreads, 1) k_est(const __grid_constant__ 
     const uint32_t first = total / nb * b + min(b, total % nb), items = total / nb + (b < total % nb ? 1u : 0u);
     if (items) w.seek(first);
 
-    if (warp == 9) {
+    if (warp == kMmaWarp + 1) {
         // ---- the rows: one thread, TMA ----
         if (lane == 0) {
             uint32_t g = 0;
@@ -195,11 +216,11 @@ __global__ void __launch_bounds__(kEstThreads, 1) k_est(const __grid_constant__ 
                 for (uint32_t h = g > kEstStages ? g - kEstStages : 0; h < g; h++)
                     mbar_wait(smem_u32(&s.full_a[h % kEstStages]), (h / kEstStages) & 1u);
         }
-    } else if (warp >= 10) {
+    } else if (warp >= kMmaWarp + 2) {
         // ---- the queries: two warps, thread p copies 16-byte unit p % 8 of rows p / 8 + 8 r ----
-        const int p = tid - 320, unit = p & 7, row0 = p >> 3;
+        const int p = tid - 32 * (kMmaWarp + 2), unit = p & 7, row0 = p >> 3;
         uint32_t g = 0;
-        constexpr uint32_t kLag = 2;  // stages whose copies may be in flight
+        constexpr uint32_t kLag = RANGES ? 1 : 2;  // stages whose copies may be in flight
         bool ok = true;
         auto landed = [&](uint32_t h) {  // stage h's copies of this warp have landed
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -241,16 +262,16 @@ __global__ void __launch_bounds__(kEstThreads, 1) k_est(const __grid_constant__ 
         asm volatile("cp.async.wait_all;" ::: "memory");
         if (ok)
             for (uint32_t h = g > kLag ? g - kLag : 0; h < g; h++) landed(h);
-    } else if (warp == 8) {
+    } else if (warp == kMmaWarp) {
         // ---- MMA issue: one thread ----
         if (lane == 0) {
-            constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kEstN >> 3) << 17) |
-                                        ((uint32_t)(kEstM >> 4) << 24);
+            // F32 accumulate, FP16 A and B, both K-major
+            constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(kEstN >> 3) << 17) | ((uint32_t)(kEstM >> 4) << 24);
             uint32_t g = 0;
             bool ok = true;
             for (uint32_t i = 0; i < items && ok; i++) {
-                const uint32_t acc = i & 1u;
-                if (!est_wait(s, s.acc_empty[acc], ((i >> 1) & 1u) ^ 1u)) break;
+                const uint32_t acc = i % kAccs;
+                if (!est_wait(s, s.acc_empty[acc], ((i / kAccs) & 1u) ^ 1u)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;");
                 for (int kc = 0; kc < nk; kc++, g++) {
                     const uint32_t st = g % kEstStages, ph = (g / kEstStages) & 1u;
@@ -281,11 +302,14 @@ __global__ void __launch_bounds__(kEstThreads, 1) k_est(const __grid_constant__ 
             }
         }
     } else {
-        // ---- epilogue ----
-        const int rl = (warp & 3) * 32 + lane, half = warp >> 2;
-        const unsigned lt = (1u << lane) - 1u;
+        // ---- epilogue: group `group` takes items group, group + kGroups, ... ----
+        const int group = warp / (kEpiThreads / 32), gt = tid - group * kEpiThreads;  // thread in the group
+        const int gw = gt >> 5, rl = (gw & 3) * 32 + lane, half = gw >> 2;
+        EstGroup& G = s.grp[group];
         const int l = RANGES ? 0 : (LT ? LT : a.l);
         constexpr int LM = RANGES ? 1 : (LT ? LT : kMaxDims);
+        float* box0 = s_box + (size_t)group * 2 * kEstN * 2 * l;
+        unsigned char* step0 = s_step + (size_t)group * 2 * kEstN * kEstM;
         // the next item's row and column constants, loaded one item ahead
         float4 rc = make_float4(INFINITY, 0.f, 0.f, 0.f), cc = make_float4(0.f, 0.f, INFINITY, 0.f);
         uint32_t qid = 0, lohi = 0, delta = 0;
@@ -299,8 +323,8 @@ __global__ void __launch_bounds__(kEstThreads, 1) k_est(const __grid_constant__ 
 #pragma unroll
                 for (int i = 0; i < LM; i++) lab[i] = i < l ? __ldg(a.labels + br * l + i) : 0.f;
             }
-            if (tid < kEstN) {
-                const uint32_t c = w.j * kEstN + tid;
+            if (gt < kEstN) {
+                const uint32_t c = w.j * kEstN + gt;
                 cc = make_float4(0.f, 0.f, INFINITY, 0.f);
                 qid = 0xffffffffu;  // a column without a query keeps nothing
                 lohi = 0;
@@ -318,139 +342,194 @@ __global__ void __launch_bounds__(kEstThreads, 1) k_est(const __grid_constant__ 
                 }
             }
         };
-        if (items) fetch();
+        auto skip = [&](uint32_t i, uint32_t n) {  // n items on from item i, as far as there are items
+            for (uint32_t k = 0; k < n && i + k + 1 < items; k++) w.next();
+        };
+        skip(0, (uint32_t)group);
+        if ((uint32_t)group < items) fetch();
         uint32_t base_reg = 0, prev_row0 = 0;
         bool ok = true;
-        auto write_kept = [&](uint32_t i, uint32_t row0) {  // the kept rows of item i
-            const int ms = i & 1, cs = i % kSlots;
-#pragma unroll 1
-            for (int c = warp * 16; c < warp * 16 + 16; c++) {
-                const uint4 m = s.mask[ms][c];
-                if (!(m.x | m.y | m.z | m.w)) continue;
-                const uint32_t word[4] = {m.x, m.y, m.z, m.w};
-                uint32_t at = s.base[ms][c];
-                const uint32_t q = s.qid[cs][c];
+        // the kept rows of the group's item number n, shared out evenly: kept row f of the item
+        // is bit f - (the kept rows of the columns before) of its column's mask
+        auto write_kept = [&](uint32_t n, uint32_t row0) {
+            const int ms = n & 1, cs = n % kSlots;
+            const uint32_t s0 = G.wsum[ms][0], s1 = s0 + G.wsum[ms][1], s2 = s1 + G.wsum[ms][2], all = s2 + G.wsum[ms][3];
+            for (uint32_t f = gt; f < all; f += kEpiThreads) {
+                const int q4 = (f >= s0) + (f >= s1) + (f >= s2);
+                const uint32_t k = f - (q4 == 0 ? 0u : (q4 == 1 ? s0 : (q4 == 2 ? s1 : s2)));
+                int c = 32 * q4;  // the last of the 32 columns with pre <= k
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    if ((word[k] >> lane) & 1u) {
-                        const uint32_t slot = at + __popc(word[k] & lt), row = row0 + 32 * k + lane;
-                        if (RANGES) {
-                            const uint64_t o = s.off[cs][c] + slot;
-                            a.prow[o] = row + s.delta[cs][c];
-                            a.drow[o] = row;
-                        } else if (slot < a.cap) {
-                            a.list[(uint64_t)q * a.cap + slot] = a.row0 + row * a.row_step;
-                        }
+                for (int st = 16; st > 0; st >>= 1)
+                    if (G.pre[ms][c + st] <= k) c += st;
+                const uint4 m = G.mask[ms][c];
+                uint32_t bit = k - G.pre[ms][c];  // the bit's rank in the mask
+                const uint32_t slot = G.base[ms][c] + bit;
+                const uint32_t p0 = __popc(m.x), p1 = p0 + __popc(m.y), p2 = p1 + __popc(m.z);
+                const int wd = (bit >= p0) + (bit >= p1) + (bit >= p2);
+                uint32_t x = wd == 0 ? m.x : (wd == 1 ? m.y : (wd == 2 ? m.z : m.w));
+                bit -= wd == 0 ? 0u : (wd == 1 ? p0 : (wd == 2 ? p1 : p2));
+                uint32_t at = 0;  // the position of set bit number `bit` of x
+#pragma unroll
+                for (int st = 16; st > 0; st >>= 1) {
+                    const uint32_t below = __popc(x & ((1u << st) - 1u));
+                    if (bit >= below) {
+                        bit -= below;
+                        at += st;
+                        x >>= st;
                     }
-                    at += __popc(word[k]);
+                }
+                const uint32_t row = row0 + 32u * wd + at;
+                if (RANGES) {
+                    const uint64_t o = G.off[cs][c] + slot;
+                    a.prow[o] = row + G.delta[cs][c];
+                    reinterpret_cast<unsigned char*>(a.drow + G.off[cs][c])[slot] =
+                        step0[((size_t)ms * kEstN + c) * kEstM + 32 * wd + at];
+                } else if (slot < a.cap) {
+                    a.list[(uint64_t)G.qid[cs][c] * a.cap + slot] = a.row0 + row * a.row_step;
                 }
             }
         };
-        for (uint32_t i = 0; i < items; i++) {
-            const int cs = i % kSlots, ms = i & 1;
-            const uint32_t row0 = w.t * kEstM;
-            if (tid < kEstN) {
-                s.col[cs][tid] = cc;
-                s.qid[cs][tid] = qid;
+        uint32_t n = 0;  // the group's items so far
+        for (uint32_t i = group; i < items; i += kGroups, n++) {
+            const int cs = n % kSlots, ms = n & 1;
+            const uint32_t row0 = w.t * kEstM, acc = i % kAccs;
+            if (gt < kEstN) {
+                float* ab = reinterpret_cast<float*>(&G.ab[cs][gt >> 1]);
+                ab[gt & 1] = cc.x;
+                ab[2 + (gt & 1)] = cc.y;
+                float* zs = reinterpret_cast<float*>(&G.zs[cs][gt >> 1]);
+                zs[gt & 1] = cc.z;
+                zs[2 + (gt & 1)] = cc.w;
+                // (2^23 + 1: the sum's low byte is the rounded step, never below zero for a kept row)
+                if (RANGES) reinterpret_cast<float*>(&G.sb[cs][gt >> 1])[gt & 1] = fmaf(-cc.z, cc.w, 8388609.f);
+                G.qid[cs][gt] = qid;
                 if (RANGES) {
-                    s.off[cs][tid] = off;
-                    s.delta[cs][tid] = delta;
-                    s.lohi[cs][tid] = lohi;
+                    G.off[cs][gt] = off;
+                    G.delta[cs][gt] = delta;
+                    G.lohi[cs][gt] = lohi;
                 }
             }
             if constexpr (!RANGES) {  // the columns' label boxes (read in this item only)
                 const uint32_t c0 = w.j * kEstN;
-                float* bx = s_box + (size_t)ms * kEstN * 2 * l;
-                for (int e = tid; e < kEstN * 2 * l; e += kEpiThreads)
+                float* bx = box0 + (size_t)ms * kEstN * 2 * l;
+                for (int e = gt; e < kEstN * 2 * l; e += kEpiThreads)
                     bx[e] = c0 + e / (2 * l) < a.nq ? __ldg(a.boxes + (uint64_t)c0 * 2 * l + e) : 0.f;
             }
-            const float xn = rc.x, xm = rc.y, rx = rc.z;
+            const float2 xn = make_float2(-rc.x, -rc.x), xm = make_float2(rc.y, rc.y), rx = make_float2(rc.z, rc.z);
             float lb[LM];
 #pragma unroll
             for (int k = 0; k < LM; k++) lb[k] = RANGES ? 0.f : lab[k];
-            epi_bar();
-            if (i + 1 < items) {
-                w.next();
+            epi_bar(group);
+            if (i + kGroups < items) {
+                skip(i, kGroups);
                 fetch();
             }
-            if (ok) ok = est_wait(s, s.acc_full[ms], (i >> 1) & 1u);
+            if (ok) ok = est_wait(s, s.acc_full[acc], (i / kAccs) & 1u);
             ok = __all_sync(0xffffffffu, ok);
             asm volatile("tcgen05.fence::after_thread_sync;");
-#pragma unroll
+#pragma unroll 1
             for (int h = 0; h < 2; h++) {
                 const int cb = half * 64 + h * 32;
-                uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(ms * kEstN + cb), v);
-                if (h == 1) {  // this warp has read its part of the accumulator
-                    asm volatile("tcgen05.fence::before_thread_sync;");
-                    __syncwarp();
-                    if (lane == 0) est_arrive(s.acc_empty[ms]);
-                }
-                uint32_t mine = 0;
+                const uint32_t taddr = tmem + ((uint32_t)((gw & 3) * 32) << 16) + acc * kEstN + (uint32_t)cb;
 #pragma unroll
-                for (int c = 0; c < 32; c++) {
-                    const float4 q = s.col[cs][cb + c];
-                    float x = fmaf(2.f, __uint_as_float(v[c]), -xn);
-                    x = fmaf(q.x, xm, x);
-                    x = fmaf(q.y, rx, x);
-                    bool keep = !(x < q.z);  // (NaN: no bound, kept)
-                    unsigned bal = __ballot_sync(0xffffffffu, keep);
-                    if constexpr (!RANGES) {
-                        if (bal) {
-                            const float* bx = s_box + ((size_t)ms * kEstN + cb + c) * 2 * l;
+                for (int hh = 0; hh < 2; hh++) {
+                    uint32_t v[16];
+                    tmem_ld16(taddr + 16 * hh, v);
+                    tmem_wait();
+                    if (h == 1 && hh == 1) {  // this warp has read its part of the accumulator
+                        asm volatile("tcgen05.fence::before_thread_sync;");
+                        __syncwarp();
+                        if (lane == 0) est_arrive(s.acc_empty[acc]);
+                    }
 #pragma unroll
-                            for (int k = 0; k < LM; k++)
-                                if (k < l && (lb[k] < bx[2 * k] || lb[k] > bx[2 * k + 1])) keep = false;
-                            bal = __ballot_sync(0xffffffffu, keep);
+                    for (int c = 0; c < 16; c += 2) {
+                        const int col = cb + 16 * hh + c;
+                        const float4 q = G.ab[cs][col >> 1];
+                        const float4 z = G.zs[cs][col >> 1];
+                        float2 x = fma2(make_float2(2.f, 2.f),
+                                        make_float2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), xn);
+                        x = fma2(make_float2(q.x, q.y), xm, x);
+                        x = fma2(make_float2(q.z, q.w), rx, x);
+                        float2 st = x;
+                        if (RANGES) {
+                            st = fma2(x, make_float2(z.z, z.w), G.sb[cs][col >> 1]);
+                            st.x = fminf(st.x, 8388608.f + 255.f);
+                            st.y = fminf(st.y, 8388608.f + 255.f);
+                        }
+#pragma unroll
+                        for (int u = 0; u < 2; u++) {
+                            bool keep = !((u ? x.y : x.x) < (u ? z.y : z.x));  // (NaN: no bound, kept)
+                            unsigned bal = __ballot_sync(0xffffffffu, keep);
+                            if constexpr (!RANGES) {
+                                if (bal) {
+                                    const float* bx = box0 + ((size_t)ms * kEstN + col + u) * 2 * l;
+#pragma unroll
+                                    for (int k = 0; k < LM; k++)
+                                        if (k < l && (lb[k] < bx[2 * k] || lb[k] > bx[2 * k + 1])) keep = false;
+                                    bal = __ballot_sync(0xffffffffu, keep);
+                                }
+                            }
+                            if (lane == 0)
+                                reinterpret_cast<uint32_t*>(&G.mask[ms][col + u])[gw & 3] = bal;
+                            if (RANGES && keep)
+                                step0[((size_t)ms * kEstN + col + u) * kEstM + rl] =
+                                    (unsigned char)__float_as_uint(u ? st.y : st.x);
                         }
                     }
-                    if (lane == c) mine = bal;
                 }
-                reinterpret_cast<uint32_t*>(&s.mask[ms][cb + lane])[warp & 3] = ok ? mine : 0u;
             }
-            if (i > 0 && tid < kEstN) s.base[ms ^ 1][tid] = base_reg;
-            epi_bar();
-            if (tid < kEstN) {
-                uint4 m = s.mask[ms][tid];
-                if (s.qid[cs][tid] == 0xffffffffu) {
+            if (n > 0 && gt < kEstN) G.base[ms ^ 1][gt] = base_reg;
+            epi_bar(group);
+            if (n > 0) write_kept(n - 1, prev_row0);
+            if (gt < kEstN) {
+                uint4 m = G.mask[ms][gt];
+                if (G.qid[cs][gt] == 0xffffffffu || !ok) {
                     m = make_uint4(0u, 0u, 0u, 0u);
-                    s.mask[ms][tid] = m;
+                    G.mask[ms][gt] = m;
                 } else if (RANGES) {  // the rows of the entry's range
-                    const uint32_t r = s.lohi[cs][tid];
+                    const uint32_t r = G.lohi[cs][gt];
                     const int lo = (int)(r & 0xffffu), hi = (int)(r >> 16);
                     auto part = [&](uint32_t x, int k) {
                         const int a0 = min(max(lo - 32 * k, 0), 32), a1 = min(max(hi - 32 * k, 0), 32);
-                        const uint32_t below = a1 >= 32 ? ~0u : (1u << a1) - 1u, skip = a0 >= 32 ? ~0u : (1u << a0) - 1u;
-                        return x & below & ~skip;
+                        const uint32_t below = a1 >= 32 ? ~0u : (1u << a1) - 1u, skip0 = a0 >= 32 ? ~0u : (1u << a0) - 1u;
+                        return x & below & ~skip0;
                     };
                     m = make_uint4(part(m.x, 0), part(m.y, 1), part(m.z, 2), part(m.w, 3));
-                    s.mask[ms][tid] = m;
+                    G.mask[ms][gt] = m;
                 }
-                const uint32_t n = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
-                if (n) base_reg = atomicAdd(a.cnt + s.qid[cs][tid], n);
+                const uint32_t kept = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+                if (kept) base_reg = atomicAdd(a.cnt + G.qid[cs][gt], kept);
+                uint32_t inc = kept;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= o) inc += y;
+                }
+                G.pre[ms][gt] = inc - kept;
+                if (lane == 31) G.wsum[ms][gw] = inc;
             }
-            if (i > 0) write_kept(i - 1, prev_row0);
             prev_row0 = row0;
         }
-        if (items) {
-            epi_bar();
-            if (tid < kEstN) s.base[(items - 1) & 1][tid] = base_reg;
-            epi_bar();
-            write_kept(items - 1, prev_row0);
+        if (n > 0) {
+            epi_bar(group);
+            if (gt < kEstN) G.base[(n - 1) & 1][gt] = base_reg;
+            epi_bar(group);
+            write_kept(n - 1, prev_row0);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (tid == 0 && s.fail) atomicExch(err, 1);
-    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kEstN));
+    if (warp == kMmaWarp)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kAccs * kEstN));
 }
 
 template <bool RANGES, int LT>
 void launch_est(const EstArgs& a, const void* rows, int ld, int* err, cudaStream_t st) {
     const CUtensorMap map = bf16_rows_map(rows, a.n_rows, ld, kEstM);
-    const size_t sm = 1024 + (size_t)kEstStages * 2 * kChunkBytes + sizeof(EstShared) + 16 +
-                      (RANGES ? 0 : sizeof(float) * 2 * kEstN * 2 * a.l);
+    const size_t sm = 1024 + (size_t)est_stages(RANGES) * 2 * kChunkBytes + sizeof(EstShared) + 16 +
+                      (RANGES ? (size_t)kGroups * 2 * kEstN * kEstM : sizeof(float) * kGroups * 2 * kEstN * 2 * a.l);
     auto kern = k_est<RANGES, LT>;
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     kern<<<(unsigned)sm_count(), kEstThreads, sm, st>>>(map, a, ld, (ld + 63) / 64, err);

@@ -104,8 +104,9 @@ struct IndexDev {
     const float* pq_centers;
     const uint32_t* prefix;        // dense prefix counts (nullptr when the rows form or prefix16 is used)
     const uint16_t* prefix16;      // the dense counts in 16 bits, kept when no list exceeds 65535 points
-    const uint16_t* decoded;       // [n x d] the points' PQ approximations in BF16, pool order (nullptr: not kept)
+    const uint16_t* decoded;       // [n x d] the points' PQ approximations in FP16, pool order (nullptr: not kept)
     const float4* decoded_c;       // [n] their constants for the distance estimates (hdg_est.cuh)
+    const uint32_t* decoded_max;   // [3] float bits: the constants' largest |x|^2, |x| and rx
     const uint64_t* prefix_off;    // compressed rows (nullptr when dense)
     const uint64_t* prefix_rows;
 };
@@ -178,7 +179,7 @@ struct hdg_index {
     hdg::IndexDev dev{};
     hdg::DeviceBuffer arena;       // all index arrays
     hdg::DeviceBuffer decoded;     // derived at upload, not stored in the index file: the points'
-                                   // PQ approximations in BF16 and their estimate constants
+                                   // PQ approximations in FP16 and their estimate constants
     hdg::DeviceBuffer map_buf;     // filter interval map
     // query contexts by stream (the last one used serves hdg_debug_fetch)
     std::map<void*, std::unique_ptr<hdg::QueryCtx>> ctxs;

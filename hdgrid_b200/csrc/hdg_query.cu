@@ -23,13 +23,11 @@
 //                exact f32 re-rank and top-k (refine.cu:36-120).
 // There is no dense [q x max_row_len] candidate table and one host round trip per batch
 // (the candidate total and the batch-wide budget).
-#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <functional>
 #include <type_traits>
 
 #include "hdg_device.cuh"
@@ -87,16 +85,15 @@ struct Workspace {
     float* dist;             // [sum of candidates]
     uint32_t* spos;          // [sum of candidates] candidate position of each entry of a compact row
     // the estimate pass of post-filter queries (nullptr: not run)
-    uint32_t* prq;           // [q] 0: every candidate scanned; 1: only the candidates its estimate keeps; 2: scanned
-                             //     in full after all (the threshold turned out too low)
-    float* thr;              // [q] ADC threshold: every candidate at or below it is kept
-    uint32_t* nle;           // [q] kept candidates whose ADC distance is at or below the threshold
+    uint32_t* prq;           // [q] 1: the ADC runs on the candidates that the estimates leave open only
     float4* est_qc;          // [q] constants of the estimate test
-    int round;               // 2: the scan and select of the prq == 2 queries
+    int* est_w;              // [q] steps by which an ADC distance can differ from its bound
+    uint32_t* est_in;        // [q] candidates sure to be selected (at the start of the query's selection)
+    uint32_t* est_row;       // [q] entries of the row before the open candidates
     float* S;                // [q x (C + L)] tensor-core dot products (nullptr: exact path only)
     uint64_t ldS;
     float* qnorm;            // [q] squared query norms
-    void* qbf;               // [q x d] bf16 queries
+    void* qbf;               // [q x d] bf16 queries of the coarse GEMM, then FP16 ones of the estimate pass
     int* gemm_err;           // tensor-core wait expiry flag
     float* feats;            // [q x 48] learned-schedule features
     uint32_t* lq_ps;         // [q] lists to probe predicted by the learned schedule
@@ -128,9 +125,12 @@ __device__ __forceinline__ bool q_prefilter(const Workspace& w, uint64_t qi) {
 // true when query qi's row is compact: the predicate pass lists its survivors (position and
 // pool row), the ADC scan replaces each pool row by the survivor's distance
 __device__ __forceinline__ bool compacts(const Workspace& w, uint64_t qi) { return w.surv_list && q_prefilter(w, qi); }
-// true when query qi's row holds only the candidates that the estimate pass kept (positions and
-// pool rows, as a compacting query's survivors)
+// true when the ADC of query qi runs only on the candidates that its estimates leave open (positions
+// and pool rows, as a compacting query's survivors, est_row entries into the row)
 __device__ __forceinline__ bool pruned(const Workspace& w, uint64_t qi) { return w.prq && w.prq[qi] == 1; }
+__device__ __forceinline__ uint64_t row_of(const Workspace& w, uint64_t qi) {
+    return w.qoff[qi] + (pruned(w, qi) ? w.est_row[qi] : 0u);
+}
 // Candidate budget n_cand of query qi given the batch's beta and max_row_len: the query's k for
 // the reference pre-filter schedule (exps0 <= 1), exps0 * k for the single-dim schedule and the
 // predicate-first schedule, and the reference's min(exps0 * k * beta, max_row_len) for the
@@ -1469,7 +1469,6 @@ __global__ void __launch_bounds__(1024) k_scan_plan(uint64_t q, Workspace w) {
     const uint64_t b = t * per, e = min(q, b + per);
     const uint32_t chunk = scan_chunk(w);
     auto n_items = [&](uint64_t i) {
-        if (w.round == 2) return w.prq[i] == 2 ? (w.qstat[i * 4] + chunk - 1) / chunk : 0u;
         uint32_t c = compacts(w, i) || pruned(w, i) ? w.cand_count[i] : w.qstat[i * 4];
         // a compact row that its budget takes whole needs no ADC distance (the select takes
         // every survivor and the re-rank orders them), unless the distances are the output
@@ -1479,7 +1478,7 @@ __global__ void __launch_bounds__(1024) k_scan_plan(uint64_t q, Workspace w) {
     };
     // such a row's survivors all count as passed (the ADC scan counts them for the others)
     for (uint64_t i = b; i < e; i++)
-        if (w.round != 2 && compacts(w, i) && w.mode != kPre && w.cand_count[i] <= w.qbud[i]) w.nfin[i] = w.cand_count[i];
+        if (compacts(w, i) && w.mode != kPre && w.cand_count[i] <= w.qbud[i]) w.nfin[i] = w.cand_count[i];
     unsigned long long items = 0;
     for (uint64_t i = b; i < e; i++) items += n_items(i);
     unsigned long long tot = 0;
@@ -1526,8 +1525,7 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
         const int item = s.item;
         if (item >= (int)n_items) break;
         const int qq = s.query;
-        const bool prn = pruned(w, qq), compact = compacts(w, qq) || prn;
-        const float thr = prn ? w.thr[qq] : 0.f;
+        const bool compact = compacts(w, qq) || pruned(w, qq);
         const uint32_t total = compact ? w.cand_count[qq] : w.qstat[(uint64_t)qq * 4];
         const uint32_t e0 = (uint32_t)(item - w.item_off[qq]) * chunk;
         if (e0 >= total) {  // a query cut by the distance capacity
@@ -1566,10 +1564,10 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
             cur = qq;
         }
         const uint32_t e1 = min(total, e0 + chunk);
-        float* dst = w.dist + w.qoff[qq];
+        float* dst = w.dist + row_of(w, qq);
         const uint32_t* srow = reinterpret_cast<const uint32_t*>(dst);  // compact: the survivors' pool rows
-        const uint32_t* sp = w.spos + w.qoff[qq];
-        uint32_t kmin = 0xffffffffu, kmax = 0u, nf = 0, nl = 0;
+        const uint32_t* sp = w.spos + row_of(w, qq);
+        uint32_t kmin = 0xffffffffu, kmax = 0u, nf = 0;
         // each warp takes a contiguous span of the item (a multiple of 32 * CPT entries, so in
         // a full row position mod 32 stays the lane), so a lane's walk to its candidate's range
         // crosses few range boundaries per step
@@ -1653,7 +1651,6 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
                     kmin = min(kmin, key);
                     kmax = max(kmax, key);
                     nf++;
-                    nl += sum[u] <= thr ? 1u : 0u;
                 }
                 dst[e] = sum[u];
             }
@@ -1668,10 +1665,6 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
             atomicMin(&w.mm[2 * qq], kmin);
             atomicMax(&w.mm[2 * qq + 1], kmax);
             atomicAdd(&w.nfin[qq], nf);
-        }
-        if (prn) {
-            nl = __reduce_add_sync(0xffffffffu, nl);
-            if (lane == 0 && nl) atomicAdd(&w.nle[qq], nl);
         }
         __syncthreads();
     }
@@ -1845,7 +1838,8 @@ __global__ void __launch_bounds__(NT) k_select(IndexDev D, int Ps, int Kcap, int
     uint64_t* s_sel = s_bbuf + kBCap;                                        // [sel_cap] (sorted mode)
     const int sel_cap = sorted_out ? (int)next_pow2_dev((uint32_t)max(Kcap, 2)) : 0;
     // this query's budget: its k for the sorted pre-filter output, else the candidate budget
-    const int K = sorted_out ? (int)q_k(w, blockIdx.x) : (int)q_budget(w, blockIdx.x);
+    const int K = (sorted_out ? (int)q_k(w, blockIdx.x) : (int)q_budget(w, blockIdx.x)) -
+                  (pruned(w, blockIdx.x) ? (int)w.est_in[blockIdx.x] : 0);
     uint32_t* s_pre = reinterpret_cast<uint32_t*>(s_sel + sel_cap);        // [Ps + 1]
     uint32_t* s_start = s_pre + Ps + 1;                                      // [Ps]
     __shared__ uint32_t s_warp[32];
@@ -1857,25 +1851,14 @@ __global__ void __launch_bounds__(NT) k_select(IndexDev D, int Ps, int Kcap, int
     // A predicate-first query of the predicate pass has a compact row: its survivors' distances
     // in arrival order with their candidate positions beside them (cand_count entries); any
     // other query's row holds one distance per candidate position.
-    // A query of the estimate pass has a compact row too: the candidates its estimates kept.  They
-    // hold its K smallest if K of them lie at or below the threshold; else (or when the pass
-    // reports an expired wait) the query is marked, scanned in full and selected in round 2.
-    if (w.round == 2 && w.prq[qi] != 2) return;
+    // A query of the estimate pass has a compact row too: the candidates that its estimates leave
+    // open; the sure ones are selected already.
     const bool prn = pruned(w, qi), compact = compacts(w, qi) || prn;
-    if (prn && ((uint32_t)K > w.nle[qi] || *w.gemm_err != 0)) {
-        __syncthreads();  // every thread has read prq
-        if (t == 0) {
-            w.prq[qi] = 2;
-            w.nfin[qi] = 0;
-            w.mm[2 * qi] = 0xffffffffu;
-            w.mm[2 * qi + 1] = 0u;
-        }
-        return;
-    }
+    const uint32_t sure = prn ? w.est_in[qi] : 0u;
     if (!sorted_out && takes_row(w, qi)) return;  // the selection is the row (cand_count entries)
     const uint32_t total = compact ? w.cand_count[qi] : w.qstat[qi * 4];
-    const float* dist = w.dist + w.qoff[qi];
-    const uint32_t* prow = compact ? w.spos + w.qoff[qi] : nullptr;
+    const float* dist = w.dist + row_of(w, qi);
+    const uint32_t* prow = compact ? w.spos + row_of(w, qi) : nullptr;
     {
         const uint32_t* rpre = w.range_pre + qi * (Ps + 1);
         for (int i = t; i <= Ps; i += blockDim.x) s_pre[i] = rpre[i];
@@ -1885,7 +1868,7 @@ __global__ void __launch_bounds__(NT) k_select(IndexDev D, int Ps, int Kcap, int
     __syncthreads();
     const uint32_t nfin = w.nfin[qi];
     const uint32_t need0 = min((uint32_t)K, nfin);
-    uint32_t* sel_dst = sorted_out ? nullptr : w.cand_pool + w.soff[qi];
+    uint32_t* sel_dst = sorted_out ? nullptr : w.cand_pool + w.soff[qi] + sure;
     // candidate position of row entry e (e < total)
     auto posof = [&](uint32_t e) { return prow ? prow[e] : e; };
     // Selected entries are recorded by candidate position; positions become pool slots once the
@@ -2116,9 +2099,8 @@ __global__ void __launch_bounds__(NT) k_select(IndexDev D, int Ps, int Kcap, int
     __syncthreads();
     const uint32_t nsel = s_out;
     if (!sorted_out) {
-        uint32_t* pool = w.cand_pool + w.soff[qi];
-        for (uint32_t i = t; i < nsel; i += blockDim.x) pool[i] = pos_to_pool(s_pre, s_start, Ps, pool[i]);
-        if (t == 0) w.cand_count[qi] = nsel;
+        for (uint32_t i = t; i < nsel; i += blockDim.x) sel_dst[i] = pos_to_pool(s_pre, s_start, Ps, sel_dst[i]);
+        if (t == 0) w.cand_count[qi] = sure + nsel;
         return;
     }
     const int n2 = (int)next_pow2_dev((uint32_t)max((int)nsel, 2));
@@ -2473,17 +2455,20 @@ __global__ void __launch_bounds__(kThreads, 5) k_refine(IndexDev D, const float*
 // ------------------------------------------------------------------------------------
 // The post-filter schedule needs the n_cand smallest ADC distances of a query's candidates, a few
 // percent of them.  An ADC distance is the distance to the candidate's PQ approximation, so a
-// tensor-core product of queries and approximations bounds it from below (hdg_est.cuh):
+// tensor-core product of queries and approximations bounds it from both sides (hdg_est.cuh):
 //   k_est_thr    a threshold per query from a strided sample of its candidates' ADC distances: a
 //                sample rank past n_cand's share by four standard deviations;
 //   k_est_count / k_est_scan / k_est_fill   the (query, range) entries of every tile of kEstM pool
 //                rows, so that a tile meets only the queries whose ranges touch it;
-//   k_est        every candidate whose bound is not above the threshold goes to its query's row;
-//   k_scan_fast  the exact ADC of those (the compact-row path);
-//   k_select     if n_cand of them lie at or below the threshold, the n_cand smallest are among
-//                them: the selection is the full scan's.  A query whose threshold was too low is
-//                scanned in full (round 2).
-// 10,000 queries x 227,000 candidates x 32 subspaces (n_cand 9,384): EST_FIG.
+//   k_est        every candidate whose lower bound is not above the threshold goes to its query's
+//                row, with the bound's depth below the threshold in steps;
+//   k_est_pick   with v the n_cand-th smallest bound and w the most an ADC distance can exceed its
+//                bound by: a candidate w and more below v is among the n_cand smallest, one more
+//                than w above v is not; those in between are left open.  When v + w passes the
+//                threshold (candidates outside the row could matter) the query is scanned in full;
+//   k_scan_fast / k_select   the exact ADC of the open candidates and the smallest of them.
+// The selection is the full scan's.  10,000 queries x 227,000 candidates x 32 subspaces (n_cand
+// 9,384), estimate to select: 20.4 ms in full (a full scan, a select over every distance), EST_FIG.
 constexpr int kThrThreads = 512;
 constexpr uint32_t kThrMax = 4096;  // sampled candidates at most
 constexpr int kThrBins = 2048;
@@ -2498,30 +2483,28 @@ __global__ void __launch_bounds__(kThrThreads) k_est_thr(IndexDev D, int R, cons
     __shared__ unsigned long long s_scan[32];
     __shared__ float s_red[3];
     __shared__ uint32_t s_mm[2];
-    __shared__ int s_bin;
+    __shared__ int s_bin, s_bin_lo;
     const uint64_t qi = blockIdx.x;
     const int t = threadIdx.x, lane = t & 31;
     const uint32_t N = w.qstat[qi * 4];
     const uint32_t K = w.qbud[qi];
     // sample size: the cost of a sampled candidate against the extra candidates that a coarser
     // threshold lets through, about 2.5 (5 sqrt(K N))^(2/3) of either
-    uint32_t ms = 0, rank = 0;
+    uint32_t ms = 0, rank = 0, rank_lo = 1;
     if (N >= 4096 && (uint64_t)K * 3 <= N) {
         ms = (uint32_t)powf(5.f * sqrtf((float)K * (float)N), 2.f / 3.f);
         ms = min(kThrMax, max(512u, ms));
         const float r = (float)K * (float)ms / (float)N;
         rank = (uint32_t)(r + 4.f * sqrtf(r) + 4.f);
+        rank_lo = (uint32_t)fmaxf(1.f, r - 5.f * sqrtf(r) - 2.f);
     }
-    if (t == 0) {
-        w.prq[qi] = 0;
-        w.nle[qi] = 0;
-    }
+    if (t == 0) w.prq[qi] = 0;
     if (ms == 0 || rank >= ms) return;  // block-uniform
     if (t == 0) {
         s_mm[0] = 0xffffffffu;
         s_mm[1] = 0u;
         s_red[0] = s_red[1] = s_red[2] = 0.f;
-        s_bin = -1;
+        s_bin = s_bin_lo = -1;
     }
     if (w.lut16) {
         const uint2* src = reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(w.lut) + qi * G * kCodes * 32);
@@ -2544,7 +2527,9 @@ __global__ void __launch_bounds__(kThrThreads) k_est_thr(IndexDev D, int R, cons
     {
         float qn = 0.f, q2 = 0.f, rq = 0.f;
         for (int i = t; i < (int)D.d; i += kThrThreads) {
-            const float v = queries[qi * D.d + i], h = __bfloat162float(__float2bfloat16_rn(v)), e = v - h;
+            const __half hv = __float2half_rn(queries[qi * D.d + i]);
+            const float v = queries[qi * D.d + i], h = __half2float(hv), e = v - h;
+            reinterpret_cast<__half*>(w.qbf)[qi * D.d + i] = hv;  // (the coarse GEMM's BF16 copy is no longer needed)
             qn = fmaf(v, v, qn);
             q2 = fmaf(h, h, q2);
             rq = fmaf(e, e, rq);
@@ -2619,24 +2604,151 @@ __global__ void __launch_bounds__(kThrThreads) k_est_thr(IndexDev D, int R, cons
     }
     unsigned long long tot = 0;
     uint32_t run = (uint32_t)block_inclusive_sum(sum, s_scan, &tot) - sum;
-    if (run < rank && rank <= run + sum) {
-        int i = 0;
-        while (i < kPer - 1 && run + c[i] < rank) run += c[i++];
-        s_bin = t * kPer + i;
-    }
+    auto bin_of = [&](uint32_t r, int* bin) {
+        if (run < r && r <= run + sum) {
+            uint32_t x = run;
+            int i = 0;
+            while (i < kPer - 1 && x + c[i] < r) x += c[i++];
+            *bin = t * kPer + i;
+        }
+    };
+    bin_of(rank, &s_bin);
+    bin_of(rank_lo, &s_bin_lo);
     __syncthreads();
-    if (t == 0 && s_bin >= 0) {
+    if (t == 0 && s_bin >= 0 && s_bin_lo >= 0) {
         const float T = s_bin == kThrBins - 1 || !(inv > 0.f) ? hi : lo + (float)(s_bin + 1) / inv;
         const float qn = s_red[0], qh = sqrtf(s_red[1]) * (1.f + kEstSlack), rq = sqrtf(s_red[2]) * (1.f + kEstSlack);
-        // the bound holds for the distance itself: an ADC distance at or below T may be off by its
-        // own rounding -- FP32 sums, and with FP16 tables each entry by 2^-11 (or 2^-25)
-        const float Tb = w.lut16 ? T * (1.f + 1.1e-3f) + 1e-7f * (float)D.M : T * (1.f + kEstSlack);
-        if (T < INFINITY) {
-            w.thr[qi] = T;
-            w.est_qc[qi] = make_float4(2.f * (rq + kEstAcc * (float)D.d * sqrtf(qn)) * (1.f + kEstSlack), 2.f * qh,
-                                       qn * (1.f - kEstSlack) - Tb, 0.f);
+        // the bounds hold for the distance itself: an ADC distance differs from it by its own
+        // rounding -- FP32 sums, and with FP16 tables each entry by 2^-11 (or 2^-25)
+        const float xm2 = __uint_as_float(D.decoded_max[0]), xm = __uint_as_float(D.decoded_max[1]),
+                    rm = __uint_as_float(D.decoded_max[2]);
+        const float adc = w.lut16 ? 1.1e-3f * T + 1e-7f * (float)D.M : kEstSlack * T;
+        const float ca = 2.f * (rq + kEstAcc * (float)D.d * sqrtf(qn)) * (1.f + kEstSlack), cb = 2.f * qh;
+        const float wide = 2.f * (ca * xm + cb * rm) + 4.f * kEstSlack * (qn + xm2) + 2.f * adc;
+        // the steps run from the sample rank five standard deviations below n_cand's share (the
+        // n_cand-th bound lies there or above, but for a rare sample) less twice the bounds' width;
+        // rows are kept up to T, the width and the steps' rounding past it, so that the n_cand-th
+        // bound lies that much below the threshold
+        const float Tl = (inv > 0.f ? lo + (float)s_bin_lo / inv : lo) - 2.f * wide;
+        const float Tb = Tl + (T + wide - Tl) * (253.f / 246.f), z = qn * (1.f - kEstSlack) - Tb;
+        const float steps = 253.f / (Tb - Tl);
+        const float ws = wide * steps + 4.f;    // and the steps' own rounding, on both sides
+        // (a NaN or an extreme norm anywhere in the index fails these tests; FP16 entries of a distance
+        // at or below T must not overflow)
+        if (T < INFINITY && Tb > Tl && ws < 120.f && fabsf(z) * steps < 1e6f && qn + xm2 < 1e30f &&
+            (!w.lut16 || T < 6e4f)) {
+            w.est_qc[qi] = make_float4(ca, cb, z, steps);
+            w.est_w[qi] = (int)ws + 1;
             w.prq[qi] = 1;
         }
+    }
+}
+
+// The sure and the open candidates of each query of the pass: the kept candidates' steps counted
+// per value, the value that holds the n_cand-th smallest bound, then one pass that appends the sure
+// ones to the selection and the open ones -- position and pool row -- behind the row's entries.
+constexpr int kPickThreads = 256;
+__global__ void __launch_bounds__(kPickThreads) k_est_pick(int R, Workspace w) {
+    extern __shared__ uint32_t s_pre[];  // [R + 1], then [R] range starts
+    uint32_t* s_start = s_pre + R + 1;
+    __shared__ uint32_t s_hist[kPickThreads / 32][256];
+    __shared__ int s_v;
+    __shared__ uint32_t s_in, s_open, s_cnt[2];
+    const uint64_t qi = blockIdx.x;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (w.prq[qi] != 1) return;
+    const uint32_t N = w.qstat[qi * 4], K = w.qbud[qi], ne = w.cand_count[qi];
+    const uint64_t row = w.qoff[qi];
+    const unsigned char* st = reinterpret_cast<const unsigned char*>(w.dist + row);
+    const bool err = *w.gemm_err != 0;
+    for (int i = lane; i < 256; i += 32) s_hist[warp][i] = 0;
+    if (t == 0) {
+        s_v = 0;
+        s_in = s_open = s_cnt[0] = s_cnt[1] = 0;
+    }
+    __syncthreads();
+    const int wd = w.est_w[qi];
+    // (rows start at any 4-byte boundary: words of four steps)
+    const uint32_t* st4 = reinterpret_cast<const uint32_t*>(st);
+    for (uint32_t i = t; 4 * i < ne; i += kPickThreads) {
+        const uint32_t x = __ldg(st4 + i);
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++)
+            if (4 * i + u < ne) atomicAdd(&s_hist[warp][(x >> (8 * u)) & 255u], 1u);
+    }
+    __syncthreads();
+    uint32_t c = 0;
+    {  // thread t holds value 255 - t: the bounds from the smallest on
+        for (int k = 0; k < kPickThreads / 32; k++) c += s_hist[k][255 - t];
+        __syncthreads();
+        s_hist[0][t] = c;
+        __syncthreads();
+        if (t < 32) {
+            uint32_t sum = 0, x[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) sum += x[k] = s_hist[0][8 * t + k];
+            uint32_t inc = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (t >= o) inc += y;
+            }
+            uint32_t run = inc - sum;
+            if (run < K && K <= inc) {
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    if (run < K && K <= run + x[k]) s_v = 255 - (8 * t + k);
+                    run += x[k];
+                }
+            }
+        }
+        __syncthreads();
+    }
+    const int v = s_v, lo = v - wd, hi = v + wd;  // open: steps lo .. hi (255 holds every smaller bound)
+    {
+        const int val = 255 - t;
+        const uint32_t in = val > hi ? c : 0u, op = val >= lo && val <= hi ? c : 0u;
+        if (in) atomicAdd(&s_in, in);
+        if (op) atomicAdd(&s_open, op);
+    }
+    __syncthreads();
+    // the open candidates' entries go behind the row's (position, step) entries
+    const uint32_t n_open = s_open, n_in = s_in;
+    if (err || v == 0 || lo < 1 || ne + n_open > N) {
+        __syncthreads();
+        if (t == 0) {
+            w.prq[qi] = 0;
+            w.cand_count[qi] = 0;
+        }
+        return;
+    }
+    for (int i = t; i <= R; i += kPickThreads) s_pre[i] = w.range_pre[qi * (R + 1) + i];
+    for (int i = t; i < R; i += kPickThreads) s_start[i] = w.range_start[qi * R + i];
+    __syncthreads();
+    uint32_t* prow = w.spos + row;
+    uint32_t* open_row = reinterpret_cast<uint32_t*>(w.dist + row) + ne;
+    uint32_t* sel = w.cand_pool + w.soff[qi];
+    for (uint32_t i0 = 0; 4 * i0 < ne; i0 += kPickThreads) {  // block-uniform bound
+        const uint32_t i = i0 + t;
+        const uint32_t x = 4 * i < ne ? __ldg(st4 + i) : 0u;
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+            const uint32_t e = 4 * i + u;
+            const int val = e < ne ? (int)((x >> (8 * u)) & 255u) : 0;  // (steps are at least 1)
+            const bool in = val > hi, op = val >= lo && val <= hi;
+            const uint32_t p = in || op ? prow[e] : 0u;
+            const uint32_t a = warp_reserve(in, &s_cnt[0]), b = warp_reserve(op, &s_cnt[1]);
+            if (in) sel[a] = p;
+            if (op) prow[ne + b] = p;
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = t; i < n_in; i += kPickThreads) sel[i] = pos_to_pool(s_pre, s_start, R, sel[i]);
+    for (uint32_t i = t; i < n_open; i += kPickThreads) open_row[i] = pos_to_pool(s_pre, s_start, R, prow[ne + i]);
+    if (t == 0) {
+        w.est_in[qi] = n_in;
+        w.est_row[qi] = ne;
+        w.cand_count[qi] = n_open;
     }
 }
 
@@ -3107,7 +3219,8 @@ static void estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const Quer
         off += align_up(bytes, 256);
         return o;
     };
-    const size_t o_prq = take(q * 4), o_thr = take(q * 4), o_nle = take(q * 4), o_qc = take(q * sizeof(float4));
+    const size_t o_prq = take(q * 4), o_w = take(q * 4), o_in = take(q * 4), o_row = take(q * 4),
+                 o_qc = take(q * sizeof(float4));
     const size_t o_diff = take((tiles + 1) * 4ull), o_eo = take((tiles + 1) * 4ull), o_no = take((tiles + 1) * 4ull),
                  o_cur = take((tiles + 1) * 4ull), o_ent = take(std::max<uint64_t>(entries, 1) * sizeof(uint4));
     if (cx.est_buf.bytes < off) {
@@ -3116,8 +3229,9 @@ static void estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const Quer
     }
     char* b = static_cast<char*>(cx.est_buf.ptr);
     w.prq = reinterpret_cast<uint32_t*>(b + o_prq);
-    w.thr = reinterpret_cast<float*>(b + o_thr);
-    w.nle = reinterpret_cast<uint32_t*>(b + o_nle);
+    w.est_w = reinterpret_cast<int*>(b + o_w);
+    w.est_in = reinterpret_cast<uint32_t*>(b + o_in);
+    w.est_row = reinterpret_cast<uint32_t*>(b + o_row);
     w.est_qc = reinterpret_cast<float4*>(b + o_qc);
     int* diff = reinterpret_cast<int*>(b + o_diff);
     EstArgs a{};
@@ -3135,7 +3249,7 @@ static void estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const Quer
     a.nt_off = nt_off;
     a.ent = ent;
     a.qoff = w.qoff;
-    a.drow = reinterpret_cast<uint32_t*>(w.dist);
+    a.drow = w.dist;
     a.prow = w.spos;
     a.cnt = w.cand_count;
     CK(cudaMemsetAsync(diff, 0, (tiles + 1) * 4ull, st));
@@ -3156,6 +3270,8 @@ static void estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const Quer
     k_est_fill<<<blocks, 256, 0, st>>>(q, R, w, cursor, ent);
     CK_LAUNCH();
     est_ranges(a, D.decoded, (int)D.d, w.gemm_err, st);
+    k_est_pick<<<(unsigned)q, kPickThreads, sizeof(uint32_t) * (2 * R + 1), st>>>(R, w);
+    CK_LAUNCH();
     k_scan_plan<<<1, 1024, 0, st>>>(q, w);
     CK_LAUNCH();
 }
@@ -3206,7 +3322,6 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     w.exps0 = (uint32_t)std::min<uint64_t>(exps0, 1u << 20);
     w.chunk = (uint32_t)P.scan_chunk;
     w.scan_items = 8 * (uint32_t)sm_count();
-    w.round = 1;
     w.cap = sync_sizing ? ~0ull : cx.dist_buf.bytes / 4;
     if (sync_sizing) w.sel_cap = ~0ull;  // sized after k_batch
     const FilterDev f = filter_dev(idx);
@@ -3300,7 +3415,6 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     // candidate ranges per query: one per probed list, or n_split per list when is_split
     const int R = Ps * w.nsplit;
     const size_t sm_tab = sizeof(uint32_t) * (2 * R + 1);
-    std::function<void(const Workspace&)> scan;  // the ADC scan as launched
     if (!sync_sizing || lazy || sc[3] > 0) {
         if (fast && (pre || w.qsched)) {
             // the predicate pass of the predicate-first queries, then the ADC items that
@@ -3342,12 +3456,8 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
         const bool prune = sync_sizing && !lazy && mode == kPost && !w.qsched && fast && D.decoded && sc[0] >= kEstMinCands &&
                            sc[0] / q >= kEstMinRow && cx.pinned[9] < (1ull << 32);
         if (prune) {
-            if (!use_gemm) {
-                rows_to_bf16(c.queries, q, (int)D.d, w.qbf, w.qnorm, st);
-                launches++;
-            }
             estimate_pass(idx, cx, w, c, R, G, cx.pinned[9], st);
-            launches += 6;
+            launches += 7;
             tm.mark("estimate");
         }
         if (fast) {
@@ -3358,8 +3468,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             auto launch = [&](auto kern, int nt) {
                 CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
                 const int blocks = sm_count() * occupancy_blocks(kern, nt, sm);
-                scan = [=](const Workspace& ww) { kern<<<blocks, nt, sm, st>>>(D, R, q, ww); };
-                scan(w);
+                kern<<<blocks, nt, sm, st>>>(D, R, q, w);
             };
             if (G == 1) {
                 if (cpt == 1) launch(k_scan_fast<1, 512, 1>, 512);
@@ -3392,17 +3501,6 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     auto launch_sel = [&](auto kern, int nt) {
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_sel));
         kern<<<(unsigned)q, nt, sm_sel, st>>>(D, R, (int)k, sorted_out, w, c.dist, c.ids, (int)k);
-        if (!w.prq) return;
-        // queries whose threshold was too low (usually none): scanned and selected in full
-        CK_LAUNCH();
-        w.round = 2;
-        k_scan_plan<<<1, 1024, 0, st>>>(q, w);
-        CK_LAUNCH();
-        scan(w);
-        CK_LAUNCH();
-        kern<<<(unsigned)q, nt, sm_sel, st>>>(D, R, (int)k, sorted_out, w, c.dist, c.ids, (int)k);
-        w.round = 1;
-        launches += 3;
     };
     if (q <= (uint64_t)sm_count()) launch_sel(k_select<kSelThreadsFew, 8>, kSelThreadsFew);
     else launch_sel(k_select<kSelThreads, 4>, kSelThreads);
