@@ -1508,17 +1508,14 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
     const uint32_t n_items = w.item_off[q], chunk = scan_chunk(w);
     int cur = -1;
     for (;;) {
-        if (t == 0) {
-            const int item = (int)atomicAdd(w.counter, 1u);
-            s.item = item;
-            if (item < (int)n_items) {  // largest query with item_off <= item
-                int lo = 0, hi = (int)q - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (w.item_off[mid] <= (uint32_t)item) lo = mid;
-                    else hi = mid - 1;
-                }
-                s.query = lo;
+        if (t < 32) {  // the item's query: the last one with item_off <= item, by 32-way rounds
+            int item = 0;
+            if (t == 0) item = (int)atomicAdd(w.counter, 1u);
+            item = __shfl_sync(0xffffffffu, item, 0);
+            const int qf = item < (int)n_items ? warp_find_le(w.item_off, (int)q, (uint32_t)item) : 0;
+            if (t == 0) {
+                s.item = item;
+                s.query = qf;
             }
         }
         __syncthreads();
@@ -1691,17 +1688,14 @@ __global__ void __launch_bounds__(512) k_scan_generic(IndexDev D, int G, int Ps,
     };
     int cur = -1;
     for (;;) {
-        if (t == 0) {
-            const int item = (int)atomicAdd(w.counter, 1u);
-            s.item = item;
-            if (item < (int)n_items) {
-                int lo = 0, hi = (int)q - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (w.item_off[mid] <= (uint32_t)item) lo = mid;
-                    else hi = mid - 1;
-                }
-                s.query = lo;
+        if (t < 32) {  // the item's query: the last one with item_off <= item, by 32-way rounds
+            int item = 0;
+            if (t == 0) item = (int)atomicAdd(w.counter, 1u);
+            item = __shfl_sync(0xffffffffu, item, 0);
+            const int qf = item < (int)n_items ? warp_find_le(w.item_off, (int)q, (uint32_t)item) : 0;
+            if (t == 0) {
+                s.item = item;
+                s.query = qf;
             }
         }
         __syncthreads();
@@ -2218,17 +2212,14 @@ __global__ void __launch_bounds__(kThreads, 5) k_refine(IndexDev D, const float*
     const uint32_t n_items = w.ritem_off[q];
     int cur = -1;
     for (;;) {
-        if (t == 0) {
-            const int item = (int)atomicAdd(&w.counter[1], 1u);
-            s_item = item;
-            if (item < (int)n_items) {  // largest query with ritem_off <= item
-                int lo = 0, hi = (int)q - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (w.ritem_off[mid] <= (uint32_t)item) lo = mid;
-                    else hi = mid - 1;
-                }
-                s_qi = lo;
+        if (t < 32) {  // the item's query: the last one with ritem_off <= item, by 32-way rounds
+            int item = 0;
+            if (t == 0) item = (int)atomicAdd(&w.counter[1], 1u);
+            item = __shfl_sync(0xffffffffu, item, 0);
+            const int qf = item < (int)n_items ? warp_find_le(w.ritem_off, (int)q, (uint32_t)item) : 0;
+            if (t == 0) {
+                s_item = item;
+                s_qi = qf;
             }
         }
         __syncthreads();
