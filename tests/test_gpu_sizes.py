@@ -248,3 +248,38 @@ def test_estimate_pass_threshold_too_low(cuda):
     idx.query(hg.query_input_t(b, q, ql), hg.query_output_t(*out[0]))
     nfin = np.frombuffer(idx.debug_fetch("nfin").tobytes(), np.uint32)[:nq]
     assert np.all(nfin == n), nfin
+
+
+# the tensor-core path: one and several query tiles, row tiles with remainders, K with a remainder
+# chunk, label dims of both forms, samples without k passing rows, more passing rows than a list holds
+@pytest.mark.parametrize("q,k,n,d,l,kind", [
+    (64, 10, 32768, 128, 4, "mixed"), (130, 100, 70001, 96, 4, "mixed"), (257, 256, 40000, 100, 2, "mixed"),
+    (65, 1, 50000, 33, 8, "mixed"), (100, 100, 33000, 200, 1, "rare"), (70, 100, 60000, 16, 4, "same"),
+    (64, 50, 40000, 64, 1, "sorted")])
+def test_bruteforce_tensor_path(cuda, q, k, n, d, l, kind):
+    import torch
+    import hdgrid_b200 as hg
+    rng = np.random.default_rng(q + n)
+    base = rng.standard_normal((n, d), dtype=np.float32)
+    qs = rng.standard_normal((q, d), dtype=np.float32)
+    if kind == "same":  # every row at one distance: every bound ties, ids decide
+        base[:] = base[0]
+    if kind == "sorted":  # the near rows lie together: a strided sample sees few of them
+        base[:20000] *= np.float32(0.01)
+        qs *= np.float32(0.01)
+    lab = rng.integers(0, 1000, (n, l)).astype(np.float32)
+    lo = np.where(rng.random((q, l)) < 0.6, 0, rng.integers(0, 1000, (q, l))).astype(np.float32)
+    hi = np.where(rng.random((q, l)) < 0.6, 1000, lo + rng.integers(0, 300, (q, l))).astype(np.float32)
+    if kind == "rare":
+        hi = lo + 1
+    box = np.stack([lo, hi], axis=2).reshape(q, 2 * l).copy()
+    t = [torch.from_numpy(x).to(cuda) for x in (base, lab, qs, box)]
+    dist = torch.full((q, k), -1.0, device=cuda)
+    ids = torch.full((q, k), 7, dtype=torch.int64, device=cuda)
+    hg.bruteforce_knn(*t, k, dist, ids)
+    # in groups below the batch rule: the direct path, the same arithmetic and order
+    d2, i2 = torch.empty_like(dist), torch.empty_like(ids)
+    for a in range(0, q, 30):
+        b = min(q, a + 30)
+        hg.bruteforce_knn(t[0], t[1], t[2][a:b].contiguous(), t[3][a:b].contiguous(), k, d2[a:b], i2[a:b])
+    assert torch.equal(ids, i2) and torch.equal(dist, d2)
