@@ -10,13 +10,15 @@
 //
 // Epilogue of an item: thread = row, loop over columns (queries), two at a time in packed FP32
 // FMAs against the queries' constants, broadcast from shared memory; a ballot per column and warp
-// gives the column's 128-bit mask.  Two threads per column then reserve the kept rows' slots with
-// one atomic, whose latency runs under the group's next item, after whose masks they walk the
-// mask's bits and write the kept rows.
-// Bound: the epilogue's issue slots (about 7 instructions per column and warp, and the writes).
-// 145,000 items of K = 128 (10,000 queries x 227,000 candidates): 6.6 ms with one epilogue group
-// and a warp per column writing its kept rows (15,000 warp instructions an item, half of them for
-// the writes, 35 % issue), K_EST_MS as it stands.  Every wait is bounded: on expiry the kernel sets
+// gives the column's 128-bit mask.  One thread per column then reserves the kept rows' slots with
+// one atomic, whose latency runs under the group's next item, after whose masks the group writes
+// the kept rows, shared out evenly over its threads (a prefix over the columns, the n-th set bit).
+// Bound: the epilogue's issue slots, 12,700 warp instructions per item at about 2 per clock.
+// 154,000 items of K = 128 (10,000 queries x 227,000 candidates): 6.6 ms with one epilogue group
+// and a warp per column writing its kept rows (15,000 instructions, 35 % issue), 4.1 ms with two
+// groups and the even sharing, 5.0 ms with the steps as well.  A thread per column walking its mask
+// took 11.4 ms (64-deep loops where a query is near); TMA gather4 instead of cp.async left this
+// case alone and took 0.9 ms more at K = 384.  Every wait is bounded: on expiry the kernel sets
 // *err, lets its copies land, frees TMEM and returns.
 #include <cuda.h>
 

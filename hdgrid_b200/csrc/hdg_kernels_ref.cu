@@ -412,7 +412,8 @@ void recover_filters_noalloc(const FilterDev& f0, const float* host_map, const f
 // Bound: with many queries the shared-memory reads of the passing rows (16 bytes per pair and four
 // dimensions), with few the read of the base set.
 // One block per 32 queries that computed every pair and tested the labels afterwards took 352 ms
-// on 1,000 queries x 1 M x 128 (32 blocks, 10 % of the pairs pass); this takes BF_MS.
+// on 1,000 queries x 1 M x 128 (32 blocks, 10 % of the pairs pass); this takes 19.1 ms there and
+// 0.31 ms for 8 queries.  Large batches go through bruteforce_est instead.
 constexpr int kBfThreads = 512, kBfWarps = kBfThreads / 32;
 
 __device__ void warp_bitonic_sort(uint64_t* keys, int n) {
@@ -712,8 +713,9 @@ __global__ void __launch_bounds__(256) k_bf_merge(const uint64_t* __restrict__ p
 // the labels leave (about kBfRatio * k per query) are computed exactly, in the same FMA chain as
 // k_bruteforce; the last level is the whole set.  A query with more rows left than its list holds
 // goes through k_bf_full.
-// 1,000 queries x 1 M x 128: 19.1 ms with k_bruteforce, BF_EST_MS this way.
-constexpr uint64_t kBfEstQueries = 64, kBfEstRows = 32768;
+// 1,000 queries x 1 M x 128: 19.1 ms with k_bruteforce, 4.3 ms this way (1.9 ms of it k_est, 0.9
+// k_bf_exact).
+constexpr uint64_t kBfEstQueries = 32, kBfEstPairs = 12000000;
 constexpr uint64_t kBfRatio = 16;
 constexpr uint64_t kBfRowsMax = 1ull << 18;  // rows converted at a time (64 MB at 128 dims)
 
@@ -970,8 +972,10 @@ void bruteforce_knn(const float* data, uint64_t n, uint32_t d, const float* labe
     HDG_REQUIRE(l >= 1 && l <= (uint32_t)kMaxDims && d >= 1, HDG_ERR_INVALID_ARG, "bad dims");
     HDG_REQUIRE(n < (1ull << 32), HDG_ERR_INVALID_ARG, "n must be < 2^32");
     if (!q) return;
-    // enough queries to share a pass over the base set, and a base set worth it: BF_RULE
-    if (q >= kBfEstQueries && n >= kBfEstRows && d <= 4096) {
+    // enough queries to share a pass over the base set, and enough pairs for its levels' launches
+    // (k 100, d 128; this path / k_bruteforce, us: 63 x 50,000 224 / 205, 32 x 200,000 395 / 326,
+    // 63 x 200,000 397 / 461, 16 x 1 M 757 / 410, 32 x 1 M 832 / 880, 63 x 1 M 842 / 1,431)
+    if (q >= kBfEstQueries && q * n >= kBfEstPairs && d <= 4096) {
         for (uint64_t a = 0; a < q; a += 4096) {
             const uint32_t nb = (uint32_t)std::min<uint64_t>(4096, q - a);
             bruteforce_est(data, n, d, labels, l, queries + a * d, nb, ranges + a * 2 * l, k, dist + a * k, ids + a * k, st);

@@ -253,9 +253,9 @@ def test_estimate_pass_threshold_too_low(cuda):
 # the tensor-core path: one and several query tiles, row tiles with remainders, K with a remainder
 # chunk, label dims of both forms, samples without k passing rows, more passing rows than a list holds
 @pytest.mark.parametrize("q,k,n,d,l,kind", [
-    (64, 10, 32768, 128, 4, "mixed"), (130, 100, 70001, 96, 4, "mixed"), (257, 256, 40000, 100, 2, "mixed"),
-    (65, 1, 50000, 33, 8, "mixed"), (100, 100, 33000, 200, 1, "rare"), (70, 100, 60000, 16, 4, "same"),
-    (64, 50, 40000, 64, 1, "sorted")])
+    (64, 10, 187500, 128, 4, "mixed"), (130, 100, 92311, 96, 4, "mixed"), (257, 256, 46700, 100, 2, "mixed"),
+    (65, 1, 185000, 33, 8, "mixed"), (100, 100, 120001, 200, 1, "rare"), (70, 100, 171500, 16, 4, "same"),
+    (64, 50, 187501, 64, 1, "sorted"), (32, 100, 375000, 32, 3, "mixed")])
 def test_bruteforce_tensor_path(cuda, q, k, n, d, l, kind):
     import torch
     import hdgrid_b200 as hg
@@ -265,7 +265,7 @@ def test_bruteforce_tensor_path(cuda, q, k, n, d, l, kind):
     if kind == "same":  # every row at one distance: every bound ties, ids decide
         base[:] = base[0]
     if kind == "sorted":  # the near rows lie together: a strided sample sees few of them
-        base[:20000] *= np.float32(0.01)
+        base[:60000] *= np.float32(0.01)
         qs *= np.float32(0.01)
     lab = rng.integers(0, 1000, (n, l)).astype(np.float32)
     lo = np.where(rng.random((q, l)) < 0.6, 0, rng.integers(0, 1000, (q, l))).astype(np.float32)
@@ -279,7 +279,7 @@ def test_bruteforce_tensor_path(cuda, q, k, n, d, l, kind):
     hg.bruteforce_knn(*t, k, dist, ids)
     # in groups below the batch rule: the direct path, the same arithmetic and order
     d2, i2 = torch.empty_like(dist), torch.empty_like(ids)
-    for a in range(0, q, 30):
-        b = min(q, a + 30)
+    for a in range(0, q, 31):
+        b = min(q, a + 31)
         hg.bruteforce_knn(t[0], t[1], t[2][a:b].contiguous(), t[3][a:b].contiguous(), k, d2[a:b], i2[a:b])
     assert torch.equal(ids, i2) and torch.equal(dist, d2)
