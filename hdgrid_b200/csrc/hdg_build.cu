@@ -21,6 +21,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <numeric>
 #include <random>
 #include <type_traits>
@@ -662,10 +663,253 @@ __global__ void k_to_bf16(const float* __restrict__ x, uint64_t n, __nv_bfloat16
 }
 
 // ------------------------------------------------------------------------------------
+// stable radix sort of (u64 key, u32 value) pairs, 8 bits per pass from the lowest
+// ------------------------------------------------------------------------------------
+// Per pass: a digit histogram per block of kRsTile pairs, one exclusive scan over (digit, block), and
+// a scatter in which a block ranks its pairs in order: a warp takes consecutive pairs, lanes with
+// the same digit find one another by match, and a prefix over the warps gives the block order.
+// Bound: the scatter's reads and writes of 12 bytes per pair and pass.
+constexpr int kRsThreads = 256, kRsPer = 16, kRsTile = kRsThreads * kRsPer;
+
+__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint64_t* __restrict__ keys, uint64_t n, int shift,
+                                                        uint32_t blocks, uint32_t* __restrict__ hist) {
+    __shared__ uint32_t s_h[256];
+    s_h[threadIdx.x] = 0;
+    __syncthreads();
+    const uint64_t b0 = (uint64_t)blockIdx.x * kRsTile;
+    for (int u = 0; u < kRsPer; u++) {
+        const uint64_t e = b0 + u * kRsThreads + threadIdx.x;
+        if (e < n) atomicAdd(&s_h[(keys[e] >> shift) & 255u], 1u);
+    }
+    __syncthreads();
+    hist[(uint64_t)threadIdx.x * blocks + blockIdx.x] = s_h[threadIdx.x];
+}
+
+// exclusive scan in place, one block
+__global__ void __launch_bounds__(1024) k_rs_scan(uint32_t* __restrict__ a, uint64_t n) {
+    __shared__ uint32_t s_w[32], s_run;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (t == 0) s_run = 0;
+    __syncthreads();
+    for (uint64_t b0 = 0; b0 < n; b0 += 4096) {
+        uint32_t v[4], sum = 0;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint64_t e = b0 + 4ull * t + u;
+            v[u] = e < n ? a[e] : 0u;
+            sum += v[u];
+        }
+        uint32_t x = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_w[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t y = s_w[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t z = __shfl_up_sync(0xffffffffu, y, o);
+                if (lane >= o) y += z;
+            }
+            s_w[lane] = y;
+        }
+        __syncthreads();
+        uint32_t run = s_run + x - sum + (warp ? s_w[warp - 1] : 0u);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint64_t e = b0 + 4ull * t + u;
+            if (e < n) a[e] = run;
+            run += v[u];
+        }
+        __syncthreads();
+        if (t == 1023) s_run = run;
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint64_t* __restrict__ keys,
+                                                           const uint32_t* __restrict__ vals, uint64_t n, int shift,
+                                                           uint32_t blocks, const uint32_t* __restrict__ off,
+                                                           uint64_t* __restrict__ out_keys,
+                                                           uint32_t* __restrict__ out_vals) {
+    constexpr int NW = kRsThreads / 32;
+    __shared__ uint32_t s_c[NW][256];  // pairs of each digit so far in the warp, then before the warp
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    for (int i = t; i < NW * 256; i += kRsThreads) (&s_c[0][0])[i] = 0;
+    __syncthreads();
+    // warp w holds pairs [w * 32 * kRsPer, +32 * kRsPer) of the tile, 32 per round
+    const uint64_t b0 = (uint64_t)blockIdx.x * kRsTile + (uint64_t)warp * 32 * kRsPer + lane;
+    uint64_t k[kRsPer];
+    uint32_t rank[kRsPer];
+#pragma unroll
+    for (int u = 0; u < kRsPer; u++) {
+        const uint64_t e = b0 + 32 * u;
+        const bool v = e < n;
+        k[u] = v ? keys[e] : 0ull;
+        const unsigned live = __ballot_sync(0xffffffffu, v);
+        const uint32_t d = (uint32_t)(k[u] >> shift) & 255u;
+        const unsigned same = __match_any_sync(0xffffffffu, v ? d : 256u + lane) & live;
+        uint32_t before = 0;
+        if (v) before = s_c[warp][d];
+        rank[u] = before + __popc(same & ((1u << lane) - 1u));
+        __syncwarp();
+        if (v && lane == __ffs((int)same) - 1) s_c[warp][d] = before + __popc(same);
+        __syncwarp();
+    }
+    __syncthreads();
+    {
+        uint32_t run = 0;
+#pragma unroll
+        for (int w = 0; w < NW; w++) {
+            const uint32_t c = s_c[w][t];
+            s_c[w][t] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kRsPer; u++) {
+        const uint64_t e = b0 + 32 * u;
+        if (e >= n) continue;
+        const uint32_t d = (uint32_t)(k[u] >> shift) & 255u;
+        const uint32_t at = off[(uint64_t)d * blocks + blockIdx.x] + s_c[warp][d] + rank[u];
+        out_keys[at] = k[u];
+        out_vals[at] = vals[e];
+    }
+}
+
+__global__ void k_iota(uint32_t* __restrict__ a, uint64_t n) {
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < n) a[e] = (uint32_t)e;
+}
+__global__ void k_gather_list(const int* __restrict__ list_of, const uint32_t* __restrict__ ids, uint64_t n,
+                              uint64_t* __restrict__ out) {
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < n) out[e] = (uint64_t)(uint32_t)list_of[ids[e]];
+}
+__global__ void k_gather_z(const uint64_t* __restrict__ z, const uint32_t* __restrict__ ids, uint64_t n,
+                           uint64_t* __restrict__ out) {
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < n) out[e] = z[ids[e]];
+}
+// every point's list under its new number, and the lists' sizes
+__global__ void k_renumber(int* __restrict__ list_of, uint64_t n, const int* __restrict__ new_of_old,
+                           uint32_t* __restrict__ sizes) {
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n) return;
+    const int j = new_of_old[list_of[e]];
+    list_of[e] = j;
+    atomicAdd(&sizes[j], 1u);
+}
+__global__ void k_narrow16(const uint32_t* __restrict__ a, uint64_t n, uint16_t* __restrict__ out) {
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < n) out[e] = (uint16_t)a[e];
+}
+// Smallest and largest label of dim blockIdx.y (as ordered keys; NaN left out) and whether any is NaN
+__global__ void __launch_bounds__(256) k_label_range(const float* __restrict__ labels, uint64_t n, int l,
+                                                     uint32_t* __restrict__ mn, uint32_t* __restrict__ mx,
+                                                     uint32_t* __restrict__ nan) {
+    const int i = blockIdx.y;
+    uint32_t lo = 0xffffffffu, hi = 0u, bad = 0u;
+    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
+        const float x = labels[r * l + i];
+        if (isnan(x)) {
+            bad = 1u;
+        } else {
+            const uint32_t k = float_key(x);
+            lo = min(lo, k);
+            hi = max(hi, k);
+        }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(&mn[i], lo);
+        atomicMax(&mx[i], hi);
+        if (bad) atomicOr(nan, 1u);
+    }
+}
+// The strided sample of one label dim as sort keys (NaN last)
+__global__ void k_rank_sample(const float* __restrict__ labels, uint64_t step, uint64_t m, int l, int i,
+                              uint64_t* __restrict__ keys) {
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= m) return;
+    const float x = labels[e * step * l + i];
+    keys[e] = isnan(x) ? 0xffffffffull : (uint64_t)float_key(x);
+}
+
+// ------------------------------------------------------------------------------------
 // host helpers
 // ------------------------------------------------------------------------------------
 
 static unsigned blocks_for(uint64_t n, unsigned per) { return (unsigned)((n + per - 1) / per); }
+
+// Sorts (keys, vals) by the low `bits` bits of the keys, stably; the result is in keys / vals.
+struct RadixSort {
+    DevMem<uint64_t> k2;
+    DevMem<uint32_t> v2, hist;
+    uint64_t n;
+    uint32_t blocks;
+    explicit RadixSort(uint64_t count)
+        : k2(count), v2(count), hist(256ull * ((count + kRsTile - 1) / kRsTile)), n(count),
+          blocks((uint32_t)((count + kRsTile - 1) / kRsTile)) {}
+    void sort(uint64_t* keys, uint32_t* vals, int bits, cudaStream_t st) {
+        uint64_t *ka = keys, *kb = k2.p;
+        uint32_t *va = vals, *vb = v2.p;
+        for (int shift = 0; shift < bits; shift += 8) {
+            k_rs_hist<<<blocks, kRsThreads, 0, st>>>(ka, n, shift, blocks, hist.p);
+            k_rs_scan<<<1, 1024, 0, st>>>(hist.p, 256ull * blocks);
+            k_rs_scatter<<<blocks, kRsThreads, 0, st>>>(ka, va, n, shift, blocks, hist.p, kb, vb);
+            CK_LAUNCH();
+            std::swap(ka, kb);
+            std::swap(va, vb);
+        }
+        if (ka != keys) {
+            CK(cudaMemcpyAsync(keys, ka, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, st));
+            CK(cudaMemcpyAsync(vals, va, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st));
+        }
+    }
+};
+
+static float ordered_float(uint32_t key) {  // the inverse of float_key
+    const uint32_t u = (key & 0x80000000u) ? (key & 0x7fffffffu) : ~key;
+    float f;
+    std::memcpy(&f, &u, 4);
+    return f;
+}
+
+// Thresholds of one label dim from its sorted sample (NaN labels already left out): the distinct
+// values when they fit in `stride` thresholds, else the sample's quantiles
+static uint32_t thresholds_of(const std::vector<float>& v, uint32_t stride, float* t) {
+    std::vector<float> u(v);
+    u.erase(std::unique(u.begin(), u.end()), u.end());
+    uint32_t m = 0;
+    if (u.size() <= stride + 1) {
+        for (size_t k = 1; k < u.size(); k++) t[m++] = u[k];
+    } else {
+        for (uint32_t k = 1; k <= stride; k++) {
+            const float x = v[(size_t)((uint64_t)k * v.size() / (stride + 1))];
+            if (m == 0 || x > t[m - 1]) t[m++] = x;
+        }
+    }
+    return m;
+}
+
+// What the build still holds on the device when it uploads the index: the arena takes these
+// instead of the host copies (nullptr: from the host)
+struct DeviceArrays {
+    const uint64_t* zcodes;
+    const uint32_t* ids;
+    const uint8_t* codes;    // pool-ordered rows
+    const float* labels;     // pool order
+    const uint32_t* prefix;  // dense counts (nullptr: the compressed rows)
+    uint32_t labels_nan;
+};
+static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArrays* src);
 
 // Lloyd k-means on device rows Xs [ns x d]; centres initialised from the first k rows.
 // Returns the centres (device, [k x d]).
@@ -885,15 +1129,25 @@ void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, co
     const int iters = (int)(P.kmeans_iters ? P.kmeans_iters : 20);
 
     // ---- 1. grid shape -------------------------------------------------------------
-    std::vector<float> hl(n * l);
-    CK(cudaMemcpyAsync(hl.data(), d_labels, sizeof(float) * n * l, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
     std::vector<float> mins(l, INFINITY), maxs(l, -INFINITY);
-    for (uint64_t r = 0; r < n; r++)
-        for (uint32_t i = 0; i < l; i++) {
-            mins[i] = std::min(mins[i], hl[r * l + i]);
-            maxs[i] = std::max(maxs[i], hl[r * l + i]);
-        }
+    uint32_t labels_nan = 0;
+    {
+        std::vector<uint32_t> hr(2 * l + 1, 0u);
+        std::fill(hr.begin(), hr.begin() + l, 0xffffffffu);
+        DevMem<uint32_t> r(2 * l + 1);
+        CK(cudaMemcpyAsync(r.p, hr.data(), sizeof(uint32_t) * hr.size(), cudaMemcpyHostToDevice, st));
+        k_label_range<<<dim3(std::min(blocks_for(n, 256), 1024u), l), 256, 0, st>>>(d_labels, n, (int)l, r.p, r.p + l,
+                                                                                   r.p + 2 * l);
+        CK_LAUNCH();
+        CK(cudaMemcpyAsync(hr.data(), r.p, sizeof(uint32_t) * hr.size(), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        for (uint32_t i = 0; i < l; i++)
+            if (hr[i] <= hr[l + i]) {  // (no label but NaN: the dim keeps inf / -inf)
+                mins[i] = ordered_float(hr[i]);
+                maxs[i] = ordered_float(hr[l + i]);
+            }
+        labels_nan = hr[2 * l];
+    }
     H.grid = compute_grid_shape(mins, maxs, l, P.max_grids, P.label_mask);
     const GridMeta& g = H.grid;
     // per-list prefix counts: the dense cells x lists array while it stays small, else the
@@ -1002,39 +1256,44 @@ void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, co
     // ---- 5. cells, Morton codes, pool order ---------------------------------------------
     DevMem<uint64_t> zc(n), cell(n);
     k_point_cells<<<blocks_for(n, 256), 256, 0, st>>>(d_labels, n, g, zc.p, cell.p);
-    std::vector<uint64_t> hz(n);
-    std::vector<int> hlist(n);
-    CK(cudaMemcpyAsync(hz.data(), zc.p, sizeof(uint64_t) * n, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(hlist.data(), list_of_id.p, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    for (uint64_t r = 0; r < n; r++) hlist[r] = new_of_old[hlist[r]];
-    H.list_off.assign(L + 1, 0);
-    for (uint64_t r = 0; r < n; r++) H.list_off[hlist[r] + 1]++;
-    for (uint64_t j = 0; j < L; j++) H.list_off[j + 1] += H.list_off[j];
-    H.ids.resize(n);
+    // pool order: by list, Morton code, id -- a stable sort of the ids by code, then by list
+    DevMem<uint32_t> dids(n);
+    DevMem<uint64_t> dz(n);
     {
-        std::vector<uint32_t> fill(H.list_off.begin(), H.list_off.end() - 1);
-        for (uint64_t r = 0; r < n; r++) H.ids[fill[hlist[r]]++] = (uint32_t)r;  // ascending ids per list
-#pragma omp parallel for schedule(dynamic, 16)
-        for (int64_t j = 0; j < (int64_t)L; j++) {
-            auto b = H.ids.begin() + H.list_off[j], e = H.ids.begin() + H.list_off[j + 1];
-            std::stable_sort(b, e, [&](uint32_t a, uint32_t c) { return hz[a] < hz[c]; });
-        }
+        DevMem<int> d_new(L);
+        DevMem<uint32_t> sizes(L);
+        CK(cudaMemcpyAsync(d_new.p, new_of_old.data(), sizeof(int) * L, cudaMemcpyHostToDevice, st));
+        CK(cudaMemsetAsync(sizes.p, 0, sizeof(uint32_t) * L, st));
+        k_renumber<<<blocks_for(n, 256), 256, 0, st>>>(list_of_id.p, n, d_new.p, sizes.p);
+        k_iota<<<blocks_for(n, 256), 256, 0, st>>>(dids.p, n);
+        CK(cudaMemcpyAsync(dz.p, zc.p, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, st));
+        RadixSort rs(n);
+        int valid = 0, lbits = 0;
+        for (int i = 0; i < g.l; i++) valid += (g.morton_valid_map >> i) & 1;
+        while ((1ull << lbits) < L) lbits++;
+        rs.sort(dz.p, dids.p, valid * g.morton_max_bits, st);
+        k_gather_list<<<blocks_for(n, 256), 256, 0, st>>>(list_of_id.p, dids.p, n, dz.p);
+        rs.sort(dz.p, dids.p, lbits, st);
+        k_gather_z<<<blocks_for(n, 256), 256, 0, st>>>(zc.p, dids.p, n, dz.p);
+        CK_LAUNCH();
+        std::vector<uint32_t> hs(L);
+        H.ids.resize(n);
+        H.zcodes.resize(n);
+        CK(cudaMemcpyAsync(hs.data(), sizes.p, sizeof(uint32_t) * L, cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(H.ids.data(), dids.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(H.zcodes.data(), dz.p, sizeof(uint64_t) * n, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        H.list_off.assign(L + 1, 0);
+        for (uint64_t j = 0; j < L; j++) H.list_off[j + 1] = H.list_off[j] + hs[j];
     }
-    H.zcodes.resize(n);
-    for (uint64_t r = 0; r < n; r++) H.zcodes[r] = hz[H.ids[r]];
 
     // ---- 6. prefix counts ------------------------------------------------------------------
+    DevMem<uint32_t> prefix(rows_form ? 0 : g.tot_cells * L);
     if (rows_form) {
-        DevMem<int> dl(n);
-        CK(cudaMemcpyAsync(dl.p, hlist.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st));
-        build_prefix_rows(g, cell.p, dl.p, n, (uint32_t)L, H, st);
+        build_prefix_rows(g, cell.p, list_of_id.p, n, (uint32_t)L, H, st);
     } else {
-        DevMem<uint32_t> prefix(g.tot_cells * L);
-        DevMem<int> dl(n);
-        CK(cudaMemcpyAsync(dl.p, hlist.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st));
         CK(cudaMemsetAsync(prefix.p, 0, sizeof(uint32_t) * g.tot_cells * L, st));
-        k_count_cells<<<blocks_for(n, 256), 256, 0, st>>>(cell.p, dl.p, n, (uint32_t)L, prefix.p);
+        k_count_cells<<<blocks_for(n, 256), 256, 0, st>>>(cell.p, list_of_id.p, n, (uint32_t)L, prefix.p);
         for (int a = 0; a < g.l; a++) {
             const uint64_t inner = g.cell_stride[a];
             const uint64_t lines = g.tot_cells / (uint64_t)g.grid_dims[a] * L;
@@ -1048,22 +1307,18 @@ void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, co
     }
 
     // ---- pool-ordered codes and labels ---------------------------------------------------
-    {
-        DevMem<uint32_t> dids(n);
-        CK(cudaMemcpyAsync(dids.p, H.ids.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, st));
-        DevMem<uint8_t> codes(n * H.M_pad);
-        DevMem<float> labels(n * l);
-        k_gather_codes_labels<<<blocks_for(n, 256), 256, 0, st>>>(codes_by_id.p, (int)H.M_pad, d_labels,
-                                                                 (int)l, dids.p, n, codes.p, labels.p);
-        H.codes.resize(n * H.M_pad);
-        H.labels.resize(n * l);
-        CK(cudaMemcpyAsync(H.codes.data(), codes.p, H.codes.size(), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(H.labels.data(), labels.p, sizeof(float) * H.labels.size(),
-                           cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-    }
+    DevMem<uint8_t> codes(n * H.M_pad);
+    DevMem<float> labels(n * l);
+    k_gather_codes_labels<<<blocks_for(n, 256), 256, 0, st>>>(codes_by_id.p, (int)H.M_pad, d_labels, (int)l, dids.p, n,
+                                                             codes.p, labels.p);
     CK_LAUNCH();
-    upload_index(idx, st);
+    H.codes.resize(n * H.M_pad);
+    H.labels.resize(n * l);
+    CK(cudaMemcpyAsync(H.codes.data(), codes.p, H.codes.size(), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(H.labels.data(), labels.p, sizeof(float) * H.labels.size(), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    const DeviceArrays src{dz.p, dids.p, codes.p, labels.p, rows_form ? nullptr : prefix.p, labels_nan};
+    upload_index_from(idx, st, &src);
 }
 
 // Label-rank thresholds of n rows of l label dims (host memory, row-major [n][l]): per dim,
@@ -1092,18 +1347,7 @@ void label_rank_thresholds(const float* labels, uint64_t n, int l, int bits, flo
         }
         mn[i] = lo;
         mx[i] = hi;
-        std::vector<float> u(v);
-        u.erase(std::unique(u.begin(), u.end()), u.end());
-        float* t = thr + (size_t)i * stride;
-        uint32_t m = 0;
-        if (u.size() <= stride + 1) {
-            for (size_t k = 1; k < u.size(); k++) t[m++] = u[k];
-        } else {
-            for (uint32_t k = 1; k <= stride; k++) {
-                const float x = v[(size_t)((uint64_t)k * v.size() / (stride + 1))];
-                if (m == 0 || x > t[m - 1]) t[m++] = x;
-            }
-        }
+        const uint32_t m = thresholds_of(v, stride, thr + (size_t)i * stride);
         n_thr[i] = m;
     }
 }
@@ -1112,7 +1356,10 @@ constexpr uint64_t kDecodedMax = 16ull << 30;
 constexpr uint64_t kDecodedMinPoints = 16384;  // smaller sets never reach the estimate pass
 
 // Copy the host index into one device arena and fill idx->dev.
-void upload_index(hdg_index* idx, cudaStream_t st) {
+void upload_index(hdg_index* idx, cudaStream_t st) { upload_index_from(idx, st, nullptr); }
+
+// src: arrays that the build still holds on the device, copied there instead of from the host
+static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArrays* src) {
     HostIndex& H = idx->host;
     struct Part {
         const void* src;
@@ -1142,7 +1389,43 @@ void upload_index(hdg_index* idx, cudaStream_t st) {
     std::vector<float> rthr((size_t)H.l * rstride);
     uint32_t rn[kMaxDims] = {0};
     float rmin[kMaxDims] = {0.f}, rmax[kMaxDims] = {0.f};
-    if (rbits) label_rank_thresholds(H.labels.data(), H.n, (int)H.l, rbits, rthr.data(), rn, rmin, rmax);
+    if (rbits && !src) {
+        label_rank_thresholds(H.labels.data(), H.n, (int)H.l, rbits, rthr.data(), rn, rmin, rmax);
+    } else if (rbits) {
+        // the same from the device's labels: the strided sample sorted there, dim by dim
+        const uint64_t step = std::max<uint64_t>(1, H.n / 262144), m = (H.n + step - 1) / step;
+        const uint32_t l = (uint32_t)H.l;
+        DevMem<uint64_t> keys(m);
+        DevMem<uint32_t> vals(m);
+        RadixSort rs(m);
+        std::vector<uint64_t> hk(m);
+        std::vector<float> v;
+        std::vector<uint32_t> hr(2 * l + 1, 0u);
+        std::fill(hr.begin(), hr.begin() + l, 0xffffffffu);
+        DevMem<uint32_t> rg(2 * l + 1);
+        CK(cudaMemcpyAsync(rg.p, hr.data(), sizeof(uint32_t) * hr.size(), cudaMemcpyHostToDevice, st));
+        k_label_range<<<dim3(std::min(blocks_for(H.n, 256), 1024u), l), 256, 0, st>>>(src->labels, H.n, (int)l, rg.p, rg.p + l,
+                                                                                     rg.p + 2 * l);
+        CK_LAUNCH();
+        CK(cudaMemcpyAsync(hr.data(), rg.p, sizeof(uint32_t) * hr.size(), cudaMemcpyDeviceToHost, st));
+        for (uint32_t i = 0; i < l; i++) {
+            k_rank_sample<<<blocks_for(m, 256), 256, 0, st>>>(src->labels, step, m, (int)l, (int)i, keys.p);
+            k_iota<<<blocks_for(m, 256), 256, 0, st>>>(vals.p, m);
+            CK_LAUNCH();
+            rs.sort(keys.p, vals.p, 32, st);
+            CK(cudaMemcpyAsync(hk.data(), keys.p, sizeof(uint64_t) * m, cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            v.clear();
+            for (uint64_t k : hk) {
+                if (k == 0xffffffffull) break;  // NaN labels sort last
+                v.push_back(ordered_float((uint32_t)k));
+            }
+            rn[i] = thresholds_of(v, rstride, rthr.data() + (size_t)i * rstride);
+            const bool any = hr[i] <= hr[l + i];
+            rmin[i] = any ? ordered_float(hr[i]) : INFINITY;
+            rmax[i] = any ? ordered_float(hr[l + i]) : -INFINITY;
+        }
+    }
     const size_t o_z = reserve(H.zcodes.size() * 8), o_id = reserve(H.ids.size() * 4);
     const size_t o_pk = reserve(rbits ? H.n * 4 : 0), o_rt = reserve(rthr.size() * 4);
     const size_t o_code = reserve(H.codes.size() + 64), o_lab = reserve(H.labels.size() * 4);
@@ -1159,6 +1442,11 @@ void upload_index(hdg_index* idx, cudaStream_t st) {
         if (bytes) CK(cudaMemcpyAsync(base + off, src, bytes, cudaMemcpyHostToDevice, st));
         return base + off;
     };
+    auto keep = [&](size_t off, const void* dev, const void* host, size_t bytes) {
+        if (dev && bytes) CK(cudaMemcpyAsync(base + off, dev, bytes, cudaMemcpyDeviceToDevice, st));
+        else up(off, host, bytes);
+        return base + off;
+    };
     D.centers = (const float*)up(o_c, H.centers.data(), H.centers.size() * 4);
     D.sub_centers = (const float*)up(o_sc, H.sub_centers.data(), H.sub_centers.size() * 4);
     cb = (uint16_t*)(base + o_cb);
@@ -1166,23 +1454,23 @@ void upload_index(hdg_index* idx, cudaStream_t st) {
     cn = (float*)(base + o_cn);
     D.cluster_off = (const uint32_t*)up(o_co, H.cluster_off.data(), H.cluster_off.size() * 4);
     D.list_off = (const uint32_t*)up(o_lo, H.list_off.data(), H.list_off.size() * 4);
-    D.zcodes = (const uint64_t*)up(o_z, H.zcodes.data(), H.zcodes.size() * 8);
-    D.ids = (const uint32_t*)up(o_id, H.ids.data(), H.ids.size() * 4);
-    D.labels_nan = std::any_of(H.labels.begin(), H.labels.end(), [](float v) { return std::isnan(v); }) ? 1u : 0u;
+    D.zcodes = (const uint64_t*)keep(o_z, src ? src->zcodes : nullptr, H.zcodes.data(), H.zcodes.size() * 8);
+    D.ids = (const uint32_t*)keep(o_id, src ? src->ids : nullptr, H.ids.data(), H.ids.size() * 4);
+    D.labels_nan = src ? src->labels_nan : std::any_of(H.labels.begin(), H.labels.end(), [](float v) { return std::isnan(v); }) ? 1u : 0u;
     {
         // pool-ordered rows -> 16-byte chunk planes (the scan's coalesced layout)
-        DevMem<uint8_t> rows(std::max<size_t>(H.codes.size(), 16));
+        DevMem<uint8_t> rows(src ? 0 : std::max<size_t>(H.codes.size(), 16));
         if (!H.codes.empty()) {
-            CK(cudaMemcpyAsync(rows.p, H.codes.data(), H.codes.size(), cudaMemcpyHostToDevice, st));
+            if (!src) CK(cudaMemcpyAsync(rows.p, H.codes.data(), H.codes.size(), cudaMemcpyHostToDevice, st));
             const uint64_t chunks = H.M_pad / 16;
             k_interleave_codes<<<blocks_for(H.n * chunks, 256), 256, 0, st>>>(
-                reinterpret_cast<const uint4*>(rows.p), H.n, (uint32_t)chunks, reinterpret_cast<uint4*>(base + o_code));
+                reinterpret_cast<const uint4*>(src ? src->codes : rows.p), H.n, (uint32_t)chunks, reinterpret_cast<uint4*>(base + o_code));
             CK_LAUNCH();
         }
         CK(cudaStreamSynchronize(st));
         D.codes = (const uint8_t*)(base + o_code);
     }
-    D.labels = (const float*)up(o_lab, H.labels.data(), H.labels.size() * 4);
+    D.labels = (const float*)keep(o_lab, src ? src->labels : nullptr, H.labels.data(), H.labels.size() * 4);
     D.rank_bits = (uint32_t)rbits;
     D.rank_stride = rstride;
     D.rank_guard = D.rank_full = 0;
@@ -1212,14 +1500,19 @@ void upload_index(hdg_index* idx, cudaStream_t st) {
     } else {
         D.prefix = nullptr;
         D.prefix16 = nullptr;
-        if (pre16) {
+        if (pre16 && src && src->prefix) {
+            k_narrow16<<<blocks_for(H.prefix.size(), 256), 256, 0, st>>>(src->prefix, H.prefix.size(),
+                                                                        reinterpret_cast<uint16_t*>(base + o_pre));
+            CK_LAUNCH();
+            D.prefix16 = reinterpret_cast<const uint16_t*>(base + o_pre);
+        } else if (pre16) {
             std::vector<uint16_t> p16(H.prefix.size());
 #pragma omp parallel for
             for (int64_t i = 0; i < (int64_t)H.prefix.size(); i++) p16[i] = (uint16_t)H.prefix[i];
             D.prefix16 = (const uint16_t*)up(o_pre, p16.data(), p16.size() * 2);
             CK(cudaStreamSynchronize(st));  // p16 is read by the copy
         } else {
-            D.prefix = (const uint32_t*)up(o_pre, H.prefix.data(), H.prefix.size() * 4);
+            D.prefix = (const uint32_t*)keep(o_pre, src ? src->prefix : nullptr, H.prefix.data(), H.prefix.size() * 4);
         }
         D.prefix_off = D.prefix_rows = nullptr;
     }
