@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <numeric>
 #include <random>
 #include <type_traits>
@@ -907,6 +908,7 @@ struct DeviceArrays {
     const uint8_t* codes;    // pool-ordered rows
     const float* labels;     // pool order
     const uint32_t* prefix;  // dense counts (nullptr: the compressed rows)
+    const uint64_t *prefix_off, *prefix_rows;
     uint32_t labels_nan;
 };
 static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArrays* src);
@@ -1065,7 +1067,8 @@ constexpr uint64_t kDensePrefixMax = 2ull << 30;
 // counts each row's change points (their exclusive sum over rows t * L + j gives the offsets),
 // a second round rebuilds each chunk and writes the (z << 32 | value) pairs.
 static void build_prefix_rows(const GridMeta& g, const uint64_t* d_cell, const int* d_list, uint64_t n, uint32_t L,
-                              HostIndex& H, cudaStream_t st) {
+                              std::unique_ptr<DevMem<uint64_t>>& off, std::unique_ptr<DevMem<uint64_t>>& rows,
+                              uint64_t& entries, cudaStream_t st) {
     const uint32_t Dd = (uint32_t)g.grid_dims[g.diff_dim];
     HDG_REQUIRE(g.cell_stride[g.diff_dim] == 1 && Dd >= 1 && g.tot_cells % Dd == 0, HDG_ERR_STATE,
                 "diff dim of the grid is not its last dim of size > 1");
@@ -1089,16 +1092,14 @@ static void build_prefix_rows(const GridMeta& g, const uint64_t* d_cell, const i
     std::vector<uint64_t> hc(T * L);
     CK(cudaMemcpyAsync(hc.data(), cnt.p, sizeof(uint64_t) * hc.size(), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    H.prefix_off.assign(T * L + 1, 0);
-    for (uint64_t r = 0; r < T * L; r++) H.prefix_off[r + 1] = H.prefix_off[r] + hc[r];
-    const uint64_t E = H.prefix_off.back();
-    DevMem<uint64_t> off(T * L + 1), rows(std::max<uint64_t>(E, 1));
-    CK(cudaMemcpyAsync(off.p, H.prefix_off.data(), sizeof(uint64_t) * (T * L + 1), cudaMemcpyHostToDevice, st));
-    for (uint32_t j0 = 0; j0 < L; j0 += B) chunk(j0, std::min(B, L - j0), off.p, rows.p);
-    H.prefix_rows.resize(E);
-    if (E) CK(cudaMemcpyAsync(H.prefix_rows.data(), rows.p, sizeof(uint64_t) * E, cudaMemcpyDeviceToHost, st));
+    std::vector<uint64_t> ho(T * L + 1, 0);
+    for (uint64_t r = 0; r < T * L; r++) ho[r + 1] = ho[r] + hc[r];
+    entries = ho.back();
+    off.reset(new DevMem<uint64_t>(T * L + 1));
+    rows.reset(new DevMem<uint64_t>(std::max<uint64_t>(entries, 1)));
+    CK(cudaMemcpyAsync(off->p, ho.data(), sizeof(uint64_t) * (T * L + 1), cudaMemcpyHostToDevice, st));
+    for (uint32_t j0 = 0; j0 < L; j0 += B) chunk(j0, std::min(B, L - j0), off->p, rows->p);
     CK(cudaStreamSynchronize(st));
-    H.prefix.clear();
 }
 
 void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, const float* d_labels,
@@ -1277,11 +1278,7 @@ void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, co
         k_gather_z<<<blocks_for(n, 256), 256, 0, st>>>(zc.p, dids.p, n, dz.p);
         CK_LAUNCH();
         std::vector<uint32_t> hs(L);
-        H.ids.resize(n);
-        H.zcodes.resize(n);
         CK(cudaMemcpyAsync(hs.data(), sizes.p, sizeof(uint32_t) * L, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(H.ids.data(), dids.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(H.zcodes.data(), dz.p, sizeof(uint64_t) * n, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         H.list_off.assign(L + 1, 0);
         for (uint64_t j = 0; j < L; j++) H.list_off[j + 1] = H.list_off[j] + hs[j];
@@ -1289,8 +1286,9 @@ void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, co
 
     // ---- 6. prefix counts ------------------------------------------------------------------
     DevMem<uint32_t> prefix(rows_form ? 0 : g.tot_cells * L);
+    std::unique_ptr<DevMem<uint64_t>> row_off, rows;  // the compressed form
     if (rows_form) {
-        build_prefix_rows(g, cell.p, list_of_id.p, n, (uint32_t)L, H, st);
+        build_prefix_rows(g, cell.p, list_of_id.p, n, (uint32_t)L, row_off, rows, H.prefix_entries, st);
     } else {
         CK(cudaMemsetAsync(prefix.p, 0, sizeof(uint32_t) * g.tot_cells * L, st));
         k_count_cells<<<blocks_for(n, 256), 256, 0, st>>>(cell.p, list_of_id.p, n, (uint32_t)L, prefix.p);
@@ -1300,10 +1298,7 @@ void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, co
             k_scan_axis<<<blocks_for(lines, 256), 256, 0, st>>>(prefix.p, lines, inner, g.grid_dims[a],
                                                                 (uint32_t)L);
         }
-        H.prefix.resize(g.tot_cells * L);
-        CK(cudaMemcpyAsync(H.prefix.data(), prefix.p, sizeof(uint32_t) * H.prefix.size(),
-                           cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
+        CK_LAUNCH();
     }
 
     // ---- pool-ordered codes and labels ---------------------------------------------------
@@ -1312,12 +1307,8 @@ void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, co
     k_gather_codes_labels<<<blocks_for(n, 256), 256, 0, st>>>(codes_by_id.p, (int)H.M_pad, d_labels, (int)l, dids.p, n,
                                                              codes.p, labels.p);
     CK_LAUNCH();
-    H.codes.resize(n * H.M_pad);
-    H.labels.resize(n * l);
-    CK(cudaMemcpyAsync(H.codes.data(), codes.p, H.codes.size(), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(H.labels.data(), labels.p, sizeof(float) * H.labels.size(), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    const DeviceArrays src{dz.p, dids.p, codes.p, labels.p, rows_form ? nullptr : prefix.p, labels_nan};
+    const DeviceArrays src{dz.p,       dids.p,     codes.p, labels.p, rows_form ? nullptr : prefix.p,
+                           rows_form ? row_off->p : nullptr, rows_form ? rows->p : nullptr, labels_nan};
     upload_index_from(idx, st, &src);
 }
 
@@ -1361,6 +1352,12 @@ void upload_index(hdg_index* idx, cudaStream_t st) { upload_index_from(idx, st, 
 // src: arrays that the build still holds on the device, copied there instead of from the host
 static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArrays* src) {
     HostIndex& H = idx->host;
+    // element counts of the large arrays, wherever they are
+    const uint64_t n_dense = src ? (src->prefix ? H.grid.tot_cells * H.n_lists : 0) : H.prefix.size();
+    const uint64_t n_off = src ? (src->prefix_off ? H.grid.tot_cells / (uint64_t)H.grid.grid_dims[H.grid.diff_dim] * H.n_lists + 1 : 0)
+                               : H.prefix_off.size();
+    if (!src) H.prefix_entries = H.prefix_rows.size();
+    const uint64_t n_rows = n_off ? H.prefix_entries : 0;
     struct Part {
         const void* src;
         size_t bytes;
@@ -1384,7 +1381,7 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
     const size_t o_co = reserve(H.cluster_off.size() * 4), o_lo = reserve(H.list_off.size() * 4);
     GridMeta gp = H.grid;
     // label-rank thresholds, so that a rank box is about as tight as the labels
-    const int rbits = H.n && !H.labels.empty() ? rank_bits_for((int)H.l) : 0;
+    const int rbits = H.n ? rank_bits_for((int)H.l) : 0;
     const uint32_t rstride = rbits ? (1u << rbits) - 1u : 0u;
     std::vector<float> rthr((size_t)H.l * rstride);
     uint32_t rn[kMaxDims] = {0};
@@ -1426,15 +1423,15 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
             rmax[i] = any ? ordered_float(hr[l + i]) : -INFINITY;
         }
     }
-    const size_t o_z = reserve(H.zcodes.size() * 8), o_id = reserve(H.ids.size() * 4);
+    const size_t o_z = reserve(H.n * 8), o_id = reserve(H.n * 4);
     const size_t o_pk = reserve(rbits ? H.n * 4 : 0), o_rt = reserve(rthr.size() * 4);
-    const size_t o_code = reserve(H.codes.size() + 64), o_lab = reserve(H.labels.size() * 4);
+    const size_t o_code = reserve(H.n * H.M_pad + 64), o_lab = reserve(H.n * H.l * 4);
     // a dense prefix count never exceeds its list's size: 16 bits suffice when no list passes 65535
     uint32_t max_list = 0;
     for (uint64_t j = 0; j + 1 < H.list_off.size(); j++) max_list = std::max(max_list, H.list_off[j + 1] - H.list_off[j]);
-    const bool pre16 = !H.prefix.empty() && max_list <= 0xffffu;
-    const size_t o_pq = reserve(H.pq_centers.size() * 4), o_pre = reserve(H.prefix.size() * (pre16 ? 2 : 4));
-    const size_t o_poff = reserve(H.prefix_off.size() * 8), o_prow = reserve(H.prefix_rows.size() * 8);
+    const bool pre16 = n_dense && max_list <= 0xffffu;
+    const size_t o_pq = reserve(H.pq_centers.size() * 4), o_pre = reserve(n_dense * (pre16 ? 2 : 4));
+    const size_t o_poff = reserve(n_off * 8), o_prow = reserve(n_rows * 8);
     idx->arena.reset();
     idx->arena.ensure(total);
     char* base = static_cast<char*>(idx->arena.ptr);
@@ -1454,13 +1451,13 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
     cn = (float*)(base + o_cn);
     D.cluster_off = (const uint32_t*)up(o_co, H.cluster_off.data(), H.cluster_off.size() * 4);
     D.list_off = (const uint32_t*)up(o_lo, H.list_off.data(), H.list_off.size() * 4);
-    D.zcodes = (const uint64_t*)keep(o_z, src ? src->zcodes : nullptr, H.zcodes.data(), H.zcodes.size() * 8);
-    D.ids = (const uint32_t*)keep(o_id, src ? src->ids : nullptr, H.ids.data(), H.ids.size() * 4);
+    D.zcodes = (const uint64_t*)keep(o_z, src ? src->zcodes : nullptr, H.zcodes.data(), H.n * 8);
+    D.ids = (const uint32_t*)keep(o_id, src ? src->ids : nullptr, H.ids.data(), H.n * 4);
     D.labels_nan = src ? src->labels_nan : std::any_of(H.labels.begin(), H.labels.end(), [](float v) { return std::isnan(v); }) ? 1u : 0u;
     {
         // pool-ordered rows -> 16-byte chunk planes (the scan's coalesced layout)
         DevMem<uint8_t> rows(src ? 0 : std::max<size_t>(H.codes.size(), 16));
-        if (!H.codes.empty()) {
+        if (H.n) {
             if (!src) CK(cudaMemcpyAsync(rows.p, H.codes.data(), H.codes.size(), cudaMemcpyHostToDevice, st));
             const uint64_t chunks = H.M_pad / 16;
             k_interleave_codes<<<blocks_for(H.n * chunks, 256), 256, 0, st>>>(
@@ -1470,7 +1467,7 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
         CK(cudaStreamSynchronize(st));
         D.codes = (const uint8_t*)(base + o_code);
     }
-    D.labels = (const float*)keep(o_lab, src ? src->labels : nullptr, H.labels.data(), H.labels.size() * 4);
+    D.labels = (const float*)keep(o_lab, src ? src->labels : nullptr, H.labels.data(), H.n * H.l * 4);
     D.rank_bits = (uint32_t)rbits;
     D.rank_stride = rstride;
     D.rank_guard = D.rank_full = 0;
@@ -1492,17 +1489,16 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
         CK(cudaStreamSynchronize(st));  // rthr is read by the copy
     }
     D.pq_centers = (const float*)up(o_pq, H.pq_centers.data(), H.pq_centers.size() * 4);
-    if (!H.prefix_off.empty()) {  // the compressed rows form
+    if (n_off) {  // the compressed rows form
         D.prefix = nullptr;
         D.prefix16 = nullptr;
-        D.prefix_off = (const uint64_t*)up(o_poff, H.prefix_off.data(), H.prefix_off.size() * 8);
-        D.prefix_rows = (const uint64_t*)up(o_prow, H.prefix_rows.data(), H.prefix_rows.size() * 8);
+        D.prefix_off = (const uint64_t*)keep(o_poff, src ? src->prefix_off : nullptr, H.prefix_off.data(), n_off * 8);
+        D.prefix_rows = (const uint64_t*)keep(o_prow, src ? src->prefix_rows : nullptr, H.prefix_rows.data(), n_rows * 8);
     } else {
         D.prefix = nullptr;
         D.prefix16 = nullptr;
         if (pre16 && src && src->prefix) {
-            k_narrow16<<<blocks_for(H.prefix.size(), 256), 256, 0, st>>>(src->prefix, H.prefix.size(),
-                                                                        reinterpret_cast<uint16_t*>(base + o_pre));
+            k_narrow16<<<blocks_for(n_dense, 256), 256, 0, st>>>(src->prefix, n_dense, reinterpret_cast<uint16_t*>(base + o_pre));
             CK_LAUNCH();
             D.prefix16 = reinterpret_cast<const uint16_t*>(base + o_pre);
         } else if (pre16) {
@@ -1512,7 +1508,7 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
             D.prefix16 = (const uint16_t*)up(o_pre, p16.data(), p16.size() * 2);
             CK(cudaStreamSynchronize(st));  // p16 is read by the copy
         } else {
-            D.prefix = (const uint32_t*)keep(o_pre, src ? src->prefix : nullptr, H.prefix.data(), H.prefix.size() * 4);
+            D.prefix = (const uint32_t*)keep(o_pre, src ? src->prefix : nullptr, H.prefix.data(), n_dense * 4);
         }
         D.prefix_off = D.prefix_rows = nullptr;
     }
@@ -1562,6 +1558,48 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
     CK_LAUNCH();
     idx->built = true;
     (void)offs;
+    // the device holds the one copy from here on
+    std::vector<uint32_t>().swap(H.ids);
+    std::vector<uint32_t>().swap(H.prefix);
+    std::vector<uint64_t>().swap(H.prefix_off);
+    std::vector<uint64_t>().swap(H.prefix_rows);
+    std::vector<uint64_t>().swap(H.zcodes);
+    std::vector<uint8_t>().swap(H.codes);
+    std::vector<float>().swap(H.labels);
+}
+
+HostIndex fetch_host(const hdg_index* idx) {
+    HostIndex H = idx->host;
+    const IndexDev& D = idx->dev;
+    auto down = [](auto& v, const void* src, uint64_t count) {
+        v.resize(count);
+        if (count) CK(cudaMemcpy(v.data(), src, count * sizeof(v[0]), cudaMemcpyDeviceToHost));
+    };
+    down(H.ids, D.ids, H.n);
+    down(H.zcodes, D.zcodes, H.n);
+    down(H.labels, D.labels, H.n * H.l);
+    {  // chunk planes back to rows
+        std::vector<uint8_t> planes;
+        down(planes, D.codes, H.n * H.M_pad);
+        H.codes.resize(H.n * H.M_pad);
+        const uint64_t chunks = H.M_pad / 16;
+#pragma omp parallel for
+        for (int64_t r = 0; r < (int64_t)H.n; r++)
+            for (uint64_t j = 0; j < chunks; j++)
+                std::memcpy(&H.codes[(uint64_t)r * H.M_pad + 16 * j], &planes[(j * H.n + (uint64_t)r) * 16], 16);
+    }
+    const uint64_t cells = H.grid.tot_cells * H.n_lists;
+    if (D.prefix_off) {
+        down(H.prefix_off, D.prefix_off, H.grid.tot_cells / (uint64_t)H.grid.grid_dims[H.grid.diff_dim] * H.n_lists + 1);
+        down(H.prefix_rows, D.prefix_rows, H.prefix_entries);
+    } else if (D.prefix16) {
+        std::vector<uint16_t> p16;
+        down(p16, D.prefix16, cells);
+        H.prefix.assign(p16.begin(), p16.end());
+    } else {
+        down(H.prefix, D.prefix, cells);
+    }
+    return H;
 }
 
 }  // namespace hdg

@@ -111,9 +111,13 @@ struct IndexDev {
     const uint64_t* prefix_rows;
 };
 
-// Host-side copy of every index array (build output, save/load payload).
+// Host side of the index: its sizes and small arrays.  The arrays that grow with the points or the
+// grid (ids, prefix*, zcodes, codes, labels) are filled while an index is read from a file and
+// emptied once they are on the device, which holds the one copy; hdg_save reads them back
+// (fetch_host).
 struct HostIndex {
     uint64_t n = 0, d = 0, l = 0, M = 0, M_pad = 0, pq_len = 0, n_lists = 0, C = 0;
+    uint64_t prefix_entries = 0;  // change points of the compressed prefix rows (0: dense counts)
     GridMeta grid;
     std::vector<float> centers, sub_centers, pq_centers;
     std::vector<uint32_t> cluster_off, list_off, ids, prefix;

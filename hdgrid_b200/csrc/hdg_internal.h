@@ -37,6 +37,8 @@ GridMeta compute_grid_shape(const std::vector<float>& mins, const std::vector<fl
 void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, const float* d_labels,
                  uint32_t l, cudaStream_t st);
 void upload_index(hdg_index* idx, cudaStream_t st);
+// a host copy of the index, its large arrays read back from the device
+HostIndex fetch_host(const hdg_index* idx);
 void upload_filter(hdg_index* idx);
 FilterDev filter_dev(const hdg_index* idx);
 void reserve_workspace(hdg_index* idx, uint64_t q, cudaStream_t st = nullptr);

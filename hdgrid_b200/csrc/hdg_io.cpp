@@ -100,7 +100,7 @@ void save_index(const hdg_index* idx, const std::string& path) {
     for (int i = 0; i < kMaxDims; i++) w.put<int32_t>(fs.div_value[i]);
     w.put<uint32_t>((uint32_t)fs.interval_map.size());
     for (float x : fs.interval_map) w.put<float>(x);
-    const HostIndex& H = idx->host;
+    const HostIndex H = fetch_host(idx);
     for (uint64_t v : {H.n, H.d, H.l, H.M, H.M_pad, H.pq_len, H.n_lists, H.C}) w.put<uint64_t>(v);
     const GridMeta& g = H.grid;
     w.put<int32_t>(g.l);
