@@ -112,7 +112,17 @@ struct Workspace {
     uint64_t cap;            // distance-buffer capacity in candidates
 };
 
+constexpr uint64_t kChainQueries = 4096;
+
 enum ScanMode { kPre = 0, kPost = 1, kL1 = 2 };
+
+// Every kernel of the query path begins with this: the next kernel of the stream may be brought up
+// (its blocks resident and waiting at the same point), and this one waits until the kernel before
+// it has ended.  Kernels launched without the attribute (launch_next) start after it anyway.
+__device__ __forceinline__ void chain_start() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 __device__ __forceinline__ uint32_t q_k(const Workspace& w, uint64_t qi) {
     return w.qk ? max(1u, min(w.qk[qi], w.k_max)) : w.k_max;
@@ -231,12 +241,14 @@ __device__ __forceinline__ unsigned long long block_inclusive_sum(unsigned long 
 __global__ void __launch_bounds__(kThreads) k_prologue(IndexDev D, GridMeta g, FilterDev f,
                                                        const float* __restrict__ qlabels,
                                                        int label_cols, Workspace w) {
+    chain_start();
     extern __shared__ uint32_t s_counts[];  // [L]
     __shared__ float s_box[2 * kMaxDims];
     __shared__ int s_cells[2 * kMaxDims];
     __shared__ uint64_t s_corner[1 << kMaxDims];
     __shared__ int s_sign[1 << kMaxDims];
     __shared__ uint32_t s_rank[4];
+    __shared__ uint32_t s_count[kMaxDims][3];
     const uint64_t qi = blockIdx.x;
     const int t = threadIdx.x;
     const int l = g.l;
@@ -252,33 +264,19 @@ __global__ void __launch_bounds__(kThreads) k_prologue(IndexDev D, GridMeta g, F
         w.box[qi * 2 * l + 2 * t + 1] = hi;
     }
     __syncthreads();
-    if (t < l && D.rankpack) {
-        // The rank box of label dim t: a rank below that of lo holds labels below a threshold
-        // <= lo, a rank above that of hi labels at or above a threshold > hi.  The inner box:
-        // ranks whose labels all lie in [lo, hi] -- above the rank of the largest threshold
-        // below lo (or every rank when the dim's smallest label is >= lo), and below the rank
-        // of hi (or every rank when its largest label is <= hi).  NaN bounds reject nothing.
-        const float blo = s_box[2 * t], bhi = s_box[2 * t + 1];
-        const float* thr = D.rank_thr + (uint64_t)t * D.rank_stride;
-        const uint32_t n = D.rank_n[t];
-        auto count = [&](float x, bool le) {  // thresholds <= x (le) or < x
-            uint32_t a = 0, b = n;
-            while (a < b) {
-                const uint32_t m = (a + b) >> 1;
-                if (le ? thr[m] <= x : thr[m] < x) a = m + 1;
-                else b = m;
-            }
-            return a;
-        };
-        const uint32_t rlo = isnan(blo) ? 0u : count(blo, true), rhi = isnan(bhi) ? n : count(bhi, true);
-        const int ilo = isnan(blo) || D.rank_min[t] >= blo ? 0 : (int)count(blo, false) + 1;
-        const int ihi = isnan(bhi) || D.rank_max[t] <= bhi ? (int)n : (int)rhi - 1;
-        const bool empty = ilo > ihi;  // no rank is sure to pass: the field's box [1, 0]
-        const int off = t * (int)(D.rank_bits + 1);
-        if (rlo) atomicOr(&s_rank[0], rlo << off);
-        atomicOr(&s_rank[1], rhi << off);
-        if (empty || ilo) atomicOr(&s_rank[2], (empty ? 1u : (uint32_t)ilo) << off);
-        if (!empty && ihi) atomicOr(&s_rank[3], (uint32_t)ihi << off);
+    // The threshold counts behind the rank boxes, one binary search per thread: thresholds <= lo,
+    // <= hi and < lo of every dim (one after another they were 36 dependent loads on 12-bit ranks)
+    if (D.rankpack && t >= 32 && t < 32 + 3 * l) {
+        const int i = (t - 32) / 3, what = (t - 32) % 3;
+        const float x = s_box[2 * i + (what == 1 ? 1 : 0)];
+        const float* thr = D.rank_thr + (uint64_t)i * D.rank_stride;
+        uint32_t a = 0, b = isnan(x) ? 0u : D.rank_n[i];
+        while (a < b) {
+            const uint32_t m = (a + b) >> 1;
+            if (what != 2 ? thr[m] <= x : thr[m] < x) a = m + 1;
+            else b = m;
+        }
+        s_count[i][what] = a;
     }
     if (t < l) {
         const int od = g.shuffle[t];
@@ -288,6 +286,25 @@ __global__ void __launch_bounds__(kThreads) k_prologue(IndexDev D, GridMeta g, F
         s_cells[2 * t + 1] = hi;
         w.cells[qi * 2 * l + 2 * t] = lo;
         w.cells[qi * 2 * l + 2 * t + 1] = hi;
+    }
+    __syncthreads();
+    if (t < l && D.rankpack) {
+        // The rank box of label dim t: a rank below that of lo holds labels below a threshold
+        // <= lo, a rank above that of hi labels at or above a threshold > hi.  The inner box:
+        // ranks whose labels all lie in [lo, hi] -- above the rank of the largest threshold
+        // below lo (or every rank when the dim's smallest label is >= lo), and below the rank
+        // of hi (or every rank when its largest label is <= hi).  NaN bounds reject nothing.
+        const float blo = s_box[2 * t], bhi = s_box[2 * t + 1];
+        const uint32_t n = D.rank_n[t];
+        const uint32_t rlo = isnan(blo) ? 0u : s_count[t][0], rhi = isnan(bhi) ? n : s_count[t][1];
+        const int ilo = isnan(blo) || D.rank_min[t] >= blo ? 0 : (int)s_count[t][2] + 1;
+        const int ihi = isnan(bhi) || D.rank_max[t] <= bhi ? (int)n : (int)rhi - 1;
+        const bool empty = ilo > ihi;  // no rank is sure to pass: the field's box [1, 0]
+        const int off = t * (int)(D.rank_bits + 1);
+        if (rlo) atomicOr(&s_rank[0], rlo << off);
+        atomicOr(&s_rank[1], rhi << off);
+        if (empty || ilo) atomicOr(&s_rank[2], (empty ? 1u : (uint32_t)ilo) << off);
+        if (!empty && ihi) atomicOr(&s_rank[3], (uint32_t)ihi << off);
     }
     __syncthreads();
     if (t == 0) {
@@ -546,6 +563,7 @@ constexpr int kCoarseThreads = 128;
 __global__ void __launch_bounds__(kCoarseThreads) k_coarse(IndexDev D, GridMeta g, const float* __restrict__ queries,
                                                      int Pc, int Ps, int sort_n1, int sort_n2,
                                                      Workspace w) {
+    chain_start();
     extern __shared__ uint64_t s_keys[];  // [max(sort_n1, sort_n2)], then the bands' lows, the query vector
     float* s_lo = reinterpret_cast<float*>(s_keys + max(sort_n1, sort_n2));
     float* s_q = s_lo + max(sort_n1, sort_n2);
@@ -805,6 +823,7 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(IndexDev D, GridMeta 
 // k_batch: per-query candidate offsets and work items, batch sums (one block)
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
+    chain_start();
     __shared__ unsigned long long s_tot[32], s_items[32], s_pitems[32], s_sel[32];
     __shared__ unsigned long long s_red[4], s_drop[2];
     __shared__ float s_beta;
@@ -973,6 +992,7 @@ __device__ __forceinline__ void store_lut(float* lut, int f16, uint64_t i, float
 // 32 -> 8 us (1 query), 100 -> 27 us (1,000) and 192 -> 131 us (10,000, M = 32).
 __global__ void __launch_bounds__(512) k_lut(IndexDev D, const float* __restrict__ queries, uint64_t q, int G,
                                              float* __restrict__ lut, int f16, const uint32_t* __restrict__ item_off) {
+    chain_start();
     extern __shared__ float smem_lut[];
     // a block none of whose queries has ADC work stages nothing
     {
@@ -1034,6 +1054,7 @@ static int lut_slices(uint64_t q, int G, int sms) {
 __global__ void __launch_bounds__(256) k_lut_plain(IndexDev D, const float* __restrict__ queries, int G,
                                                    float* __restrict__ lut, int f16,
                                                    const uint32_t* __restrict__ item_off) {
+    chain_start();
     extern __shared__ float s_q[];     // [d]
     __shared__ float s_t[kCodes][33];  // [c][j]
     const uint64_t qi = blockIdx.x;
@@ -1500,6 +1521,7 @@ __global__ void __launch_bounds__(1024) k_scan_plan(uint64_t q, Workspace w) {
 template <int G, int NT, int CPT>
 __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(IndexDev D, int Ps, uint64_t q,
                                                                                  Workspace w) {
+    chain_start();
     extern __shared__ __align__(16) float s_lut[];  // [G][256][64]
     uint32_t* s_pre = reinterpret_cast<uint32_t*>(s_lut + G * kCodes * 64);  // [Ps + 1]
     uint32_t* s_start = s_pre + Ps + 1;                                       // [Ps]
@@ -1673,6 +1695,7 @@ __global__ void __launch_bounds__(NT, (G == 1 && CPT == 1) ? 2 : 1) k_scan_fast(
 // the item and walks the ranges.  2.7 M candidates x 25 subspaces: 125 -> 66 us.
 __global__ void __launch_bounds__(512) k_scan_generic(IndexDev D, int G, int Ps, int pre, int lbl, uint64_t q,
                                                       Workspace w) {
+    chain_start();
     extern __shared__ __align__(16) float s_lut[];  // [32 G][256], swizzled
     uint32_t* s_pre = reinterpret_cast<uint32_t*>(s_lut + G * kCodes * 32);
     uint32_t* s_start = s_pre + Ps + 1;
@@ -1826,6 +1849,7 @@ template <int NT, int U>
 __global__ void __launch_bounds__(NT) k_select(IndexDev D, int Ps, int Kcap, int sorted_out, Workspace w,
                                                         float* __restrict__ out_dist,
                                                         uint64_t* __restrict__ out_ids, int k_out) {
+    chain_start();
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t* s_hist = reinterpret_cast<uint32_t*>(smem);                   // [kBins]
     uint64_t* s_bbuf = reinterpret_cast<uint64_t*>(s_hist + kBins);         // [kBCap]
@@ -2126,6 +2150,7 @@ constexpr uint32_t kRefChunk = 4096;
 
 
 __global__ void __launch_bounds__(1024) k_refine_plan(uint64_t q, Workspace w) {
+    chain_start();
     __shared__ unsigned long long s_w[32];
     const int t = threadIdx.x;
     const uint64_t per = (q + blockDim.x - 1) / blockDim.x;
@@ -2196,6 +2221,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_refine(IndexDev D, const float*
                                                      const float* __restrict__ data, int cap, int apply_pred,
                                                      int lbl, uint64_t q, Workspace w, float* __restrict__ out_dist,
                                                      uint64_t* __restrict__ out_ids, int k_out) {
+    chain_start();
     extern __shared__ __align__(16) unsigned char smem[];
     uint64_t* s_keys = reinterpret_cast<uint64_t*>(smem);           // [cap]
     float* s_q = reinterpret_cast<float*>(s_keys + cap);             // [d]
@@ -3063,6 +3089,25 @@ struct StageTimer {
     }
 };
 
+// Launches a kernel of the query path; with `chain`, as a programmatic dependent of the kernel before
+// it on the stream: its launch and its blocks' start overlap that kernel's run.  Used for batches of
+// up to kChainQueries queries, whose kernels are not much longer than a launch (one query: 67 -> 58
+// us, with the prologue's searches side by side).
+template <typename... P, typename... A>
+void launch_next(bool chain, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = chain ? 1 : 0;
+    CK(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+}
+
 template <typename K>
 int occupancy_blocks(K kernel, int threads, size_t smem) {
     int nb = 0;
@@ -3316,6 +3361,8 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     w.cap = sync_sizing ? ~0ull : cx.dist_buf.bytes / 4;
     if (sync_sizing) w.sel_cap = ~0ull;  // sized after k_batch
     const FilterDev f = filter_dev(idx);
+    // programmatic launches: small batches of the plain path (stage events would sit between them)
+    const bool chain = sync_sizing && P.break_down == 0 && q <= kChainQueries;
     StageTimer tm(idx, st, P.break_down != 0 && (sync_sizing || capture), capture ? &capture->stage_ev : nullptr,
                   capture ? &capture->stage_names : nullptr);
 
@@ -3323,7 +3370,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     if (sm_pro > 48 * 1024)
         CK(cudaFuncSetAttribute(k_prologue, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_pro));
     uint64_t launches = 0;  // kernels of this query, reported in the stats
-    k_prologue<<<(unsigned)q, kThreads, sm_pro, st>>>(D, idx->grid, f, c.qlabels, (int)c.label_cols, w);
+    launch_next(false, k_prologue, dim3((unsigned)q), kThreads, sm_pro, st, D, idx->grid, f, c.qlabels, (int)c.label_cols, w);
     CK_LAUNCH();
     launches++;
     tm.mark("prologue");
@@ -3357,13 +3404,14 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
         tm.mark("learned");
     }
 
-    k_coarse<<<(unsigned)q, kCoarseThreads, sm_co, st>>>(D, idx->grid, c.queries, Pc, Ps, sort_n1, sort_n2, w);
+    launch_next(chain && !use_gemm && !w.qps, k_coarse, dim3((unsigned)q), kCoarseThreads, sm_co, st, D, idx->grid, c.queries, Pc,
+                Ps, sort_n1, sort_n2, w);
     CK_LAUNCH();
     launches++;
     tm.mark("coarse");
 
     // candidate offsets, work items, batch sums, beta and the per-query budgets' inputs
-    k_batch<<<1, 1024, 0, st>>>(q, w);
+    launch_next(chain, k_batch, dim3(1), 1024, 0, st, q, w);
     CK_LAUNCH();
     launches++;
     uint64_t sc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -3406,8 +3454,9 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     // candidate ranges per query: one per probed list, or n_split per list when is_split
     const int R = Ps * w.nsplit;
     const size_t sm_tab = sizeof(uint32_t) * (2 * R + 1);
-    if (!sync_sizing || lazy || sc[3] > 0) {
-        if (fast && (pre || w.qsched)) {
+    const bool scanned = !sync_sizing || lazy || sc[3] > 0, pre_pass = fast && (pre || w.qsched);
+    if (scanned) {
+        if (pre_pass) {
             // the predicate pass of the predicate-first queries, then the ADC items that
             // follow from their survivors
             const bool lab4 = l == 4 && (reinterpret_cast<uintptr_t>(D.labels) & 15) == 0;
@@ -3432,11 +3481,11 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
                 const int slices = lut_slices(q, (int)G, sm_count());
                 const size_t sm = sizeof(float) * (kCodes / slices) * D.pq_len * 33;
                 CK(cudaFuncSetAttribute(k_lut, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-                k_lut<<<dim3((unsigned)((q + kLutQ - 1) / kLutQ), G, slices), 512, sm, st>>>(D, c.queries, q, (int)G,
-                                                                                            w.lut, w.lut16, w.item_off);
+                launch_next(chain && lazy && !pre_pass, k_lut, dim3((unsigned)((q + kLutQ - 1) / kLutQ), G, slices), 512, sm,
+                            st, D, c.queries, q, (int)G, w.lut, w.lut16, w.item_off);
             } else {
-                k_lut_plain<<<dim3((unsigned)q, G), 256, sizeof(float) * D.d, st>>>(D, c.queries, (int)G, w.lut,
-                                                                                  w.lut16, w.item_off);
+                launch_next(false, k_lut_plain, dim3((unsigned)q, G), 256, sizeof(float) * D.d, st, D, c.queries, (int)G,
+                            w.lut, w.lut16, w.item_off);
             }
             CK_LAUNCH();
             launches++;
@@ -3459,7 +3508,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             auto launch = [&](auto kern, int nt) {
                 CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
                 const int blocks = sm_count() * occupancy_blocks(kern, nt, sm);
-                kern<<<blocks, nt, sm, st>>>(D, R, q, w);
+                launch_next(chain && !prune, kern, dim3((unsigned)blocks), nt, sm, st, D, R, q, w);
             };
             if (G == 1) {
                 if (cpt == 1) launch(k_scan_fast<1, 512, 1>, 512);
@@ -3479,7 +3528,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             HDG_REQUIRE(sm <= 227 * 1024, HDG_ERR_UNSUPPORTED, "scan tables exceed shared memory");
             CK(cudaFuncSetAttribute(k_scan_generic, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
             const int blocks = sm_count() * occupancy_blocks(k_scan_generic, 512, sm);
-            k_scan_generic<<<blocks, 512, sm, st>>>(D, (int)G, R, pre, l, q, w);
+            launch_next(chain, k_scan_generic, dim3((unsigned)blocks), 512, sm, st, D, (int)G, R, pre, l, q, w);
         }
         CK_LAUNCH();
         launches++;
@@ -3491,7 +3540,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
                           (sorted_out ? sizeof(uint64_t) * next_pow2(std::max<uint32_t>(k, 2)) : 0) + sm_tab + 16;
     auto launch_sel = [&](auto kern, int nt) {
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_sel));
-        kern<<<(unsigned)q, nt, sm_sel, st>>>(D, R, (int)k, sorted_out, w, c.dist, c.ids, (int)k);
+        launch_next(chain && scanned, kern, dim3((unsigned)q), nt, sm_sel, st, D, R, (int)k, sorted_out, w, c.dist, c.ids, (int)k);
     };
     if (q <= (uint64_t)sm_count()) launch_sel(k_select<kSelThreadsFew, 8>, kSelThreadsFew);
     else launch_sel(k_select<kSelThreads, 4>, kSelThreads);
@@ -3499,7 +3548,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     launches++;
     tm.mark("select");
     if (mode != kPre) {
-        k_refine_plan<<<1, 1024, 0, st>>>(q, w);
+        launch_next(chain, k_refine_plan, dim3(1), 1024, 0, st, q, w);
         CK_LAUNCH();
         const int rcap = (int)next_pow2(k + 4 * kThreads);  // rounds of rcap - k exact distances
         const size_t sm_ref = sizeof(uint64_t) * rcap + sizeof(float) * D.d + 16;
@@ -3507,8 +3556,8 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
         // persistent over the refine items; no more CTAs than queries are useful for small batches
         const uint64_t blocks = std::min<uint64_t>((uint64_t)sm_count() * occupancy_blocks(k_refine, kThreads, sm_ref),
                                                    q + (cx.sel_buf.bytes / 4) / kRefChunk + 1);
-        k_refine<<<(unsigned)blocks, kThreads, sm_ref, st>>>(D, c.queries, c.data, rcap, mode == kPost ? 1 : 0, l, q,
-                                                            w, c.dist, c.ids, (int)k);
+        launch_next(chain, k_refine, dim3((unsigned)blocks), kThreads, sm_ref, st, D, c.queries, c.data, rcap,
+                    mode == kPost ? 1 : 0, l, q, w, c.dist, c.ids, (int)k);
         CK_LAUNCH();
         launches += 2;
         tm.mark("refine");
