@@ -458,7 +458,10 @@ def run_hdgrid(args):
     if pred_pass and p0["exps0"] > 1:
         bud_q = np.frombuffer(idx.debug_fetch("budget").tobytes(), np.uint32)[:nq].astype(np.uint64)
         adc_q = pre_q & (pass_q > bud_q)
-    pred_bytes, adc_bytes = algorithmic_scan_bytes(cand_q, np.where(pre_q & ~adc_q, 0, pass_q), pre_q, info["M"],
+    # with the estimate pass the ADC of a post-filter query covers only the candidates that its
+    # bounds left open (its finite distances)
+    scan_q = np.where(pre_q, cand_q, pass_q) if "estimate" in stage_ms else cand_q
+    pred_bytes, adc_bytes = algorithmic_scan_bytes(scan_q, np.where(pre_q & ~adc_q, 0, pass_q), pre_q, info["M"],
                                                    info["l"], read_q, chk_q, info["rank_pack_bytes"])
     pass_share = float(pass_q[pre_q].sum() / max(1, cand_q[pre_q].sum())) if pre_q.any() else None
     launches_per_step = int(stats["launches"])
@@ -545,7 +548,7 @@ def run_hdgrid(args):
         other = {"kernel": "k_scan_fast", "kernel_ms": scan_avg, "algorithmic_bytes": adc_bytes,
                  "achieved": adc_bytes / (scan_avg / 1e3) / 1e9}
     else:
-        kern, k_ms, k_bytes, k_cand = "k_scan_fast", scan_avg, adc_bytes, cand
+        kern, k_ms, k_bytes, k_cand = "k_scan_fast", scan_avg, adc_bytes, int(scan_q.sum())
         other = ({"kernel": "k_pre_scan", "kernel_ms": pred_avg, "algorithmic_bytes": pred_bytes,
                   "achieved": pred_bytes / (pred_avg / 1e3) / 1e9} if pred_avg > 0 else None)
     per_cand = k_bytes / max(k_cand, 1)

@@ -151,7 +151,6 @@ struct QueryCtx {
     uint64_t work_queries = 0;
     std::map<std::string, std::pair<size_t, size_t>> layout;  // name -> (offset, bytes)
     GraphState* graphs = nullptr;   // QUERY_GRAPH=1: graphs keyed by pointers and sizes
-    uint64_t* pinned = nullptr;     // [16] the batch scalars and the GEMM status word, read back per call
     // the last call's scalars, still on the device (a call that needed no host read)
     struct Lazy {
         bool pending = false;
@@ -167,7 +166,6 @@ struct QueryCtx {
     QueryCtx& operator=(const QueryCtx&) = delete;
     ~QueryCtx() {
         release_graphs(graphs);
-        if (pinned) cudaFreeHost(pinned);
         if (lazy.done) cudaEventDestroy(lazy.done);
     }
 };

@@ -2485,7 +2485,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_refine(IndexDev D, const float*
 //                threshold (candidates outside the row could matter) the query is scanned in full;
 //   k_scan_fast / k_select   the exact ADC of the open candidates and the smallest of them.
 // The selection is the full scan's.  10,000 queries x 227,000 candidates x 32 subspaces (n_cand
-// 9,384), estimate to select: 20.4 ms in full (a full scan, a select over every distance), EST_FIG.
+// 9,384), estimate to select: 20.4 ms in full (a full scan, a select over every distance), 7.3 ms this way.
 constexpr int kThrThreads = 512;
 constexpr uint32_t kThrMax = 4096;  // sampled candidates at most
 constexpr int kThrBins = 2048;
@@ -3248,9 +3248,12 @@ static void resolve_lazy(hdg_index* idx, QueryCtx& cx) {
     fill_stats(idx, cx.lazy.q, cx.lazy.k, cx.lazy.mode, cx.lazy.exps0, sc, cx.lazy.launches);
 }
 
-// The estimate pass pays from this many candidates in the batch and on the average query:
-// EST_RULE
-constexpr uint64_t kEstMinCands = 32ull << 20, kEstMinRow = 8192;
+// The estimate pass pays from this many candidates in the batch, on the average query and per
+// selected one.  With it / without, us, at (candidates, per query, per selected): 30 M, 60,000, 6.4:
+// 781 / 784; 117 M, 58,500, 6.2: 1,670 / 2,051; 74 M, 36,900, 6.7: 2,813 / 3,237; 60 M, 60,300, 21:
+// 1,467 / 2,092; 46 M, 228,000, 23: 840 / 1,147; but 18 M, 36,700, 6.8: 1,161 / 1,108; 73 M, 14,600,
+// 5.5: 3,499 / 3,425; 98 M, 24,600, 2.6: 2,362 / 2,345; 26 M, 5,200, 2.3: 2,314 / 2,029.
+constexpr uint64_t kEstMinCands = 32ull << 20, kEstMinRow = 8192, kEstMinRatio = 6;
 
 // Thresholds, row-tile entries (`entries` of them at most), estimates and the scan's work items.
 static void estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const QueryCall& c, int R, uint32_t G,
@@ -3423,7 +3426,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     launch_next(chain, k_batch, dim3(1), 1024, 0, st, q, w);
     CK_LAUNCH();
     launches++;
-    uint64_t sc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    uint64_t sc[10] = {0};  // the batch scalars, the GEMM status word, the row-tile sum
     // no host read: a small batch whose caller needs no totals and whose coarse stage has no
     // tensor-core status to report
     bool lazy = sync_sizing && !use_gemm && !coarse_out && P.break_down == 0 && q * (uint64_t)D.n <= kUnsizedPairs;
@@ -3438,11 +3441,10 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             if (!cx.lazy.done) CK(cudaEventCreateWithFlags(&cx.lazy.done, cudaEventDisableTiming));
             CK(cudaEventRecord(cx.lazy.done, st));
         } else {
-            if (!cx.pinned) CK(cudaMallocHost(reinterpret_cast<void**>(&cx.pinned), 16 * sizeof(uint64_t)));
-            CK(cudaMemcpyAsync(cx.pinned, w.scal, 10 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+            // (one copy; to ordinary memory, since page-locking it costs a new context milliseconds)
+            CK(cudaMemcpyAsync(sc, w.scal, sizeof(sc), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
-            std::memcpy(sc, cx.pinned, sizeof(sc));
-            HDG_REQUIRE((uint32_t)cx.pinned[8] == 0, HDG_ERR_TIMEOUT, "tensor-core wait expired in the coarse GEMM");
+            HDG_REQUIRE((uint32_t)sc[8] == 0, HDG_ERR_TIMEOUT, "tensor-core wait expired in the coarse GEMM");
             coarse = sc[0];
             selected = sc[7];
         }
@@ -3503,9 +3505,9 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
         // post-filter queries with many more candidates than budget: the estimate pass (not in a
         // captured graph, whose entry count is not known)
         const bool prune = sync_sizing && !lazy && mode == kPost && !w.qsched && fast && D.decoded && sc[0] >= kEstMinCands &&
-                           sc[0] / q >= kEstMinRow && cx.pinned[9] < (1ull << 32);
+                           sc[0] / q >= kEstMinRow && sc[0] >= kEstMinRatio * sc[7] && sc[9] < (1ull << 32);
         if (prune) {
-            estimate_pass(idx, cx, w, c, R, G, cx.pinned[9], st);
+            estimate_pass(idx, cx, w, c, R, G, sc[9], st);
             launches += 7;
             tm.mark("estimate");
         }

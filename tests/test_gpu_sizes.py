@@ -205,7 +205,7 @@ def _plain_and_full(cuda, ws, k, conf=()):
 def test_estimate_pass_equals_full_scan(cuda, case):
     import torch
     if case in ("m96", "fp16"):
-        ws = datasets.config2(scale=0.4, n_queries=2001, max_grids=30_000, lut_fp16=1 if case == "fp16" else 0)
+        ws = datasets.config2(scale=0.4, n_queries=2001, max_grids=30_000, exps0=2, lut_fp16=1 if case == "fp16" else 0)
     else:
         ws = datasets.config4(scale=0.04, n_queries=129 if case == "few" else 1500, clusters=16, sub_clusters=8,
                               n_list=16, sub_lists=100, exps0=8, max_grids=16384, pq_dim=64 if case == "m64" else 32,
