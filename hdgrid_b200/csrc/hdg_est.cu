@@ -383,9 +383,8 @@ __global__ void __launch_bounds__(kEstThreads, 1) k_est(const __grid_constant__ 
                 const uint32_t row = row0 + 32u * wd + at;
                 if (RANGES) {
                     const uint64_t o = G.off[cs][c] + slot;
-                    a.prow[o] = row + G.delta[cs][c];
-                    reinterpret_cast<unsigned char*>(a.drow + G.off[cs][c])[slot] =
-                        step0[((size_t)ms * kEstN + c) * kEstM + 32 * wd + at];
+                    a.prow[o] = (row + G.delta[cs][c]) |
+                                ((uint32_t)step0[((size_t)ms * kEstN + c) * kEstM + 32 * wd + at] << 24);
                 } else if (slot < a.cap) {
                     a.list[(uint64_t)G.qid[cs][c] * a.cap + slot] = a.row0 + row * a.row_step;
                 }

@@ -41,10 +41,11 @@ struct EstArgs {
     const uint32_t* ent_off;   // [tiles + 1]
     const uint32_t* nt_off;    // [tiles + 1] prefix of the entries' query tiles
     const uint4* ent;          // {query, first row | last row + 1 << 16 in the tile, position - pool row, 0}
-    const uint64_t* qoff;      // row of each query in dist / spos
-    uint32_t* prow;            // candidate positions of the kept rows
-    float* drow;               // and, a byte each from the start of the query's row, their steps:
+    const uint64_t* qoff;      // row of each query in prow
+    uint32_t* prow;            // kept rows: candidate position (below 2^24) | step << 24, the step
                                // 1 + (t - bound) * steps per unit, rounded, at most 255
+                               // (one word: with the steps as bytes beside the positions the
+                               // 10,000 x 227,000-candidate batch took 11.6 ms, 11.1 so)
     // every query against every row (k_est<false>), label boxes tested on the way
     uint32_t nq;
     uint32_t row0, row_step;   // base row of row r: row0 + r * row_step

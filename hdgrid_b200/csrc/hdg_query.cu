@@ -2685,7 +2685,6 @@ __global__ void __launch_bounds__(kPickThreads) k_est_pick(int R, Workspace w) {
     if (w.prq[qi] != 1) return;
     const uint32_t N = w.qstat[qi * 4], K = w.qbud[qi], ne = w.cand_count[qi];
     const uint64_t row = w.qoff[qi];
-    const unsigned char* st = reinterpret_cast<const unsigned char*>(w.dist + row);
     const bool err = *w.gemm_err != 0;
     for (int i = lane; i < 256; i += 32) s_hist[warp][i] = 0;
     if (t == 0) {
@@ -2694,13 +2693,14 @@ __global__ void __launch_bounds__(kPickThreads) k_est_pick(int R, Workspace w) {
     }
     __syncthreads();
     const int wd = w.est_w[qi];
-    // (rows start at any 4-byte boundary: words of four steps)
-    const uint32_t* st4 = reinterpret_cast<const uint32_t*>(st);
-    for (uint32_t i = t; 4 * i < ne; i += kPickThreads) {
-        const uint32_t x = __ldg(st4 + i);
+    uint32_t* prow = w.spos + row;  // position | step << 24
+    for (uint32_t e0 = t; e0 < ne; e0 += 4 * kPickThreads) {
+        uint32_t x[4];
 #pragma unroll
-        for (uint32_t u = 0; u < 4; u++)
-            if (4 * i + u < ne) atomicAdd(&s_hist[warp][(x >> (8 * u)) & 255u], 1u);
+        for (int u = 0; u < 4; u++) x[u] = e0 + u * kPickThreads < ne ? prow[e0 + u * kPickThreads] : 0u;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (e0 + u * kPickThreads < ne) atomicAdd(&s_hist[warp][x[u] >> 24], 1u);
     }
     __syncthreads();
     uint32_t c = 0;
@@ -2751,18 +2751,18 @@ __global__ void __launch_bounds__(kPickThreads) k_est_pick(int R, Workspace w) {
     for (int i = t; i <= R; i += kPickThreads) s_pre[i] = w.range_pre[qi * (R + 1) + i];
     for (int i = t; i < R; i += kPickThreads) s_start[i] = w.range_start[qi * R + i];
     __syncthreads();
-    uint32_t* prow = w.spos + row;
     uint32_t* open_row = reinterpret_cast<uint32_t*>(w.dist + row) + ne;
     uint32_t* sel = w.cand_pool + w.soff[qi];
-    for (uint32_t i0 = 0; 4 * i0 < ne; i0 += kPickThreads) {  // block-uniform bound
-        const uint32_t i = i0 + t;
-        const uint32_t x = 4 * i < ne ? __ldg(st4 + i) : 0u;
+    for (uint32_t e0 = 0; e0 < ne; e0 += 4 * kPickThreads) {  // block-uniform bound
+        uint32_t x[4];
 #pragma unroll
-        for (uint32_t u = 0; u < 4; u++) {
-            const uint32_t e = 4 * i + u;
-            const int val = e < ne ? (int)((x >> (8 * u)) & 255u) : 0;  // (steps are at least 1)
-            const bool in = val > hi, op = val >= lo && val <= hi;
-            const uint32_t p = in || op ? prow[e] : 0u;
+        for (int u = 0; u < 4; u++) x[u] = e0 + t + u * kPickThreads < ne ? prow[e0 + t + u * kPickThreads] : 0u;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const bool v = e0 + t + u * kPickThreads < ne;
+            const int val = (int)(x[u] >> 24);
+            const uint32_t p = x[u] & 0xffffffu;
+            const bool in = v && val > hi, op = v && val >= lo && val <= hi;
             const uint32_t a = warp_reserve(in, &s_cnt[0]), b = warp_reserve(op, &s_cnt[1]);
             if (in) sel[a] = p;
             if (op) prow[ne + b] = p;
@@ -3297,7 +3297,6 @@ static void estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const Quer
     a.nt_off = nt_off;
     a.ent = ent;
     a.qoff = w.qoff;
-    a.drow = w.dist;
     a.prow = w.spos;
     a.cnt = w.cand_count;
     CK(cudaMemsetAsync(diff, 0, (tiles + 1) * 4ull, st));
@@ -3505,7 +3504,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
         // post-filter queries with many more candidates than budget: the estimate pass (not in a
         // captured graph, whose entry count is not known)
         const bool prune = sync_sizing && !lazy && mode == kPost && !w.qsched && fast && D.decoded && sc[0] >= kEstMinCands &&
-                           sc[0] / q >= kEstMinRow && sc[0] >= kEstMinRatio * sc[7] && sc[9] < (1ull << 32);
+                           sc[0] / q >= kEstMinRow && sc[0] >= kEstMinRatio * sc[7] && sc[2] < (1u << 24) && sc[9] < (1ull << 32);
         if (prune) {
             estimate_pass(idx, cx, w, c, R, G, sc[9], st);
             launches += 7;
