@@ -462,6 +462,42 @@ __global__ void k_pack_ranks(const float* __restrict__ labels, uint64_t n, int l
     out[r] = packed;
 }
 
+// The ranks' bit planes (IndexDev::rank_planes).  A warp takes 256 rows: a ballot per plane and
+// word leaves lane v the eight words of plane v, written as one 32-byte sector.
+__global__ void __launch_bounds__(256) k_rank_planes(IndexDev D, uint64_t n, uint32_t* __restrict__ out) {
+    const uint64_t w0 = ((uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * 8;  // first word
+    const int lane = threadIdx.x & 31;
+    if (w0 >= D.plane_words) return;
+    uint32_t c[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const uint64_t r = (w0 + k) * 32 + lane;
+        c[k] = r < n ? __ldg(D.rankpack + r) : 0u;
+    }
+    for (uint32_t i = 0; i < D.l; i++) {
+        const uint32_t off = i * (D.rank_bits + 1), mask = (1u << D.rank_bits) - 1u;
+        const uint32_t planes = D.rank_n[i] >> D.plane_shift;
+        for (uint32_t v0 = 0; v0 < planes; v0 += 32) {
+            uint32_t word[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const uint32_t x = ((c[k] >> off) & mask) >> D.plane_shift;
+                word[k] = 0;
+#pragma unroll
+                for (uint32_t v = 0; v < 32; v++) {
+                    const uint32_t b = __ballot_sync(0xffffffffu, x <= v0 + v);
+                    if (lane == (int)v) word[k] = b;
+                }
+            }
+            if (v0 + lane < planes) {
+                uint4* o = reinterpret_cast<uint4*>(out + (D.plane_off[i] + v0 + lane) * D.plane_words + w0);
+                o[0] = make_uint4(word[0], word[1], word[2], word[3]);
+                o[1] = make_uint4(word[4], word[5], word[6], word[7]);
+            }
+        }
+    }
+}
+
 // codes [n][chunks] (16-byte chunks, row-major) -> [chunks][n]: chunk j of point p at j*n + p
 __global__ void k_interleave_codes(const uint4* __restrict__ rows, uint64_t n, uint32_t chunks,
                                    uint4* __restrict__ out) {
@@ -1344,6 +1380,7 @@ void label_rank_thresholds(const float* labels, uint64_t n, int l, int bits, flo
 }
 
 constexpr uint64_t kDecodedMax = 16ull << 30;
+constexpr uint64_t kPlanes = 512, kPlanesMax = 8ull << 30;  // label-rank bit planes: at most 64 bytes per point
 constexpr uint64_t kDecodedMinPoints = 16384;  // smaller sets never reach the estimate pass
 
 // Copy the host index into one device arena and fill idx->dev.
@@ -1532,6 +1569,28 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
     D.S_max = 0;
     for (uint64_t c = 0; c < H.C; c++)
         D.S_max = std::max<uint32_t>(D.S_max, H.cluster_off[c + 1] - H.cluster_off[c]);
+    // the ranks' bit planes: up to kPlanes of them in all, a bit of resolution less for as long as
+    // they would take more than kPlanesMax bytes
+    D.rank_planes = nullptr;
+    idx->planes.reset();
+    if (rbits && !D.labels_nan) {
+        D.plane_words = align_up((H.n + 31) / 32, 8);
+        D.plane_shift = 0;
+        while ((H.l << rbits) >> D.plane_shift > kPlanes) D.plane_shift++;
+        uint64_t planes = 0;
+        for (;; D.plane_shift++) {
+            planes = 0;
+            for (uint64_t i = 0; i < H.l; i++) {
+                D.plane_off[i] = (uint32_t)planes;
+                planes += rn[i] >> D.plane_shift;
+            }
+            if (planes * D.plane_words * 4 <= kPlanesMax) break;
+        }
+        idx->planes.ensure(std::max<uint64_t>(planes * D.plane_words * 4, 16));
+        k_rank_planes<<<blocks_for(D.plane_words, 64), 256, 0, st>>>(D, H.n, static_cast<uint32_t*>(idx->planes.ptr));
+        CK_LAUNCH();
+        D.rank_planes = static_cast<const uint32_t*>(idx->planes.ptr);
+    }
     // the estimate pass of the post-filter scan reads the points' PQ approximations as tensor-core
     // operands (2 d + 16 bytes per point; not kept past kDecodedMax, where the full scan runs)
     D.decoded = nullptr;

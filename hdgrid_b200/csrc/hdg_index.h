@@ -97,6 +97,12 @@ struct IndexDev {
     uint32_t rank_n[kMaxDims];
     float rank_min[kMaxDims], rank_max[kMaxDims];
     uint32_t rank_bits, rank_stride, rank_guard, rank_full;
+    // The same ranks as bit planes, for the predicate pass (derived at upload; nullptr with NaN
+    // labels): bit row % 32 of word row / 32 of plane plane_off[i] + v says that the row's rank of
+    // dim i, shifted right by plane_shift, is at most v (v below the dim's largest such value).
+    const uint32_t* rank_planes;
+    uint64_t plane_words;          // words of a plane (a multiple of 8)
+    uint32_t plane_shift, plane_off[kMaxDims];
     uint32_t labels_nan;           // some label is NaN (passes every label test, in any cell)
     const uint32_t* ids;
     const uint8_t* codes;
@@ -180,6 +186,7 @@ struct hdg_index {
     hdg::GridMeta grid;
     hdg::IndexDev dev{};
     hdg::DeviceBuffer arena;       // all index arrays
+    hdg::DeviceBuffer planes;      // derived at upload: the label ranks' bit planes
     hdg::DeviceBuffer decoded;     // derived at upload, not stored in the index file: the points'
                                    // PQ approximations in FP16 and their estimate constants
     hdg::DeviceBuffer map_buf;     // filter interval map

@@ -42,7 +42,7 @@ constexpr uint32_t kChunk = 32768;  // default most candidates per scan work ite
 constexpr uint32_t kChunkMin = 1024;
 constexpr int kBins = 4096;         // select histogram
 constexpr int kBCap = 4096;         // boundary-bin buffer of the select
-constexpr uint32_t kPreChunk = 8192; // candidates per work item of the predicate pass
+constexpr uint32_t kPreChunk = 16384, kPreChunkMin = 1024;  // candidates per work item of the predicate pass
 
 struct Workspace {
     float* box;              // [q x 2l]
@@ -173,6 +173,7 @@ __device__ __forceinline__ bool takes_row(const Workspace& w, uint64_t qi) {
 }
 // Candidates per scan work item (k_batch sets the word)
 __device__ __forceinline__ uint32_t scan_chunk(const Workspace& w) { return w.counter[3]; }
+__device__ __forceinline__ uint32_t pre_chunk(const Workspace& w) { return w.counter[4]; }
 // The selected candidates (pool rows) of query qi: its row of the selection buffer, or its
 // distance row when it takes the row whole
 __device__ __forceinline__ uint32_t* sel_row(const Workspace& w, uint64_t qi) {
@@ -839,23 +840,25 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
     // that leaves at most scan_items items.  A small batch then fills the SMs (37 queries of
     // 73,000 candidates ran as 111 items of up to 32,768 in 325 us, in 125 us this way); a large one keeps long
     // items, since each loads its query's LUT.
-    if (w.chunk) {
-        if (t == 0) s_chunk = w.chunk;
-        __syncthreads();
-    } else {
+    // Predicate items likewise, for 16 times as many items (a warp each): 64 queries of 47,000
+    // candidates took 188 us as items of 8,192.
+    __shared__ uint32_t s_pchunk;
+    {
         unsigned long long c = 0, all = 0;
         for (uint64_t i = b; i < e; i++) c += w.qstat[i * 4];
         block_inclusive_sum(c, s_tot, &all);
         if (t == 0) {
-            uint32_t ch = kChunkMin;
+            uint32_t ch = kChunkMin, pc = kPreChunkMin;
             while (ch < kChunk && (unsigned long long)ch * w.scan_items < all) ch *= 2;
-            s_chunk = ch;
+            while (pc < kPreChunk && (unsigned long long)pc * w.scan_items * 16u < all) pc *= 2;
+            s_chunk = w.chunk ? w.chunk : ch;
+            s_pchunk = pc;
         }
         __syncthreads();
     }
-    const uint32_t chunk = s_chunk;
+    const uint32_t chunk = s_chunk, pchunk = s_pchunk;
     auto n_items = [&](uint64_t i, uint32_t c) { return compacts(w, i) ? 0u : (c + chunk - 1) / chunk; };
-    auto n_pitems = [&](uint64_t i, uint32_t c) { return compacts(w, i) ? (c + kPreChunk - 1) / kPreChunk : 0u; };
+    auto n_pitems = [&](uint64_t i, uint32_t c) { return compacts(w, i) ? (c + pchunk - 1) / pchunk : 0u; };
     unsigned long long cand = 0, items = 0, pitems = 0, exact = 0, mx = 0, rtiles = 0;
     for (uint64_t i = b; i < e; i++) {
         rtiles += w.qtiles[i];
@@ -926,6 +929,7 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
         w.counter[0] = 0;
         w.counter[2] = 0;
         w.counter[3] = chunk;
+        w.counter[4] = pchunk;
     }
     __syncthreads();
     // each query's budget n_cand, now that the batch's beta and max_row are known, and the
@@ -1148,21 +1152,21 @@ __device__ __forceinline__ void scan_load_query(const Workspace& w, int Ps, int 
 // A predicate-first query (query_prefilter, prefiltering.cu:36-51; the learned schedule's
 // predicate-first flag) keeps only its candidates that pass the label predicate
 // (filter.cu:30-64), and only those need an ADC distance.  This pass runs before the ADC scan:
-// one warp per work item (kPreChunk consecutive candidate positions of one query), no
-// shared-memory LUT, so it runs at full occupancy and streams the candidates' packed label
-// ranks and labels.  A lane tests positions lane, lane + 32, ... of every step of 32 * J:
-//   1. the candidate's label ranks against the query's rank box, all dims in one guarded-field
-//      range test: a rank outside the box proves that the label test fails, so the candidate
-//      is rejected without reading its labels;
-//   2. the labels of the other candidates against the query's f32 box, 128 per batch from a
-//      per-warp queue, so that a batch's label loads are all useful;
-//   3. the survivors are staged per warp and appended to the query's row 32 at a time -- the
-//      candidate position into spos and the pool row into the distance slot, which the ADC
-//      scan then overwrites with the survivor's distance.
+// one warp per work item (pre_chunk consecutive candidate positions of one query), no
+// shared-memory LUT.  A lane takes words of 32 pool rows and tests their label ranks by bit planes,
+// the two at the ends of every constrained dim's box ANDed:
+//   1. against the query's rank box: a rank outside it proves that the label test fails;
+//   2. against its inner box: a rank inside proves that the test passes (a survivor);
+//   3. only the rows between the two have their labels read, up to 128 per batch from a per-warp
+//      queue, so that a batch's label loads are all useful;
+//   4. the survivors are staged per warp and appended to the query's row -- the candidate position
+//      into spos and the pool row into the distance slot, which the ADC scan then overwrites with
+//      the survivor's distance.
 // The row's order depends on timing; the distance of each survivor does not (the ADC order
 // follows its position) and the select orders ties by position.
 constexpr int kPreThreads = 256;
-constexpr int kPreRingWords = 4 * 128 + 2 * 512 + 2 * 64;  // shared words per warp: labels, queue, survivors
+// shared words per warp: labels, queue, survivors, ranges, planes
+constexpr int kPreRingWords = 4 * 128 + 2 * 256 + 2 * 128 + 4 * 32 + 2 * 4 * kMaxDims;
 
 // Largest i in [0, n) with a[i] <= key (a nondecreasing, a[0] <= key), by 32-way rounds.
 // Every lane of the warp calls it and gets the answer.
@@ -1196,6 +1200,27 @@ __device__ __forceinline__ void ring_push(uint32_t* ring, uint32_t& t, bool f, u
     t += __popc(bal);
 }
 
+// Appends the rows of every lane's word m (first row p32, position - row delta; n of them in the
+// warp) in row order.  All lanes.
+template <uint32_t SIZE>
+__device__ __forceinline__ void push_own(uint32_t* ring, uint32_t& t, uint32_t m, uint32_t n, uint32_t p32, uint32_t delta) {
+    const int lane = threadIdx.x & 31;
+    uint32_t at = __popc(m);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += y;
+    }
+    at += t - __popc(m);
+    for (; m; m &= m - 1u, at++) {
+        const uint32_t p = p32 + (uint32_t)__ffs((int)m) - 1u, s = at & (SIZE - 1);
+        ring[s] = p + delta;
+        ring[SIZE + s] = p;
+    }
+    __syncwarp();
+    t += n;
+}
+
 // 16-byte asynchronous global -> shared copy (cp.async, cached in L2 only) and its groups
 __device__ __forceinline__ void cp16_async(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
@@ -1205,27 +1230,242 @@ __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// One predicate-pass work item: positions [e0, e1) of one query (R ranges, prefix pre, starts
-// start; r0 the range of e0).  CHECK: test the rank box first (lo_f / hi_g / gd: the box's low
-// ranks, its high ranks with the guard bits set, the guard bits), LAB4: four 16-byte-aligned
-// label dims.  qr: [2][512] ring of rank-passed candidates (without CHECK: of survivors), sr:
-// [2][64] survivor ring, lst: [128] staged labels (LAB4).  n_chk / n_read: candidates whose
-// ranks / labels were read (warp totals).
-template <bool CHECK, bool LAB4>
-__device__ __forceinline__ void pre_span(const IndexDev& D, int lbl, const float* bx_s, uint32_t lo_f, uint32_t hi_g,
-                                         uint32_t gd,
-                                         const uint32_t* pre, const uint32_t* start, int R, int r0, uint32_t e0,
-                                         uint32_t e1, uint32_t* qr, uint32_t* sr, float4* lst, uint32_t* ctr,
-                                         uint32_t* drow, uint32_t* prow, uint32_t& n_read, uint32_t& n_chk) {
-    constexpr int J = 8;  // windows of 32 positions in one step
-    constexpr uint32_t QS = 512, SS = 64, LB = 128;
+// m (<= 32) entries from a ring's head to the query's row: position into spos, pool row into the
+// distance slot.  All lanes.
+__device__ __forceinline__ void pre_flush(const uint32_t* ring, uint32_t size, uint32_t h, int m, uint32_t* ctr,
+                                          uint32_t* drow, uint32_t* prow) {
     const int lane = threadIdx.x & 31;
-    const uint32_t* ranks = D.rankpack;
+    __syncwarp();
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(ctr, (uint32_t)m);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (lane < m) {
+        const uint32_t s = (h + lane) & (size - 1);
+        prow[at + lane] = ring[s];
+        drow[at + lane] = ring[size + s];
+    }
+    __syncwarp();
+}
+
+// the label predicate (a NaN label passes, as in the reference); bx_s: the query's box in shared memory
+__device__ __forceinline__ bool pre_box4(const float* bx_s, const float4& v) {
+    const float4 b0 = reinterpret_cast<const float4*>(bx_s)[0], b1 = reinterpret_cast<const float4*>(bx_s)[1];
+    return !(v.x < b0.x || v.x > b0.y) && !(v.y < b0.z || v.y > b0.w) && !(v.z < b1.x || v.z > b1.y) &&
+           !(v.w < b1.z || v.w > b1.w);
+}
+template <bool LAB4>
+__device__ __forceinline__ bool pre_label_ok(const IndexDev& D, int lbl, const float* bx_s, uint32_t p) {
+    if (LAB4) return pre_box4(bx_s, __ldg(reinterpret_cast<const float4*>(D.labels) + p));
+    bool ok = true;
+    const float* lab = D.labels + (uint64_t)p * lbl;
+    for (int i = 0; i < lbl; i++) {
+        const float v = __ldg(lab + i);
+        if (v < bx_s[2 * i] || v > bx_s[2 * i + 1]) ok = false;
+    }
+    return ok;
+}
+
+// The planes of one rank box: first words p[0 .. n), those from n_hi on to be inverted.
+struct PreBox {
+    const uint32_t* const* p;
+    int n_hi, n;
+};
+__device__ __forceinline__ uint32_t pre_word(const PreBox& x, uint32_t w) {
+    uint32_t m = 0xffffffffu;
+    for (int k = 0; k < x.n; k += 4) {
+        uint32_t v[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            v[i] = k + i < x.n ? __ldg(x.p[k + i] + w) ^ (k + i < x.n_hi ? 0u : 0xffffffffu) : 0xffffffffu;
+        m &= v[0] & v[1] & v[2] & v[3];
+    }
+    return m;
+}
+
+// One predicate-pass work item by the ranks' bit planes: positions [e0, e1) of one query (R ranges,
+// prefix pre, starts start; r0 the range of e0), outer / inner: its rank boxes (has_inner: some rank
+// passes for sure).  LAB4: four 16-byte-aligned label dims.  qr: [2][256] ring of candidates whose
+// labels decide, sr: [2][128] survivor ring, lst: [128] staged labels (LAB4), rt: [32] ranges.
+// n_read: candidates whose labels were read.
+template <bool LAB4>
+__device__ __forceinline__ void pre_bits(const IndexDev& D, int lbl, const float* bx_s, const PreBox& outer,
+                                         const PreBox& inner, bool has_inner, const uint32_t* pre, const uint32_t* start, int R, int r0, uint32_t e0,
+                                         uint32_t e1, uint32_t* qr, uint32_t* sr, float4* lst, uint4* rt, uint32_t* ctr,
+                                         uint32_t* drow, uint32_t* prow, uint32_t& n_read) {
+    constexpr uint32_t QS = 256, SS = 128, LB = 128;
+    const int lane = threadIdx.x & 31;
+    const float4* lab4 = reinterpret_cast<const float4*>(D.labels);
+    uint32_t sh = 0, st = 0;
+    auto stage_surv = [&](bool f, uint32_t e, uint32_t p) {
+        ring_push<SS>(sr, st, f, e, p);
+        if (st - sh >= 32) {
+            pre_flush(sr, SS, sh, 32, ctr, drow, prow);
+            sh += 32;
+        }
+    };
+    // qr holds [qh, qi) whose labels are on their way into lst, then [qi, qt) queued.  issue() starts
+    // a batch's 16-byte label copies (cp.async: no registers held while they fly), consume() tests a
+    // batch once its copies have landed.
+    uint32_t qh = 0, qi = 0, qt = 0;
+    auto issue = [&]() {
+        const uint32_t m = qt - qi;  // at most LB
+        __syncwarp();                // the pushes of every lane are visible
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t k = lane + 32u * u;
+            if (LAB4 && k < m) cp16_async(lst + k, lab4 + qr[QS + ((qi + k) & (QS - 1))]);
+        }
+        if (LAB4) cp_commit();
+        qi = qt;
+    };
+    auto consume = [&]() {
+        const uint32_t m = qi - qh;
+        if (LAB4) cp_wait<0>();
+        __syncwarp();  // every lane's copies have landed
+#pragma unroll 1
+        for (uint32_t k0 = 0; k0 < m; k0 += 32) {
+            const uint32_t k = k0 + lane;
+            const bool v = k < m;
+            const uint32_t s = (qh + k) & (QS - 1);
+            const uint32_t e = v ? qr[s] : 0u, p = v ? qr[QS + s] : 0u;
+            bool ok = false;
+            if (v) ok = LAB4 ? pre_box4(bx_s, lst[k]) : pre_label_ok<LAB4>(D, lbl, bx_s, p);
+            stage_surv(ok, e, p);
+        }
+        qh = qi;
+        __syncwarp();  // lst and the consumed ring slots are free again
+    };
+    // Ranges come 32 at a time, the non-empty ones of them as rt[j] = {first word - words before, first
+    // row, end row, position - row}; lane j keeps the words before range j (first).  A step is 32 of
+    // their words, one per lane.
+    int rnext = r0;
+    uint32_t first = 0xffffffffu, total = 0, t0 = 0, done = 0;  // done: ranges that begin before word t0
+    uint32_t m = 0, p32 = 0, delta = 0;                         // the lane's word: open rows, its first row
+    for (bool more = true;;) {
+        while (qt - qi <= LB - 64u) {
+            // the open rows in row order (so that the survivors' codes are read in order): a lane's own
+            // rows one after another while they are few, else word by word with a lane per row
+            const uint32_t open = __reduce_add_sync(0xffffffffu, __popc(m));
+            if (open > 64) {
+                unsigned nz = __ballot_sync(0xffffffffu, m != 0);
+                while (nz && qt - qi <= LB - 32u) {
+                    const int j = __ffs((int)nz) - 1;
+                    const uint32_t mj = __shfl_sync(0xffffffffu, m, j), pj = __shfl_sync(0xffffffffu, p32, j) + lane;
+                    const uint32_t dj = __shfl_sync(0xffffffffu, delta, j);
+                    if (mj >> lane & 1u) {
+                        const uint32_t s = (qt + __popc(mj & ((1u << lane) - 1u))) & (QS - 1);
+                        qr[s] = pj + dj;
+                        qr[QS + s] = pj;
+                    }
+                    qt += __popc(mj);
+                    if (lane == j) m = 0;
+                    nz &= nz - 1;
+                }
+                continue;
+            }
+            if (open) {
+                push_own<QS>(qr, qt, m, open, p32, delta);
+                m = 0;
+                continue;
+            }
+            if (t0 >= total) {
+                if (rnext >= R || pre[rnext] >= e1) {
+                    more = false;
+                    break;
+                }
+                const int r = rnext + lane;
+                uint32_t nw = 0, w0 = 0, p0 = 0, p1 = 0, dl = 0;
+                if (r < R) {
+                    const uint32_t f = pre[r], a = max(f, e0), b = min(pre[r + 1], e1);
+                    if (a < b) {
+                        dl = f - start[r];
+                        p0 = a - dl;
+                        p1 = b - dl;
+                        w0 = p0 >> 5;
+                        nw = ((p1 - 1u) >> 5) - w0 + 1u;
+                    }
+                }
+                uint32_t inc = nw;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= o) inc += y;
+                }
+                const unsigned some = __ballot_sync(0xffffffffu, nw != 0);
+                __syncwarp();  // the last step's reads of rt are done
+                if (nw) rt[__popc(some & ((1u << lane) - 1u))] = make_uint4(w0 - (inc - nw), p0, p1, dl);
+                total = __shfl_sync(0xffffffffu, inc, 31);
+                first = nw ? inc - nw : 0xffffffffu;
+                __syncwarp();
+                t0 = done = 0;
+                rnext += 32;
+                if (!total) continue;
+            }
+            const uint32_t starts = __reduce_or_sync(0xffffffffu, first - t0 < 32u ? 1u << (first - t0) : 0u);
+            const uint32_t u = t0 + lane;
+            uint32_t sure = 0;
+            if (u < total) {
+                const uint4 g = rt[done + __popc(starts & (0xffffffffu >> (31 - lane))) - 1u];
+                const uint32_t w = g.x + u;
+                p32 = w << 5;
+                delta = g.w;
+                m = 0xffffffffu;
+                if (g.y > p32) m <<= g.y - p32;
+                if (g.z - p32 < 32u) m &= (1u << (g.z - p32)) - 1u;
+                m &= pre_word(outer, w);
+                if (has_inner && m) {
+                    sure = m & pre_word(inner, w);
+                    m &= ~sure;
+                }
+            }
+            const uint32_t n_sure = __reduce_add_sync(0xffffffffu, __popc(sure));
+            if (n_sure > 64) {  // straight to the query's row, word by word with a lane per row
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(ctr, n_sure);
+                at = __shfl_sync(0xffffffffu, at, 0);
+                for (unsigned nz = __ballot_sync(0xffffffffu, sure != 0); nz; nz &= nz - 1) {
+                    const int j = __ffs((int)nz) - 1;
+                    const uint32_t mj = __shfl_sync(0xffffffffu, sure, j), pj = __shfl_sync(0xffffffffu, p32, j) + lane;
+                    const uint32_t dj = __shfl_sync(0xffffffffu, delta, j);
+                    if (mj >> lane & 1u) {
+                        const uint32_t s = at + __popc(mj & ((1u << lane) - 1u));
+                        prow[s] = pj + dj;
+                        drow[s] = pj;
+                    }
+                    at += __popc(mj);
+                }
+            } else if (n_sure) {
+                push_own<SS>(sr, st, sure, n_sure, p32, delta);
+                while (st - sh >= 32) {
+                    pre_flush(sr, SS, sh, 32, ctr, drow, prow);
+                    sh += 32;
+                }
+            }
+            done += __popc(starts);
+            t0 += 32;
+        }
+        if (qi != qh) consume();
+        if (qt != qi) issue();
+        else if (!more) break;
+    }
+    n_read += qt;  // every queued candidate had its labels read
+    if (st != sh) pre_flush(sr, SS, sh, (int)(st - sh), ctr, drow, prow);
+}
+
+// The same without the rank test, for an index with NaN labels (a NaN passes the label test): every
+// candidate's labels are read.  Out of line, so that the other loop stays compact in the instruction
+// cache.  qr: [2][256] ring of survivors.
+template <bool LAB4>
+__device__ __noinline__ void pre_labels(const IndexDev& D, int lbl, const float* bx_s, const uint32_t* pre,
+                                        const uint32_t* start, int R, int r0, uint32_t e0, uint32_t e1, uint32_t* qr,
+                                        uint32_t* ctr, uint32_t* drow, uint32_t* prow) {
+    constexpr int J = 4;  // windows of 32 positions in one step: as many label loads in flight
+    constexpr uint32_t QS = 256;
+    const int lane = threadIdx.x & 31;
     const float4* lab4 = reinterpret_cast<const float4*>(D.labels);
     // Position -> pool row (warp-uniform state): the current range rc holds positions up to
-    // nb1 (pool row = bc + position), the next non-empty range from nb1 up to nb2 (bn).  A step
-    // with at most one range start inside reads the two bases; a window with more (ranges
-    // shorter than 32) walks per lane.
+    // nb1 (pool row = bc + position), the next non-empty range from nb1 up to nb2 (bn).  A window
+    // with two or more range starts walks per lane.
     int rc = r0, rn = r0;
     uint32_t nb1 = pre[r0 + 1], bc = start[r0] - pre[r0], nb2 = 0xffffffffu, bn = 0;
     const uint32_t total = pre[R];
@@ -1245,199 +1485,53 @@ __device__ __forceinline__ void pre_span(const IndexDev& D, int lbl, const float
             find_next();
         }
     };
-    // (the box stays in shared memory: the label tests are rare and the registers go to loads in flight)
-    auto box4 = [&](const float4& v) {
-        const float4 b0 = reinterpret_cast<const float4*>(bx_s)[0], b1 = reinterpret_cast<const float4*>(bx_s)[1];
-        return !(v.x < b0.x || v.x > b0.y) && !(v.y < b0.z || v.y > b0.w) && !(v.z < b1.x || v.z > b1.y) &&
-               !(v.w < b1.z || v.w > b1.w);
-    };
-    // the label predicate of the candidate at pool row p (a NaN label passes, as in the reference)
-    auto label_ok = [&](uint32_t p) -> bool {
-        if (LAB4) return box4(__ldg(lab4 + p));
-        bool ok = true;
-        const float* lab = D.labels + (uint64_t)p * lbl;
-        for (int i = 0; i < lbl; i++) {
-            const float v = __ldg(lab + i);
-            if (v < bx_s[2 * i] || v > bx_s[2 * i + 1]) ok = false;
-        }
-        return ok;
-    };
-    // m (<= 32) entries from a ring's head to the query's row: position into spos, pool row
-    // into the distance slot
-    auto flush = [&](const uint32_t* ring, uint32_t size, uint32_t h, int m) {
-        __syncwarp();
-        uint32_t at = 0;
-        if (lane == 0) at = atomicAdd(ctr, (uint32_t)m);
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (lane < m) {
-            const uint32_t s = (h + lane) & (size - 1);
-            prow[at + lane] = ring[s];
-            drow[at + lane] = ring[size + s];
-        }
-        __syncwarp();
-    };
-    uint32_t sh = 0, st = 0;
-    auto stage_surv = [&](bool f, uint32_t e, uint32_t p) {
-        ring_push<SS>(sr, st, f, e, p);
-        if (st - sh >= 32) {
-            flush(sr, SS, sh, 32);
-            sh += 32;
-        }
-    };
-    // Label batches (CHECK): qr holds [qh, qi) whose labels are on their way into lst, then
-    // [qi, qt) queued.  issue() starts the next batch's 16-byte label copies (cp.async: no
-    // registers held while they fly), consume() tests a batch once its copies have landed.
-    uint32_t qh = 0, qi = 0, qt = 0;
-    auto issue = [&](uint32_t m) {
-        __syncwarp();  // the pushes of every lane are visible
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const uint32_t k = lane + 32u * u;
-            if (LAB4 && k < m) cp16_async(lst + k, lab4 + qr[QS + ((qi + k) & (QS - 1))]);
-        }
-        if (LAB4) cp_commit();
-        qi += m;
-    };
-    auto consume = [&]() {
-        const uint32_t m = qi - qh;
-        if (LAB4) cp_wait<0>();
-        __syncwarp();  // every lane's copies have landed
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const uint32_t k = lane + 32u * u;
-            const bool v = k < m;
-            const uint32_t s = (qh + k) & (QS - 1);
-            const uint32_t e = v ? qr[s] : 0u, p = v ? qr[QS + s] : 0u;
-            bool ok = false;
-            if (v) ok = LAB4 ? box4(lst[k]) : label_ok(p);
-            stage_surv(ok, e, p);
-        }
-        qh = qi;
-        __syncwarp();  // lst and the consumed ring slots are free again
-    };
-    // one pass past the last step drains the queue (a single copy of the label-batch code)
-    for (uint32_t eb = e0;; eb += 32u * J) {
-        const bool last_pass = eb >= e1;
-        if (CHECK) {
-            // test the batch in flight, start the next one; drain more only when the ring has no
-            // room for this step's pushes (or, after the last step, until it is empty)
-            for (;;) {
-                if (qi != qh) consume();
-                const uint32_t pend = qt - qh;
-                if (pend >= LB || (last_pass && pend > 0)) issue(min(LB, pend));
-                if (last_pass ? qi == qh : qt - qh <= QS - 32u * J) break;
-            }
-        }
-        if (last_pass) break;
+    uint32_t qh = 0, qt = 0;
+    for (uint32_t eb = e0; eb < e1; eb += 32u * J) {
         uint32_t pp[J];
         bool pv[J];
-        const uint32_t last = min(e1, eb + 32u * J) - 1;  // the step's last position
-        if (last < nb1 && eb + 32u * J <= e1) {  // a whole step inside the current range
 #pragma unroll
-            for (int j = 0; j < J; j++) {
-                pv[j] = true;
-                pp[j] = bc + eb + 32u * j + lane;
+        for (int j = 0; j < J; j++) {
+            const uint32_t p = eb + 32u * j, e = p + lane;  // the window [p, p + 32)
+            pv[j] = e < e1;
+            uint32_t base;
+            if (p + 31u < nb2) {
+                base = e < nb1 ? bc : bn;
+            } else {  // two or more ranges start inside the window
+                int r = rc;
+                if (pv[j])
+                    while (pre[r + 1] <= e) r++;
+                base = start[r] - pre[r];
             }
-            advance_to(eb + 32u * J);
-        } else if (last < nb2) {  // at most one range starts inside the step
+            pp[j] = pv[j] ? base + e : 0u;
+            advance_to(p + 32u);
+        }
+        if (LAB4) {
+            float4 v[J];
 #pragma unroll
-            for (int j = 0; j < J; j++) {
-                const uint32_t e = eb + 32u * j + lane;
-                pv[j] = e < e1;
-                pp[j] = pv[j] ? (e < nb1 ? bc : bn) + e : 0u;
-            }
-            advance_to(eb + 32u * J);
+            for (int j = 0; j < J; j++) v[j] = pv[j] ? __ldg(lab4 + pp[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < J; j++)
+                ring_push<QS>(qr, qt, pv[j] && pre_box4(bx_s, v[j]), eb + 32u * j + lane, pp[j]);
         } else {
 #pragma unroll
-            for (int j = 0; j < J; j++) {
-                const uint32_t p = eb + 32u * j, e = p + lane;  // the window [p, p + 32)
-                pv[j] = e < e1;
-                uint32_t base;
-                if (p + 31u < nb2) {
-                    base = e < nb1 ? bc : bn;
-                } else {  // two or more ranges start inside the window
-                    int r = rc;
-                    if (pv[j])
-                        while (pre[r + 1] <= e) r++;
-                    base = start[r] - pre[r];
-                }
-                pp[j] = pv[j] ? base + e : 0u;
-                advance_to(p + 32u);
-            }
+            for (int j = 0; j < J; j++)
+                ring_push<QS>(qr, qt, pv[j] && pre_label_ok<LAB4>(D, lbl, bx_s, pp[j]), eb + 32u * j + lane, pp[j]);
         }
-        if constexpr (CHECK) {
-            uint32_t c[J];
-#pragma unroll
-            for (int j = 0; j < J; j++) c[j] = pv[j] ? __ldg(ranks + pp[j]) : 0u;
-#pragma unroll
-            for (int j = 0; j < J; j++) {
-                // every field at or above its low bound and at or below its high bound: the
-                // guard bit above a field survives both subtractions exactly then
-                const uint32_t t = ((c[j] | gd) - lo_f) & (hi_g - c[j]);
-                ring_push<QS>(qr, qt, pv[j] && (t & gd) == gd, eb + 32u * j + lane, pp[j]);
-            }
-        } else {
-            if (LAB4) {
-                // four 16-byte label loads in flight at a time
-#pragma unroll
-                for (int j0 = 0; j0 < J; j0 += 4) {
-                    float4 v[4];
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        v[j] = pv[j0 + j] ? __ldg(lab4 + pp[j0 + j]) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        ring_push<QS>(qr, qt, pv[j0 + j] && box4(v[j]), eb + 32u * (j0 + j) + lane, pp[j0 + j]);
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < J; j++)
-                    ring_push<QS>(qr, qt, pv[j] && label_ok(pp[j]), eb + 32u * j + lane, pp[j]);
-            }
-            while (qt - qh >= 32) {
-                flush(qr, QS, qh, 32);
-                qh += 32;
-            }
+        while (qt - qh >= 32) {
+            pre_flush(qr, QS, qh, 32, ctr, drow, prow);
+            qh += 32;
         }
     }
-    if (CHECK) {
-        n_read += qt;  // every rank-passed candidate had its labels read
-        n_chk += e1 - e0;
-        for (;;) {
-            if (qi != qh) consume();
-            if (qt == qh) break;
-            issue(min(LB, qt - qh));
-        }
-        if (st != sh) flush(sr, SS, sh, (int)(st - sh));
-    } else {
-        n_read += e1 - e0;
-        while (qt != qh) {
-            const int m = (int)min(32u, qt - qh);
-            flush(qr, QS, qh, m);
-            qh += (uint32_t)m;
-        }
-    }
-}
-
-// The pass without the rank test (queries with most candidates inside the cell box, or an index
-// with NaN labels) is called out of line, so that the hot loop with the test stays compact in
-// the instruction cache
-template <bool LAB4>
-__device__ __noinline__ void pre_span_labels(const IndexDev& D, int lbl, const float* bx_s, const uint32_t* pre,
-                                             const uint32_t* start, int R, int r0, uint32_t e0, uint32_t e1,
-                                             uint32_t* qr, uint32_t* sr, float4* lst, uint32_t* ctr, uint32_t* drow,
-                                             uint32_t* prow, uint32_t& n_read, uint32_t& n_chk) {
-    pre_span<false, LAB4>(D, lbl, bx_s, 0u, 0u, 0u, pre, start, R, r0, e0, e1, qr, sr, lst, ctr, drow, prow, n_read,
-                          n_chk);
+    if (qt != qh) pre_flush(qr, QS, qh, (int)(qt - qh), ctr, drow, prow);
 }
 
 template <bool LAB4>
 __global__ void __launch_bounds__(kPreThreads, 4) k_pre_scan(IndexDev D, int R, int lbl, uint64_t q, Workspace w) {
     constexpr int NW = kPreThreads / 32;
-    extern __shared__ __align__(16) uint32_t s_rings[];  // per warp: staged labels, queue ring, survivor ring
+    extern __shared__ __align__(16) uint32_t s_rings[];  // per warp: staged labels, ranges, planes, queue ring, survivor ring
     __shared__ __align__(16) float s_bx[NW][2 * kMaxDims];
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const uint32_t n_items = w.pitem_off[q];
+    const uint32_t n_items = w.pitem_off[q], chunk = pre_chunk(w);
     for (;;) {
         __syncwarp();  // the previous item's reads of the warp's tables are done
         uint32_t item = 0;
@@ -1446,19 +1540,47 @@ __global__ void __launch_bounds__(kPreThreads, 4) k_pre_scan(IndexDev D, int R, 
         if (item >= n_items) break;
         const int qq = warp_find_le(w.pitem_off, (int)q, item);
         const uint32_t total = w.qstat[(uint64_t)qq * 4];
-        const uint32_t e0 = (item - w.pitem_off[qq]) * kPreChunk;
+        const uint32_t e0 = (item - w.pitem_off[qq]) * chunk;
         if (e0 >= total) continue;  // a query cut by a capacity
-        const uint32_t e1 = min(total, e0 + kPreChunk);
+        const uint32_t e1 = min(total, e0 + chunk);
         if (lane < 2 * lbl) s_bx[wp][lane] = w.box[(uint64_t)qq * 2 * lbl + lane];
-        // The query's rank box (label ranks: see IndexDev) rejects a candidate whose labels
-        // must fail without reading them.  Skipped when it rejects nothing, when the index holds
-        // NaN labels (a NaN passes the label test), or when the query's count of points in its
-        // cell box over the probed lists says that most candidates pass anyway.
-        const uint32_t inbox = w.qstat[(uint64_t)qq * 4 + 1];
-        const uint32_t rlo = w.rank_box[4 * qq], rhi = w.rank_box[4 * qq + 1];
-        const bool use = D.rankpack && !D.labels_nan && (rlo != 0 || rhi != (D.rank_full | D.rank_guard)) &&
-                         (uint64_t)inbox * 16 < (uint64_t)total * 12;
-        __syncwarp();  // s_bx is written
+        const bool use = D.rank_planes != nullptr;
+        float4* lst = reinterpret_cast<float4*>(s_rings + (size_t)wp * kPreRingWords);
+        uint4* rt = reinterpret_cast<uint4*>(lst + 128);
+        const uint32_t** pl = reinterpret_cast<const uint32_t**>(rt + 32);
+        uint32_t* qr = reinterpret_cast<uint32_t*>(pl + 4 * kMaxDims);
+        uint32_t* sr = qr + 2 * 256;
+        // lane i: the planes of dim i's bounds, absent where a bound excludes no (shifted) rank
+        auto planes_of = [&](uint32_t a, uint32_t b, const uint32_t** out) {
+            bool hi = false, lo = false;
+            const uint32_t *ph = nullptr, *plo = nullptr;
+            if (lane < lbl) {
+                hi = b < D.rank_n[lane] >> D.plane_shift;
+                lo = a > 0;
+                ph = D.rank_planes + ((uint64_t)D.plane_off[lane] + b) * D.plane_words;
+                plo = D.rank_planes + ((uint64_t)D.plane_off[lane] + a - 1u) * D.plane_words;
+            }
+            const unsigned bh = __ballot_sync(0xffffffffu, hi), bl = __ballot_sync(0xffffffffu, lo);
+            const unsigned below = (1u << lane) - 1u;
+            const int n_hi = __popc(bh);
+            if (hi) out[__popc(bh & below)] = ph;
+            if (lo) out[n_hi + __popc(bl & below)] = plo;
+            return PreBox{out, n_hi, n_hi + __popc(bl)};
+        };
+        PreBox outer{}, inner{};
+        bool has_inner = false;
+        if (use) {
+            const uint32_t sft = D.plane_shift, mask = (1u << D.rank_bits) - 1u;
+            const uint32_t off = lane < lbl ? lane * (D.rank_bits + 1) : 0u, top = lane < lbl ? D.rank_n[lane] : 0u;
+            auto field = [&](int k) { return (w.rank_box[4 * qq + k] >> off) & mask; };
+            outer = planes_of(field(0) >> sft, field(1) >> sft, pl);
+            // the inner box in shifted ranks: those whose every rank lies in it
+            const uint32_t il = field(2), ih = field(3), a = (il + (1u << sft) - 1u) >> sft;
+            const uint32_t b1 = ih >= top ? (top >> sft) + 1u : (ih + 1u) >> sft;  // one past the last
+            has_inner = __all_sync(0xffffffffu, lane >= lbl || (il <= ih && a < b1));
+            if (has_inner) inner = planes_of(a, b1 - 1u, pl + 2 * kMaxDims);
+        }
+        __syncwarp();  // s_bx and pl are written
         const uint32_t* pre = w.range_pre + (uint64_t)qq * (R + 1);
         const uint32_t* start = w.range_start + (uint64_t)qq * R;
         const int r0 = warp_find_le(pre, R, e0);
@@ -1467,15 +1589,13 @@ __global__ void __launch_bounds__(kPreThreads, 4) k_pre_scan(IndexDev D, int R, 
         uint32_t* prow = w.spos + w.qoff[qq];
         uint32_t n_read = 0, n_chk = 0;
         const float* bxs = s_bx[wp];
-        float4* lst = reinterpret_cast<float4*>(s_rings + (size_t)wp * kPreRingWords);
-        uint32_t* qr = reinterpret_cast<uint32_t*>(lst + 128);
-        uint32_t* sr = qr + 2 * 512;
-        if (use)
-            pre_span<true, LAB4>(D, lbl, bxs, rlo, rhi, D.rank_guard, pre, start, R, r0, e0, e1, qr, sr, lst, ctr,
-                                 drow, prow, n_read, n_chk);
-        else
-            pre_span_labels<LAB4>(D, lbl, bxs, pre, start, R, r0, e0, e1, qr, sr, lst, ctr, drow, prow, n_read,
-                                  n_chk);
+        if (use) {
+            pre_bits<LAB4>(D, lbl, bxs, outer, inner, has_inner, pre, start, R, r0, e0, e1, qr, sr, lst, rt, ctr, drow, prow, n_read);
+            n_chk = e1 - e0;
+        } else {
+            pre_labels<LAB4>(D, lbl, bxs, pre, start, R, r0, e0, e1, qr, ctr, drow, prow);
+            n_read = e1 - e0;
+        }
         if (lane == 0 && n_read) atomicAdd(&w.lab_read[qq], n_read);
         if (lane == 0 && n_chk) atomicAdd(&w.rank_read[qq], n_chk);
     }
@@ -2910,7 +3030,7 @@ static Workspace carve(hdg_index* idx, QueryCtx& cx, uint64_t q, bool record) {
     w.nfin = (uint32_t*)take("nfin", q * 4);
     w.lab_read = (uint32_t*)take("labels_read", q * 4);
     w.rank_read = (uint32_t*)take("ranks_read", q * 4);
-    w.counter = (uint32_t*)take("counter", 16);
+    w.counter = (uint32_t*)take("counter", 32);
     w.lut16 = P.lut_fp16 != 0;
     w.lut = (float*)take("lut", q * G * kCodes * 32 * (w.lut16 ? 2 : 4));
     w.cand_count = (uint32_t*)take("cand_count", q * 4);

@@ -283,3 +283,31 @@ def test_bruteforce_tensor_path(cuda, q, k, n, d, l, kind):
         b = min(q, a + 31)
         hg.bruteforce_knn(t[0], t[1], t[2][a:b].contiguous(), t[3][a:b].contiguous(), k, d2[a:b], i2[a:b])
     assert torch.equal(ids, i2) and torch.equal(dist, d2)
+
+
+# the predicate pass by bit planes: rank fields of 12 to 3 bits (one plane a rank, or shifted where
+# the planes would be too many), ranges of a few rows to whole lists, labels of few values, NaN
+# labels (which take the pass without ranks); ids and distances equal the oracle's
+@pytest.mark.parametrize("l", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("labels", ["spread", "few", "nan"])
+def test_predicate_pass_planes(cuda, l, labels):
+    from tests.test_gpu_parity import INV, _parity
+    ws = dict(datasets.config4(scale=0.002, n_queries=70, clusters=8, sub_clusters=4, n_list=6, sub_lists=20,
+                               max_grids=2048, exps0=1))
+    n, q = ws["base"].shape[0], ws["queries"].shape[0]
+    rng = np.random.default_rng(l)
+    hi = {"spread": 1_000_000, "few": 6, "nan": 1_000_000}[labels]
+    lab = rng.integers(0, hi, (n, l)).astype(np.float32)
+    if labels == "nan":
+        lab[rng.random((n, l)) < 0.01] = np.nan
+    a = rng.integers(0, hi, (q, l, 2)).astype(np.float32)
+    box = np.sort(a, axis=2)  # from one value to most of the range
+    box[:5] = [0, hi]         # nothing excluded
+    box[5:10, 0] = [hi + 1, hi + 2]  # nothing passes
+    ws["labels"], ws["query_labels"] = lab, box.reshape(q, 2 * l).copy()
+    ws["filter_conf"] = f"l = {l}\n" + "".join(f"filter{i}:\n\ttype = 3\n" for i in range(l))
+    idx, r = _parity(ws, cuda, exact_ids=True, adc_rotated=True)
+    valid = r["g_ids"] != INV
+    assert valid.any()
+    assert np.array_equal(r["g_ids"], r["o_ids"])
+    assert np.array_equal(r["g_dist"][valid].view(np.uint32), r["o_dist"][valid].view(np.uint32))
