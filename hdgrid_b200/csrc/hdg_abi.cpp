@@ -34,6 +34,15 @@ void DeviceBuffer::ensure(size_t b) {
     ptr = p;
     bytes = b;
 }
+bool DeviceBuffer::try_ensure(size_t b) {
+    try {
+        ensure(b);
+    } catch (const Error& e) {
+        if (e.status != HDG_ERR_OOM) throw;
+        return false;
+    }
+    return true;
+}
 
 template <typename F>
 static hdg_status guarded(F&& f) {

@@ -1586,10 +1586,12 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
             }
             if (planes * D.plane_words * 4 <= kPlanesMax) break;
         }
-        idx->planes.ensure(std::max<uint64_t>(planes * D.plane_words * 4, 16));
-        k_rank_planes<<<blocks_for(D.plane_words, 64), 256, 0, st>>>(D, H.n, static_cast<uint32_t*>(idx->planes.ptr));
-        CK_LAUNCH();
-        D.rank_planes = static_cast<const uint32_t*>(idx->planes.ptr);
+        // (without room for them the predicate pass reads every candidate's labels)
+        if (idx->planes.try_ensure(std::max<uint64_t>(planes * D.plane_words * 4, 16))) {
+            k_rank_planes<<<blocks_for(D.plane_words, 64), 256, 0, st>>>(D, H.n, static_cast<uint32_t*>(idx->planes.ptr));
+            CK_LAUNCH();
+            D.rank_planes = static_cast<const uint32_t*>(idx->planes.ptr);
+        }
     }
     // the estimate pass of the post-filter scan reads the points' PQ approximations as tensor-core
     // operands (2 d + 16 bytes per point; not kept past kDecodedMax, where the full scan runs)
@@ -1599,9 +1601,8 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
     idx->decoded.reset();
     const uint64_t dec = align_up((uint64_t)H.n * H.d * 2, 256);
     if (H.d % 8 == 0 && H.M % 32 == 0 && H.M <= 96 && H.M * H.pq_len == H.d && H.n >= kDecodedMinPoints &&
-        dec <= kDecodedMax) {
+        dec <= kDecodedMax && idx->decoded.try_ensure(dec + (uint64_t)H.n * sizeof(float4) + 16)) {
         const uint64_t cst = (uint64_t)H.n * sizeof(float4);
-        idx->decoded.ensure(dec + cst + 16);
         char* p = static_cast<char*>(idx->decoded.ptr);
         uint32_t* mx = reinterpret_cast<uint32_t*>(p + dec + cst);
         CK(cudaMemsetAsync(mx, 0, 16, st));

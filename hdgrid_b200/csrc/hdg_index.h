@@ -138,6 +138,7 @@ struct DeviceBuffer {
     size_t bytes = 0;
     void reset();
     void ensure(size_t b);  // grow-only cudaMalloc
+    bool try_ensure(size_t b);  // the same; false when the memory is not there
     ~DeviceBuffer() { reset(); }
 };
 

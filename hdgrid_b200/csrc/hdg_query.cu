@@ -3072,11 +3072,25 @@ static void ensure_part_buf(QueryCtx& cx, uint64_t q, uint32_t k) {
 }
 
 // The per-candidate rows: one f32 distance and one u32 position per candidate, same capacity.
-static void resize_rows(QueryCtx& cx, size_t bytes) {
+static bool resize_rows(QueryCtx& cx, size_t bytes) {
     cx.dist_buf.reset();
     cx.pos_buf.reset();
-    cx.dist_buf.ensure(bytes);
-    cx.pos_buf.ensure(bytes);
+    // (dist_buf last: its size is the capacity of both)
+    return cx.pos_buf.try_ensure(bytes) && cx.dist_buf.try_ensure(bytes);
+}
+
+// Rows and selection of at least the given bytes, a quarter more when the memory is there.
+static void resize_candidates(QueryCtx& cx, size_t rows, size_t sel) {
+    bool ok = cx.dist_buf.bytes >= rows || resize_rows(cx, rows * 5 / 4);
+    if (ok && cx.sel_buf.bytes < sel) {
+        cx.sel_buf.reset();
+        ok = cx.sel_buf.try_ensure(sel * 5 / 4);
+    }
+    if (ok) return;
+    for (DeviceBuffer* b : {&cx.dist_buf, &cx.pos_buf, &cx.sel_buf, &cx.est_buf}) b->reset();
+    cx.sel_buf.ensure(sel);
+    cx.pos_buf.ensure(rows);
+    cx.dist_buf.ensure(rows);
 }
 
 static size_t workspace_bytes(hdg_index* idx, QueryCtx& cx, uint64_t q) {
@@ -3110,14 +3124,10 @@ constexpr uint64_t kUnsizedPairs = 16ull << 20;
 
 // Candidate buffers of a batch whose totals are known to be at most coarse / selected entries
 static void ensure_candidates(QueryCtx& cx, uint64_t q, uint32_t k, uint64_t coarse, uint64_t selected) {
-    if (cx.dist_buf.bytes < std::max<uint64_t>(coarse, 1) * 4) {
-        invalidate_ctx_graphs(cx);  // their distance pointer dies with the old buffer
-        resize_rows(cx, std::max<uint64_t>(coarse, 1) * 4 * 5 / 4);
-    }
-    if (cx.sel_buf.bytes < std::max<uint64_t>(selected, 1) * 4) {
-        invalidate_ctx_graphs(cx);  // and their selection pointer with this one
-        cx.sel_buf.reset();
-        cx.sel_buf.ensure(std::max<uint64_t>(selected, 1) * 4 * 5 / 4);
+    const size_t rows = std::max<uint64_t>(coarse, 1) * 4, sel = std::max<uint64_t>(selected, 1) * 4;
+    if (cx.dist_buf.bytes < rows || cx.sel_buf.bytes < sel) {
+        invalidate_ctx_graphs(cx);  // their distance and selection pointers die with the old buffers
+        resize_candidates(cx, rows, sel);
     }
     ensure_part_buf(cx, q, k);
 }
@@ -3376,7 +3386,8 @@ static void resolve_lazy(hdg_index* idx, QueryCtx& cx) {
 constexpr uint64_t kEstMinCands = 32ull << 20, kEstMinRow = 8192, kEstMinRatio = 6;
 
 // Thresholds, row-tile entries (`entries` of them at most), estimates and the scan's work items.
-static void estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const QueryCall& c, int R, uint32_t G,
+// False, and nothing enqueued, when its memory is not there.
+static bool estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const QueryCall& c, int R, uint32_t G,
                           uint64_t entries, cudaStream_t st) {
     const IndexDev& D = idx->dev;
     const uint64_t q = c.q;
@@ -3393,7 +3404,7 @@ static void estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const Quer
                  o_cur = take((tiles + 1) * 4ull), o_ent = take(std::max<uint64_t>(entries, 1) * sizeof(uint4));
     if (cx.est_buf.bytes < off) {
         cx.est_buf.reset();
-        cx.est_buf.ensure(off + off / 4);
+        if (!cx.est_buf.try_ensure(off + off / 4)) return false;
     }
     char* b = static_cast<char*>(cx.est_buf.ptr);
     w.prq = reinterpret_cast<uint32_t*>(b + o_prq);
@@ -3441,6 +3452,7 @@ static void estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const Quer
     CK_LAUNCH();
     k_scan_plan<<<1, 1024, 0, st>>>(q, w);
     CK_LAUNCH();
+    return true;
 }
 
 // Enqueues one query batch on st.  sync_sizing: one host read after k_batch sizes the
@@ -3623,10 +3635,10 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
         }
         // post-filter queries with many more candidates than budget: the estimate pass (not in a
         // captured graph, whose entry count is not known)
-        const bool prune = sync_sizing && !lazy && mode == kPost && !w.qsched && fast && D.decoded && sc[0] >= kEstMinCands &&
+        bool prune = sync_sizing && !lazy && mode == kPost && !w.qsched && fast && D.decoded && sc[0] >= kEstMinCands &&
                            sc[0] / q >= kEstMinRow && sc[0] >= kEstMinRatio * sc[7] && sc[2] < (1u << 24) && sc[9] < (1ull << 32);
+        if (prune) prune = estimate_pass(idx, cx, w, c, R, G, sc[9], st);
         if (prune) {
-            estimate_pass(idx, cx, w, c, R, G, sc[9], st);
             launches += 7;
             tm.mark("estimate");
         }
@@ -3783,17 +3795,16 @@ void run_query(hdg_index* idx, const float* d_queries, uint64_t q, const float* 
         uint64_t coarse = 0, selected = 0;
         enqueue_query(idx, cx, c, st, true, nullptr, nullptr, nullptr, &coarse, &selected);
         const uint64_t need = std::max<uint64_t>(coarse, 1) * 4 * 5 / 4;  // 1.25x this batch
-        if (cx.dist_buf.bytes < need) {
-            invalidate_ctx_graphs(cx);
-            resize_rows(cx, need);
-        }
         const uint64_t need_sel = std::max<uint64_t>(selected, 1) * 4 * 5 / 4;
-        if (cx.sel_buf.bytes < need_sel) {
+        if (cx.dist_buf.bytes < need || cx.sel_buf.bytes < need_sel) {
             invalidate_ctx_graphs(cx);
-            cx.sel_buf.reset();
-            cx.sel_buf.ensure(need_sel);
+            if (cx.dist_buf.bytes < need) resize_rows(cx, need);
+            if (cx.sel_buf.bytes < need_sel) {
+                cx.sel_buf.reset();
+                cx.sel_buf.try_ensure(need_sel);
+            }
         }
-        ensure_part_buf(cx, q, k);
+        ensure_candidates(cx, q, k, coarse, selected);  // without the quarter, where it was not there
         make_graph_key(idx, cx, c, key);
         CK(cudaStreamSynchronize(st));
         GraphEntry e;
