@@ -304,9 +304,9 @@ def algorithmic_scan_bytes(cand_q, pass_q, pre_q, M: int, l: int, read_q=None, c
     A post-filter query: M code bytes per candidate, in the ADC scan.  A predicate-first query
     with the predicate inside the ADC scan (read_q None): 4*l label bytes per candidate plus M
     code bytes per candidate that passes, all in the ADC scan.  A predicate-first query of the
-    predicate pass: cbytes of packed label ranks per candidate whose ranks it tested (chk_q)
-    and 4*l label bytes per candidate whose labels it read (read_q), then M code bytes per
-    survivor in the ADC scan."""
+    predicate pass: cbytes (per query) of label-rank bit planes per candidate whose ranks it
+    tested (chk_q) and 4*l label bytes per candidate whose labels it read (read_q), then M code
+    bytes per survivor in the ADC scan."""
     cand_q = np.asarray(cand_q, np.float64)
     pass_q = np.asarray(pass_q, np.float64)
     pre = np.asarray(pre_q, bool)
@@ -316,6 +316,17 @@ def algorithmic_scan_bytes(cand_q, pass_q, pre_q, M: int, l: int, read_q=None, c
     read_q = np.asarray(read_q, np.float64)
     chk_q = np.zeros_like(read_q) if chk_q is None else np.asarray(chk_q, np.float64)
     return float((chk_q * cbytes + read_q * (4 * l))[pre].sum()), adc
+
+
+def rank_plane_bytes(rank_box, l: int, bits: int):
+    """Bytes of label-rank bit planes per candidate of each query: a bit for every bound of its
+    rank box (rank_box [q x 4], fields of `bits` bits and a guard bit) that excludes some rank."""
+    lo, hi = rank_box[:, 0].astype(np.int64), rank_box[:, 1].astype(np.int64)
+    planes = np.zeros(len(rank_box))
+    for i in range(l):
+        a, b = [(x >> (i * (bits + 1))) & ((1 << bits) - 1) for x in (lo, hi)]
+        planes += (a > 0) + (b < b.max()).astype(np.float64)
+    return planes / 8
 
 
 def refine_algorithmic_bytes(sel_q, pre_q, rows_q, lab_q, l: int, d: int, rank_bytes: int) -> float:
@@ -445,11 +456,14 @@ def run_hdgrid(args):
     if learned:
         pre_q = np.frombuffer(idx.debug_fetch("learned_schedule").tobytes(), np.uint8)[:nq] == 1
     pass_q = np.frombuffer(idx.debug_fetch("nfin").tobytes(), np.uint32)[:nq].astype(np.uint64)
-    # the predicate pass (the fast ADC path: M a multiple of 32, at most 96) counts the packed
-    # label ranks and labels it read per query
+    # the predicate pass (the fast ADC path: M a multiple of 32, at most 96) counts the candidates
+    # whose label ranks it tested, 32 to a word of bit planes, and those whose labels it read
     pred_pass = info["M"] % 32 == 0 and info["M"] <= 96
     read_q = chk_q = None
+    plane_bytes = 0.0
     if pred_pass:
+        rank_box = np.frombuffer(idx.debug_fetch("rank_box").tobytes(), np.uint32).reshape(-1, 4)[:nq]
+        plane_bytes = rank_plane_bytes(rank_box, info["l"], info["rank_bits"])
         read_q = np.frombuffer(idx.debug_fetch("labels_read").tobytes(), np.uint32)[:nq].astype(np.uint64)
         chk_q = np.frombuffer(idx.debug_fetch("ranks_read").tobytes(), np.uint32)[:nq].astype(np.uint64)
     # a predicate-first query whose budget takes every survivor needs no ADC (the re-rank
@@ -462,7 +476,7 @@ def run_hdgrid(args):
     # bounds left open (its finite distances)
     scan_q = np.where(pre_q, cand_q, pass_q) if "estimate" in stage_ms else cand_q
     pred_bytes, adc_bytes = algorithmic_scan_bytes(scan_q, np.where(pre_q & ~adc_q, 0, pass_q), pre_q, info["M"],
-                                                   info["l"], read_q, chk_q, info["rank_pack_bytes"])
+                                                   info["l"], read_q, chk_q, plane_bytes)
     pass_share = float(pass_q[pre_q].sum() / max(1, cand_q[pre_q].sum())) if pre_q.any() else None
     launches_per_step = int(stats["launches"])
     # the re-rank: every selected entry's pool -> id lookup (4 B); for a post-filter query, its

@@ -42,7 +42,7 @@ constexpr uint32_t kChunk = 32768;  // default most candidates per scan work ite
 constexpr uint32_t kChunkMin = 1024;
 constexpr int kBins = 4096;         // select histogram
 constexpr int kBCap = 4096;         // boundary-bin buffer of the select
-constexpr uint32_t kPreChunk = 16384, kPreChunkMin = 1024;  // candidates per work item of the predicate pass
+constexpr uint32_t kPreChunk = 32768, kPreChunkMin = 1024;  // candidates per work item of the predicate pass
 
 struct Workspace {
     float* box;              // [q x 2l]
@@ -840,8 +840,11 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
     // that leaves at most scan_items items.  A small batch then fills the SMs (37 queries of
     // 73,000 candidates ran as 111 items of up to 32,768 in 325 us, in 125 us this way); a large one keeps long
     // items, since each loads its query's LUT.
-    // Predicate items likewise, for 16 times as many items (a warp each): 64 queries of 47,000
-    // candidates took 188 us as items of 8,192.
+    // Predicate items likewise, for 64 times as many items (a warp each, 16 per resident warp): an
+    // item costs some 4 us of searches before its first word, a long one leaves a tail.  Predicate
+    // stage, us, at items of 16,384 / 8,192 / 4,096 / 2,048: 2 G candidates 1,307 / 1,405 / 1,649 /
+    // 2,183; 1 G 1,263 / 1,262 / 1,364 / 1,648; 161 M 265 / 199 / 186 / 211; 3 M (1,024) 38, as items of
+    // 8,192 188.
     __shared__ uint32_t s_pchunk;
     {
         unsigned long long c = 0, all = 0;
@@ -850,7 +853,7 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
         if (t == 0) {
             uint32_t ch = kChunkMin, pc = kPreChunkMin;
             while (ch < kChunk && (unsigned long long)ch * w.scan_items < all) ch *= 2;
-            while (pc < kPreChunk && (unsigned long long)pc * w.scan_items * 16u < all) pc *= 2;
+            while (pc < kPreChunk && (unsigned long long)pc * w.scan_items * 64u < all) pc *= 2;
             s_chunk = w.chunk ? w.chunk : ch;
             s_pchunk = pc;
         }
@@ -1162,6 +1165,12 @@ __device__ __forceinline__ void scan_load_query(const Workspace& w, int Ps, int 
 //   4. the survivors are staged per warp and appended to the query's row -- the candidate position
 //      into spos and the pool row into the distance slot, which the ADC scan then overwrites with
 //      the survivor's distance.
+// Bound: latency of the plane words (ncu, 161 M candidates of 2,000 queries: issue slots 39 % busy, a third
+// of the stalls on loads; DRAM 1.8 B per candidate on 10 M points, 2.7 TB/s).  One packed rank word per
+// candidate took 2,505 us for 1.9 G candidates of 10,000 queries (issue and L2 latency), planes with
+// the labels of every row inside the outer box 1,305, the inner box as well 1,790 -> 1,263 on 1 G
+// candidates of which a third pass; survivors pushed a bit per word and lane, out of row order, cost the
+// ADC scan 2,558 against 2,017.
 // The row's order depends on timing; the distance of each survivor does not (the ADC order
 // follows its position) and the select orders ties by position.
 constexpr int kPreThreads = 256;

@@ -225,7 +225,7 @@ int hdg_last_stage_times(const hdg_index* index, float* ms, const char** names, 
  * Names: "box", "cells", "zrange", "list_counts", "cluster_counts", "probe_clusters",
  * "probe_lists", "range_start", "range_len", "cand_count", "budget", "sel_off", "scalars",
  * "qoff", "qstat", "labels_read" (candidates of the predicate pass whose labels were read),
- * "ranks_read" (candidates of the predicate pass whose packed label ranks were read),
+ * "ranks_read" (candidates of the predicate pass whose label ranks were tested),
  * "rank_box" (per query: the label-rank box and its inner box, four words), "refine_rows"
  * (rows the re-rank computed exactly), "refine_labels_read" (selected entries whose labels
  * the re-rank read), "distances" (the f32 ADC distance of every scanned candidate, query rows
