@@ -1507,16 +1507,13 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
     D.labels = (const float*)keep(o_lab, src ? src->labels : nullptr, H.labels.data(), H.n * H.l * 4);
     D.rank_bits = (uint32_t)rbits;
     D.rank_stride = rstride;
-    D.rank_guard = D.rank_full = 0;
+    D.rank_guard = 0;
     for (int i = 0; i < kMaxDims; i++) {
         D.rank_n[i] = i < (int)H.l ? rn[i] : 0u;
         D.rank_min[i] = i < (int)H.l ? rmin[i] : 0.f;
         D.rank_max[i] = i < (int)H.l ? rmax[i] : 0.f;
     }
-    for (int i = 0; rbits && i < (int)H.l; i++) {
-        D.rank_guard |= 1u << (i * (rbits + 1) + rbits);
-        D.rank_full |= rn[i] << (i * (rbits + 1));
-    }
+    for (int i = 0; rbits && i < (int)H.l; i++) D.rank_guard |= 1u << (i * (rbits + 1) + rbits);
     D.rank_thr = rbits ? (const float*)up(o_rt, rthr.data(), rthr.size() * 4) : nullptr;
     D.rankpack = rbits ? reinterpret_cast<const uint32_t*>(base + o_pk) : nullptr;
     if (rbits) {

@@ -87,7 +87,7 @@ struct IndexDev {
     // 2^rank_bits - 1 ascending thresholds rank_thr[i * rank_stride + k], k < rank_n[i]; a
     // label's rank is the number of thresholds at or below it.  rankpack holds every point's
     // ranks in pool order, dim i in bits [i * (rank_bits + 1), +rank_bits) with a zero guard bit
-    // above (rank_guard = the guard bits; rank_full = every rank_n[i] in its field).  The labels
+    // above (rank_guard = the guard bits).  The labels
     // of rank r lie in [thr[r - 1], thr[r]), with rank_min / rank_max (the smallest and largest
     // label of the dim) closing the two ends.  A rank outside the query's rank box proves that
     // the label test fails; a rank inside its inner box proves that it passes.  Only the others
@@ -96,7 +96,7 @@ struct IndexDev {
     const float* rank_thr;
     uint32_t rank_n[kMaxDims];
     float rank_min[kMaxDims], rank_max[kMaxDims];
-    uint32_t rank_bits, rank_stride, rank_guard, rank_full;
+    uint32_t rank_bits, rank_stride, rank_guard;
     // The same ranks as bit planes, for the predicate pass (derived at upload; nullptr with NaN
     // labels): bit row % 32 of word row / 32 of plane plane_off[i] + v says that the row's rank of
     // dim i, shifted right by plane_shift, is at most v (v below the dim's largest such value).

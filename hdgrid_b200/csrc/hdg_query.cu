@@ -42,7 +42,7 @@ constexpr uint32_t kChunk = 32768;  // default most candidates per scan work ite
 constexpr uint32_t kChunkMin = 1024;
 constexpr int kBins = 4096;         // select histogram
 constexpr int kBCap = 4096;         // boundary-bin buffer of the select
-constexpr uint32_t kPreChunk = 32768, kPreChunkMin = 1024;  // candidates per work item of the predicate pass
+constexpr uint32_t kPreChunk = 16384, kPreChunkMin = 1024;  // candidates per work item of the predicate pass
 
 struct Workspace {
     float* box;              // [q x 2l]
@@ -1170,7 +1170,8 @@ __device__ __forceinline__ void scan_load_query(const Workspace& w, int Ps, int 
 // candidate took 2,505 us for 1.9 G candidates of 10,000 queries (issue and L2 latency), planes with
 // the labels of every row inside the outer box 1,305, the inner box as well 1,790 -> 1,263 on 1 G
 // candidates of which a third pass; survivors pushed a bit per word and lane, out of row order, cost the
-// ADC scan 2,558 against 2,017.
+// ADC scan 2,558 against 2,017.  Slower on 10 M points (1,308): the inner box's words of every lane, open
+// rows or not (1,398), five blocks per SM with spills (1,438), items of up to 32,768 (1,321).
 // The row's order depends on timing; the distance of each survivor does not (the ADC order
 // follows its position) and the select orders ties by position.
 constexpr int kPreThreads = 256;

@@ -246,8 +246,8 @@ typedef struct hdg_index_info {
     int32_t morton_dims, morton_max_bits, morton_valid_map, diff_dim;
     uint64_t device_bytes;
     uint64_t prefix_entries;  /* change points of the compressed prefix rows; 0 = dense form */
-    uint64_t rank_pack_bytes; /* bytes per point of the packed label ranks that the predicate pass
-                               * reads before the labels (4; 0 = not kept) */
+    uint64_t rank_pack_bytes; /* bytes per point of the packed label ranks, tested
+                               * before the labels (4; 0 = not kept) */
     uint64_t rank_bits;       /* bits per label dim of a packed rank (2^bits - 1 thresholds at most) */
 } hdg_index_info;
 hdg_status hdg_get_info(const hdg_index* index, hdg_index_info* out);
