@@ -487,8 +487,10 @@ __global__ void __launch_bounds__(kEstThreads, 1) k_est(const __grid_constant__ 
                 if (G.qid[cs][gt] == 0xffffffffu || !ok) {
                     m = make_uint4(0u, 0u, 0u, 0u);
                     G.mask[ms][gt] = m;
-                } else if (RANGES) {  // the rows of the entry's range
-                    const uint32_t r = G.lohi[cs][gt];
+                } else if (RANGES || row0 + kEstM > a.n_rows) {
+                    // the rows of the entry's range, or those that the last tile has: a bound that is not
+                    // finite keeps its whole column, the rows past the end with it
+                    const uint32_t r = RANGES ? G.lohi[cs][gt] : (a.n_rows - row0) << 16;
                     const int lo = (int)(r & 0xffffu), hi = (int)(r >> 16);
                     auto part = [&](uint32_t x, int k) {
                         const int a0 = min(max(lo - 32 * k, 0), 32), a1 = min(max(hi - 32 * k, 0), 32);

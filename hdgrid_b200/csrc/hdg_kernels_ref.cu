@@ -774,7 +774,7 @@ __global__ void k_bf_queries(const float* __restrict__ queries, uint32_t d, uint
 // Exact distances of a query's listed rows.  Not the last level: the query's threshold from the
 // k-th smallest.  Last level: the k smallest, ascending.  A thread computes one row at a time.
 constexpr int kBfExactThreads = 256;
-__global__ void __launch_bounds__(kBfExactThreads) k_bf_exact(const float* __restrict__ data, uint32_t d,
+__global__ void __launch_bounds__(kBfExactThreads) k_bf_exact(const float* __restrict__ data, uint32_t n, uint32_t d,
                                                               const float* __restrict__ queries, uint32_t k,
                                                               const uint32_t* __restrict__ list, uint32_t cap,
                                                               uint32_t* __restrict__ cnt, int vec, int last,
@@ -801,14 +801,14 @@ __global__ void __launch_bounds__(kBfExactThreads) k_bf_exact(const float* __res
         for (int u = 0; u < 2; u++) {
             const int e = e0 + u * kBfExactThreads;
             id[u] = __ldg(list + q * cap + (e < c ? e : e0));
-            row[u] = data + (uint64_t)id[u] * d;
+            row[u] = data + (uint64_t)min(id[u], n - 1) * d;
         }
         if (vec) bf_dist<true, 2>(s_q, row, (int)d, acc);
         else bf_dist<false, 2>(s_q, row, (int)d, acc);
 #pragma unroll
         for (int u = 0; u < 2; u++)
             if (e0 + u * kBfExactThreads < c)
-                s_keys[e0 + u * kBfExactThreads] = ((uint64_t)float_key(acc[u]) << 32) | id[u];
+                s_keys[e0 + u * kBfExactThreads] = id[u] < n ? ((uint64_t)float_key(acc[u]) << 32) | id[u] : ~0ull;
     }
     __syncthreads();
     if (!last) {
@@ -829,8 +829,8 @@ __global__ void __launch_bounds__(kBfExactThreads) k_bf_exact(const float* __res
     block_bitonic_sort(s_keys, n2);
     for (int i = t; i < (int)k; i += kBfExactThreads) {
         const uint64_t key = i < m ? s_keys[i] : ~0ull;
-        out_dist[q * k + i] = i < m ? key_float((uint32_t)(key >> 32)) : INFINITY;
-        out_ids[q * k + i] = i < m ? (uint64_t)(uint32_t)key : ~0ull;
+        out_dist[q * k + i] = i < m && key != ~0ull ? key_float((uint32_t)(key >> 32)) : INFINITY;
+        out_ids[q * k + i] = i < m && key != ~0ull ? (uint64_t)(uint32_t)key : ~0ull;
     }
 }
 
@@ -951,7 +951,7 @@ static void bruteforce_est(const float* data, uint64_t n, uint32_t d, const floa
                 a.row_step = (uint32_t)step;
                 est_all(a, rows, (int)ld, err, st);
             }
-            k_bf_exact<<<nq, kBfExactThreads, sm, st>>>(data, d, queries, k, list, cap, cnt, vec, step == 1 ? 1 : 0, qn, qc,
+            k_bf_exact<<<nq, kBfExactThreads, sm, st>>>(data, (uint32_t)n, d, queries, k, list, cap, cnt, vec, step == 1 ? 1 : 0, qn, qc,
                                                        dist, ids);
             CK_LAUNCH();
             if (step == 1) break;

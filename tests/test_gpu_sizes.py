@@ -285,6 +285,38 @@ def test_bruteforce_tensor_path(cuda, q, k, n, d, l, kind):
     assert torch.equal(ids, i2) and torch.equal(dist, d2)
 
 
+# the same with components that FP16 cannot hold, infinities and NaN in queries and base rows, the
+# last row tile of every level a part of one and its last row inside the boxes
+@pytest.mark.parametrize("n", [187500, 187507, 187649])
+def test_bruteforce_tensor_path_not_finite(cuda, n):
+    import torch
+    import hdgrid_b200 as hg
+    q, k, d, l = 64, 10, 128, 4
+    rng = np.random.default_rng(n)
+    base = rng.standard_normal((n, d), dtype=np.float32)
+    qs = rng.standard_normal((q, d), dtype=np.float32)
+    lab = rng.integers(0, 1000, (n, l)).astype(np.float32)
+    box = np.tile(np.array([0, 1000], np.float32), (q, l))  # every row passes ...
+    box[40:, 0] = 700                                       # ... or about a third
+    lab[-1] = 800
+    for i, v in enumerate((70_000.0, -65_520.0, np.inf, -np.inf, np.nan, 3e19, -3e38, 0.0)):
+        qs[5 * i, i] = v
+        qs[5 * i + 1] = v
+        qs[56 + i, d - 1] = v
+    for i, v in enumerate((70_000.0, -1e30, np.inf, -np.inf, np.nan)):
+        base[rng.integers(0, n, 40), i] = v
+    t = [torch.from_numpy(x).to(cuda) for x in (base, lab, qs, box)]
+    dist = torch.full((q, k), -1.0, device=cuda)
+    ids = torch.full((q, k), 7, dtype=torch.int64, device=cuda)
+    hg.bruteforce_knn(*t, k, dist, ids)
+    d2, i2 = torch.empty_like(dist), torch.empty_like(ids)
+    for a in range(0, q, 31):  # the direct path
+        b = min(q, a + 31)
+        hg.bruteforce_knn(t[0], t[1], t[2][a:b].contiguous(), t[3][a:b].contiguous(), k, d2[a:b], i2[a:b])
+    assert int(ids.max()) < n
+    assert torch.equal(ids, i2) and torch.equal(dist.view(torch.int32), d2.view(torch.int32))
+
+
 # the predicate pass by bit planes: rank fields of 12 to 3 bits (one plane a rank, or shifted where
 # the planes would be too many), ranges of a few rows to whole lists, labels of few values, NaN
 # labels (which take the pass without ranks); ids and distances equal the oracle's
