@@ -294,7 +294,7 @@ static void pq_assign(const float* X, uint64_t n, int d, int M, int pq_len, cons
     auto go = [&](auto plc) {
         constexpr int PL = decltype(plc)::value;
         constexpr size_t sm = sizeof(float) * pq_mb(PL) * kCodes * PL;
-        CK(cudaFuncSetAttribute(k_pq_assign<PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        allow_smem(k_pq_assign<PL>);
         k_pq_assign<PL><<<dim3((unsigned)((n + 2 * kPqThreads - 1) / (2 * kPqThreads)),
                                (unsigned)((M + pq_mb(PL) - 1) / pq_mb(PL))),
                           kPqThreads, sm, st>>>(X, n, d, M, cb, out, out_stride, out_int);

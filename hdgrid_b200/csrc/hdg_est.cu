@@ -534,7 +534,7 @@ void launch_est(const EstArgs& a, const void* rows, int ld, int* err, cudaStream
     const size_t sm = 1024 + (size_t)est_stages(RANGES) * 2 * kChunkBytes + sizeof(EstShared) + 16 +
                       (RANGES ? (size_t)kGroups * 2 * kEstN * kEstM : sizeof(float) * kGroups * 2 * kEstN * 2 * a.l);
     auto kern = k_est<RANGES, LT>;
-    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    allow_smem(kern);
     kern<<<(unsigned)sm_count(), kEstThreads, sm, st>>>(map, a, ld, (ld + 63) / 64, err);
     CK_LAUNCH();
 }

@@ -383,7 +383,7 @@ void umma_dot_tma(const void* A_bf16, uint64_t rows, const void* B_bf16, uint64_
     auto launch = [&](auto kern, uint32_t bn) {
         const CUtensorMap mb = bf16_rows_map(B_bf16, cols, d, bn);
         const int sm = (int)(kTStages * (kTileA + bn * GK * 2) + 1024);
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+        allow_smem(kern);
         dim3 grid((unsigned)row_tiles, (unsigned)((cols + bn - 1) / bn));
         kern<<<grid, kGemmThreads, sm, st>>>(ma, rows, mb, cols, d, out, ldo, err);
     };
@@ -410,7 +410,7 @@ void umma_dot_cp_async(const void* A_bf16, uint64_t rows, const void* B_bf16, ui
     HDG_REQUIRE(d % 8 == 0, HDG_ERR_UNSUPPORTED, "tensor-core coarse GEMM needs d % 8 == 0");
     if (!rows || !cols) return;
     const int sm = (int)umma_smem_bytes();
-    CK(cudaFuncSetAttribute(k_umma_dot, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    allow_smem(k_umma_dot);
     dim3 grid((unsigned)((rows + GM - 1) / GM), (unsigned)((cols + GN - 1) / GN));
     k_umma_dot<<<grid, kGemmThreads, sm, st>>>(static_cast<const __nv_bfloat16*>(A_bf16), rows,
                                                static_cast<const __nv_bfloat16*>(B_bf16), cols, d, out, ldo, err);

@@ -47,6 +47,15 @@ void run_query(hdg_index* idx, const float* d_queries, uint64_t q, const float* 
                cudaStream_t st, const uint32_t* d_k = nullptr, const uint32_t* d_nprobe = nullptr,
                const uint8_t* d_sched = nullptr);
 int sm_count();  // SMs of the current device
+constexpr size_t kBlockSmem = 227 * 1024;  // shared memory of a block, static and dynamic
+// Before a launch with dynamic shared memory: lets the kernel use all that a block may have.  Always
+// the same limit, whatever this launch needs: the limit belongs to the kernel, and a smaller one set
+// by another thread's call would fail a launch that is about to happen.
+void allow_smem(const void* kernel);
+template <typename... P>
+void allow_smem(void (*kernel)(P...)) {
+    allow_smem(reinterpret_cast<const void*>(kernel));
+}
 // per-dim label-rank thresholds and label ranges of a base set (hdg_build.cu)
 void label_rank_thresholds(const float* labels, uint64_t n, int l, int bits, float* thr, uint32_t* n_thr, float* mn,
                            float* mx);

@@ -293,7 +293,7 @@ void pq_adc(const uint8_t* codebook, uint64_t tot_data, const float* lut, uint64
     if (!indices && n_codes == 256 && pq_dim >= 1 && nq <= 0x7fffffffull) {
         auto launch = [&](auto kern, int qb) {
             const size_t sm = adc_smem(pq_dim, qb);
-            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            allow_smem(kern);
             int occ = 0;
             CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kAdcThreads, sm));
             // one span of tiles per resident block, no block with fewer tiles than warps
@@ -303,10 +303,9 @@ void pq_adc(const uint8_t* codebook, uint64_t tot_data, const float* lut, uint64
                                                             n_cand, dist);
             CK_LAUNCH();
         };
-        const size_t most = 227 * 1024;
-        if (nq >= 3 && adc_smem(pq_dim, 4) <= most) return launch(k_pq_adc_all<4>, 4);
-        if (nq >= 2 && adc_smem(pq_dim, 2) <= most) return launch(k_pq_adc_all<2>, 2);
-        if (adc_smem(pq_dim, 1) <= most) return launch(k_pq_adc_all<1>, 1);
+        if (nq >= 3 && adc_smem(pq_dim, 4) <= kBlockSmem) return launch(k_pq_adc_all<4>, 4);
+        if (nq >= 2 && adc_smem(pq_dim, 2) <= kBlockSmem) return launch(k_pq_adc_all<2>, 2);
+        if (adc_smem(pq_dim, 1) <= kBlockSmem) return launch(k_pq_adc_all<1>, 1);
     }
     k_pq_adc<<<nblk(nq * n_cand, 256), 256, 0, st>>>(codebook, tot_data, lut, nq, pq_dim, n_codes, indices,
                                                       n_cand, dist);
@@ -935,7 +934,7 @@ static void bruteforce_est(const float* data, uint64_t n, uint32_t d, const floa
         a.cap = cap;
         a.cnt = cnt;
         const size_t sm = sizeof(uint64_t) * cap + sizeof(float) * d;
-        CK(cudaFuncSetAttribute(k_bf_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        allow_smem(k_bf_exact);
         const int vec = d % 4 == 0 && (reinterpret_cast<uintptr_t>(data) & 15) == 0;
         uint64_t step = 1;  // the coarsest sample: as many rows as a list holds
         while ((n + step - 1) / step > cap) step *= kBfRatio;
@@ -997,14 +996,13 @@ void bruteforce_knn(const float* data, uint64_t n, uint32_t d, const float* labe
     }
     // the longest tile whose two buffers fit, its rows padded to an odd number of bank groups;
     // rows too long for that are read from global memory, and so are queries of extreme length
-    const size_t most = 227 * 1024;
     b.pitch = vec ? (int)(d + (d / 4 % 2 ? 0 : 4)) : (int)(d | 1);
-    for (b.rows = 128; b.rows >= 32 && bf_smem(b, d, l) > most; b.rows /= 2) {
+    for (b.rows = 128; b.rows >= 32 && bf_smem(b, d, l) > kBlockSmem; b.rows /= 2) {
     }
     if (b.rows < 32) {
         b.rows = 128;
         b.pitch = 0;
-        if (bf_smem(b, d, l) > most) {
+        if (bf_smem(b, d, l) > kBlockSmem) {
             b.staged_q = 0;
             vec = false;
         }
@@ -1029,7 +1027,7 @@ void bruteforce_knn(const float* data, uint64_t n, uint32_t d, const float* labe
         uint64_t* part = nullptr;
         CK(cudaMallocAsync(reinterpret_cast<void**>(&part), sizeof(uint64_t) * nb * spans * k, st));
         auto launch = [&](auto kern) {
-            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            allow_smem(kern);
             kern<<<(unsigned)(groups * spans), kBfThreads, sm, st>>>(data, n, d, labels, l, queries + a * d, nb,
                                                                     ranges + a * 2 * l, k, b, part);
             CK_LAUNCH();
@@ -1107,7 +1105,7 @@ void merge_topk(const float* dist, const uint64_t* ids, uint64_t q, uint32_t k, 
     HDG_REQUIRE(k >= 1 && nb >= 1 && (uint64_t)k * nb <= 8192, HDG_ERR_UNSUPPORTED, "k * n_batches must be <= 8192");
     const int n2 = (int)next_pow2(std::max<uint32_t>(k * nb, 2));
     const size_t sm = sizeof(uint64_t) * (n2 + (size_t)k * nb);
-    CK(cudaFuncSetAttribute(k_merge_topk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    allow_smem(k_merge_topk);
     k_merge_topk<<<(unsigned)q, 256, sm, st>>>(dist, ids, k, nb, offsets, n2, out_dist, out_ids);
     CK_LAUNCH();
 }

@@ -516,7 +516,7 @@ int launch_mlp(const ModelPtrs& mp, const float* x, uint64_t n, const FwdOut& o,
     auto go = [&](auto tsc) {
         constexpr int TS = decltype(tsc)::value;
         constexpr size_t sm = forward_smem<TS, GRAD>();
-        CK(cudaFuncSetAttribute(k_mlp<TS, GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        allow_smem(k_mlp<TS, GRAD>);
         const int blocks = std::max(1, mlp_blocks(n, TS));
         k_mlp<TS, GRAD><<<blocks, kFwdThreads, sm, st>>>(Params{mp.master, mp.w}, x, n, o);
         CK_LAUNCH();
@@ -564,7 +564,7 @@ void learned_features(hdg_index* idx, const float* d_queries, uint64_t q, const 
     const int sort_n = (int)next_pow2(std::max<uint32_t>(D.C, 16));
     const size_t sm = (sizeof(uint64_t) + sizeof(uint32_t) + sizeof(float)) * sort_n + sizeof(float) * D.d;
     HDG_REQUIRE(sm <= 200 * 1024, HDG_ERR_UNSUPPORTED, "feature kernel does not fit shared memory");
-    CK(cudaFuncSetAttribute(k_features, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    allow_smem(k_features);
     k_features<<<(unsigned)q, 128, sm, st>>>(D, idx->grid, d_queries, box, cc, qk, k_max, sort_n, S, ldS, qnorm,
                                              feats);
     CK_LAUNCH();

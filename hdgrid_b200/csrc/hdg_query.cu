@@ -28,6 +28,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <type_traits>
 
 #include "hdg_device.cuh"
@@ -3276,6 +3278,23 @@ int sm_count() {
     return n;
 }
 
+void allow_smem(const void* kernel) {
+    static std::mutex mu;
+    static std::map<const void*, int> fixed;  // the kernels' static shared memory (part of the code)
+    int bytes;
+    {
+        std::lock_guard<std::mutex> g(mu);
+        auto it = fixed.find(kernel);
+        if (it == fixed.end()) {
+            cudaFuncAttributes a;
+            CK(cudaFuncGetAttributes(&a, kernel));
+            it = fixed.emplace(kernel, (int)a.sharedSizeBytes).first;
+        }
+        bytes = (int)kBlockSmem - it->second;
+    }
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+}
+
 struct QueryCall {
     const float* queries;
     uint64_t q;
@@ -3443,7 +3462,7 @@ static bool estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const Quer
     CK(cudaMemsetAsync(diff, 0, (tiles + 1) * 4ull, st));
     const size_t sm = sizeof(uint32_t) * (G * kCodes * 16 + kThrMax + kThrBins + 2 * R + 1);
     auto thr = [&](auto kern) {
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        allow_smem(kern);
         kern<<<(unsigned)q, kThrThreads, sm, st>>>(D, R, c.queries, w);
         CK_LAUNCH();
     };
@@ -3520,8 +3539,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
                   capture ? &capture->stage_names : nullptr);
 
     const size_t sm_pro = sizeof(uint32_t) * D.n_lists;
-    if (sm_pro > 48 * 1024)
-        CK(cudaFuncSetAttribute(k_prologue, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_pro));
+    if (sm_pro > 48 * 1024) allow_smem(k_prologue);
     uint64_t launches = 0;  // kernels of this query, reported in the stats
     launch_next(false, k_prologue, dim3((unsigned)q), kThreads, sm_pro, st, D, idx->grid, f, c.qlabels, (int)c.label_cols, w);
     CK_LAUNCH();
@@ -3532,7 +3550,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     const size_t sm_co = (sizeof(uint64_t) + sizeof(float)) * std::max(sort_n1, sort_n2) + sizeof(float) * D.d;
     HDG_REQUIRE(sm_co <= 200 * 1024, HDG_ERR_UNSUPPORTED, "coarse selection does not fit shared memory");
     if (sm_co > 48 * 1024)
-        CK(cudaFuncSetAttribute(k_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_co));
+        allow_smem(k_coarse);
     // tensor-core estimates of every query-centroid dot product, used to prune the exact
     // ranking when n_list or sub_lists leaves part of the candidates out (COARSE_BF16=1)
     const bool use_gemm = P.coarse_bf16 != 0 && D.d % 8 == 0 && (Pc < (int)D.C || Ps < Pc * (int)D.S_max);
@@ -3614,7 +3632,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             const bool lab4 = l == 4 && (reinterpret_cast<uintptr_t>(D.labels) & 15) == 0;
             auto launch_pre = [&](auto kern) {
                 const size_t smp = sizeof(uint32_t) * kPreRingWords * (kPreThreads / 32);
-                CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smp));
+                allow_smem(kern);
                 const int blocks = sm_count() * occupancy_blocks(kern, kPreThreads, smp);
                 kern<<<blocks, kPreThreads, smp, st>>>(D, R, l, q, w);
             };
@@ -3632,7 +3650,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             if (D.pq_len <= (uint32_t)kLutMaxPqLen) {
                 const int slices = lut_slices(q, (int)G, sm_count());
                 const size_t sm = sizeof(float) * (kCodes / slices) * D.pq_len * 33;
-                CK(cudaFuncSetAttribute(k_lut, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+                allow_smem(k_lut);
                 launch_next(chain && lazy && !pre_pass, k_lut, dim3((unsigned)((q + kLutQ - 1) / kLutQ), G, slices), 512, sm,
                             st, D, c.queries, q, (int)G, w.lut, w.lut16, w.item_off);
             } else {
@@ -3656,9 +3674,9 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             // threads x candidates-per-thread (SCAN_CPT, chosen by the autotuner; 0 = 1)
             const int cpt = (P.scan_cpt == 1 || P.scan_cpt == 2 || P.scan_cpt == 4) ? (int)P.scan_cpt : 1;
             const size_t sm = sizeof(float) * G * kCodes * 64 + sm_tab;
-            HDG_REQUIRE(sm <= 227 * 1024, HDG_ERR_UNSUPPORTED, "scan tables exceed shared memory");
+            HDG_REQUIRE(sm <= kBlockSmem, HDG_ERR_UNSUPPORTED, "scan tables exceed shared memory");
             auto launch = [&](auto kern, int nt) {
-                CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+                allow_smem(kern);
                 const int blocks = sm_count() * occupancy_blocks(kern, nt, sm);
                 launch_next(chain && !prune, kern, dim3((unsigned)blocks), nt, sm, st, D, R, q, w);
             };
@@ -3677,8 +3695,8 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             }
         } else {
             const size_t sm = sizeof(float) * G * kCodes * 32 + sm_tab;
-            HDG_REQUIRE(sm <= 227 * 1024, HDG_ERR_UNSUPPORTED, "scan tables exceed shared memory");
-            CK(cudaFuncSetAttribute(k_scan_generic, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            HDG_REQUIRE(sm <= kBlockSmem, HDG_ERR_UNSUPPORTED, "scan tables exceed shared memory");
+            allow_smem(k_scan_generic);
             const int blocks = sm_count() * occupancy_blocks(k_scan_generic, 512, sm);
             launch_next(chain, k_scan_generic, dim3((unsigned)blocks), 512, sm, st, D, (int)G, R, pre, l, q, w);
         }
@@ -3691,7 +3709,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     const size_t sm_sel = sizeof(uint32_t) * kBins + sizeof(uint64_t) * kBCap +
                           (sorted_out ? sizeof(uint64_t) * next_pow2(std::max<uint32_t>(k, 2)) : 0) + sm_tab + 16;
     auto launch_sel = [&](auto kern, int nt) {
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_sel));
+        allow_smem(kern);
         launch_next(chain && scanned, kern, dim3((unsigned)q), nt, sm_sel, st, D, R, (int)k, sorted_out, w, c.dist, c.ids, (int)k);
     };
     if (q <= (uint64_t)sm_count()) launch_sel(k_select<kSelThreadsFew, 8>, kSelThreadsFew);
@@ -3704,7 +3722,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
         CK_LAUNCH();
         const int rcap = (int)next_pow2(k + 4 * kThreads);  // rounds of rcap - k exact distances
         const size_t sm_ref = sizeof(uint64_t) * rcap + sizeof(float) * D.d + 16;
-        CK(cudaFuncSetAttribute(k_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ref));
+        allow_smem(k_refine);
         // persistent over the refine items; no more CTAs than queries are useful for small batches
         const uint64_t blocks = std::min<uint64_t>((uint64_t)sm_count() * occupancy_blocks(k_refine, kThreads, sm_ref),
                                                    q + (cx.sel_buf.bytes / 4) / kRefChunk + 1);
@@ -3871,8 +3889,7 @@ void query_features(hdg_index* idx, const float* d_queries, uint64_t q, const fl
     Workspace w = carve(idx, cx, q, true);
     const FilterDev f = filter_dev(idx);
     const size_t sm_pro = sizeof(uint32_t) * D.n_lists;
-    if (sm_pro > 48 * 1024)
-        CK(cudaFuncSetAttribute(k_prologue, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_pro));
+    if (sm_pro > 48 * 1024) allow_smem(k_prologue);
     k_prologue<<<(unsigned)q, kThreads, sm_pro, st>>>(D, idx->grid, f, d_query_labels, (int)label_cols, w);
     CK_LAUNCH();
     learned_features(idx, d_queries, q, w.box, w.cluster_counts, d_k, k_max, d_feats, st);

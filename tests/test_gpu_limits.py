@@ -1,0 +1,115 @@
+"""Calls at the limits of their resources: little free device memory, several host threads,
+buffers left by larger calls, candidate ranges near the shared-memory limit."""
+import threading
+
+import numpy as np
+import pytest
+
+from hdgrid_b200 import datasets
+from tests.helpers import build_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def _in_threads(*calls):
+    """Runs the calls at the same time, each in a thread of its own; their exceptions."""
+    errors = []
+
+    def run(f):
+        try:
+            f()
+        except Exception as e:  # noqa: BLE001 (reported to the test)
+            errors.append(e)
+
+    ts = [threading.Thread(target=run, args=(f,)) for f in calls]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    return errors
+
+
+def _range_ws(n, q, l=4, d=32, m=32, **conf):
+    """Points with l integer labels below 1,000 and range filters: half of every dim, or a fiftieth of the one."""
+    rng = np.random.default_rng(n + q)
+    lab = rng.integers(0, 1000, (n, l)).astype(np.float32)
+    lo = rng.integers(0, 500, (q, l)).astype(np.float32)
+    box = np.stack([lo, lo + (500 if l > 1 else 20)], axis=2).reshape(q, 2 * l).copy()
+    c = dict(clusters=8, sub_clusters=8, pq_dim=m, max_grids=256, filter_dim=2, n_list=8, sub_lists=64, exps0=4, topk=10)
+    c.update(conf)
+    return dict(base=rng.standard_normal((n, d), dtype=np.float32), labels=lab,
+                queries=rng.standard_normal((q, d), dtype=np.float32), query_labels=box,
+                hdgrid_conf=datasets.hdgrid_conf(**c),
+                filter_conf=f"l = {l}\n" + "".join(f"filter{i}:\n\ttype = 3\n" for i in range(l)), k=int(c["topk"]))
+
+
+def _io(ws, base, k, cuda, q0=0, q1=None):
+    """The queries [q0, q1) of a workload as call arguments: (distances, ids, query input, query output)."""
+    import torch
+    import hdgrid_b200 as hg
+    q = torch.from_numpy(ws["queries"][q0:q1].copy()).to(cuda)
+    ql = torch.from_numpy(ws["query_labels"][q0:q1].copy()).to(cuda)
+    d = torch.full((q.shape[0], k), -1.0, device=cuda)
+    i = torch.full((q.shape[0], k), 7, dtype=torch.int64, device=cuda)
+    return d, i, hg.query_input_t(base, q, ql), hg.query_output_t(d, i)
+
+
+# batches whose kernels ask for different amounts of shared memory, from two threads on two streams
+@pytest.mark.parametrize("what", ["query", "bruteforce", "bruteforce_batch", "pq_adc"])
+def test_threads_with_different_sizes(cuda, what):
+    import torch
+    import hdgrid_b200 as hg
+    rng = np.random.default_rng(4)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    calls, outs = [], []
+    if what == "query":  # subspaces of 16 dims: table slices of 34 KB for one query, 135 KB for 5,000
+        ws = _range_ws(2000, 5000, d=512)
+        idx, base, _ = build_gpu(ws, cuda)
+        for n in (1, 5000):
+            d, i, qin, qout = _io(ws, base, 10, cuda, 0, n)
+            outs.append((d, i))
+            calls.append(lambda st, a=qin, b=qout: idx.query(a, b, stream=st))
+        repeat = 300
+    elif what == "pq_adc":
+        for m in (8, 64):
+            codes = torch.from_numpy(rng.integers(0, 256, (m, 5000), dtype=np.uint8)).to(cuda)
+            lut = torch.rand((4, m, 256), device=cuda)
+            d = torch.zeros((4, 5000), device=cuda)
+            outs.append((d,))
+            calls.append(lambda st, a=codes, b=lut, c=d, m=m: hg.pq_adc(a, 5000, b, 4, m, 256, None, 5000, c, stream=st))
+        repeat = 2000
+    else:
+        q, n = (4, 2000) if what == "bruteforce" else (64, 190000)
+        for dim, l, k in ((16, 1, 5), (96, 5, 200)):
+            x = [torch.randn((n, dim), device=cuda), torch.rand((n, l), device=cuda), torch.randn((q, dim), device=cuda),
+                 torch.tensor([0.0, 0.7] * l, device=cuda).repeat(q, 1)]
+            d = torch.zeros((q, k), device=cuda)
+            i = torch.zeros((q, k), dtype=torch.int64, device=cuda)
+            outs.append((d, i))
+            calls.append(lambda st, x=x, k=k, d=d, i=i: hg.bruteforce_knn(*x, k, d, i, stream=st))
+        repeat = 2000 if what == "bruteforce" else 200
+    torch.cuda.synchronize()
+    want = []
+    for c, o, st in zip(calls, outs, streams):
+        c(st)
+        torch.cuda.synchronize()
+        want.append([x.clone() for x in o])
+
+    done = threading.Event()
+
+    def loop(c, st, first):
+        try:
+            n = 0
+            while not done.is_set() if first else n < repeat:  # the first for as long as the second
+                c(st)
+                n += 1
+                if n % 64 == 0:
+                    st.synchronize()
+            st.synchronize()
+        finally:
+            done.set()
+
+    errors = _in_threads(*(lambda a=a: loop(*a) for a in zip(calls, streams, (True, False))))
+    assert not errors, errors[0]
+    for w, o in zip(want, outs):
+        assert all(torch.equal(a, b) for a, b in zip(w, o))
