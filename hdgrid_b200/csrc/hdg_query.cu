@@ -3414,6 +3414,12 @@ static void resolve_lazy(hdg_index* idx, QueryCtx& cx) {
 // 5.5: 3,499 / 3,425; 98 M, 24,600, 2.6: 2,362 / 2,345; 26 M, 5,200, 2.3: 2,314 / 2,029.
 constexpr uint64_t kEstMinCands = 32ull << 20, kEstMinRow = 8192, kEstMinRatio = 6;
 
+// Dynamic shared memory of the pass's kernels that hold a query's R candidate ranges
+static size_t est_thr_smem(uint32_t G, int R) { return sizeof(uint32_t) * (G * kCodes * 16 + kThrMax + kThrBins + 2 * (size_t)R + 1); }
+static size_t est_pick_smem(int R) { return sizeof(uint32_t) * (2 * (size_t)R + 1); }
+// (with up to 10 KB of static tables beside them)
+static bool est_fits(uint32_t G, int R) { return std::max(est_thr_smem(G, R), est_pick_smem(R)) + 10 * 1024 <= kBlockSmem; }
+
 // Thresholds, row-tile entries (`entries` of them at most), estimates and the scan's work items.
 // False, and nothing enqueued, when its memory is not there.
 static bool estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const QueryCall& c, int R, uint32_t G,
@@ -3460,7 +3466,7 @@ static bool estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const Quer
     a.prow = w.spos;
     a.cnt = w.cand_count;
     CK(cudaMemsetAsync(diff, 0, (tiles + 1) * 4ull, st));
-    const size_t sm = sizeof(uint32_t) * (G * kCodes * 16 + kThrMax + kThrBins + 2 * R + 1);
+    const size_t sm = est_thr_smem(G, R);
     auto thr = [&](auto kern) {
         allow_smem(kern);
         kern<<<(unsigned)q, kThrThreads, sm, st>>>(D, R, c.queries, w);
@@ -3477,7 +3483,8 @@ static bool estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const Quer
     k_est_fill<<<blocks, 256, 0, st>>>(q, R, w, cursor, ent);
     CK_LAUNCH();
     est_ranges(a, D.decoded, (int)D.d, w.gemm_err, st);
-    k_est_pick<<<(unsigned)q, kPickThreads, sizeof(uint32_t) * (2 * R + 1), st>>>(R, w);
+    allow_smem(k_est_pick);
+    k_est_pick<<<(unsigned)q, kPickThreads, est_pick_smem(R), st>>>(R, w);
     CK_LAUNCH();
     k_scan_plan<<<1, 1024, 0, st>>>(q, w);
     CK_LAUNCH();
@@ -3664,7 +3671,8 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
         // post-filter queries with many more candidates than budget: the estimate pass (not in a
         // captured graph, whose entry count is not known)
         bool prune = sync_sizing && !lazy && mode == kPost && !w.qsched && fast && D.decoded && sc[0] >= kEstMinCands &&
-                           sc[0] / q >= kEstMinRow && sc[0] >= kEstMinRatio * sc[7] && sc[2] < (1u << 24) && sc[9] < (1ull << 32);
+                     sc[0] / q >= kEstMinRow && sc[0] >= kEstMinRatio * sc[7] && sc[2] < (1u << 24) && sc[9] < (1ull << 32) &&
+                     est_fits(G, R);
         if (prune) prune = estimate_pass(idx, cx, w, c, R, G, sc[9], st);
         if (prune) {
             launches += 7;

@@ -113,3 +113,25 @@ def test_threads_with_different_sizes(cuda, what):
     assert not errors, errors[0]
     for w, o in zip(want, outs):
         assert all(torch.equal(a, b) for a, b in zip(w, o))
+
+
+def test_estimate_pass_many_ranges(cuda):
+    """2,048 lists in three parts each: 6,144 ranges per query."""
+    import torch
+    ws = datasets.config4(scale=0.04, n_queries=129, clusters=64, sub_clusters=32, n_list=64, sub_lists=2048, exps0=2,
+                          max_grids=1024, pq_dim=32, topk=10, is_split=1, n_split=3)
+    ws["query_labels"][:, 0::2] = 0
+    ws["query_labels"][:, 1::2] = 1_000_000
+    idx, base, _ = build_gpu(ws, cuda)
+    d, i, qin, qout = _io(ws, base, 10, cuda)
+    idx.set_param("BREAK_DOWN", 1)
+    idx.query(qin, qout)
+    assert "estimate" in idx.stage_times()
+    want = d.clone(), i.clone()
+    idx.set_param("QUERY_GRAPH", 1)  # the replay scans every candidate
+    idx.query(qin, qout)
+    d.fill_(-1.0)
+    idx.query(qin, qout)
+    idx.status()
+    torch.cuda.synchronize()
+    assert torch.equal(d, want[0]) and torch.equal(i, want[1])
