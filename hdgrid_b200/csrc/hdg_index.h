@@ -154,7 +154,7 @@ struct QueryCtx {
     DeviceBuffer pos_buf;           // u32 candidate positions of compact rows (same capacity)
     DeviceBuffer sel_buf;           // u32 selected candidates: min(n_cand, candidates) per query
     DeviceBuffer part_buf;          // u64 best keys of the refine work items
-    DeviceBuffer est_buf;           // thresholds and row-tile entries of the estimate pass
+    DeviceBuffer est_buf;           // thresholds and row-tile entries of the estimate pass (where dist_buf has no room)
     uint64_t work_queries = 0;
     std::map<std::string, std::pair<size_t, size_t>> layout;  // name -> (offset, bytes)
     GraphState* graphs = nullptr;   // QUERY_GRAPH=1: graphs keyed by pointers and sizes

@@ -3420,10 +3420,10 @@ static size_t est_pick_smem(int R) { return sizeof(uint32_t) * (2 * (size_t)R + 
 // (with up to 10 KB of static tables beside them)
 static bool est_fits(uint32_t G, int R) { return std::max(est_thr_smem(G, R), est_pick_smem(R)) + 10 * 1024 <= kBlockSmem; }
 
-// Thresholds, row-tile entries (`entries` of them at most), estimates and the scan's work items.
-// False, and nothing enqueued, when its memory is not there.
+// Thresholds, row-tile entries (`entries` of them at most), estimates and the scan's work items of a
+// batch of `cands` candidates.  False, and nothing enqueued, when its memory is not there.
 static bool estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const QueryCall& c, int R, uint32_t G,
-                          uint64_t entries, cudaStream_t st) {
+                          uint64_t entries, uint64_t cands, cudaStream_t st) {
     const IndexDev& D = idx->dev;
     const uint64_t q = c.q;
     const uint32_t tiles = (D.n + kEstM - 1) / kEstM;
@@ -3437,11 +3437,20 @@ static bool estimate_pass(hdg_index* idx, QueryCtx& cx, Workspace& w, const Quer
                  o_qc = take(q * sizeof(float4));
     const size_t o_diff = take((tiles + 1) * 4ull), o_eo = take((tiles + 1) * 4ull), o_no = take((tiles + 1) * 4ull),
                  o_cur = take((tiles + 1) * 4ull), o_ent = take(std::max<uint64_t>(entries, 1) * sizeof(uint4));
-    if (cx.est_buf.bytes < off) {
-        cx.est_buf.reset();
-        if (!cx.est_buf.try_ensure(off + off / 4)) return false;
+    // In the part of the rows that this batch leaves unused when it is large enough (the quarter more
+    // of a batch of this size, or what a larger one left: then there may be no other memory), else in a
+    // buffer of its own
+    const size_t used = align_up(std::max<uint64_t>(cands, 1) * 4, 256);
+    char* b = nullptr;
+    if (cx.dist_buf.bytes >= used + off) {
+        b = static_cast<char*>(cx.dist_buf.ptr) + used;
+    } else {
+        if (cx.est_buf.bytes < off) {
+            cx.est_buf.reset();
+            if (!cx.est_buf.try_ensure(off + off / 4) && !cx.est_buf.try_ensure(off)) return false;
+        }
+        b = static_cast<char*>(cx.est_buf.ptr);
     }
-    char* b = static_cast<char*>(cx.est_buf.ptr);
     w.prq = reinterpret_cast<uint32_t*>(b + o_prq);
     w.est_w = reinterpret_cast<int*>(b + o_w);
     w.est_in = reinterpret_cast<uint32_t*>(b + o_in);
@@ -3673,7 +3682,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
         bool prune = sync_sizing && !lazy && mode == kPost && !w.qsched && fast && D.decoded && sc[0] >= kEstMinCands &&
                      sc[0] / q >= kEstMinRow && sc[0] >= kEstMinRatio * sc[7] && sc[2] < (1u << 24) && sc[9] < (1ull << 32) &&
                      est_fits(G, R);
-        if (prune) prune = estimate_pass(idx, cx, w, c, R, G, sc[9], st);
+        if (prune) prune = estimate_pass(idx, cx, w, c, R, G, sc[9], sc[0], st);
         if (prune) {
             launches += 7;
             tm.mark("estimate");

@@ -1,5 +1,6 @@
 """Calls at the limits of their resources: little free device memory, several host threads,
 buffers left by larger calls, candidate ranges near the shared-memory limit."""
+import contextlib
 import threading
 
 import numpy as np
@@ -9,6 +10,29 @@ from hdgrid_b200 import datasets
 from tests.helpers import build_gpu
 
 pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+@contextlib.contextmanager
+def only_free(n_bytes: int):
+    """Takes device memory until n_bytes of it (give or take 4 MB) are free."""
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = []
+    for step in (64 * MB, 2 * MB):
+        while True:
+            over = torch.cuda.mem_get_info()[0] - n_bytes
+            if over < step:
+                break
+            held.append(torch.empty(over // step * step, dtype=torch.uint8, device="cuda"))
+    try:
+        yield
+    finally:
+        torch.cuda.synchronize()
+        held.clear()
+        torch.cuda.empty_cache()
 
 
 def _in_threads(*calls):
@@ -113,6 +137,32 @@ def test_threads_with_different_sizes(cuda, what):
     assert not errors, errors[0]
     for w, o in zip(want, outs):
         assert all(torch.equal(a, b) for a, b in zip(w, o))
+
+
+def test_estimate_pass_after_a_larger_batch(cuda):
+    """The candidate rows of a larger batch hold the memory: the entries of the estimate pass go
+    into the part of them that a smaller batch leaves unused."""
+    import torch
+    ws = datasets.config4(scale=0.04, n_queries=1500, clusters=16, sub_clusters=8, n_list=16, sub_lists=100, exps0=8,
+                          max_grids=16384, pq_dim=32)
+    idx, base, _ = build_gpu(ws, cuda)
+    a, b = _io(ws, base, 100, cuda), _io(ws, base, 100, cuda, 0, 900)
+    idx.set_param("BREAK_DOWN", 1)
+    idx.query(b[2], b[3])
+    assert "estimate" in idx.stage_times()
+    want = b[0].clone(), b[1].clone()
+    idx, base, _ = build_gpu(ws, cuda)  # (new buffers)
+    idx.set_param("BREAK_DOWN", 1)
+    idx.set_param("EXPS0", 4096)  # budgets of most of the candidates: no estimate pass
+    idx.query(a[2], a[3])
+    assert "estimate" not in idx.stage_times()
+    idx.set_param("EXPS0", 8)
+    with only_free(2 * MB):
+        idx.query(b[2], b[3])
+        stages = idx.stage_times()
+        torch.cuda.synchronize()
+    assert "estimate" in stages, stages
+    assert torch.equal(b[0], want[0]) and torch.equal(b[1], want[1])
 
 
 def test_estimate_pass_many_ranges(cuda):
