@@ -1583,7 +1583,7 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
             }
             if (planes * D.plane_words * 4 <= kPlanesMax) break;
         }
-        // (without room for them the predicate pass reads every candidate's labels)
+        // (without room for them the predicate pass tests the packed ranks, one candidate at a time)
         if (idx->planes.try_ensure(std::max<uint64_t>(planes * D.plane_words * 4, 16))) {
             k_rank_planes<<<blocks_for(D.plane_words, 64), 256, 0, st>>>(D, H.n, static_cast<uint32_t*>(idx->planes.ptr));
             CK_LAUNCH();

@@ -1464,13 +1464,15 @@ __device__ __forceinline__ void pre_bits(const IndexDev& D, int lbl, const float
     if (st != sh) pre_flush(sr, SS, sh, (int)(st - sh), ctr, drow, prow);
 }
 
-// The same without the rank test, for an index with NaN labels (a NaN passes the label test): every
-// candidate's labels are read.  Out of line, so that the other loop stays compact in the instruction
-// cache.  qr: [2][256] ring of survivors.
-template <bool LAB4>
-__device__ __noinline__ void pre_labels(const IndexDev& D, int lbl, const float* bx_s, const uint32_t* pre,
-                                        const uint32_t* start, int R, int r0, uint32_t e0, uint32_t e1, uint32_t* qr,
-                                        uint32_t* ctr, uint32_t* drow, uint32_t* prow) {
+// The same position by position, where there are no bit planes: with RANKS (no memory for the planes)
+// the packed ranks are tested against the outer and the inner box (rb: rank_box, high words with the
+// guard bits gd) before labels are read; without (NaN labels: a NaN passes the label test) every
+// candidate's labels are.  qr: [2][256] ring of survivors.  Returns the candidates whose labels were
+// read.
+template <bool LAB4, bool RANKS>
+__device__ __forceinline__ uint32_t pre_labels(const IndexDev& D, int lbl, const float* bx_s, uint4 rb, const uint32_t* pre,
+                                               const uint32_t* start, int R, int r0, uint32_t e0, uint32_t e1, uint32_t* qr,
+                                               uint32_t* ctr, uint32_t* drow, uint32_t* prow) {
     constexpr int J = 4;  // windows of 32 positions in one step: as many label loads in flight
     constexpr uint32_t QS = 256;
     const int lane = threadIdx.x & 31;
@@ -1497,7 +1499,8 @@ __device__ __noinline__ void pre_labels(const IndexDev& D, int lbl, const float*
             find_next();
         }
     };
-    uint32_t qh = 0, qt = 0;
+    const uint32_t gd = D.rank_guard;
+    uint32_t qh = 0, qt = 0, n_read = 0;
     for (uint32_t eb = e0; eb < e1; eb += 32u * J) {
         uint32_t pp[J];
         bool pv[J];
@@ -1517,17 +1520,36 @@ __device__ __noinline__ void pre_labels(const IndexDev& D, int lbl, const float*
             pp[j] = pv[j] ? base + e : 0u;
             advance_to(p + 32u);
         }
+        bool sure[J];  // pass without a look at their labels; pv: the labels decide
+#pragma unroll
+        for (int j = 0; j < J; j++) sure[j] = false;
+        if (RANKS) {
+            uint32_t c[J];
+#pragma unroll
+            for (int j = 0; j < J; j++) c[j] = pv[j] ? __ldg(D.rankpack + pp[j]) : 0u;
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                // every field at or above its low bound and at or below its high bound: the guard bit
+                // above a field survives both subtractions exactly then
+                auto inside = [&](uint32_t lo, uint32_t hi) { return ((((c[j] | gd) - lo) & (hi - c[j])) & gd) == gd; };
+                sure[j] = pv[j] && inside(rb.z, rb.w);
+                pv[j] = pv[j] && !sure[j] && inside(rb.x, rb.y);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < J; j++) n_read += __popc(__ballot_sync(0xffffffffu, pv[j]));
         if (LAB4) {
             float4 v[J];
 #pragma unroll
             for (int j = 0; j < J; j++) v[j] = pv[j] ? __ldg(lab4 + pp[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int j = 0; j < J; j++)
-                ring_push<QS>(qr, qt, pv[j] && pre_box4(bx_s, v[j]), eb + 32u * j + lane, pp[j]);
+                ring_push<QS>(qr, qt, sure[j] || (pv[j] && pre_box4(bx_s, v[j])), eb + 32u * j + lane, pp[j]);
         } else {
 #pragma unroll
             for (int j = 0; j < J; j++)
-                ring_push<QS>(qr, qt, pv[j] && pre_label_ok<LAB4>(D, lbl, bx_s, pp[j]), eb + 32u * j + lane, pp[j]);
+                ring_push<QS>(qr, qt, sure[j] || (pv[j] && pre_label_ok<LAB4>(D, lbl, bx_s, pp[j])), eb + 32u * j + lane,
+                              pp[j]);
         }
         while (qt - qh >= 32) {
             pre_flush(qr, QS, qh, 32, ctr, drow, prow);
@@ -1535,9 +1557,14 @@ __device__ __noinline__ void pre_labels(const IndexDev& D, int lbl, const float*
         }
     }
     if (qt != qh) pre_flush(qr, QS, qh, (int)(qt - qh), ctr, drow, prow);
+    return n_read;
 }
 
-template <bool LAB4>
+// What a candidate is tested by before its labels: bit planes, packed ranks, nothing.  Kernels of their
+// own: the planes' loop is compact in the instruction cache (with the others called out of line beside
+// it 5,431 us for the 10 M point batch of the learned schedule, 5,351 so).
+enum PreTest { kPlaneTest, kRankTest, kLabelTest };
+template <bool LAB4, int TEST>
 __global__ void __launch_bounds__(kPreThreads, 4) k_pre_scan(IndexDev D, int R, int lbl, uint64_t q, Workspace w) {
     constexpr int NW = kPreThreads / 32;
     extern __shared__ __align__(16) uint32_t s_rings[];  // per warp: staged labels, ranges, planes, queue ring, survivor ring
@@ -1556,7 +1583,6 @@ __global__ void __launch_bounds__(kPreThreads, 4) k_pre_scan(IndexDev D, int R, 
         if (e0 >= total) continue;  // a query cut by a capacity
         const uint32_t e1 = min(total, e0 + chunk);
         if (lane < 2 * lbl) s_bx[wp][lane] = w.box[(uint64_t)qq * 2 * lbl + lane];
-        const bool use = D.rank_planes != nullptr;
         float4* lst = reinterpret_cast<float4*>(s_rings + (size_t)wp * kPreRingWords);
         uint4* rt = reinterpret_cast<uint4*>(lst + 128);
         const uint32_t** pl = reinterpret_cast<const uint32_t**>(rt + 32);
@@ -1581,7 +1607,7 @@ __global__ void __launch_bounds__(kPreThreads, 4) k_pre_scan(IndexDev D, int R, 
         };
         PreBox outer{}, inner{};
         bool has_inner = false;
-        if (use) {
+        if (TEST == kPlaneTest) {
             const uint32_t sft = D.plane_shift, mask = (1u << D.rank_bits) - 1u;
             const uint32_t off = lane < lbl ? lane * (D.rank_bits + 1) : 0u, top = lane < lbl ? D.rank_n[lane] : 0u;
             auto field = [&](int k) { return (w.rank_box[4 * qq + k] >> off) & mask; };
@@ -1601,13 +1627,13 @@ __global__ void __launch_bounds__(kPreThreads, 4) k_pre_scan(IndexDev D, int R, 
         uint32_t* prow = w.spos + w.qoff[qq];
         uint32_t n_read = 0, n_chk = 0;
         const float* bxs = s_bx[wp];
-        if (use) {
+        if constexpr (TEST == kPlaneTest) {
             pre_bits<LAB4>(D, lbl, bxs, outer, inner, has_inner, pre, start, R, r0, e0, e1, qr, sr, lst, rt, ctr, drow, prow, n_read);
-            n_chk = e1 - e0;
         } else {
-            pre_labels<LAB4>(D, lbl, bxs, pre, start, R, r0, e0, e1, qr, ctr, drow, prow);
-            n_read = e1 - e0;
+            const uint4 rb = make_uint4(w.rank_box[4 * qq], w.rank_box[4 * qq + 1], w.rank_box[4 * qq + 2], w.rank_box[4 * qq + 3]);
+            n_read = pre_labels<LAB4, TEST == kRankTest>(D, lbl, bxs, rb, pre, start, R, r0, e0, e1, qr, ctr, drow, prow);
         }
+        if (TEST != kLabelTest) n_chk = e1 - e0;
         if (lane == 0 && n_read) atomicAdd(&w.lab_read[qq], n_read);
         if (lane == 0 && n_chk) atomicAdd(&w.rank_read[qq], n_chk);
     }
@@ -3652,8 +3678,9 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
                 const int blocks = sm_count() * occupancy_blocks(kern, kPreThreads, smp);
                 kern<<<blocks, kPreThreads, smp, st>>>(D, R, l, q, w);
             };
-            if (lab4) launch_pre(k_pre_scan<true>);
-            else launch_pre(k_pre_scan<false>);
+            if (D.rank_planes) lab4 ? launch_pre(k_pre_scan<true, kPlaneTest>) : launch_pre(k_pre_scan<false, kPlaneTest>);
+            else if (D.rankpack && !D.labels_nan) lab4 ? launch_pre(k_pre_scan<true, kRankTest>) : launch_pre(k_pre_scan<false, kRankTest>);
+            else lab4 ? launch_pre(k_pre_scan<true, kLabelTest>) : launch_pre(k_pre_scan<false, kLabelTest>);
             CK_LAUNCH();
             k_scan_plan<<<1, 1024, 0, st>>>(q, w);
             CK_LAUNCH();

@@ -165,6 +165,32 @@ def test_estimate_pass_after_a_larger_batch(cuda):
     assert torch.equal(b[0], want[0]) and torch.equal(b[1], want[1])
 
 
+def test_ranks_tested_without_planes(cuda, tmp_path):
+    """An index loaded with no room for the rank planes still rejects candidates by their packed
+    ranks before it reads labels."""
+    import torch
+    import hdgrid_b200 as hg
+    n, q = 2_000_000, 2
+    ws = _range_ws(n, q, exps0=1)
+    idx, base, _ = build_gpu(ws, cuda)
+    d, i, qin, qout = _io(ws, base, 10, cuda)
+    idx.query(qin, qout)
+    torch.cuda.synchronize()
+    want = d.clone(), i.clone()
+    path = str(tmp_path / "index.hdg")
+    idx.save(path)
+    del idx
+    with only_free(n * (64 + 32) + 24 * MB):  # arena and code rows; the planes are another 64 a point
+        idx = hg.SuperGridIndex.load(path)
+        idx.query(qin, qout)
+        torch.cuda.synchronize()
+    total = idx.last_query_stats()["coarse_total"]
+    read = np.frombuffer(idx.debug_fetch("labels_read").tobytes(), np.uint32)[:q].astype(np.int64).sum()
+    tested = np.frombuffer(idx.debug_fetch("ranks_read").tobytes(), np.uint32)[:q].astype(np.int64).sum()
+    assert torch.equal(d, want[0]) and torch.equal(i, want[1])
+    assert tested == total and read < total // 2, (tested, read, total)
+
+
 def test_estimate_pass_many_ranges(cuda):
     """2,048 lists in three parts each: 6,144 ranges per query."""
     import torch
