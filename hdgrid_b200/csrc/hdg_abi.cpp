@@ -390,7 +390,7 @@ hdg_status hdg_get_info(const hdg_index* index, hdg_index_info* out) {
         out->morton_max_bits = H.grid.morton_max_bits;
         out->morton_valid_map = H.grid.morton_valid_map;
         out->diff_dim = H.grid.diff_dim;
-        out->device_bytes = index->arena.bytes;
+        out->device_bytes = index->arena.bytes + index->planes.bytes + index->decoded.bytes;
         out->prefix_entries = index->host.prefix_entries;
         out->rank_pack_bytes = index->dev.rankpack ? 4 : 0;
         out->rank_bits = index->dev.rank_bits;

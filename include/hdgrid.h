@@ -244,7 +244,7 @@ typedef struct hdg_index_info {
     uint64_t label_left[HDG_MAX_LABEL_DIMS];
     uint64_t label_span[HDG_MAX_LABEL_DIMS];
     int32_t morton_dims, morton_max_bits, morton_valid_map, diff_dim;
-    uint64_t device_bytes;
+    uint64_t device_bytes;    /* every index array; the query workspaces are not among them */
     uint64_t prefix_entries;  /* change points of the compressed prefix rows; 0 = dense form */
     uint64_t rank_pack_bytes; /* bytes per point of the packed label ranks, tested
                                * before the labels (4; 0 = not kept) */

@@ -165,6 +165,23 @@ def test_estimate_pass_after_a_larger_batch(cuda):
     assert torch.equal(b[0], want[0]) and torch.equal(b[1], want[1])
 
 
+def test_device_bytes_counts_every_index_array(cuda):
+    import torch
+    n = 1_000_000
+    ws = _range_ws(n, 8, d=128)
+    torch.cuda.synchronize()
+    base = torch.from_numpy(ws["base"]).to(cuda)
+    labels = torch.from_numpy(ws["labels"]).to(cuda)
+    import hdgrid_b200 as hg
+    idx = hg.SuperGridIndex.from_text(ws["hdgrid_conf"], ws["filter_conf"])
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    idx.build(hg.build_input_t(base, labels))
+    torch.cuda.synchronize()
+    used = before - torch.cuda.mem_get_info()[0]
+    assert abs(idx.info()["device_bytes"] - used) < 32 * MB, (idx.info()["device_bytes"], used)
+
+
 def test_ranks_tested_without_planes(cuda, tmp_path):
     """An index loaded with no room for the rank planes still rejects candidates by their packed
     ranks before it reads labels."""
