@@ -1379,6 +1379,14 @@ void label_rank_thresholds(const float* labels, uint64_t n, int l, int bits, flo
     }
 }
 
+// The index's optional buffers (decoded vectors, rank planes) speed calls up that run without them too.
+// They are kept while each takes at most a quarter of the memory that is free, and given back to a
+// call that has no room otherwise (release_optional).
+static bool optional_room(uint64_t bytes) {
+    size_t free = 0, total = 0;
+    CK(cudaMemGetInfo(&free, &total));
+    return bytes <= free / 4;
+}
 constexpr uint64_t kDecodedMax = 16ull << 30;
 constexpr uint64_t kPlanes = 512, kPlanesMax = 8ull << 30;  // label-rank bit planes: at most 64 bytes per point
 constexpr uint64_t kDecodedMinPoints = 16384;  // smaller sets never reach the estimate pass
@@ -1469,6 +1477,8 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
     const bool pre16 = n_dense && max_list <= 0xffffu;
     const size_t o_pq = reserve(H.pq_centers.size() * 4), o_pre = reserve(n_dense * (pre16 ? 2 : 4));
     const size_t o_poff = reserve(n_off * 8), o_prow = reserve(n_rows * 8);
+    idx->planes.reset();
+    idx->decoded.reset();
     idx->arena.reset();
     idx->arena.ensure(total);
     char* base = static_cast<char*>(idx->arena.ptr);
@@ -1568,8 +1578,6 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
         D.S_max = std::max<uint32_t>(D.S_max, H.cluster_off[c + 1] - H.cluster_off[c]);
     // the ranks' bit planes: up to kPlanes of them in all, a bit of resolution less for as long as
     // they would take more than kPlanesMax bytes
-    D.rank_planes = nullptr;
-    idx->planes.reset();
     if (rbits && !D.labels_nan) {
         D.plane_words = align_up((H.n + 31) / 32, 8);
         D.plane_shift = 0;
@@ -1584,21 +1592,19 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
             if (planes * D.plane_words * 4 <= kPlanesMax) break;
         }
         // (without room for them the predicate pass tests the packed ranks, one candidate at a time)
-        if (idx->planes.try_ensure(std::max<uint64_t>(planes * D.plane_words * 4, 16))) {
+        if (optional_room(planes * D.plane_words * 4) && idx->planes.try_ensure(std::max<uint64_t>(planes * D.plane_words * 4, 16))) {
             k_rank_planes<<<blocks_for(D.plane_words, 64), 256, 0, st>>>(D, H.n, static_cast<uint32_t*>(idx->planes.ptr));
             CK_LAUNCH();
             D.rank_planes = static_cast<const uint32_t*>(idx->planes.ptr);
         }
     }
     // the estimate pass of the post-filter scan reads the points' PQ approximations as tensor-core
-    // operands (2 d + 16 bytes per point; not kept past kDecodedMax, where the full scan runs)
-    D.decoded = nullptr;
-    D.decoded_c = nullptr;
-    D.decoded_max = nullptr;
-    idx->decoded.reset();
+    // operands (2 d + 16 bytes per point; not kept past kDecodedMax, where the full scan runs, nor with one
+    // label dim, whose schedule has no such scan)
     const uint64_t dec = align_up((uint64_t)H.n * H.d * 2, 256);
-    if (H.d % 8 == 0 && H.M % 32 == 0 && H.M <= 96 && H.M * H.pq_len == H.d && H.n >= kDecodedMinPoints &&
-        dec <= kDecodedMax && idx->decoded.try_ensure(dec + (uint64_t)H.n * sizeof(float4) + 16)) {
+    if (H.l > 1 && H.d % 8 == 0 && H.M % 32 == 0 && H.M <= 96 && H.M * H.pq_len == H.d && H.n >= kDecodedMinPoints &&
+        dec <= kDecodedMax && optional_room(dec + (uint64_t)H.n * sizeof(float4) + 16) &&
+        idx->decoded.try_ensure(dec + (uint64_t)H.n * sizeof(float4) + 16)) {
         const uint64_t cst = (uint64_t)H.n * sizeof(float4);
         char* p = static_cast<char*>(idx->decoded.ptr);
         uint32_t* mx = reinterpret_cast<uint32_t*>(p + dec + cst);

@@ -3179,13 +3179,47 @@ static QueryCtx& query_ctx(hdg_index* idx, cudaStream_t st) {
     return *slot;
 }
 
-void reserve_workspace(hdg_index* idx, uint64_t q, cudaStream_t st) {
+// Gives back one of the index's optional buffers: the decoded vectors (the estimate pass is left out
+// from then on), then the rank planes (the packed ranks are tested instead).  No context's mutex may be
+// held: none of them is enqueueing a call, which would read their addresses, while it is at work; the
+// launched ones have ended when cudaFree returns.  False: nothing left to give.
+static bool release_optional(hdg_index* idx) {
+    std::lock_guard<std::mutex> g(idx->ctx_mu);
+    std::vector<std::unique_lock<std::mutex>> held;
+    for (auto& kv : idx->ctxs) held.emplace_back(kv.second->mu);
+    DeviceBuffer& b = idx->decoded.ptr ? idx->decoded : idx->planes;
+    if (!b.ptr) return false;
+    for (auto& kv : idx->ctxs) invalidate_ctx_graphs(*kv.second);  // (they hold its address)
+    if (&b == &idx->planes) idx->dev.rank_planes = nullptr;
+    else idx->dev.decoded = nullptr, idx->dev.decoded_c = nullptr, idx->dev.decoded_max = nullptr;
+    b.reset();
+    return true;
+}
+
+// f(), again without the optional buffers where it ran out of device memory.
+template <typename F>
+static void with_room(hdg_index* idx, F&& f) {
+    for (;;) {
+        try {
+            f();
+            return;
+        } catch (const Error& e) {
+            if (e.status != HDG_ERR_OOM || !release_optional(idx)) throw;
+        }
+    }
+}
+
+static void reserve_once(hdg_index* idx, uint64_t q, cudaStream_t st) {
     QueryCtx& cx = query_ctx(idx, st);
     std::lock_guard<std::mutex> g(cx.mu);
     reserve_ctx(idx, cx, q);
     // a small batch's candidate buffers too: its calls then allocate nothing
     const uint64_t pairs = q * (uint64_t)idx->dev.n, k = idx->params.topk;
     if (pairs <= kUnsizedPairs && k >= 1 && k <= 2048) ensure_candidates(cx, q, (uint32_t)k, pairs, pairs);
+}
+
+void reserve_workspace(hdg_index* idx, uint64_t q, cudaStream_t st) {
+    with_room(idx, [&] { reserve_once(idx, q, st); });
 }
 
 FilterDev filter_dev(const hdg_index* idx) {
@@ -3834,10 +3868,9 @@ static void make_graph_key(const hdg_index* idx, const QueryCtx& cx, const Query
     std::memcpy(key, v, sizeof(v));
 }
 
-void run_query(hdg_index* idx, const float* d_queries, uint64_t q, const float* d_query_labels,
-               uint32_t label_cols, const float* d_data, uint32_t k, float* d_dist, uint64_t* d_ids,
-               cudaStream_t st, const uint32_t* d_k, const uint32_t* d_nprobe, const uint8_t* d_sched) {
-    const QueryCall c{d_queries, q, d_query_labels, label_cols, d_data, k, d_dist, d_ids, d_k, d_nprobe, d_sched};
+static void query_once(hdg_index* idx, const QueryCall& c, cudaStream_t st) {
+    const uint64_t q = c.q;
+    const uint32_t k = c.k;
     QueryCtx& cx = query_ctx(idx, st);
     std::lock_guard<std::mutex> lock(cx.mu);  // one query at a time per stream
     if (idx->params.query_graph == 0) {
@@ -3917,8 +3950,15 @@ void run_query(hdg_index* idx, const float* d_queries, uint64_t q, const float* 
     idx->lazy_ctx = nullptr;
 }
 
-void query_features(hdg_index* idx, const float* d_queries, uint64_t q, const float* d_query_labels,
-                    uint32_t label_cols, const uint32_t* d_k, uint32_t k_max, float* d_feats, cudaStream_t st) {
+void run_query(hdg_index* idx, const float* d_queries, uint64_t q, const float* d_query_labels,
+               uint32_t label_cols, const float* d_data, uint32_t k, float* d_dist, uint64_t* d_ids,
+               cudaStream_t st, const uint32_t* d_k, const uint32_t* d_nprobe, const uint8_t* d_sched) {
+    const QueryCall c{d_queries, q, d_query_labels, label_cols, d_data, k, d_dist, d_ids, d_k, d_nprobe, d_sched};
+    with_room(idx, [&] { query_once(idx, c, st); });
+}
+
+static void features_once(hdg_index* idx, const float* d_queries, uint64_t q, const float* d_query_labels,
+                          uint32_t label_cols, const uint32_t* d_k, uint32_t k_max, float* d_feats, cudaStream_t st) {
     HDG_REQUIRE(idx->built, HDG_ERR_STATE, "index not built");
     HDG_REQUIRE(q > 0 && q < (1ull << 31), HDG_ERR_INVALID_ARG, "query count out of range");
     HDG_REQUIRE(d_queries && d_query_labels && d_feats, HDG_ERR_INVALID_ARG, "null pointer");
@@ -3939,14 +3979,16 @@ void query_features(hdg_index* idx, const float* d_queries, uint64_t q, const fl
     learned_features(idx, d_queries, q, w.box, w.cluster_counts, d_k, k_max, d_feats, st);
 }
 
-void autotune_query(hdg_index* idx, const float* d_queries, uint64_t q, const float* d_query_labels,
-                    uint32_t label_cols, const float* d_data, uint32_t k, float* d_dist, uint64_t* d_ids,
-                    cudaStream_t st, float* best_ms) {
+void query_features(hdg_index* idx, const float* d_queries, uint64_t q, const float* d_query_labels,
+                    uint32_t label_cols, const uint32_t* d_k, uint32_t k_max, float* d_feats, cudaStream_t st) {
+    with_room(idx, [&] { features_once(idx, d_queries, q, d_query_labels, label_cols, d_k, k_max, d_feats, st); });
+}
+
+static void autotune_once(hdg_index* idx, const QueryCall& c, cudaStream_t st, float* best_ms) {
     hdg_params& P = idx->params;
     const uint64_t saved_bd = P.break_down, saved_graph = P.query_graph;
     P.break_down = 1;
     P.query_graph = 0;
-    const QueryCall c{d_queries, q, d_query_labels, label_cols, d_data, k, d_dist, d_ids, nullptr, nullptr, nullptr};
     float best = INFINITY;
     uint64_t best_cpt = 1, best_chunk = kChunk;
     QueryCtx& cx = query_ctx(idx, st);
@@ -3986,6 +4028,13 @@ void autotune_query(hdg_index* idx, const float* d_queries, uint64_t q, const fl
     lock.unlock();
     invalidate_graphs(idx);
     if (best_ms) *best_ms = best;
+}
+
+void autotune_query(hdg_index* idx, const float* d_queries, uint64_t q, const float* d_query_labels,
+                    uint32_t label_cols, const float* d_data, uint32_t k, float* d_dist, uint64_t* d_ids,
+                    cudaStream_t st, float* best_ms) {
+    const QueryCall c{d_queries, q, d_query_labels, label_cols, d_data, k, d_dist, d_ids, nullptr, nullptr, nullptr};
+    with_room(idx, [&] { autotune_once(idx, c, st, best_ms); });
 }
 
 }  // namespace hdg

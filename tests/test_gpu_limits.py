@@ -165,6 +165,73 @@ def test_estimate_pass_after_a_larger_batch(cuda):
     assert torch.equal(b[0], want[0]) and torch.equal(b[1], want[1])
 
 
+def test_optional_buffers_make_room(cuda):
+    """A batch whose rows need the memory of the decoded vectors and the rank planes gets it."""
+    import torch
+    n, q = 400_000, 600
+    ws = _range_ws(n, q, d=128, exps0=2)
+    idx, base, _ = build_gpu(ws, cuda)
+    d, i, qin, qout = _io(ws, base, 10, cuda)
+    idx.query(qin, qout)
+    torch.cuda.synchronize()
+    want = d.clone(), i.clone()
+    cands, sel = idx.last_query_stats()["coarse_total"], int(np.frombuffer(idx.debug_fetch("sel_off").tobytes(), np.uint64)[q])
+    del idx, qin, qout
+    idx, base, _ = build_gpu(ws, cuda)
+    d, i, qin, qout = _io(ws, base, 10, cuda)
+    idx.reserve(q)
+    rows = 8 * cands + 4 * sel + (sel // 4096 + q + 1) * 80
+    optional = idx.info()["device_bytes"]
+    with only_free(rows - 16 * MB):  # (the planes' 64 bytes a point are 25 MB, the decoded vectors 109 MB)
+        idx.query(qin, qout)
+        torch.cuda.synchronize()
+    assert idx.info()["device_bytes"] < optional
+    assert torch.equal(d, want[0]) and torch.equal(i, want[1])
+
+
+def test_room_made_while_another_thread_queries(cuda):
+    """The optional buffers go while calls of another stream, captured and plain, are on their way."""
+    import torch
+    n, q = 400_000, 600
+    ws = _range_ws(n, q, d=128, exps0=2)
+    idx, base, _ = build_gpu(ws, cuda)
+    big, small = _io(ws, base, 10, cuda), _io(ws, base, 10, cuda, 0, 20)
+    side = torch.cuda.Stream()
+    for graph in (0, 1):
+        idx.set_param("QUERY_GRAPH", graph)
+        for _ in range(2):
+            idx.query(small[2], small[3], stream=side)
+    idx.status()
+    torch.cuda.synchronize()
+    want = small[0].clone(), small[1].clone()
+    idx.reserve(q)
+    before = idx.info()["device_bytes"]
+    done = threading.Event()
+
+    def loop():
+        n_calls = 0
+        while not done.is_set() or n_calls < 20:
+            idx.query(small[2], small[3], stream=side)
+            n_calls += 1
+        idx.status()
+        side.synchronize()
+
+    def large():
+        try:
+            idx.query(big[2], big[3])
+            torch.cuda.synchronize()
+        finally:
+            done.set()
+
+    # the rows of 600 queries take about 1.3 GB: the decoded vectors, then the planes make room for them
+    with only_free(1200 * MB):
+        errors = _in_threads(loop, large)
+        torch.cuda.synchronize()
+    assert not errors, errors[0]
+    assert idx.info()["device_bytes"] < before
+    assert torch.equal(small[0], want[0]) and torch.equal(small[1], want[1])
+
+
 def test_device_bytes_counts_every_index_array(cuda):
     import torch
     n = 1_000_000
