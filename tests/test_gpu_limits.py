@@ -295,3 +295,20 @@ def test_estimate_pass_many_ranges(cuda):
     idx.status()
     torch.cuda.synchronize()
     assert torch.equal(d, want[0]) and torch.equal(i, want[1])
+
+
+@pytest.mark.parametrize("scale", [1e6, 1e-7])
+def test_no_estimate_pass_of_a_useless_scale(cuda, scale):
+    """PQ approximations that FP16 cannot hold bound nothing: they are not kept and a batch goes
+    straight to the full scan."""
+    import torch
+    ws = datasets.config4(scale=0.04, n_queries=1500, clusters=16, sub_clusters=8, n_list=16, sub_lists=100, exps0=8,
+                          max_grids=16384, pq_dim=32)
+    ws["base"] *= np.float32(scale)
+    ws["queries"] *= np.float32(scale)
+    idx, base, _ = build_gpu(ws, cuda)
+    d, i, qin, qout = _io(ws, base, 100, cuda)
+    idx.set_param("BREAK_DOWN", 1)
+    idx.query(qin, qout)
+    idx.query(qin, qout)
+    assert "estimate" not in idx.stage_times()
