@@ -407,7 +407,8 @@ void recover_filters_noalloc(const FilterDev& f0, const float* host_map, const f
 // tests the tile's labels first, packs the rows that pass into a list and only then computes
 // distances, one (query, row) pair per lane, in dimension order as one FMA chain.  A key below the
 // query's running k-th goes to the query's buffer, which a warp sort cuts back to k when it fills.
-// An item leaves its k best keys per query; k_bf_merge takes the k smallest over the spans.
+// An item leaves its k best keys per query; k_bf_merge takes the k smallest over the spans (with one
+// span, where there is no memory for the keys, they are the answer).
 // Bound: with many queries the shared-memory reads of the passing rows (16 bytes per pair and four
 // dimensions), with few the read of the base set.
 // One block per 32 queries that computed every pair and tested the labels afterwards took 352 ms
@@ -499,7 +500,8 @@ __global__ void __launch_bounds__(kBfThreads) k_bruteforce(const float* __restri
                                                            const float* __restrict__ labels, uint32_t l,
                                                            const float* __restrict__ queries, uint64_t nq,
                                                            const float* __restrict__ ranges, uint32_t k, BfShape b,
-                                                           uint64_t* __restrict__ part) {
+                                                           uint64_t* __restrict__ part, float* __restrict__ out_dist,
+                                                           uint64_t* __restrict__ out_ids) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int R = b.rows, dq = (int)(d + 3) / 4 * 4;
@@ -652,9 +654,16 @@ __global__ void __launch_bounds__(kBfThreads) k_bruteforce(const float* __restri
     for (int o = 0; o < kOwn; o++) {
         const int qq = (warp / b.share) * own + o;
         if (o >= own || qq >= nqb || sub) continue;
-        uint64_t* dst = part + ((q0 + qq) * b.spans + span) * k;
         const uint64_t* buf = s_buf + (size_t)(warp * own + o) * b.cap;
-        for (int i = lane; i < (int)k; i += 32) dst[i] = buf[i];
+        for (int i = lane; i < (int)k; i += 32) {
+            const uint64_t key = buf[i];
+            if (part) {
+                part[((q0 + qq) * b.spans + span) * k + i] = key;
+            } else {  // one span: the answer
+                out_dist[(q0 + qq) * k + i] = key != ~0ull ? key_float((uint32_t)(key >> 32)) : INFINITY;
+                out_ids[(q0 + qq) * k + i] = key != ~0ull ? (uint64_t)(uint32_t)key : ~0ull;
+            }
+        }
     }
 }
 
@@ -893,7 +902,20 @@ __global__ void __launch_bounds__(kBfExactThreads) k_bf_full(const float* __rest
     }
 }
 
-static void bruteforce_est(const float* data, uint64_t n, uint32_t d, const float* labels, uint32_t l,
+// Stream-ordered scratch; nullptr when the memory is not there
+static void* scratch(size_t bytes, cudaStream_t st) {
+    void* p = nullptr;
+    const cudaError_t e = cudaMallocAsync(&p, bytes, st);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    CK(e);
+    return p;
+}
+
+// False, and nothing enqueued, when its memory is not there.
+static bool bruteforce_est(const float* data, uint64_t n, uint32_t d, const float* labels, uint32_t l,
                            const float* queries, uint32_t nq, const float* ranges, uint32_t k, float* dist,
                            uint64_t* ids, cudaStream_t st) {
     const uint32_t ld = (d + 7) / 8 * 8, cap = (uint32_t)(3 * kBfRatio * k + 2048);
@@ -907,8 +929,8 @@ static void bruteforce_est(const float* data, uint64_t n, uint32_t d, const floa
     const size_t o_rows = take(rows_max * ld * 2), o_rc = take(rows_max * sizeof(float4)), o_q = take((size_t)nq * ld * 2),
                  o_qc = take(nq * sizeof(float4)), o_qn = take(nq * 4ull), o_list = take((size_t)nq * cap * 4),
                  o_cnt = take(nq * 4ull + 4);
-    char* b = nullptr;
-    CK(cudaMallocAsync(reinterpret_cast<void**>(&b), off, st));
+    char* b = static_cast<char*>(scratch(off, st));
+    if (!b) return false;
     try {
         uint16_t* rows = reinterpret_cast<uint16_t*>(b + o_rows);
         uint16_t* qh = reinterpret_cast<uint16_t*>(b + o_q);
@@ -962,6 +984,7 @@ static void bruteforce_est(const float* data, uint64_t n, uint32_t d, const floa
         throw;
     }
     CK(cudaFreeAsync(b, st));
+    return true;
 }
 
 void bruteforce_knn(const float* data, uint64_t n, uint32_t d, const float* labels, uint32_t l,
@@ -975,11 +998,17 @@ void bruteforce_knn(const float* data, uint64_t n, uint32_t d, const float* labe
     // (k 100, d 128; this path / k_bruteforce, us: 63 x 50,000 224 / 205, 32 x 200,000 395 / 326,
     // 63 x 200,000 397 / 461, 16 x 1 M 757 / 410, 32 x 1 M 832 / 880, 63 x 1 M 842 / 1,431)
     if (q >= kBfEstQueries && q * n >= kBfEstPairs && d <= 4096) {
-        for (uint64_t a = 0; a < q; a += 4096) {
+        uint64_t a = 0;
+        for (; a < q; a += 4096) {
             const uint32_t nb = (uint32_t)std::min<uint64_t>(4096, q - a);
-            bruteforce_est(data, n, d, labels, l, queries + a * d, nb, ranges + a * 2 * l, k, dist + a * k, ids + a * k, st);
+            if (!bruteforce_est(data, n, d, labels, l, queries + a * d, nb, ranges + a * 2 * l, k, dist + a * k, ids + a * k, st)) break;
         }
-        return;
+        if (a >= q) return;
+        queries += a * d;  // the rest without its scratch
+        ranges += a * 2 * l;
+        dist += a * k;
+        ids += a * k;
+        q -= a;
     }
     bool vec = d % 4 == 0 && (reinterpret_cast<uintptr_t>(data) & 15) == 0;
     BfShape b{};
@@ -1023,26 +1052,28 @@ void bruteforce_knn(const float* data, uint64_t n, uint32_t d, const float* labe
                 spans = c;
             }
         }
+        uint64_t* part = static_cast<uint64_t*>(scratch(sizeof(uint64_t) * nb * spans * k, st));
+        if (!part) spans = 1;
         b.spans = (uint32_t)spans;
-        uint64_t* part = nullptr;
-        CK(cudaMallocAsync(reinterpret_cast<void**>(&part), sizeof(uint64_t) * nb * spans * k, st));
         auto launch = [&](auto kern) {
             allow_smem(kern);
             kern<<<(unsigned)(groups * spans), kBfThreads, sm, st>>>(data, n, d, labels, l, queries + a * d, nb,
-                                                                    ranges + a * 2 * l, k, b, part);
+                                                                    ranges + a * 2 * l, k, b, part, dist + a * k, ids + a * k);
             CK_LAUNCH();
         };
         try {
             if (!b.pitch) vec ? launch(k_bruteforce<true, false, false>) : launch(k_bruteforce<false, false, false>);
             else if (vec) l == 4 ? launch(k_bruteforce<true, true, true>) : launch(k_bruteforce<true, false, true>);
             else l == 4 ? launch(k_bruteforce<false, true, true>) : launch(k_bruteforce<false, false, true>);
-            k_bf_merge<<<(unsigned)nb, 256, 0, st>>>(part, b.spans, k, dist + a * k, ids + a * k);
-            CK_LAUNCH();
+            if (part) {
+                k_bf_merge<<<(unsigned)nb, 256, 0, st>>>(part, b.spans, k, dist + a * k, ids + a * k);
+                CK_LAUNCH();
+            }
         } catch (...) {
-            cudaFreeAsync(part, st);
+            if (part) cudaFreeAsync(part, st);
             throw;
         }
-        CK(cudaFreeAsync(part, st));
+        if (part) CK(cudaFreeAsync(part, st));
     }
 }
 

@@ -1,6 +1,7 @@
 """Calls at the limits of their resources: little free device memory, several host threads,
 buffers left by larger calls, candidate ranges near the shared-memory limit."""
 import contextlib
+import ctypes as C
 import threading
 
 import numpy as np
@@ -16,23 +17,25 @@ MB = 1 << 20
 
 @contextlib.contextmanager
 def only_free(n_bytes: int):
-    """Takes device memory until n_bytes of it (give or take 4 MB) are free."""
+    """Takes device memory until n_bytes of it (give or take 2 MB) are free."""
     import torch
+    rt = C.CDLL("libcudart.so.12")  # (torch's allocator rounds small requests up)
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     held = []
-    for step in (64 * MB, 2 * MB):
-        while True:
-            over = torch.cuda.mem_get_info()[0] - n_bytes
-            if over < step:
-                break
-            held.append(torch.empty(over // step * step, dtype=torch.uint8, device="cuda"))
     try:
+        for step in (64 * MB, 2 * MB):
+            while (over := torch.cuda.mem_get_info()[0] - n_bytes) >= step:
+                p = C.c_void_p()
+                if rt.cudaMalloc(C.byref(p), C.c_size_t(over // step * step)) != 0:
+                    rt.cudaGetLastError()
+                    break
+                held.append(p)
         yield
     finally:
         torch.cuda.synchronize()
-        held.clear()
-        torch.cuda.empty_cache()
+        for p in held:
+            rt.cudaFree(p)
 
 
 def _in_threads(*calls):
@@ -219,7 +222,7 @@ def test_room_made_while_another_thread_queries(cuda):
     def large():
         try:
             idx.query(big[2], big[3])
-            torch.cuda.synchronize()
+            torch.cuda.default_stream().synchronize()  # (a device-wide wait would break the other's capture)
         finally:
             done.set()
 
@@ -295,6 +298,24 @@ def test_estimate_pass_many_ranges(cuda):
     idx.status()
     torch.cuda.synchronize()
     assert torch.equal(d, want[0]) and torch.equal(i, want[1])
+
+
+@pytest.mark.parametrize("q,k,n,d", [(64, 100, 190000, 96), (4500, 256, 2000, 16), (1, 10, 100000, 64)])
+def test_bruteforce_with_little_memory(cuda, q, k, n, d):
+    import torch
+    import hdgrid_b200 as hg
+    g = torch.Generator(device="cuda").manual_seed(q)
+    x = [torch.randn((n, d), device=cuda, generator=g), torch.rand((n, 2), device=cuda, generator=g),
+         torch.randn((q, d), device=cuda, generator=g), torch.tensor([0.0, 0.7] * 2, device=cuda).repeat(q, 1)]
+    out = []
+    for free in (None, 2 * MB):
+        dist = torch.full((q, k), -1.0, device=cuda)
+        ids = torch.full((q, k), 7, dtype=torch.int64, device=cuda)
+        with contextlib.nullcontext() if free is None else only_free(free):
+            hg.bruteforce_knn(*x, k, dist, ids)
+            torch.cuda.synchronize()
+        out.append((dist, ids))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
 
 
 @pytest.mark.parametrize("scale", [1e6, 1e-7])
