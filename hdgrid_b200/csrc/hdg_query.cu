@@ -3154,10 +3154,10 @@ static void reserve_ctx(hdg_index* idx, QueryCtx& cx, uint64_t q) {
     cx.work_queries = q;
 }
 
-// Batches of up to this many (query, point) pairs get candidate buffers for every pair (at
-// most 80 MiB each for distances, positions and selection), so the host need not read the candidate total
-// before it enqueues the scan: one query went
-// from 100 to 69 us without the wait.
+// Batches of up to this many (query, point) pairs get candidate buffers for every pair (at most
+// 80 MiB each for distances, positions and selection) when there is room for them, so the host need
+// not read the candidate total before it enqueues the scan: one query went from 100 to 69 us without
+// the wait.
 constexpr uint64_t kUnsizedPairs = 16ull << 20;
 
 // Candidate buffers of a batch whose totals are known to be at most coarse / selected entries
@@ -3168,6 +3168,17 @@ static void ensure_candidates(QueryCtx& cx, uint64_t q, uint32_t k, uint64_t coa
         resize_candidates(cx, rows, sel);
     }
     ensure_part_buf(cx, q, k);
+}
+
+// The same for every one of `pairs` (query, point) pairs; false when the memory is not there.
+static bool try_candidates(QueryCtx& cx, uint64_t q, uint32_t k, uint64_t pairs) {
+    try {
+        ensure_candidates(cx, q, k, pairs, pairs);
+    } catch (const Error& e) {
+        if (e.status != HDG_ERR_OOM) throw;
+        return false;
+    }
+    return true;
 }
 
 // The query context of a stream (created on first use); it becomes the last one used.
@@ -3213,9 +3224,9 @@ static void reserve_once(hdg_index* idx, uint64_t q, cudaStream_t st) {
     QueryCtx& cx = query_ctx(idx, st);
     std::lock_guard<std::mutex> g(cx.mu);
     reserve_ctx(idx, cx, q);
-    // a small batch's candidate buffers too: its calls then allocate nothing
+    // a small batch's candidate buffers too, if there is room: its calls then allocate nothing
     const uint64_t pairs = q * (uint64_t)idx->dev.n, k = idx->params.topk;
-    if (pairs <= kUnsizedPairs && k >= 1 && k <= 2048) ensure_candidates(cx, q, (uint32_t)k, pairs, pairs);
+    if (pairs <= kUnsizedPairs && k >= 1 && k <= 2048) try_candidates(cx, q, (uint32_t)k, pairs);
 }
 
 void reserve_workspace(hdg_index* idx, uint64_t q, cudaStream_t st) {
@@ -3670,8 +3681,9 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
         CK(cudaStreamIsCapturing(st, &cap));
         lazy = cap == cudaStreamCaptureStatusNone;
     }
+    const uint64_t pairs = q * (uint64_t)D.n;  // at most every point of every query
+    if (lazy && !try_candidates(cx, q, k, pairs)) lazy = false;  // (its candidates may find room)
     if (sync_sizing) {
-        uint64_t coarse = q * (uint64_t)D.n, selected = coarse;  // at most every point of every query
         if (lazy) {
             if (!cx.lazy.done) CK(cudaEventCreateWithFlags(&cx.lazy.done, cudaEventDisableTiming));
             CK(cudaEventRecord(cx.lazy.done, st));
@@ -3680,12 +3692,10 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
             CK(cudaMemcpyAsync(sc, w.scal, sizeof(sc), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             HDG_REQUIRE((uint32_t)sc[8] == 0, HDG_ERR_TIMEOUT, "tensor-core wait expired in the coarse GEMM");
-            coarse = sc[0];
-            selected = sc[7];
+            if (coarse_out) *coarse_out = sc[0];
+            if (sel_out) *sel_out = sc[7];
+            ensure_candidates(cx, q, k, sc[0], sc[7]);
         }
-        if (coarse_out) *coarse_out = coarse;
-        if (sel_out) *sel_out = selected;
-        ensure_candidates(cx, q, k, coarse, selected);
     } else {
         HDG_REQUIRE(cx.dist_buf.ptr && cx.sel_buf.ptr && cx.part_buf.bytes >= part_bytes(cx, q, k), HDG_ERR_STATE,
                     "no candidate buffers for a captured query");

@@ -300,6 +300,25 @@ def test_estimate_pass_many_ranges(cuda):
     assert torch.equal(d, want[0]) and torch.equal(i, want[1])
 
 
+def test_small_batch_with_little_memory(cuda):
+    """A small batch whose rows would be taken for every (query, point) pair runs with the memory
+    that its candidates need."""
+    import torch
+    n, q = 2_000_000, 8
+    ws = _range_ws(n, q, l=1)
+    idx, base, _ = build_gpu(ws, cuda)
+    d, i, qin, qout = _io(ws, base, 10, cuda)
+    idx.query(qin, qout)
+    torch.cuda.synchronize()
+    want = d.clone(), i.clone()
+    assert idx.last_query_stats()["coarse_total"] < n * q // 8
+    side = torch.cuda.Stream()
+    with only_free(48 * MB):  # 192 MB for every pair
+        idx.query(qin, qout, stream=side)
+        torch.cuda.synchronize()
+    assert torch.equal(d, want[0]) and torch.equal(i, want[1])
+
+
 @pytest.mark.parametrize("q,k,n,d", [(64, 100, 190000, 96), (4500, 256, 2000, 16), (1, 10, 100000, 64)])
 def test_bruteforce_with_little_memory(cuda, q, k, n, d):
     import torch
