@@ -107,8 +107,8 @@ struct Workspace {
     uint32_t k_max;          // output row stride
     int mode;                // batch schedule: 0 pre-filter (exps0 <= 1), 1 post-filter, 2 single dim
     uint32_t exps0;
-    uint32_t chunk;          // candidates per scan work item (SCAN_CHUNK; 0: set by k_batch from the batch)
-    uint32_t scan_items;     // work items k_batch aims at when it sets the chunk
+    uint32_t chunk;          // most candidates per scan work item (SCAN_CHUNK)
+    uint32_t scan_items;     // work items k_batch aims at when it sets the items' size
     int is_split;            // IS_SPLIT: trimmed Morton sub-ranges per probed list
     int nsplit;              // sub-ranges per probed list (n_split when is_split, else 1)
     uint64_t cap;            // distance-buffer capacity in candidates
@@ -838,8 +838,9 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
     const uint64_t b = t * per, e = min(q, b + per);
     // a predicate-first query of the predicate pass has predicate items over its candidates
     // (its ADC items follow from its survivors, k_scan_plan); any other query has ADC items
-    // Candidates per scan item: SCAN_CHUNK, or the smallest power of two from kChunkMin to kChunk
-    // that leaves at most scan_items items.  A small batch then fills the SMs (37 queries of
+    // Candidates per scan item: the smallest power of two from kChunkMin to SCAN_CHUNK (which the
+    // autotuner takes from one batch, and which bounds every other one's items only) that leaves at
+    // most scan_items items.  A small batch then fills the SMs (37 queries of
     // 73,000 candidates ran as 111 items of up to 32,768 in 325 us, in 125 us this way); a large one keeps long
     // items, since each loads its query's LUT.
     // Predicate items likewise, for 64 times as many items (a warp each, 16 per resident warp): an
@@ -854,9 +855,9 @@ __global__ void __launch_bounds__(1024) k_batch(uint64_t q, Workspace w) {
         block_inclusive_sum(c, s_tot, &all);
         if (t == 0) {
             uint32_t ch = kChunkMin, pc = kPreChunkMin;
-            while (ch < kChunk && (unsigned long long)ch * w.scan_items < all) ch *= 2;
+            while (ch < w.chunk && (unsigned long long)ch * w.scan_items < all) ch *= 2;
             while (pc < kPreChunk && (unsigned long long)pc * w.scan_items * 64u < all) pc *= 2;
-            s_chunk = w.chunk ? w.chunk : ch;
+            s_chunk = ch;
             s_pchunk = pc;
         }
         __syncthreads();
@@ -3615,7 +3616,7 @@ static void enqueue_query(hdg_index* idx, QueryCtx& cx, const QueryCall& c, cuda
     w.k_max = k;
     w.mode = mode;
     w.exps0 = (uint32_t)std::min<uint64_t>(exps0, 1u << 20);
-    w.chunk = (uint32_t)P.scan_chunk;
+    w.chunk = P.scan_chunk ? (uint32_t)std::min<uint64_t>(P.scan_chunk, 1u << 30) : kChunk;
     w.scan_items = 8 * (uint32_t)sm_count();
     w.cap = sync_sizing ? ~0ull : cx.dist_buf.bytes / 4;
     if (sync_sizing) w.sel_cap = ~0ull;  // sized after k_batch
@@ -4006,7 +4007,9 @@ static void autotune_once(hdg_index* idx, const QueryCall& c, cudaStream_t st, f
     try {
         enqueue_query(idx, cx, c, st, true, nullptr, nullptr, nullptr);  // warm-up, buffers sized
         const uint64_t cpts[3] = {1, 2, 4};
-        const uint64_t chunks[4] = {8192, 16384, 32768, 65536};
+        // the default first: another variant has to be a percent faster (on a small batch, whose items
+        // are below every one of these sizes, they are all the same)
+        const uint64_t chunks[4] = {kChunk, 8192, 16384, 65536};
         for (uint64_t cpt : cpts)
             for (uint64_t ch : chunks) {
                 P.scan_cpt = cpt;
@@ -4020,7 +4023,7 @@ static void autotune_once(hdg_index* idx, const QueryCall& c, cudaStream_t st, f
                         if (idx->stage_names[i] == "scan") s = idx->stage_ms[i];
                     t = std::min(t, s);
                 }
-                if (t < best) {
+                if (t < 0.99f * best) {
                     best = t;
                     best_cpt = cpt;
                     best_chunk = ch;

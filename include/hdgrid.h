@@ -77,8 +77,9 @@ typedef struct hdg_params {
     uint64_t kmeans_iters;  /* KMEANS_ITERS: Lloyd iterations of the index build (default 20) */
     uint64_t seed;          /* SEED: build RNG seed (default 1234) */
     uint64_t scan_cpt;      /* SCAN_CPT: ADC scan candidates per thread (1, 2 or 4; 0 = default) */
-    uint64_t scan_chunk;    /* SCAN_CHUNK: candidates per scan work item (power of two in
-                             * [4096, 262144]; 0 = 32768) -- the list/query split of the scan */
+    uint64_t scan_chunk;    /* SCAN_CHUNK: most candidates per scan work item (power of two in
+                             * [4096, 262144]; 0 = 32768) -- the list/query split of the scan;
+                             * a batch too small to fill the GPU with such items gets smaller ones */
     uint64_t query_graph;   /* QUERY_GRAPH: 1 = hdg_query replays a captured CUDA graph per
                              * (pointers, q, k); status of a replay via hdg_query_status */
     uint64_t learned;       /* LEARNED: 1 = per-query lists to probe and predicate-first flag

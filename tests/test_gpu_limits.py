@@ -300,6 +300,28 @@ def test_estimate_pass_many_ranges(cuda):
     assert torch.equal(d, want[0]) and torch.equal(i, want[1])
 
 
+def test_scan_chunk_is_the_largest_item(cuda):
+    """SCAN_CHUNK (the autotuner's choice, from one batch) bounds the scan items: a smaller batch
+    keeps the items its own size asks for."""
+    import torch
+    ws = _range_ws(200_000, 100)
+    idx, base, _ = build_gpu(ws, cuda)
+
+    def items(q, chunk):
+        idx.set_param("SCAN_CHUNK", chunk)
+        d, i, qin, qout = _io(ws, base, 10, cuda, 0, q)
+        idx.query(qin, qout)
+        torch.cuda.synchronize()
+        return int(np.frombuffer(idx.debug_fetch("item_off").tobytes(), np.uint32)[q]), d, i
+
+    auto = items(1, 0)
+    for chunk in (8192, 65536):
+        fixed = items(1, chunk)
+        assert fixed[0] == auto[0]
+        assert torch.equal(fixed[1], auto[1]) and torch.equal(fixed[2], auto[2])
+    assert items(100, 4096)[0] > items(100, 65536)[0]
+
+
 def test_small_batch_with_little_memory(cuda):
     """A small batch whose rows would be taken for every (query, point) pair runs with the memory
     that its candidates need."""
