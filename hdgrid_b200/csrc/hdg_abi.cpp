@@ -462,6 +462,9 @@ hdg_status hdg_recover_filters(const hdg_filter_spec* spec, const float* d_query
         const cudaStream_t st = static_cast<cudaStream_t>(stream);
         if (spec->n_map <= kMapArg) {
             recover_filters_arg(f, spec->interval_map, d_query_labels, n_queries, d_ranges, st);
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            CK(cudaStreamIsCapturing(st, &cap));
+            if (cap == cudaStreamCaptureStatusNone) CK(cudaStreamSynchronize(st));
             return;
         }
         DeviceBuffer map;

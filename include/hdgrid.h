@@ -273,7 +273,8 @@ hdg_status hdg_pq_adc(const uint8_t* d_codebook, uint64_t tot_data, const float*
 hdg_status hdg_label_mask(const float* d_ranges, const float* d_labels, uint32_t l,
                           uint64_t n_data, uint64_t n_queries, const uint64_t* d_indices,
                           uint64_t n_cand, int32_t* d_mask, void* stream);
-/* filters [q x 2l] f32 from the query labels and a filter spec. */
+/* filters [q x 2l] f32 from the query labels and a filter spec.  Returns once they are written
+ * (while `stream` is captured, with a map of at most 512 entries: once that is recorded). */
 hdg_status hdg_recover_filters(const hdg_filter_spec* spec, const float* d_query_labels,
                                uint64_t n_queries, float* d_ranges, void* stream);
 /* out[r][c] = sum_k a[r][k] * b[c][k] for bf16 a [rows x d] and b [cols x d] (row-major,
@@ -284,21 +285,21 @@ hdg_status hdg_recover_filters(const hdg_filter_spec* spec, const float* d_query
 hdg_status hdg_bf16_gemm(const void* d_a, uint64_t rows, const void* d_b, uint64_t cols, uint32_t d,
                          float* d_out, uint64_t ldo, void* stream);
 
-/* Allocation-free variant of hdg_recover_filters -- no counterpart in the reference.
- * For callers that must not allocate device memory while they run: a host application
- * whose own allocator owns the GPU's memory, or a serving loop that cannot afford the
- * device-wide synchronisation cudaMalloc / cudaFree may cause.  hdg_recover_filters keeps
- * a per-call device copy of the filter's interval-map table; this variant keeps it in a
- * fixed scratch array of HDG_NOALLOC_MAP_MAX floats inside the library (present on every
- * GPU that loads the library until the process exits) and allocates nothing.  The caller
- * still passes the labels and the output.  Maps longer than HDG_NOALLOC_MAP_MAX entries
- * return HDG_ERR_INVALID_ARG.  The first call on a device looks up the scratch array's
- * device address (make that device current, and make that first call before any stream
- * capture).  All calls share the one array: calls whose work overlaps on the GPU (other
- * streams, other threads) race on it and must be serialised by the caller.  The map is
- * copied from spec->interval_map on `stream` (stream-ordered): that host memory must stay
- * valid and unchanged until the call's stream work has completed.  The looked-up address
- * is kept per device ordinal for the life of the process; it does not survive a
+/* Allocation-free variant of hdg_recover_filters -- no counterpart in the reference. For
+ * callers that must not allocate device memory while they run: a host application whose own
+ * allocator owns the GPU's memory, or a serving loop that cannot afford the device-wide
+ * synchronisation cudaMalloc / cudaFree may cause.  hdg_recover_filters keeps a per-call
+ * device copy of an interval-map table of more than 512 entries, and waits; this variant
+ * keeps it in a fixed scratch array of HDG_NOALLOC_MAP_MAX floats inside the library
+ * (present on every GPU that loads the library until the process exits) and allocates
+ * nothing.  The caller still passes the labels and the output.  Maps longer than
+ * HDG_NOALLOC_MAP_MAX entries return HDG_ERR_INVALID_ARG.  The first call on a device looks
+ * up the scratch array's device address (make that device current, and make that first call
+ * before any stream capture).  All calls share the one array: calls whose work overlaps on
+ * the GPU (other streams, other threads) race on it and must be serialised by the caller.
+ * The map is copied from spec->interval_map on `stream` (stream-ordered): that host memory
+ * must stay valid and unchanged until the call's stream work has completed.  The looked-up
+ * address is kept per device ordinal for the life of the process; it does not survive a
  * cudaDeviceReset (or a primary-context reset) of that device. */
 #define HDG_NOALLOC_MAP_MAX 65536
 hdg_status hdg_recover_filters_noalloc(const hdg_filter_spec* spec, const float* d_query_labels,

@@ -374,3 +374,31 @@ def test_no_estimate_pass_of_a_useless_scale(cuda, scale):
     idx.query(qin, qout)
     idx.query(qin, qout)
     assert "estimate" not in idx.stage_times()
+
+
+@pytest.mark.parametrize("entries", [2, 600])
+def test_recover_filters_returns_with_its_result(cuda, entries):
+    import torch
+    import hdgrid_b200 as hg
+    conf = "l = 1\nfilter0:\n\ttype = 1\n\tinterval_map = [" + ", ".join(str(i) for i in range(entries)) + "]\n"
+    ql = torch.ones((100, 1), device=cuda)
+    out = torch.empty((100, 2), device=cuda)
+    a = torch.randn((8192, 8192), device=cuda)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        for _ in range(20):
+            a @ a
+    hg.recover_filters(conf, ql, out, stream=side)
+    assert side.query()  # the stream's work, the result with it, has ended
+    want = out.clone()
+    if entries > 512:
+        return
+    out.zero_()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=side):  # nothing to wait for
+        hg.recover_filters(conf, ql, out, stream=side)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
