@@ -1343,6 +1343,12 @@ void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, co
     k_gather_codes_labels<<<blocks_for(n, 256), 256, 0, st>>>(codes_by_id.p, (int)H.M_pad, d_labels, (int)l, dids.p, n,
                                                              codes.p, labels.p);
     CK_LAUNCH();
+    // the upload needs the pool-ordered arrays only: room for the arena beside them
+    codes_by_id.reset();
+    list_of_id.reset();
+    zc.reset();
+    cell.reset();
+    Xs.reset();
     const DeviceArrays src{dz.p,       dids.p,     codes.p, labels.p, rows_form ? nullptr : prefix.p,
                            rows_form ? row_off->p : nullptr, rows_form ? rows->p : nullptr, labels_nan};
     upload_index_from(idx, st, &src);

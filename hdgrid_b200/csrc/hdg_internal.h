@@ -25,9 +25,11 @@ struct DevMem {
     explicit DevMem(uint64_t count) {
         if (count) CK(cudaMalloc(reinterpret_cast<void**>(&p), sizeof(T) * count));
     }
-    ~DevMem() {
+    void reset() {
         if (p) cudaFree(p);
+        p = nullptr;
     }
+    ~DevMem() { reset(); }
     DevMem(const DevMem&) = delete;
     DevMem& operator=(const DevMem&) = delete;
 };

@@ -402,3 +402,21 @@ def test_recover_filters_returns_with_its_result(cuda, entries):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, want)
+
+
+def test_build_frees_what_its_upload_does_not_need(cuda):
+    """Beside the index the upload needs the pool-ordered arrays only: by-id codes, lists, cells
+    and Morton codes (36 bytes a point here) are gone by then."""
+    import torch
+    import hdgrid_b200 as hg
+    n = 8_000_000
+    ws = _range_ws(1000, 8, d=16, m=16)
+    base = torch.randn((n, 16), device=cuda)
+    labels = torch.randint(0, 1000, (n, 4), device=cuda).float()
+    torch.cuda.synchronize()
+    idx = hg.SuperGridIndex.from_text(ws["hdgrid_conf"], ws["filter_conf"])
+    # at the upload: code rows, labels, ids, codes, the arena of 48 a point
+    with only_free(n * 100 + 48 * MB):
+        idx.build(hg.build_input_t(base, labels))
+        torch.cuda.synchronize()
+    assert idx.info()["n"] == n
