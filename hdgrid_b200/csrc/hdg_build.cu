@@ -1388,11 +1388,18 @@ void label_rank_thresholds(const float* labels, uint64_t n, int l, int bits, flo
 // The index's optional buffers (decoded vectors, rank planes) speed calls up that run without them too.
 // They are kept while each takes at most a quarter of the memory that is free, and given back to a
 // call that has no room otherwise (release_optional).
-static bool optional_room(uint64_t bytes) {
-    size_t free = 0, total = 0;
-    CK(cudaMemGetInfo(&free, &total));
-    return bytes <= free / 4;
-}
+struct OptionalRoom {
+    size_t free = 0;
+    OptionalRoom() {
+        size_t total = 0;
+        CK(cudaMemGetInfo(&free, &total));
+    }
+    bool keep(DeviceBuffer& b, uint64_t bytes) {
+        if (bytes > free / 4 || !b.try_ensure(bytes)) return false;
+        free -= bytes;
+        return true;
+    }
+};
 constexpr uint64_t kDecodedMax = 16ull << 30;
 constexpr uint64_t kPlanes = 512, kPlanesMax = 8ull << 30;  // label-rank bit planes: at most 64 bytes per point
 constexpr uint64_t kDecodedMinPoints = 16384;  // smaller sets never reach the estimate pass
@@ -1582,6 +1589,7 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
     D.S_max = 0;
     for (uint64_t c = 0; c < H.C; c++)
         D.S_max = std::max<uint32_t>(D.S_max, H.cluster_off[c + 1] - H.cluster_off[c]);
+    OptionalRoom room;
     // the ranks' bit planes: up to kPlanes of them in all, a bit of resolution less for as long as
     // they would take more than kPlanesMax bytes
     if (rbits && !D.labels_nan) {
@@ -1598,7 +1606,7 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
             if (planes * D.plane_words * 4 <= kPlanesMax) break;
         }
         // (without room for them the predicate pass tests the packed ranks, one candidate at a time)
-        if (optional_room(planes * D.plane_words * 4) && idx->planes.try_ensure(std::max<uint64_t>(planes * D.plane_words * 4, 16))) {
+        if (room.keep(idx->planes, std::max<uint64_t>(planes * D.plane_words * 4, 16))) {
             k_rank_planes<<<blocks_for(D.plane_words, 64), 256, 0, st>>>(D, H.n, static_cast<uint32_t*>(idx->planes.ptr));
             CK_LAUNCH();
             D.rank_planes = static_cast<const uint32_t*>(idx->planes.ptr);
@@ -1609,8 +1617,7 @@ static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArray
     // label dim, whose schedule has no such scan)
     const uint64_t dec = align_up((uint64_t)H.n * H.d * 2, 256);
     if (H.l > 1 && H.d % 8 == 0 && H.M % 32 == 0 && H.M <= 96 && H.M * H.pq_len == H.d && H.n >= kDecodedMinPoints &&
-        dec <= kDecodedMax && optional_room(dec + (uint64_t)H.n * sizeof(float4) + 16) &&
-        idx->decoded.try_ensure(dec + (uint64_t)H.n * sizeof(float4) + 16)) {
+        dec <= kDecodedMax && room.keep(idx->decoded, dec + (uint64_t)H.n * sizeof(float4) + 16)) {
         const uint64_t cst = (uint64_t)H.n * sizeof(float4);
         char* p = static_cast<char*>(idx->decoded.ptr);
         uint32_t* mx = reinterpret_cast<uint32_t*>(p + dec + cst);
