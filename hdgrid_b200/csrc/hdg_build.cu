@@ -1153,8 +1153,7 @@ void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, co
     HDG_REQUIRE(n >= L && n >= 256 && n < (1ull << 32), HDG_ERR_INVALID_ARG,
                 "base set must hold at least max(256, clusters*sub_clusters) points and < 2^32");
     std::mt19937_64 rng(P.seed);
-    HostIndex& H = idx->host;
-    H = HostIndex();
+    HostIndex H;  // the index's own once its arrays exist: a build that fails before leaves the old one
     H.n = n;
     H.d = d;
     H.l = l;
@@ -1351,6 +1350,7 @@ void build_index(hdg_index* idx, const float* d_data, uint64_t n, uint32_t d, co
     Xs.reset();
     const DeviceArrays src{dz.p,       dids.p,     codes.p, labels.p, rows_form ? nullptr : prefix.p,
                            rows_form ? row_off->p : nullptr, rows_form ? rows->p : nullptr, labels_nan};
+    idx->host = std::move(H);
     upload_index_from(idx, st, &src);
 }
 
@@ -1409,6 +1409,8 @@ void upload_index(hdg_index* idx, cudaStream_t st) { upload_index_from(idx, st, 
 
 // src: arrays that the build still holds on the device, copied there instead of from the host
 static void upload_index_from(hdg_index* idx, cudaStream_t st, const DeviceArrays* src) {
+    idx->built = false;      // until every array is in place
+    invalidate_graphs(idx);  // captured graphs hold the old arrays' addresses
     HostIndex& H = idx->host;
     // element counts of the large arrays, wherever they are
     const uint64_t n_dense = src ? (src->prefix ? H.grid.tot_cells * H.n_lists : 0) : H.prefix.size();

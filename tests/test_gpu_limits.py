@@ -420,3 +420,57 @@ def test_build_frees_what_its_upload_does_not_need(cuda):
         idx.build(hg.build_input_t(base, labels))
         torch.cuda.synchronize()
     assert idx.info()["n"] == n
+
+
+def test_rebuild(cuda, tmp_path):
+    """A refused build leaves the index as it was; a new one ends the old one's captured graphs; one
+    without room for its arrays leaves no index."""
+    import torch
+    import hdgrid_b200 as hg
+    ws = _range_ws(20_000, 50)
+    idx, base, labels = build_gpu(ws, cuda)
+    d, i, qin, qout = _io(ws, base, 10, cuda)
+    idx.query(qin, qout)
+    torch.cuda.synchronize()
+    want, info = (d.clone(), i.clone()), idx.info()
+    with pytest.raises(hg.HDGError):
+        idx.build(hg.build_input_t(base, -1.0 - labels))
+    assert idx.info() == info
+    idx.save(str(tmp_path / "index.hdg"))
+    again = hg.SuperGridIndex.load(str(tmp_path / "index.hdg"))
+    for x in (idx, again):
+        d.fill_(-1.0)
+        x.query(qin, qout)
+        torch.cuda.synchronize()
+        assert torch.equal(d, want[0]) and torch.equal(i, want[1])
+    idx.set_param("QUERY_GRAPH", 1)
+    for _ in range(3):
+        idx.query(qin, qout)
+    idx.status()
+    other = base.flip(0).contiguous()
+    fresh = hg.SuperGridIndex.from_text(ws["hdgrid_conf"], ws["filter_conf"])
+    fresh.build(hg.build_input_t(other, labels))
+    base.copy_(other)  # the same addresses, other vectors
+    fresh.query(qin, qout)
+    torch.cuda.synchronize()
+    want = d.clone(), i.clone()
+    idx.build(hg.build_input_t(base, labels))
+    for _ in range(3):
+        d.fill_(-1.0)
+        idx.query(qin, qout)
+        idx.status()
+        torch.cuda.synchronize()
+        assert torch.equal(d, want[0]) and torch.equal(i, want[1])
+    n = 8_000_000
+    big = hg.build_input_t(torch.randn((n, 32), device=cuda), torch.randint(0, 1000, (n, 4), device=cuda).float())
+    with only_free(n * 118):  # pool order takes 112 a point, code rows and labels with the arena 124
+        with pytest.raises(hg.HDGError, match="OOM"):
+            idx.build(big)
+    with pytest.raises(hg.HDGError, match="not built"):
+        idx.query(qin, qout)
+    idx.build(hg.build_input_t(base, labels))
+    d.fill_(-1.0)
+    idx.query(qin, qout)
+    idx.status()
+    torch.cuda.synchronize()
+    assert torch.equal(d, want[0]) and torch.equal(i, want[1])
