@@ -3084,6 +3084,7 @@ static Workspace carve(hdg_index* idx, QueryCtx& cx, uint64_t q, bool record) {
     w.qnorm = (float*)take("qnorm", q * 4);
     w.qbf = take("qbf", q * idx->dev.d * 2);
     w.gemm_err = reinterpret_cast<int*>(w.scal + 8);  // in the scalars' padding: one copy reads both
+    if (record) cx.layout["gemm_err"] = {cx.layout["scalars"].first + 64, 16};
     w.feats = (float*)take("features", q * kMlpFeatures * 4);
     w.lq_ps = (uint32_t*)take("learned_nprobe", q * 4);
     w.lq_sched = (uint8_t*)take("learned_schedule", q);

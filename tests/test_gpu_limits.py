@@ -474,3 +474,11 @@ def test_rebuild(cuda, tmp_path):
     idx.status()
     torch.cuda.synchronize()
     assert torch.equal(d, want[0]) and torch.equal(i, want[1])
+
+
+def test_debug_fetch_gemm_err(cuda):
+    ws = _range_ws(4000, 8)
+    idx, base, _ = build_gpu(ws, cuda)
+    d, i, qin, qout = _io(ws, base, 10, cuda)
+    idx.query(qin, qout)
+    assert np.frombuffer(idx.debug_fetch("gemm_err").tobytes(), np.int32)[0] == 0
