@@ -10,6 +10,7 @@ namespace hdg {
 
 inline void check_cuda(cudaError_t e, const char* what, const char* file, int line) {
     if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here: the next launch check, or the caller's own, is not to find it
         const hdg_status s = (e == cudaErrorMemoryAllocation) ? HDG_ERR_OOM : HDG_ERR_CUDA;
         throw Error(s, std::string(what) + " failed: " + cudaGetErrorString(e) + " (" + file + ":" +
                            std::to_string(line) + ")");

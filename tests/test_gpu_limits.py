@@ -482,3 +482,24 @@ def test_debug_fetch_gemm_err(cuda):
     d, i, qin, qout = _io(ws, base, 10, cuda)
     idx.query(qin, qout)
     assert np.frombuffer(idx.debug_fetch("gemm_err").tobytes(), np.int32)[0] == 0
+
+
+def test_failed_allocation_is_reported_once(cuda):
+    """Neither torch nor the next call of the library finds the status of a build that had no room."""
+    import torch
+    import hdgrid_b200 as hg
+    ws = _range_ws(20_000, 50)
+    idx, base, labels = build_gpu(ws, cuda)
+    d, i, qin, qout = _io(ws, base, 10, cuda)
+    idx.query(qin, qout)
+    n = 2_000_000
+    big = hg.build_input_t(torch.randn((n, 32), device=cuda), torch.randint(0, 1000, (n, 4), device=cuda).float())
+    other = hg.SuperGridIndex.from_text(ws["hdgrid_conf"], ws["filter_conf"])
+    with only_free(n * 50):  # (the pool order alone takes 76 a point)
+        with pytest.raises(hg.HDGError, match="OOM"):
+            other.build(big)
+        assert float(torch.ones(8, device=cuda).sum()) == 8.0
+        with pytest.raises(hg.HDGError, match="OOM"):
+            other.build(big)
+        idx.query(qin, qout)
+    torch.cuda.synchronize()
