@@ -721,8 +721,9 @@ __global__ void __launch_bounds__(256) k_bf_merge(const uint64_t* __restrict__ p
 // the labels leave (about kBfRatio * k per query) are computed exactly, in the same FMA chain as
 // k_bruteforce; the last level is the whole set.  A query with more rows left than its list holds
 // goes through k_bf_full.
-// 1,000 queries x 1 M x 128: 19.1 ms with k_bruteforce, 4.3 ms this way (1.9 ms of it k_est, 0.9
-// k_bf_exact).
+// 1,000 queries x 1 M x 128: 19.1 ms with k_bruteforce, 3.0 to 3.9 ms this way (1.9 ms of it k_est, 0.9
+// k_bf_exact; the scratch's allocation varies).  Vectors that FP16 cannot hold bound nothing: every query
+// then goes through k_bf_full, 70 ms there (347 ms with a block per 32 queries that computed every pair).
 constexpr uint64_t kBfEstQueries = 32, kBfEstPairs = 12000000;
 constexpr uint64_t kBfRatio = 16;
 constexpr uint64_t kBfRowsMax = 1ull << 18;  // rows converted at a time (64 MB at 128 dims)

@@ -11,7 +11,7 @@
 //                [lower_bound(zlo), lower_bound(zhi+1)) inside every probed list (zorder.cu:656-685).
 //   k_batch      candidate offsets, work items and the batch sums of the post-filter budget
 //                beta (:1198-1222).
-//   k_pre_scan   predicate-first queries: label-rank box test, then the label predicate
+//   k_pre_scan   predicate-first queries: label-rank boxes, then the label predicate
 //                (filter.cu:30-64), survivors listed for the ADC (prefiltering.cu:36-51).
 //   k_lut        per query PQ lookup table (build_pq_lut_kernel, product-quantization.cu:4-35).
 //   k_scan       persistent streaming ADC over the contiguous Z-ordered candidate ranges
@@ -70,7 +70,8 @@ struct Workspace {
     uint32_t* nfin;          // [q] finite distances (predicate passed)
     uint32_t* lab_read;      // [q] candidates of the predicate pass whose labels were read
     uint32_t* rank_read;     // [q] candidates of the predicate pass whose label ranks were read
-    uint32_t* counter;       // [4] work counters: ADC scan, refine, predicate pass; [3] candidates per scan item
+    uint32_t* counter;       // [8] work counters: ADC scan, refine, predicate pass; [3] candidates per scan item,
+                             //     [4] per predicate item
     float* lut;              // [q x G x 256 x 32] f32, or __half when lut16
     int lut16;               // LUT stored in FP16 (LUT_FP16=1); the scan sums in FP32
     uint32_t* qbud;          // [q] candidate budget n_cand of each query (k_batch)
@@ -118,9 +119,11 @@ constexpr uint64_t kChainQueries = 4096;
 
 enum ScanMode { kPre = 0, kPost = 1, kL1 = 2 };
 
-// Every kernel of the query path begins with this: the next kernel of the stream may be brought up
-// (its blocks resident and waiting at the same point), and this one waits until the kernel before
-// it has ended.  Kernels launched without the attribute (launch_next) start after it anyway.
+// The kernels that launch_next may launch as programmatic dependents begin with this: the next kernel
+// of the stream may be brought up (its blocks resident and waiting at the same point), and this one
+// waits until the kernel before it has ended.  The others (k_pre_scan, k_scan_plan, the estimate
+// pass's) are always launched without the attribute and start after the kernel before them; with
+// it they would race.
 __device__ __forceinline__ void chain_start() {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -3396,7 +3399,7 @@ struct GraphState {
     std::vector<GraphEntry> entries;
     cudaStream_t stream = nullptr;  // capture and replay stream
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
-    uint64_t* pinned = nullptr;     // [8] scalars + [8] gemm status of the last replay
+    uint64_t* pinned = nullptr;     // the last replay's scalars and GEMM status word (nine words)
     bool pending = false;
     GraphEntry last;                // description of the last replay (stats)
 };

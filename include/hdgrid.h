@@ -201,15 +201,17 @@ int hdg_last_query_stats(hdg_index* index, uint64_t* out, int cap);
 /* With QUERY_GRAPH=1 hdg_query returns once the captured graph is enqueued; this waits for
  * the last replay and returns its device status: HDG_OK, HDG_ERR_TIMEOUT (a tensor-core
  * wait of the coarse GEMM expired) or HDG_ERR_OOM (the batch had more candidates than the
- * distance buffer sized at capture -- 1.25x the first batch of the shape -- and the
- * queries past it returned no results).  HDG_OK when no replay is pending.  No reference
+ * distance buffer sized at capture -- 1.25x the first batch of the shape, or that batch's
+ * own size where the memory for more was not there -- and the queries past it returned
+ * no results).  HDG_OK when no replay is pending.  No reference
  * counterpart: the reference synchronises after every stage. */
 hdg_status hdg_query_status(hdg_index* index);
 
 /* The project autotuner: runs the batch through the plain path once per scan variant --
  * threads x candidates-per-thread (SCAN_CPT 1, 2, 4) and work-item size (SCAN_CHUNK 8192 ..
  * 65536 candidates, the split of the scan between lists and queries) -- and keeps the
- * fastest scan in the index's parameters.  Outputs as hdg_query; best_scan_ms (may be
+ * fastest scan in the index's parameters (the defaults unless another is a percent faster;
+ * SCAN_CHUNK bounds the items, so smaller batches keep smaller ones).  Outputs as hdg_query; best_scan_ms (may be
  * NULL) receives the chosen variant's scan time.  Replaces the reference's memory
  * predictor (search-engine/search-engine-auto-batch.cu:178-190, 381-430, 431-490), which
  * picks batch sizes instead. */
@@ -306,7 +308,9 @@ hdg_status hdg_recover_filters_noalloc(const hdg_filter_spec* spec, const float*
                                        uint64_t n_queries, float* d_ranges, void* stream);
 
 /* Exact filtered kNN in FP32: distances of every base vector whose labels pass the
- * per-query box d_ranges [q x 2l]; k smallest, ascending, ties by lower id. */
+ * per-query box d_ranges [q x 2l]; k smallest, ascending, ties by lower id.  Takes scratch
+ * from the device's memory pool on `stream` (64 MB and more for a batch) and gives it back;
+ * without room for it the call runs slower, with the same results. */
 hdg_status hdg_bruteforce_knn(const float* d_data, uint64_t n, uint32_t d,
                               const float* d_labels, uint32_t l, const float* d_queries,
                               uint64_t q, const float* d_ranges, uint32_t k,
